@@ -23,13 +23,26 @@ __global__ void chi0_bar_seed_kernel(double *a, int64_t n, const double *w) {
     m[i] *= s;
 }
 
-// out = (in + in^T) / 2
-__global__ void sym_half_kernel(const double *in, double *out, int64_t n) {
-  const int64_t total = n * n;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t r = i / n, c = i % n;
-    out[i] = 0.5 * (in[i] + in[c * n + r]);
+// out = (in + in^T) / 2 for each n x n slice: one 32 x 32 tile and its mirror
+// per block, both halves through shared memory so that every access runs
+// along rows
+__global__ void sym_half_kernel(const double *__restrict__ in, double *__restrict__ out,
+                                int64_t n) {
+  __shared__ double lo[32][33], up[32][33];
+  if (blockIdx.x < blockIdx.y) return;
+  const int64_t base = static_cast<int64_t>(blockIdx.z) * n * n;
+  const int64_t r0 = static_cast<int64_t>(blockIdx.y) * 32, c0 = static_cast<int64_t>(blockIdx.x) * 32;
+  const int x = threadIdx.x;
+  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+    up[k][x] = r0 + k < n && c0 + x < n ? in[base + (r0 + k) * n + c0 + x] : 0.0;
+    lo[k][x] = c0 + k < n && r0 + x < n ? in[base + (c0 + k) * n + r0 + x] : 0.0;
+  }
+  __syncthreads();
+  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+    if (r0 + k < n && c0 + x < n)
+      out[base + (r0 + k) * n + c0 + x] = 0.5 * (up[k][x] + lo[x][k]);
+    if (r0 != c0 && c0 + k < n && r0 + x < n)
+      out[base + (c0 + k) * n + r0 + x] = 0.5 * (lo[k][x] + up[x][k]);
   }
 }
 
@@ -639,8 +652,10 @@ void launch_chi0_bar_seed(double *a, int64_t n, int nfreq, const double *w, cuda
   count_launch(); chi0_bar_seed_kernel<<<grid, 256, 0, st>>>(a, n, w);
 }
 
-void launch_sym_half(const double *in, double *out, int64_t n, cudaStream_t st) {
-  count_launch(); sym_half_kernel<<<blocks(n * n), 256, 0, st>>>(in, out, n);
+void launch_sym_half(const double *in, double *out, int64_t n, int batch, cudaStream_t st) {
+  const unsigned t = static_cast<unsigned>((n + 31) / 32);
+  count_launch();
+  sym_half_kernel<<<dim3(t, t, batch), dim3(32, 8), 0, st>>>(in, out, n);
 }
 
 void launch_xbar_update(const double *GoX, const double *GvX, const double *X, int64_t M,

@@ -14,6 +14,7 @@
 #include <tuple>
 #include <vector>
 
+#include "dmma.h"
 #include "internal.h"
 
 namespace mbpt {
@@ -26,7 +27,7 @@ int launch_pade_eval(const double *sigma, const double *pade_freq, int npade,
                      const double *query, int nq, double *out, cudaStream_t st);
 void launch_chi0_bar_seed(double *a, int64_t n, int nfreq, const double *scale,
                           cudaStream_t st);
-void launch_sym_half(const double *in, double *out, int64_t n, cudaStream_t st);
+void launch_sym_half(const double *in, double *out, int64_t n, int batch, cudaStream_t st);
 void launch_xbar_update(const double *GoX, const double *GvX, const double *X, int64_t M,
                         int64_t n, int64_t nocc, const double *eps, double mu, double tau,
                         double *X_bar, double *eps_bar, cudaStream_t st);
@@ -210,8 +211,9 @@ struct Dims {
 // ---------------------------------------------------------------- chi0 sweep
 struct Chi0Bufs {
   double *w;  // cosft_wt on the device
-  // fp64
+  // fp64 (Xo_s, Xv_s, Go, Y: `batch` tau points each; Gv: the int8 mode only)
   double *Xo_s, *Xv_s, *Go, *Gv, *Y, *proj;
+  int batch;
   // mixed
   bf16 *Dt_hi, *Dt_lo, *Pi_hi, *Pi_lo, *Z_hi, *Z_lo;
   float *Yo_hi, *Yo_lo, *Yv_hi, *Yv_lo;  // TF32 pairs of the G products
@@ -219,15 +221,47 @@ struct Chi0Bufs {
   double *eye;  // ntau x ntau identity for the optional proj copy
 };
 
+// Tau points per launch of the FP64 sweeps: as many as keep their grid arrays
+// within 640 MB (all of them up to M of about 1300; one where a single point
+// already fills the GPU many times over), in even batches. At M = 2400 six
+// points a launch leave 26 tiles to the busiest SM where 25.03 are the mean;
+// one point a launch would leave 6 against 5.007.
+int tau_batch(int ntau, int64_t doubles_per_tau) {
+  const int64_t cap = (int64_t{640} << 20) / 8;
+  const int64_t most = std::max<int64_t>(1, std::min<int64_t>(
+      std::min(ntau, kMaxTauBatch), cap / std::max<int64_t>(1, doubles_per_tau)));
+  const int64_t batches = (ntau + most - 1) / most;
+  return static_cast<int>((ntau + batches - 1) / batches);
+}
+
+TauList tau_list(const double *tau, int count) {
+  TauList l{};
+  for (int i = 0; i < count; ++i) l.t[i] = tau[i];
+  l.n = count;
+  return l;
+}
+
+// Transform weights from which the FP64 chi0 keeps the library's products.
+// The 16- and 18-point grids are not regularised: their weights reach 1e8-1e9
+// and cancel, so the last bits of proj(tau) move chi0 by 1e-8 of its scale,
+// and a result can only be reproduced by products summed in the reference's
+// order with both triangles formed on their own (E_c of the 16-point golden
+// system: 1e-11 relative that way, 8e-11 from mirrored halves; both are
+// rounding, but not the same rounding). From 20 points on the weights stay
+// below 1e3.
+constexpr double kAmplifyingWeight = 1e6;
+
 Chi0Bufs carve_chi0(Arena &ar, const Dims &d, int ntau, int nfreq, int mode, bool own_proj) {
   Chi0Bufs b{};
   b.w = ar.take<double>(static_cast<size_t>(nfreq) * ntau);
   if (fp64_mode(mode)) {
-    b.Xo_s = ar.take<double>(d.M * d.nocc);
-    b.Xv_s = ar.take<double>(d.M * d.nv);
-    b.Go = ar.take<double>(d.M * d.M);
-    b.Gv = ar.take<double>(d.M * d.M);
-    b.Y = ar.take<double>(d.M * d.naux);
+    b.batch = mode == MBPT_MODE_FP64 ? tau_batch(ntau, d.M * (d.M + d.naux + d.n)) : 1;
+    b.Xo_s = ar.take<double>(b.batch * d.M * d.nocc);
+    b.Xv_s = ar.take<double>(b.batch * d.M * d.nv);
+    // the library products hold one tau point's G_occ and G_virt
+    b.Go = ar.take<double>(std::max(b.batch, 2) * d.M * d.M);
+    b.Gv = ar.counting ? nullptr : b.Go + d.M * d.M;
+    b.Y = ar.take<double>(b.batch * d.M * d.naux);
     if (own_proj) b.proj = ar.take<double>(static_cast<size_t>(ntau) * d.naux * d.naux);
   } else {
     b.Dt_hi = ar.take<bf16>(d.Ap * d.Mp);
@@ -253,7 +287,31 @@ int chi0_run(const double *X, const Dims &d, const double *eps, double mu, const
   if (ar.overflow()) return MBPT_ERR_WORKSPACE;
   cudaMemcpyAsync(b.w, cw, sizeof(double) * nfreq * ntau, cudaMemcpyHostToDevice, st);
   const int64_t a2 = d.naux * d.naux;
-  if (fp64_mode(mode)) {
+  double top = 0.0;
+  for (int i = 0; i < nfreq * ntau; ++i) top = std::max(top, std::fabs(cw[i]));
+  if (mode == MBPT_MODE_FP64 && top <= kAmplifyingWeight) {
+    double *proj = proj_out ? proj_out : b.proj;
+    const int64_t mo = d.M * d.nocc, mv = d.M * d.nv, m2 = d.M * d.M, ma = d.M * d.naux;
+    for (int k = 0; k < ntau; k += b.batch) {
+      const int nb = std::min(b.batch, ntau - k);
+      launch_scaled_branches_batch(X, d.M, d.n, d.nocc, eps, mu, tau_list(tau + k, nb), b.Xo_s,
+                                   b.Xv_s, st);
+      // Pi = G_occ o G_virt, G_occ = (X_o e^{e_o tau}) X_o^T, G_virt likewise
+      // (MBPTcode space_time.py:525-526), Y = Pi D, proj = -2 D^T Y
+      int rc = dmma::hadamard_product({b.Xo_s, d.nocc, mo}, {X, d.n, 0}, d.nocc,
+                                      {b.Xv_s, d.nv, mv}, {X + d.nocc, d.n, 0}, d.nv, d.M, b.Go,
+                                      d.M, m2, nb, st);
+      if (!rc)
+        rc = dmma::gemm({b.Go, d.M, m2}, true, {D, d.naux, 0}, false, d.M, d.naux, d.M, 1.0, 0.0,
+                        b.Y, d.naux, ma, nb, false, st);
+      if (!rc)
+        rc = dmma::gemm({D, d.naux, 0}, false, {b.Y, d.naux, ma}, false, d.naux, d.naux, d.M,
+                        -2.0, 0.0, proj + k * a2, d.naux, a2, nb, true, st);
+      if (rc) return rc;
+    }
+    launch_transform<double>(proj, a2, d.naux, d.naux, d.naux, b.w, nfreq, ntau, chi0, a2,
+                             d.naux, st);
+  } else if (fp64_mode(mode)) {
     double *proj = proj_out ? proj_out : b.proj;
     cublasHandle_t h = handles(st).blas;
     for (int k = 0; k < ntau; ++k) {
@@ -1036,8 +1094,10 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
 
 // -------------------------------------------------------------------- Sigma
 struct SigmaBufs {
-  // fp64
-  double *U, *Zt, *G, *Xo_s, *Xv_s, *Xs, *R;
+  // fp64 (U, Ws, Hl, Hg, Xo_s, Xv_s: `batch` tau points each; Zt alone where
+  // W = I; Hl as G and R: the int8 mode)
+  double *U, *Ws, *Zt, *Hl, *Hg, *Xo_s, *Xv_s, *Xs, *R;
+  int batch;
   // mixed
   bf16 *D_hi, *D_lo, *W_hi, *W_lo, *U_hi, *U_lo, *Yo_hi, *Yo_lo, *Yv_hi, *Yv_lo, *Hl_hi,
       *Hl_lo, *Hg_hi, *Hg_lo, *XsT_hi, *XsT_lo;
@@ -1049,10 +1109,22 @@ int64_t pad_states(int nstates) { return round_up(nstates, 128); }
 
 SigmaBufs carve_sigma(Arena &ar, const Dims &d, int ntau, int nstates, int mode) {
   SigmaBufs b{};
-  if (fp64_mode(mode)) {
+  if (mode == MBPT_MODE_FP64) {
+    b.batch = tau_batch(ntau, d.M * (2 * d.M + d.naux + d.n) + d.naux * d.naux);
+    // Zt (W = I) takes the place of U and W
+    const int64_t uw = b.batch * d.naux * (d.M + d.naux);
+    b.U = ar.take<double>(std::max(uw, d.M * d.M));
+    b.Ws = ar.counting ? nullptr : b.U + b.batch * d.M * d.naux;
+    b.Zt = b.U;
+    b.Hl = ar.take<double>(b.batch * d.M * d.M);
+    b.Hg = ar.take<double>(b.batch * d.M * d.M);
+    b.Xo_s = ar.take<double>(b.batch * d.M * d.nocc);
+    b.Xv_s = ar.take<double>(b.batch * d.M * d.nv);
+    b.Xs = ar.take<double>(d.M * static_cast<int64_t>(nstates));
+  } else if (fp64_mode(mode)) {
     b.U = ar.take<double>(d.M * d.naux);
     b.Zt = ar.take<double>(d.M * d.M);
-    b.G = ar.take<double>(d.M * d.M);
+    b.Hl = ar.take<double>(d.M * d.M);
     b.Xo_s = ar.take<double>(d.M * d.nocc);
     b.Xv_s = ar.take<double>(d.M * d.nv);
     b.Xs = ar.take<double>(d.M * static_cast<int64_t>(nstates));
@@ -1089,7 +1161,40 @@ int sigma_run(const double *X, const Dims &d, const double *eps, double mu, cons
   if (ar.overflow()) return MBPT_ERR_WORKSPACE;
   const int64_t a2 = d.naux * d.naux;
   const int64_t S = nstates;
-  if (fp64_mode(mode)) {
+  if (mode == MBPT_MODE_FP64) {
+    launch_gather_cols_f64(X, d.M, d.n, states, S, b.Xs, st);
+    if (cudaMemsetAsync(branch, 0, sizeof(double) * 2 * ntau * S, st) != cudaSuccess)
+      return MBPT_ERR_CUDA;
+    const int64_t mo = d.M * d.nocc, mv = d.M * d.nv, m2 = d.M * d.M, ma = d.M * d.naux;
+    int rc = MBPT_OK;
+    if (!Wt)  // W = I: Zt = D D^T at every tau point
+      rc = dmma::gemm({D, d.naux, 0}, true, {D, d.naux, 0}, true, d.M, d.M, d.naux, 1.0, 0.0,
+                      b.Zt, d.M, 0, 1, true, st);
+    for (int k = 0; k < ntau && !rc; k += b.batch) {
+      const int nb = std::min(b.batch, ntau - k);
+      launch_scaled_branches_batch(X, d.M, d.n, d.nocc, eps, mu, tau_list(tau + k, nb), b.Xo_s,
+                                   b.Xv_s, st);
+      // Zt = D Wt D^T (MBPTcode imaginary_time.py:508, :513). The branch sums
+      // x^T (G o Zt) x see Zt's symmetric part only, which Wt's gives
+      if (Wt) {
+        launch_sym_half(Wt + k * a2, b.Ws, d.naux, nb, st);
+        rc = dmma::gemm({D, d.naux, 0}, true, {b.Ws, d.naux, a2}, false, d.M, d.naux, d.naux,
+                        1.0, 0.0, b.U, d.naux, ma, nb, false, st);
+        if (rc) break;
+      }
+      // H^< = G_occ o Zt and H^> = G_virt o Zt, contracted with X_s on both
+      // sides; the greater branch has a minus sign
+      rc = dmma::sigma_h(Wt ? nullptr : b.Zt, {b.U, d.naux, ma}, {D, d.naux, 0}, d.naux,
+                         {b.Xo_s, d.nocc, mo}, {X, d.n, 0}, d.nocc, {b.Xv_s, d.nv, mv},
+                         {X + d.nocc, d.n, 0}, d.nv, d.M, b.Hl, b.Hg, m2, nb, st);
+      if (!rc)
+        rc = dmma::half_quadratic(b.Hl, m2, d.M, b.Xs, S, 1.0, branch + k * S, S, nb, st);
+      if (!rc)
+        rc = dmma::half_quadratic(b.Hg, m2, d.M, b.Xs, S, -1.0, branch + (ntau + k) * S, S, nb,
+                                  st);
+    }
+    if (rc) return rc;
+  } else if (fp64_mode(mode)) {
     cublasHandle_t h = handles(st).blas;
     launch_gather_cols_f64(X, d.M, d.n, states, S, b.Xs, st);
     for (int k = 0; k < ntau; ++k) {
@@ -1105,19 +1210,19 @@ int sigma_run(const double *X, const Dims &d, const double *eps, double mu, cons
       double *out_g = branch + static_cast<int64_t>(ntau + k) * S;
       // lesser branch: G_occ o Zt contracted with X_s on both sides
       if (!gemm_mode(mode, h, false, true, d.M, d.M, d.nocc, 1.0, b.Xo_s, d.nocc, X, d.n, 0.0,
-                     b.G, d.M))
+                     b.Hl, d.M))
         return MBPT_ERR_CUDA;
-      launch_hadamard(b.G, b.Zt, d.M * d.M, st);
-      if (!gemm_mode(mode, h, false, false, d.M, S, d.M, 1.0, b.G, d.M, b.Xs, S, 0.0, b.R, S))
+      launch_hadamard(b.Hl, b.Zt, d.M * d.M, st);
+      if (!gemm_mode(mode, h, false, false, d.M, S, d.M, 1.0, b.Hl, d.M, b.Xs, S, 0.0, b.R, S))
         return MBPT_ERR_CUDA;
       cudaMemsetAsync(out_l, 0, sizeof(double) * S, st);
       launch_rowdot(b.R, S, b.Xs, S, d.M, S, 1.0, out_l, st);
       // greater branch, with its minus sign
       if (!gemm_mode(mode, h, false, true, d.M, d.M, d.nv, 1.0, b.Xv_s, d.nv, X + d.nocc, d.n,
-                     0.0, b.G, d.M))
+                     0.0, b.Hl, d.M))
         return MBPT_ERR_CUDA;
-      launch_hadamard(b.G, b.Zt, d.M * d.M, st);
-      if (!gemm_mode(mode, h, false, false, d.M, S, d.M, 1.0, b.G, d.M, b.Xs, S, 0.0, b.R, S))
+      launch_hadamard(b.Hl, b.Zt, d.M * d.M, st);
+      if (!gemm_mode(mode, h, false, false, d.M, S, d.M, 1.0, b.Hl, d.M, b.Xs, S, 0.0, b.R, S))
         return MBPT_ERR_CUDA;
       cudaMemsetAsync(out_g, 0, sizeof(double) * S, st);
       launch_rowdot(b.R, S, b.Xs, S, d.M, S, -1.0, out_g, st);
@@ -1221,7 +1326,7 @@ int back_run(const double *pbar, const double *X, const Dims &d, const double *e
   cudaMemsetAsync(D_bar, 0, sizeof(double) * d.M * d.naux, st);
   for (int k = 0; k < ntau; ++k) {
     // MBPTcode gradients/rpa/space_time_adjoint.py:196-217, one row tile
-    launch_sym_half(pbar + k * a2, b.pb, d.naux, st);
+    launch_sym_half(pbar + k * a2, b.pb, d.naux, 1, st);
     if (!gemm_mode(mode, h, false, false, d.M, d.naux, d.naux, -2.0, D, d.naux, b.pb, d.naux, 0.0,
                   b.E, d.naux))
       return MBPT_ERR_CUDA;

@@ -1,0 +1,481 @@
+// FP64 products of the sweeps on the FP64 tensor pipe (mma.sync m8n8k4 f64):
+// the N^3 products of MBPT_MODE_FP64, many tau points per launch, only the
+// tiles on and above the diagonal of a symmetric result, and the element-wise
+// and contraction steps that follow in the same kernel. Every multiply and
+// add is FP64, as in a library DGEMM.
+//
+// What bounds it: the FP64 pipe (64 FMA per clock and SM, 37 TFLOP/s; cuBLAS
+// DGEMM reaches 35.7 here). A library product cannot leave out the half of a
+// symmetric result that the other half determines, writes G_occ, G_virt and
+// Zt to memory for a pass of their own, and takes a launch per product and
+// tau point, which at M = 888 is most of the time.
+//
+// Layout: a CTA of four warps owns a 64 x BN tile (BN = 64, or 32 for few
+// columns), each warp 32 x BN/2 of it in registers. The operands come through a
+// three-stage cp.async ring of 16 K columns per stage. An operand tile lies in
+// shared memory as in global memory, [row][k] with a row stride of 20 doubles
+// or [k][row] with a stride of rows + 4: both strides are 4 modulo 16, so the
+// sixteen lanes of a fragment load's half warp (four rows, four k) fall into
+// sixteen different 8-byte banks. 128 threads and 61 KB: three CTAs per SM,
+// one's epilogue under the others' products. Rows of odd length or
+// odd origin are copied 8 bytes at a time, the others 16.
+// Measured (B200): 34.3 TFLOP/s on Pi D at M = naux = 2400, five tau points a
+// launch (cuBLAS 34.1, one point a launch); smaller warp tiles (32 x 16, more
+// warps) 32.8, two CTAs per SM with a deeper ring 32.1. The sweep with it
+// (n = 400, M = naux = 2400, 20 points): chi0 36.9 -> 27.2 ms, Sigma of 400
+// states 45.0 -> 32.0 ms; E_c at M = 888, naux = 141: 1.51 -> 0.76 ms.
+#include <algorithm>
+
+#include "dmma.h"
+
+namespace mbpt {
+namespace dmma {
+namespace {
+
+constexpr int BM = 64, BK = 16, kStages = 3, kThreads = 128;
+constexpr int kKStride = BK + 4;  // [row][k] tiles
+
+template <bool KC, int R>
+struct Tile {
+  static constexpr int kStride = KC ? kKStride : R + 4;
+  static constexpr int kDoubles = KC ? R * kKStride : BK * (R + 4);
+  __device__ static __forceinline__ int at(int r, int k) {
+    return KC ? r * kStride + k : k * kStride + r;
+  }
+};
+
+template <int BN, bool AK, bool BKC>
+struct Smem {
+  static constexpr int kA = Tile<AK, BM>::kDoubles, kB = Tile<BKC, BN>::kDoubles;
+  static constexpr int kStage = kA + kB;
+  static constexpr int kBytes = kStages * kStage * 8;
+};
+
+__device__ __forceinline__ void cp16(void *dst, const void *src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                   static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src), "r"(bytes));
+}
+__device__ __forceinline__ void cp8(void *dst, const void *src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(
+                   static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src), "r"(bytes));
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N));
+}
+
+// One operand's stream of tiles: rows [r0, r0 + R), K columns from k0 on, BK at
+// a time, zeros past `rows` and `kend`. The copies of a tile that lies inside
+// the matrix cost one pointer addition each (with the bounds worked out per
+// copy, integer instructions outnumbered the DMMAs five to one and the FP64
+// pipe was 85 % busy).
+template <bool KC, int R>
+struct Stream {
+  using T = Tile<KC, R>;
+  const double *base, *p;  // the operand; this thread's first copy of the next tile
+  int64_t ld;
+  int r0, rows, k0, kend;
+  bool wide;
+
+  __device__ __forceinline__ void start(const double *g, int64_t ld_, int r0_, int rows_,
+                                        int k0_, int kend_, bool wide_) {
+    base = g;
+    ld = ld_;
+    r0 = r0_;
+    rows = rows_;
+    k0 = k0_;
+    kend = kend_;
+    wide = wide_;
+    const int tid = threadIdx.x, w = wide ? 2 : 1;
+    const int r = KC ? tid / (BK / w) : tid % (R / w) * w;
+    const int k = KC ? tid % (BK / w) * w : tid / (R / w);
+    p = g + (KC ? static_cast<int64_t>(r0 + r) * ld + k0 + k
+                : static_cast<int64_t>(k0 + k) * ld + r0 + r);
+  }
+
+  template <int W>
+  __device__ __forceinline__ void tile(double *s) {
+    constexpr int kCopies = R * BK / W / kThreads;
+    constexpr int kRows = KC ? kThreads / (BK / W) : kThreads / (R / W);  // a copy's step
+    const int tid = threadIdx.x;
+    const int r = KC ? tid / (BK / W) : tid % (R / W) * W;
+    const int k = KC ? tid % (BK / W) * W : tid / (R / W);
+    double *dst = s + T::at(r, k);
+    constexpr int kDst = kRows * T::kStride;
+    const int64_t step = kRows * ld;
+    if (r0 + R <= rows && k0 + BK <= kend) {
+      const double *src = p;
+#pragma unroll
+      for (int i = 0; i < kCopies; ++i, src += step) {
+        if constexpr (W == 2)
+          cp16(dst + i * kDst, src, 16);
+        else
+          cp8(dst + i * kDst, src, 8);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < kCopies; ++i) {
+        const int ri = r0 + r + (KC ? i * kRows : 0), ki = k0 + k + (KC ? 0 : i * kRows);
+        const int in = KC ? (ri < rows ? min(max(kend - ki, 0), W) : 0)
+                          : (ki < kend ? min(max(rows - ri, 0), W) : 0);
+        const double *src = in ? p + i * step : base;
+        if constexpr (W == 2)
+          cp16(dst + i * kDst, src, 8 * in);
+        else
+          cp8(dst + i * kDst, src, 8 * in);
+      }
+    }
+  }
+
+  __device__ __forceinline__ void load(double *s) {
+    if (wide)
+      tile<2>(s);
+    else
+      tile<1>(s);
+    k0 += BK;
+    p += KC ? BK : BK * ld;
+  }
+};
+
+__device__ __forceinline__ void mma(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+// tile `idx` of the upper triangle of nt x nt tiles, row by row
+__device__ __forceinline__ void upper_tile(int idx, int nt, int &ti, int &tj) {
+  const double q = 2.0 * nt + 1.0;
+  int i = static_cast<int>(0.5 * (q - sqrt(q * q - 8.0 * idx)));
+  i = max(0, min(i, nt - 1));
+  auto first = [nt](int r) { return r * nt - r * (r - 1) / 2; };
+  while (i > 0 && first(i) > idx) --i;
+  while (i + 1 < nt && first(i + 1) <= idx) ++i;
+  ti = i;
+  tj = i + idx - first(i);
+}
+
+struct Args {
+  Operand a[3], b[3];
+  int k[3];
+  bool wa[3], wb[3];  // 16-byte copies
+  int m, n, tiles_m, tiles_n;
+  bool upper;
+  double alpha, beta;
+  double *c0, *c1;
+  int64_t ldc, sc;
+  const double *zt;    // SIGMA: Zt as stored (ld m) instead of the first product
+  const double *xs;    // row contraction
+  int64_t ld_xs;
+  double *out;
+  int64_t s_out;
+};
+
+enum Epi : int {
+  STORE = 0,     // C = alpha acc + beta C (upper: and its mirror)
+  PRODUCT = 1,   // C = acc0 o acc1, mirrored
+  SIGMA = 2,     // c0 = acc1 o acc0, c1 = acc2 o acc0: upper tiles, the diagonal ones halved
+  ROWDOT = 3,    // out[p] += alpha sum_r xs[r, p] acc[r, p], K from the tile's first row
+};
+
+template <int BN, bool AK, bool BKC, int EPI>
+__global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const __grid_constant__ Args p) {
+  using S = Smem<BN, AK, BKC>;
+  constexpr int NS = EPI == SIGMA ? 3 : (EPI == PRODUCT ? 2 : 1);
+  constexpr int MI = 4, NJ = BN / 16;  // 8 x 8 blocks of a warp's 32 x BN/2
+  extern __shared__ __align__(16) double sm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int wm = (warp & 1) * 32, wn = (warp >> 1) * (BN / 2);
+  int ti, tj;
+  if (p.upper) {
+    upper_tile(blockIdx.x, p.tiles_m, ti, tj);
+  } else {
+    // eight row tiles sweep the column tiles together (L2 reuse)
+    const int per = 8 * p.tiles_n, grp = blockIdx.x / per, first = grp * 8;
+    const int rows = min(8, p.tiles_m - first), in = blockIdx.x % per;
+    ti = first + in % rows;
+    tj = in / rows;
+  }
+  const int m0 = ti * BM, n0 = tj * BN;
+  const int64_t z = blockIdx.z;
+  const int k_first = EPI == ROWDOT ? m0 : 0;
+  int tiles[NS], total = 0;
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    tiles[s] = (p.k[s] - k_first + BK - 1) / BK;
+    total += tiles[s];
+  }
+  // the tiles of the products, one product after the other
+  Stream<AK, BM> fa;
+  Stream<BKC, BN> fb;
+  int fseg = EPI == SIGMA && tiles[0] == 0 ? 1 : 0, fleft = tiles[fseg], fstage = 0;
+  auto open = [&](int s) {
+    fa.start(p.a[s].p + z * p.a[s].stride, p.a[s].ld, m0, p.m, k_first, p.k[s], p.wa[s]);
+    fb.start(p.b[s].p + z * p.b[s].stride, p.b[s].ld, n0, p.n, k_first, p.k[s], p.wb[s]);
+  };
+  open(fseg);
+  auto fetch = [&] {
+    double *st = sm + fstage * S::kStage;
+    fa.load(st);
+    fb.load(st + S::kA);
+    fstage = fstage + 1 == kStages ? 0 : fstage + 1;
+    if (NS > 1 && --fleft == 0 && fseg + 1 < NS) {
+      ++fseg;
+      fleft = tiles[fseg < NS ? fseg : 0];
+      open(fseg < NS ? fseg : 0);
+    }
+  };
+  double acc[MI][NJ][2];
+  double keep[NS > 1 ? MI : 1][NS > 1 ? NJ : 1][2];
+  auto clear = [&] {
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  };
+  // an element-wise result: the tile and, above the diagonal, its mirror
+  auto store = [&](double *c, auto value, bool mirror) {
+#pragma unroll
+    for (int i = 0; i < MI; ++i) {
+      const int r = m0 + wm + 8 * i + g;
+      if (r >= p.m) continue;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int col = n0 + wn + 8 * j + 2 * t + e;
+          if (col >= p.n) continue;
+          double *at = c + z * p.sc + static_cast<int64_t>(r) * p.ldc + col;
+          const double v = value(i, j, e, at);
+          *at = v;
+          if (mirror) c[z * p.sc + static_cast<int64_t>(col) * p.ldc + r] = v;
+        }
+    }
+  };
+  clear();
+  int seg_end = tiles[0];
+  [[maybe_unused]] int seg = 0;
+  if constexpr (EPI == SIGMA) {
+    if (p.zt) {
+      seg = 1;
+      seg_end = tiles[1];
+#pragma unroll
+      for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int r = m0 + wm + 8 * i + g, col = n0 + wn + 8 * j + 2 * t + e;
+            keep[i][j][e] = r < p.m && col < p.n ? p.zt[static_cast<int64_t>(r) * p.ldc + col] : 0.0;
+          }
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < kStages - 1; ++s) {
+    if (s < total) fetch();
+    cp_commit();
+  }
+  int stage = 0;
+  for (int it = 0; it < total; ++it) {
+    cp_wait<kStages - 2>();
+    __syncthreads();
+    if (it + kStages - 1 < total) fetch();
+    cp_commit();
+    const double *sa = sm + stage * S::kStage, *sb = sa + S::kA;
+    stage = stage + 1 == kStages ? 0 : stage + 1;
+#pragma unroll
+    for (int kk = 0; kk < BK; kk += 4) {
+      double a[MI], b[NJ];
+#pragma unroll
+      for (int i = 0; i < MI; ++i) a[i] = sa[Tile<AK, BM>::at(wm + 8 * i + g, kk + t)];
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) b[j] = sb[Tile<BKC, BN>::at(wn + 8 * j + g, kk + t)];
+#pragma unroll
+      for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) mma(acc[i][j], a[i], b[j]);
+    }
+    if constexpr (NS > 1) {
+      if (it + 1 == seg_end && seg + 1 < NS) {
+        if (seg == 0) {
+#pragma unroll
+          for (int i = 0; i < MI; ++i)
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) {
+              keep[i][j][0] = acc[i][j][0];
+              keep[i][j][1] = acc[i][j][1];
+            }
+        } else {
+          const double f = ti == tj ? 0.5 : 1.0;
+          store(p.c0, [&](int i, int j, int e, double *) { return acc[i][j][e] * keep[i][j][e] * f; },
+                false);
+        }
+        clear();
+        ++seg;
+        seg_end += tiles[seg < NS ? seg : 0];
+      }
+    }
+  }
+  if constexpr (EPI == STORE) {
+    const double alpha = p.alpha, beta = p.beta;
+    store(p.c0,
+          [&](int i, int j, int e, const double *at) {
+            const double v = alpha * acc[i][j][e];
+            return beta == 0.0 ? v : v + beta * *at;
+          },
+          p.upper && tj > ti);
+  } else if constexpr (EPI == PRODUCT) {
+    store(p.c0, [&](int i, int j, int e, double *) { return acc[i][j][e] * keep[i][j][e]; },
+          tj > ti);
+  } else if constexpr (EPI == SIGMA) {
+    const double f = ti == tj ? 0.5 : 1.0;
+    store(p.c1, [&](int i, int j, int e, double *) { return acc[i][j][e] * keep[i][j][e] * f; },
+          false);
+  } else {
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int col = n0 + wn + 8 * j + 2 * t + e;
+        double s = 0.0;
+#pragma unroll
+        for (int i = 0; i < MI; ++i) {
+          const int r = m0 + wm + 8 * i + g;
+          if (r < p.m && col < p.n) s = fma(p.xs[static_cast<int64_t>(r) * p.ld_xs + col],
+                                            acc[i][j][e], s);
+        }
+#pragma unroll
+        for (int d = 4; d < 32; d <<= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+        if (g == 0 && col < p.n) atomicAdd(p.out + z * p.s_out + col, p.alpha * s);
+      }
+  }
+}
+
+bool wide(const Operand &o, int64_t batch) {
+  return (reinterpret_cast<uintptr_t>(o.p) & 15) == 0 && o.ld % 2 == 0 &&
+         (batch <= 1 || o.stride % 2 == 0);
+}
+
+template <int BN, bool AK, bool BKC, int EPI>
+int launch(Args &p, int batch, cudaStream_t st) {
+  constexpr int NS = EPI == SIGMA ? 3 : (EPI == PRODUCT ? 2 : 1);
+  using S = Smem<BN, AK, BKC>;
+  if (p.m < 1 || p.n < 1 || batch < 1 || batch > 65535) return MBPT_ERR_SHAPE;
+  for (int s = 0; s < NS; ++s) {
+    if (p.k[s] < (EPI == SIGMA && s == 0 && p.zt ? 0 : 1)) return MBPT_ERR_SHAPE;
+    p.wa[s] = wide(p.a[s], batch);
+    p.wb[s] = wide(p.b[s], batch);
+  }
+  p.tiles_m = (p.m + BM - 1) / BM;
+  p.tiles_n = (p.n + BN - 1) / BN;
+  if (p.upper && (BN != BM || p.m != p.n)) return MBPT_ERR_SHAPE;
+  const int64_t grid = p.upper ? static_cast<int64_t>(p.tiles_m) * (p.tiles_m + 1) / 2
+                               : static_cast<int64_t>(p.tiles_m) * p.tiles_n;
+  if (grid > (int64_t{1} << 30)) return MBPT_ERR_SHAPE;
+  auto kern = dmma_kernel<BN, AK, BKC, EPI>;
+  static std::atomic<uint64_t> attr{0};
+  if (!allow_smem(reinterpret_cast<const void *>(kern), S::kBytes, attr)) return MBPT_ERR_CUDA;
+  count_launch();
+  kern<<<dim3(static_cast<unsigned>(grid), 1, static_cast<unsigned>(batch)), kThreads, S::kBytes,
+         st>>>(p);
+  return cudaGetLastError() == cudaSuccess ? MBPT_OK : MBPT_ERR_CUDA;
+}
+
+// Whether 32-wide tiles pad n columns so much less than 64-wide ones that
+// their lower rate pays (33.9 against 34.3 TFLOP/s at n = 2400, where both pad
+// alike; 24.7 against 21.1 at n = 141, 160 columns against 192).
+bool narrow(int64_t n) { return round_up(n, 64) * 20 >= round_up(n, 32) * 21; }
+
+bool fits(int64_t v) { return v > 0 && v <= (int64_t{1} << 30); }
+
+}  // namespace
+
+int gemm(const Operand &a, bool a_k, const Operand &b, bool b_k, int64_t m, int64_t n, int64_t k,
+         double alpha, double beta, double *c, int64_t ldc, int64_t sc, int batch, bool upper,
+         cudaStream_t st) {
+  if (!fits(m) || !fits(n) || !fits(k)) return MBPT_ERR_SHAPE;
+  Args p{};
+  p.a[0] = a;
+  p.b[0] = b;
+  p.k[0] = static_cast<int>(k);
+  p.m = static_cast<int>(m);
+  p.n = static_cast<int>(n);
+  p.alpha = alpha;
+  p.beta = beta;
+  p.c0 = c;
+  p.ldc = ldc;
+  p.sc = sc;
+  p.upper = upper;
+  if (a_k && b_k) return launch<64, true, true, STORE>(p, batch, st);
+  if (a_k && narrow(n)) return launch<32, true, false, STORE>(p, batch, st);
+  if (a_k) return launch<64, true, false, STORE>(p, batch, st);
+  if (!b_k) return launch<64, false, false, STORE>(p, batch, st);
+  return MBPT_ERR_UNSUPPORTED;
+}
+
+int hadamard_product(const Operand &a0, const Operand &b0, int64_t k0, const Operand &a1,
+                     const Operand &b1, int64_t k1, int64_t m, double *c, int64_t ldc,
+                     int64_t sc, int batch, cudaStream_t st) {
+  if (!fits(m) || !fits(k0) || !fits(k1)) return MBPT_ERR_SHAPE;
+  Args p{};
+  p.a[0] = a0;
+  p.b[0] = b0;
+  p.a[1] = a1;
+  p.b[1] = b1;
+  p.k[0] = static_cast<int>(k0);
+  p.k[1] = static_cast<int>(k1);
+  p.m = p.n = static_cast<int>(m);
+  p.c0 = c;
+  p.ldc = ldc;
+  p.sc = sc;
+  p.upper = true;
+  return launch<64, true, true, PRODUCT>(p, batch, st);
+}
+
+int sigma_h(const double *zt, const Operand &u, const Operand &d, int64_t naux,
+            const Operand &xo_s, const Operand &xo, int64_t nocc, const Operand &xv_s,
+            const Operand &xv, int64_t nv, int64_t m, double *hl, double *hg, int64_t sh,
+            int batch, cudaStream_t st) {
+  if (!fits(m) || !fits(naux) || !fits(nocc) || !fits(nv)) return MBPT_ERR_SHAPE;
+  Args p{};
+  p.zt = zt;
+  const Operand *as[3] = {&u, &xo_s, &xv_s}, *bs[3] = {&d, &xo, &xv};
+  const int64_t ks[3] = {zt ? 0 : naux, nocc, nv};
+  for (int s = 0; s < 3; ++s) {
+    p.a[s] = *as[s];
+    p.b[s] = *bs[s];
+    p.k[s] = static_cast<int>(ks[s]);
+  }
+  p.m = p.n = static_cast<int>(m);
+  p.c0 = hl;
+  p.c1 = hg;
+  p.ldc = m;
+  p.sc = sh;
+  p.upper = true;
+  return launch<64, true, true, SIGMA>(p, batch, st);
+}
+
+int half_quadratic(const double *h, int64_t sh, int64_t m, const double *xs, int64_t ns,
+                   double sign, double *out, int64_t s_out, int batch, cudaStream_t st) {
+  if (!fits(m) || !fits(ns)) return MBPT_ERR_SHAPE;
+  Args p{};
+  p.a[0] = {h, m, sh};
+  p.b[0] = {xs, ns, 0};
+  p.k[0] = static_cast<int>(m);
+  p.m = static_cast<int>(m);
+  p.n = static_cast<int>(ns);
+  p.alpha = 2.0 * sign;
+  p.xs = xs;
+  p.ld_xs = ns;
+  p.out = out;
+  p.s_out = s_out;
+  if (narrow(ns)) return launch<32, true, false, ROWDOT>(p, batch, st);
+  return launch<64, true, false, ROWDOT>(p, batch, st);
+}
+
+}  // namespace dmma
+}  // namespace mbpt

@@ -1,0 +1,46 @@
+// FP64 products on the FP64 tensor pipe (dmma.cu), batched over tau points.
+#pragma once
+#include "internal.h"
+
+namespace mbpt {
+namespace dmma {
+
+// An FP64 operand: element (r, k) at p[r ld + k] (K contiguous) or
+// p[k ld + r] (rows contiguous), `stride` doubles between batch members
+// (0: the same for all).
+struct Operand {
+  const double *p = nullptr;
+  int64_t ld = 0, stride = 0;
+};
+
+// C (m x n, row-major, ldc) = alpha A B^T + beta C per batch member, A (m x k)
+// and B (n x k) K-contiguous (a_k, b_k) or row-contiguous (not A
+// row-contiguous with B K-contiguous). upper: the product is symmetric (m ==
+// n): the tiles on and above the diagonal are formed and mirrored.
+int gemm(const Operand &a, bool a_k, const Operand &b, bool b_k, int64_t m, int64_t n, int64_t k,
+         double alpha, double beta, double *c, int64_t ldc, int64_t sc, int batch, bool upper,
+         cudaStream_t st);
+
+// C (m x m) = (A0 B0^T) o (A1 B1^T), both symmetric: Pi = G_occ o G_virt.
+// All operands K-contiguous.
+int hadamard_product(const Operand &a0, const Operand &b0, int64_t k0, const Operand &a1,
+                     const Operand &b1, int64_t k1, int64_t m, double *c, int64_t ldc,
+                     int64_t sc, int batch, cudaStream_t st);
+
+// Zt = U D^T, hl = (Xo_s Xo^T) o Zt and hg = (Xv_s Xv^T) o Zt (all symmetric,
+// K-contiguous operands), leading dimension m, as `half_quadratic` reads
+// them: the 64 x 64 tiles on and above the diagonal only, the diagonal ones
+// times 1/2. zt not null: Zt (m x m, its upper triangle, the same for the
+// whole batch) is read instead of formed from u and d.
+int sigma_h(const double *zt, const Operand &u, const Operand &d, int64_t naux,
+            const Operand &xo_s, const Operand &xo, int64_t nocc, const Operand &xv_s,
+            const Operand &xv, int64_t nv, int64_t m, double *hl, double *hg, int64_t sh,
+            int batch, cudaStream_t st);
+
+// out[p] += sign x_p^T H x_p for the ns columns x_p of xs (m x ns) and the
+// symmetric H held as sigma_h leaves it: twice the sum over its tiles.
+int half_quadratic(const double *h, int64_t sh, int64_t m, const double *xs, int64_t ns,
+                   double sign, double *out, int64_t s_out, int batch, cudaStream_t st);
+
+}  // namespace dmma
+}  // namespace mbpt

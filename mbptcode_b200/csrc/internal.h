@@ -138,6 +138,16 @@ void launch_split_pad_tf32(const double *src, int64_t rows, int64_t cols, int64_
 void launch_scaled_branches(const double *X, int64_t M, int64_t n, int64_t nocc,
                             const double *eps, double mu, double tau, double power,
                             double *Xo_s, double *Xv_s, cudaStream_t st);
+// the tau points of one batched launch
+constexpr int kMaxTauBatch = 34;
+struct TauList {
+  double t[kMaxTauBatch];
+  int n;
+};
+// Xo_s (n taus x M x nocc) and Xv_s (n taus x M x (norb - nocc)), power 1
+void launch_scaled_branches_batch(const double *X, int64_t M, int64_t n, int64_t nocc,
+                                  const double *eps, double mu, const TauList &taus,
+                                  double *Xo_s, double *Xv_s, cudaStream_t st);
 void launch_hadamard(double *a, const double *b, int64_t n, cudaStream_t st);
 void launch_hadamard3(double *out, const double *a, const double *b, int64_t n, cudaStream_t st);
 // out[j] = sum_k w[j,k] in[k] over a rows x cols block of each slice

@@ -174,6 +174,25 @@ __global__ void scaled_branches_kernel(const double *__restrict__ X, int64_t M, 
   }
 }
 
+// The same for several tau points at once (blockIdx.y), each M x nocc and
+// M x (n - nocc), one after the other.
+__global__ void scaled_branches_batch_kernel(const double *__restrict__ X, int64_t M, int64_t n,
+                                             int64_t nocc, const double *__restrict__ eps,
+                                             double mu, const __grid_constant__ TauList taus,
+                                             double *Xo_s, double *Xv_s) {
+  const double tau = taus.t[blockIdx.y];
+  const int64_t total = M * n, nv = n - nocc;
+  double *o = Xo_s + blockIdx.y * M * nocc, *v = Xv_s + blockIdx.y * M * nv;
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t r = i / n, c = i % n;
+    if (c < nocc)
+      o[r * nocc + c] = X[i] * exp((eps[c] - mu) * tau);
+    else
+      v[r * nv + (c - nocc)] = X[i] * exp(-(eps[c] - mu) * tau);
+  }
+}
+
 __global__ void hadamard_kernel(double *a, const double *__restrict__ b, int64_t n) {
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x)
@@ -474,6 +493,14 @@ void launch_scaled_branches(const double *X, int64_t M, int64_t n, int64_t nocc,
                             double *Xo_s, double *Xv_s, cudaStream_t st) {
   count_launch(); scaled_branches_kernel<<<grid_cap(M * n), kThreads, 0, st>>>(X, M, n, nocc, eps, mu, tau,
                                                                power, Xo_s, Xv_s);
+}
+
+void launch_scaled_branches_batch(const double *X, int64_t M, int64_t n, int64_t nocc,
+                                  const double *eps, double mu, const TauList &taus,
+                                  double *Xo_s, double *Xv_s, cudaStream_t st) {
+  count_launch();
+  scaled_branches_batch_kernel<<<dim3(grid_cap(M * n), taus.n), kThreads, 0, st>>>(
+      X, M, n, nocc, eps, mu, taus, Xo_s, Xv_s);
 }
 
 void launch_hadamard(double *a, const double *b, int64_t n, cudaStream_t st) {
