@@ -121,6 +121,27 @@ __device__ __forceinline__ void tmem_ld32_s32(uint32_t addr, int (&v)[32]) {
       : "memory");
 }
 
+// Shared tile of the cutting kernels, 32 rows x 128 columns: one double of
+// padding per 16 columns and a row stride of 137, so that a half warp hits 16
+// different 8-byte banks when it writes 16 columns or 16 rows, and 15 when it
+// reads two rows at eight 16-column groups (8 lanes in one bank without).
+constexpr int kCutStride = 137;
+__device__ __forceinline__ int cut_at(int r, int c) { return r * kCutStride + c + (c >> 4); }
+
+// The next digit of t (|t| <= 127): adding 1.5 2^52 leaves rint(t), ties to
+// even, in the low word, so a digit costs FP64 additions instead of the
+// conversion unit's two instructions (16 lanes per clock and SM; the cutting
+// kernels ran at its rate: 60 us for two 2400 x 2400 operands, 8 digits; now
+// 36 us). t
+// becomes the exact remainder times the base. A t that is not finite gives
+// some byte and stays not finite.
+__device__ __forceinline__ int8_t next_digit(double &t, double base) {
+  constexpr double kMagic = 6755399441055744.0;  // 1.5 2^52
+  const double r = t + kMagic;
+  t = (t - (r - kMagic)) * base;
+  return static_cast<int8_t>(__double2loint(r));
+}
+
 enum Epi : int {
   EPI_CHOL = 0,  // the Cholesky panel: P -= product, column-major, exact diagonal
   EPI_GEMM = 1,  // C = alpha product + beta C, row-major
@@ -422,7 +443,7 @@ template <int S>
 __global__ void chol_slice_kernel(const double *A, int64_t n, int64_t mat_stride, int nmat,
                                   int j0, int nb, const double *scale, int8_t *D,
                                   int64_t npad, double *rownorm) {
-  __shared__ double tile[32][129];
+  __shared__ double tile[32 * kCutStride];
   const int f = blockIdx.y;
   const int64_t rbase = j0 + static_cast<int64_t>(blockIdx.x) * 32;
   const double *Af = A + f * mat_stride;
@@ -432,7 +453,7 @@ __global__ void chol_slice_kernel(const double *A, int64_t n, int64_t mat_stride
     const int64_t r = rbase + rr;
     // the factor is lower triangular: above the block's diagonal A still holds
     // 1 - chi0, which is not part of L
-    tile[rr][cc] = (r < n && cc < nb && r >= j0 + cc)
+    tile[cut_at(rr, cc)] = (r < n && cc < nb && r >= j0 + cc)
                        ? Af[static_cast<int64_t>(j0 + cc) * n + r] : 0.0;
   }
   __syncthreads();
@@ -444,7 +465,7 @@ __global__ void chol_slice_kernel(const double *A, int64_t n, int64_t mat_stride
   // fixed order
   double sq = 0.0;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) sq = fma(tile[rr][cg + i], tile[rr][cg + i], sq);
+  for (int i = 0; i < 16; ++i) sq = fma(tile[cut_at(rr, cg + i)], tile[cut_at(rr, cg + i)], sq);
   sq += __shfl_xor_sync(0xffffffffu, sq, 1);
   sq += __shfl_xor_sync(0xffffffffu, sq, 2);
   sq += __shfl_xor_sync(0xffffffffu, sq, 4);
@@ -456,14 +477,9 @@ __global__ void chol_slice_kernel(const double *A, int64_t n, int64_t mat_stride
   __align__(16) int8_t out[S][16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
-    double t = tile[rr][cg + i] * inv;   // |t| <= kTop
+    double t = tile[cut_at(rr, cg + i)] * inv;   // |t| <= kTop
 #pragma unroll
-    for (int q = 0; q < S; ++q) {
-      double d = rint(t);
-      d = fmin(fmax(d, -127.0), 127.0);  // non-finite input stays in range
-      out[q][i] = static_cast<int8_t>(static_cast<int>(d));
-      t = (t - d) * kBase;
-    }
+    for (int q = 0; q < S; ++q) out[q][i] = next_digit(t, kBase);
   }
   if (cg >= nb) return;
 #pragma unroll
@@ -474,83 +490,125 @@ __global__ void chol_slice_kernel(const double *A, int64_t n, int64_t mat_stride
 }
 
 
-// scale[i] = 2^e >= max_k |x(i, k)| of each row of an operand (1 for a row
-// of zeros or with a non-finite entry); x(i, k) = src[i ld + k], or
-// src[k ld + i] with trans.
-__global__ void row_scale_kernel(const double *src, int64_t rows, int64_t kdim, int64_t ld,
-                                 int trans, double *scale) {
-  const int lane = threadIdx.x & 31;
-  if (trans) {
-    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < rows;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-      double mx = 0.0;
-      for (int64_t k = 0; k < kdim; ++k) mx = fmax(mx, fabs(src[k * ld + i]));
-      int e = 0;
-      frexp(mx, &e);
-      scale[i] = (mx > 0.0 && mx < 1e300) ? ldexp(1.0, e) : 1.0;
-    }
-    return;
-  }
-  const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x >> 5) + (threadIdx.x >> 5);
-       i < rows; i += warps) {
+// An operand as the digit cutting reads it: x(i, k) = src[i ld + k], or
+// src[k ld + i] with trans. rowmax (rows, zeroed by the caller) receives the
+// bits of max_k |x(i, k)|, planes and scale the result.
+struct Source {
+  const double *src;
+  int64_t rows, kdim, ld;
+  int trans;
+  unsigned long long *rowmax;
+  double *scale;
+  int8_t *planes;
+  int64_t rows_pad, k_pad;
+};
+struct Sources {
+  Source s[2];
+};
+
+// The row maxima of one or two operands (blockIdx.z). Two passes over memory
+// (this and the cutting, the second mostly from L2) are what the scheme needs;
+// a block takes 32 rows x 256 K columns, so that both layouts are read along
+// their contiguous index with 32 loads in flight per thread and K is spread
+// over blocks: with one thread per row of a transposed operand, walking all
+// of K, a 2400 x 2400 operand took 200 us of latency; now 7 us. The maximum
+// of non-negative doubles is that of their bits; NaN counts as nothing.
+constexpr int kMaxRows = 32, kMaxK = 256;
+
+__global__ void __launch_bounds__(256) row_max_kernel(const __grid_constant__ Sources p) {
+  const Source &s = p.s[blockIdx.z];
+  const int64_t i0 = static_cast<int64_t>(blockIdx.y) * kMaxRows;
+  const int64_t k0 = static_cast<int64_t>(blockIdx.x) * kMaxK;
+  if (i0 >= s.rows || k0 >= s.kdim) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (s.trans) {
+    // lanes on rows, each warp 32 of the K columns
+    __shared__ double part[8][32];
+    const int64_t i = i0 + lane;
     double mx = 0.0;
-    for (int64_t k = lane; k < kdim; k += 32) mx = fmax(mx, fabs(src[i * ld + k]));
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) {
-      int e = 0;
-      frexp(mx, &e);
-      scale[i] = (mx > 0.0 && mx < 1e300) ? ldexp(1.0, e) : 1.0;
+    if (i < s.rows) {
+#pragma unroll 8
+      for (int q = 0; q < kMaxK / 8; ++q) {
+        const int64_t k = k0 + warp + 8 * q;
+        if (k < s.kdim) mx = fmax(mx, fabs(s.src[k * s.ld + i]));
+      }
+    }
+    part[warp][lane] = mx;
+    __syncthreads();
+    if (warp == 0 && i < s.rows) {
+#pragma unroll
+      for (int w = 1; w < 8; ++w) mx = fmax(mx, part[w][lane]);
+      if (mx > 0.0) atomicMax(s.rowmax + i, __double_as_longlong(mx));
+    }
+  } else {
+    // each warp four rows, lanes on K
+#pragma unroll
+    for (int r = 0; r < kMaxRows / 8; ++r) {
+      const int64_t i = i0 + warp * (kMaxRows / 8) + r;
+      if (i >= s.rows) break;
+      double mx = 0.0;
+#pragma unroll
+      for (int q = 0; q < kMaxK / 32; ++q) {
+        const int64_t k = k0 + lane + 32 * q;
+        if (k < s.kdim) mx = fmax(mx, fabs(s.src[i * s.ld + k]));
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      if (lane == 0 && mx > 0.0) atomicMax(s.rowmax + i, __double_as_longlong(mx));
     }
   }
 }
 
-// Digit planes of an operand (rows x kdim, row scales `scale`): plane q, row
-// i, column k at planes[(q rows_pad + i) k_pad + k], zeros beyond rows and
-// kdim up to rows_pad and k_pad. One block per 32 rows x 128 columns,
-// through shared memory so that both layouts of the source are read along
-// their contiguous index.
+// 2^e >= the row's largest magnitude (1 for a row of zeros or with an
+// infinite entry)
+__device__ __forceinline__ double scale_of(unsigned long long max_bits) {
+  const double mx = __longlong_as_double(static_cast<long long>(max_bits));
+  int e = 0;
+  frexp(mx, &e);
+  return (mx > 0.0 && mx < 1e300) ? ldexp(1.0, e) : 1.0;
+}
+
+// Digit planes of one or two operands (blockIdx.z; rows x kdim, row maxima in
+// rowmax): plane q, row i, column k at planes[(q rows_pad + i) k_pad + k],
+// zeros beyond rows and kdim up to rows_pad and k_pad, and the rows' scales.
+// One block per 32 rows x 128 columns, through shared memory so that both
+// layouts of the source are read along their contiguous index.
 template <int S>
-__global__ void operand_slice_kernel(const double *src, int64_t rows, int64_t kdim, int64_t ld,
-                                     int trans, const double *scale, int8_t *planes,
-                                     int64_t rows_pad, int64_t k_pad) {
-  __shared__ double tile[32][129];
+__global__ void __launch_bounds__(256) operand_slice_kernel(const __grid_constant__ Sources p) {
+  __shared__ double tile[32 * kCutStride];
+  const Source &s = p.s[blockIdx.z];
   const int64_t i0 = static_cast<int64_t>(blockIdx.y) * 32;
   const int64_t k0 = static_cast<int64_t>(blockIdx.x) * 128;
-  for (int t = threadIdx.x; t < 32 * 128; t += blockDim.x) {
-    int rr, kk;
-    if (trans) {
-      rr = t & 31;
-      kk = t >> 5;
-    } else {
-      rr = t >> 7;
-      kk = t & 127;
-    }
+  if (i0 >= s.rows_pad || k0 >= s.k_pad) return;
+#pragma unroll 8
+  for (int q = 0; q < 32 * 128 / 256; ++q) {
+    const int t = threadIdx.x + 256 * q;
+    const int rr = s.trans ? t & 31 : t >> 7, kk = s.trans ? t >> 5 : t & 127;
     const int64_t i = i0 + rr, k = k0 + kk;
     double v = 0.0;
-    if (i < rows && k < kdim) v = trans ? src[k * ld + i] : src[i * ld + k];
-    tile[rr][kk] = v;
+    if (i < s.rows && k < s.kdim) v = s.trans ? s.src[k * s.ld + i] : s.src[i * s.ld + k];
+    tile[cut_at(rr, kk)] = v;
   }
   __syncthreads();
   const int rr = threadIdx.x >> 3, cg = (threadIdx.x & 7) * 16;
   const int64_t i = i0 + rr;
-  if (i >= rows_pad) return;
-  const double inv = i < rows ? 64.0 / scale[i] : 0.0;
+  if (i >= s.rows_pad) return;
+  double inv = 0.0;
+  if (i < s.rows) {
+    const double sc = scale_of(s.rowmax[i]);
+    inv = 64.0 / sc;
+    if (blockIdx.x == 0 && cg == 0) s.scale[i] = sc;
+  }
   __align__(16) int8_t out[S][16];
 #pragma unroll
   for (int c = 0; c < 16; ++c) {
-    double t = tile[rr][cg + c] * inv;     // |t| <= 64
+    double t = tile[cut_at(rr, cg + c)] * inv;     // |t| <= 64
 #pragma unroll
-    for (int q = 0; q < S; ++q) {
-      double d = rint(t);
-      d = fmin(fmax(d, -127.0), 127.0);
-      out[q][c] = static_cast<int8_t>(static_cast<int>(d));
-      t = (t - d) * 128.0;
-    }
+    for (int q = 0; q < S; ++q) out[q][c] = next_digit(t, 128.0);
   }
 #pragma unroll
   for (int q = 0; q < S; ++q) {
-    int8_t *dst = planes + (static_cast<int64_t>(q) * rows_pad + i) * k_pad + k0 + cg;
+    int8_t *dst = s.planes + (static_cast<int64_t>(q) * s.rows_pad + i) * s.k_pad + k0 + cg;
     *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(out[q]);
   }
 }
@@ -692,7 +750,7 @@ int ozaki_chol_update(double *A, int64_t n, int nmat, int64_t j0, int nb, double
 size_t ozaki_gemm_scratch_bytes(int64_t m, int64_t n, int64_t k, int slices) {
   const int64_t kc = std::min<int64_t>(round_up(k, 128), kOzakiKChunk);
   const int64_t mp = round_up(m, 128), np = round_up(n, 128);
-  return static_cast<size_t>(slices) * (mp + np) * kc + 8 * (mp + np) + 4096;
+  return static_cast<size_t>(slices) * (mp + np) * kc + 16 * (mp + np) + 4096;
 }
 
 int ozaki_dgemm(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha,
@@ -718,23 +776,23 @@ int ozaki_dgemm(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha,
         (reinterpret_cast<uintptr_t>(pb + static_cast<int64_t>(slices) * np * kp) + 255) &
         ~static_cast<uintptr_t>(255));
     double *sb = sa + mp;
+    unsigned long long *ma = reinterpret_cast<unsigned long long *>(sb + np), *mb = ma + mp;
     // op(A) rows are K-contiguous unless ta; op(B) = B^T rows unless tb
-    const double *a0 = ta ? A + kb * lda : A + kb;
-    const double *b0 = tb ? B + kb : B + kb * ldb;
-    const int at = ta ? 1 : 0, bt = tb ? 0 : 1;
+    ozaki::Sources src{};
+    src.s[0] = {ta ? A + kb * lda : A + kb, m, kc, lda, ta ? 1 : 0, ma, sa, pa, mp, kp};
+    src.s[1] = {tb ? B + kb : B + kb * ldb, n, kc, ldb, tb ? 0 : 1, mb, sb, pb, np, kp};
+    if (cudaMemsetAsync(ma, 0, sizeof(unsigned long long) * (mp + np), st) != cudaSuccess)
+      return MBPT_ERR_CUDA;
+    const int64_t rmax = std::max(mp, np);
+    const dim3 gm(static_cast<unsigned>((kc + ozaki::kMaxK - 1) / ozaki::kMaxK),
+                  static_cast<unsigned>(rmax / ozaki::kMaxRows), 2);
+    const dim3 gs(static_cast<unsigned>(kp / 128), static_cast<unsigned>(rmax / 32), 2);
     count_launch(2);
-    ozaki::row_scale_kernel<<<ozaki::grid_blocks(m * 32), 256, 0, st>>>(a0, m, kc, lda, at, sa);
-    ozaki::row_scale_kernel<<<ozaki::grid_blocks(n * 32), 256, 0, st>>>(b0, n, kc, ldb, bt, sb);
-    const dim3 ga(static_cast<unsigned>(kp / 128), static_cast<unsigned>(mp / 32));
-    const dim3 gb(static_cast<unsigned>(kp / 128), static_cast<unsigned>(np / 32));
-    count_launch(2);
-    if (slices == 8) {
-      ozaki::operand_slice_kernel<8><<<ga, 256, 0, st>>>(a0, m, kc, lda, at, sa, pa, mp, kp);
-      ozaki::operand_slice_kernel<8><<<gb, 256, 0, st>>>(b0, n, kc, ldb, bt, sb, pb, np, kp);
-    } else {
-      ozaki::operand_slice_kernel<7><<<ga, 256, 0, st>>>(a0, m, kc, lda, at, sa, pa, mp, kp);
-      ozaki::operand_slice_kernel<7><<<gb, 256, 0, st>>>(b0, n, kc, ldb, bt, sb, pb, np, kp);
-    }
+    ozaki::row_max_kernel<<<gm, 256, 0, st>>>(src);
+    if (slices == 8)
+      ozaki::operand_slice_kernel<8><<<gs, 256, 0, st>>>(src);
+    else
+      ozaki::operand_slice_kernel<7><<<gs, 256, 0, st>>>(src);
     ozaki::UpdateArgs p{};
     if (!ozaki::make_operand_map(&p.tm_a, pa, kp, mp, slices, ozaki::BM) ||
         !ozaki::make_operand_map(&p.tm_b, pb, kp, np, slices, ozaki::BN))
