@@ -307,7 +307,7 @@ __global__ void scatter_cols_kernel(const double *__restrict__ T, int64_t M, int
 // n x n matrices (the lower factor, as cuSOLVER's lower-fill potrf leaves it;
 // the strict upper triangle is never written).
 constexpr int kCholNb = 128;
-constexpr int kCholStride = kCholNb + 1;  // odd: a column of s read by a warp is free of bank conflicts
+constexpr int kCholStride = kCholNb + 4;
 
 // P_f (m x nbj, column-major, ld m) <- the block column A_f[j0:, j0:j0+nbj],
 // or of I - A_f with one_minus (the factorised matrix is then I - A_f, whose
@@ -327,214 +327,265 @@ __global__ void chol_copy_panel_kernel(const double *__restrict__ A, int64_t n, 
 }
 
 // One CTA (512 threads) per matrix: the updated diagonal block (the top nbj
-// rows of P_f, padded to 128 with the identity) is factorised and inverted in
-// shared memory, blocked by 32-column sub-blocks so that the sequential part,
-// one pivot after another, stays inside one warp:
-//  * warp 0 factorises the 32 x 32 diagonal sub-block in registers (lane r
-//    holds row r; each pivot's column is broadcast by shuffles, the chain per
-//    column is one rsqrt and one FMA) and forms its inverse X_kk by forward
-//    substitution column by column (lane c holds column c);
-//  * all warps then form the rows below it, L_ik = A_ik X_kk^T, and apply the
-//    rank-32 update of the trailing lower triangle in 4 x 4 register tiles;
-//  * after the last sub-block the off-diagonal blocks of X = L^-1 follow by
-//    block rows, X_ik = -X_ii sum_{k <= j < i} L_ij X_jk.
+// rows of P_f, padded to whole sub-blocks with the identity) is factorised and
+// inverted in shared memory, by 32-column sub-blocks k:
+//  A. warp 0 factorises the 32 x 32 diagonal sub-block in registers (lane r
+//     holds row r) as U D^-1 U^T without square roots, so that the chain from
+//     pivot to pivot is one reciprocal, two shuffles and two FP64 operations;
+//     the rows' entries below a pivot are read back from shared memory as
+//     broadcasts; L_kk = U D^-1/2. Warp 1 follows it eight pivots behind
+//     with the inverse X_kk (lane c holds column c). Meanwhile the other warps
+//     of its schedulers finish the previous step: the rank-32 update of the
+//     columns past this sub-block, T_ki = sum_{i <= j < k} L_kj X_ji for
+//     every i < k, and the stores of what is final (in step 0, the loads of
+//     the later columns);
+//  B. L_ik = A_ik X_kk^T for the rows below, X_ki = -X_kk T_ki beside it;
+//  C. the update of the next sub-block's 32 columns.
+// B, C and the work beside A run as FP64 tensor-core products (m8n8k4) of 8-row
+// strips, one strip a warp.
 // The lower factor goes into A_f's diagonal block (lower triangle and
-// diagonal only), X into Linv_f (column-major, ld kCholNb, zeros above the
-// diagonal). The diagonal is sqrt(pivot), the scaling of the column below it
-// rsqrt(pivot) (within an ulp of LAPACK's 1 / sqrt). A pivot that is not
+// diagonal only), X = L^-1 into Linv_f (column-major, ld kCholNb, zeros above
+// the diagonal). The diagonal is sqrt(pivot), the scaling of the column below
+// it rsqrt(pivot) (within an ulp of LAPACK's 1 / sqrt). A pivot that is not
 // positive records info_f = its global column + 1 (the first one only), as
 // potrf does; the factor of that matrix is then not meaningful.
-// Shared memory: s (128 x kCholStride: L in the strict lower triangle, the
+// What bounds it: latency, 128 dependent pivots of about 230 cycles each.
+// Measured (B200, 20 matrices, time of the launch): 128 columns 36.9 us, 64
+// columns 18.4 us, 13 columns 11.0 us; 90, 84 and 80 us with the square root
+// on the pivots' chain, 4 x 4 register tiles for the block products (34 000
+// of 170 000 cycles in X alone) and every block padded to 128.
+// Shared memory: s (128 x kCholStride: L in the lower triangle, the
 // off-diagonal blocks of X transposed in the upper one, X[r][c] at s[c][r]),
-// the diagonal of L and of X, the four X_kk dense (kCholXStride rows), and
-// the current panel transposed (pt, reused for the block products of the
-// inverse).
+// the diagonals of L and of X, the four X_kk dense, the sub-block's U by
+// columns, and T. All strides are 4 modulo 16, which keeps a fragment load's
+// half warp (four rows, four k) in sixteen different 8-byte banks whichever
+// index runs along memory.
 constexpr int kCholSub = 32;
-constexpr int kCholXStride = kCholSub + 1;
-constexpr int kCholPtStride = kCholNb + 2;  // even: the 4 x 4 tiles read pairs
-constexpr int kCholSmemDoubles = kCholNb * kCholStride + 2 * kCholNb +
+constexpr int kCholXStride = kCholSub + 4;
+constexpr int kCholSmemDoubles = kCholNb * kCholStride + 3 * kCholNb +
                                  (kCholNb / kCholSub) * kCholSub * kCholXStride +
-                                 kCholSub * kCholPtStride;
+                                 kCholSub * kCholXStride + 3 * kCholSub * kCholXStride;
+
+// acc (8 x 32, four 8 x 8 blocks) += A B^T over 4 ksteps K columns: A(r, k) at
+// a[r ar + k ak], B(c, k) at b[c br + k bk]; blocks from nblk on are left out
+__device__ __forceinline__ void strip_product(double (&acc)[4][2], const double *a, int ar, int ak,
+                                              const double *b, int br, int bk, int ksteps,
+                                              int nblk, int lane) {
+  const double *pa = a + (lane >> 2) * ar + (lane & 3) * ak;
+  const double *pb = b + (lane >> 2) * br + (lane & 3) * bk;
+#pragma unroll 2
+  for (int q = 0; q < ksteps; ++q) {
+    const double x = pa[4 * q * ak];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j < nblk) {
+        const double y = pb[8 * j * br + 4 * q * bk];
+        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+            : "+d"(acc[j][0]), "+d"(acc[j][1])
+            : "d"(x), "d"(y));
+      }
+  }
+}
 
 __global__ void __launch_bounds__(512) chol_diag_block_kernel(
     const double *__restrict__ P, int64_t m, int nbj, double *A, int64_t n, int64_t j0,
     double *__restrict__ Linv, int *info) {
   extern __shared__ __align__(16) double sm[];
-  constexpr int ST = kCholStride, XS = kCholXStride, PT = kCholPtStride, NB = kCholNb;
+  constexpr int ST = kCholStride, XS = kCholXStride, NB = kCholNb, SB = kCholSub;
   double *s = sm;
   double *diag = s + NB * ST;                 // L_cc
   double *xdiag = diag + NB;                  // X_cc = rsqrt(pivot)
-  double *xd = xdiag + NB;                    // X_kk dense, [k][r][c]
-  double *pt = xd + (NB / kCholSub) * kCholSub * XS;  // panel transposed, [m][i]
-  double *tb = pt;                            // the inverse's block products, [k][r][c]
+  double *pinv = xdiag + NB;                  // 1 / pivot
+  double *xd = pinv + NB;                     // X_kk dense, [k][r][c]
+  double *ut = xd + (NB / SB) * SB * XS;      // U of the sub-block by columns, [c][r]
+  double *tb = ut + SB * XS;                  // T_ki, [i][r][c]
+  __shared__ double rsx[SB];
   __shared__ int bad;
   const int f = blockIdx.x, tid = threadIdx.x;
-  const int warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
+  const int warp = tid >> 5, lane = tid & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int nsub = (nbj + SB - 1) / SB, nr = nsub * SB;
   const double *p = P + static_cast<int64_t>(f) * m * nbj;
   double *a = A + static_cast<int64_t>(f) * n * n;
   if (tid == 0) bad = -1;
-  // the tile padded with the identity, zeros above the diagonal; eight
-  // independent loads in flight per thread before any store
-  for (int i0 = tid; i0 < NB * NB; i0 += 8 * blockDim.x) {
-    double v[8];
+  // columns [c0, c1) of the tile padded with the identity, zeros above the
+  // diagonal, by `count` threads (this one the id-th); eight independent loads
+  // in flight per thread before any store
+  auto load_columns = [&](int c0, int c1, int id, int count) {
+    for (int i0 = c0 * NB + id; i0 < c1 * NB; i0 += 8 * count) {
+      double v[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int i = i0 + u * blockDim.x;
-      const int c = i / NB, r = i % NB;
-      v[u] = 0.0;
-      if (i < NB * NB && r >= c)
-        v[u] = (r < nbj && c < nbj) ? p[static_cast<int64_t>(c) * m + r] : (r == c ? 1.0 : 0.0);
-    }
+      for (int u = 0; u < 8; ++u) {
+        const int i = i0 + u * count;
+        const int c = i / NB, r = i % NB;
+        v[u] = 0.0;
+        if (c < c1 && r >= c)
+          v[u] = (r < nbj && c < nbj) ? p[static_cast<int64_t>(c) * m + r] : (r == c ? 1.0 : 0.0);
+      }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int i = i0 + u * blockDim.x;
-      if (i < NB * NB) s[(i % NB) * ST + i / NB] = v[u];
+      for (int u = 0; u < 8; ++u) {
+        const int i = i0 + u * count;
+        if (i < c1 * NB) s[(i % NB) * ST + i / NB] = v[u];
+      }
     }
-  }
+  };
+  // L's column block k and X's row block k, by `count` warps (this one the
+  // id-th)
+  double *ld = Linv + static_cast<int64_t>(f) * NB * NB;
+  auto store_block = [&](int k, int id, int count) {
+    for (int c = k * SB + id; c < min(nbj, (k + 1) * SB); c += count)
+      for (int r = k * SB + lane; r < nbj; r += 32)
+        if (r >= c) a[(j0 + c) * n + j0 + r] = r == c ? diag[c] : s[r * ST + c];
+    const int r = k * SB + lane;
+    if (r < nbj)
+      for (int c = id; c < nbj; c += count) {
+        double x = 0.0;
+        if (r == c)
+          x = xdiag[c];
+        else if (r > c)
+          x = c / SB == k ? xd[(k * SB + lane) * XS + c % SB] : s[c * ST + r];
+        ld[c * NB + r] = x;
+      }
+  };
+  load_columns(0, SB, tid, 512);
   __syncthreads();
-  for (int k = 0; k < NB / kCholSub; ++k) {
-    const int b = k * kCholSub;
-    double *xk = xd + k * kCholSub * XS;
-    if (warp == 0) {
-      double *row = s + (b + lane) * ST + b;
-      double v[kCholSub];
+  // rows [r0, r0 + 8) of the trailing triangle, 32 columns from c0, minus the
+  // panel in columns [b, b + 32)
+  auto update = [&](int r0, int c0, int b) {
+    const int nblk = min(4, (r0 - c0) / 8 + 1);  // blocks on and below the diagonal
+    double acc[4][2] = {};
+    strip_product(acc, s + r0 * ST + b, ST, 1, s + c0 * ST + b, ST, 1, SB / 4, nblk, lane);
 #pragma unroll
-      for (int j = 0; j < kCholSub; ++j) v[j] = row[j];
+    for (int j = 0; j < 4; ++j)
+      if (j < nblk) {
+        double *at = s + (r0 + g) * ST + c0 + 8 * j + 2 * t;
+        at[0] -= acc[j][0];
+        at[1] -= acc[j][1];
+      }
+  };
+  // rows [8 q, 8 q + 8) of T_ki (k the current sub-block)
+  auto t_strip = [&](int k, int i, int q) {
+    double acc[4][2] = {};
+    for (int j = i; j < k; ++j) {
+      const double *l = s + (k * SB + 8 * q) * ST + j * SB;
+      if (j == i)
+        strip_product(acc, l, ST, 1, xd + i * SB * XS, 1, XS, SB / 4, 4, lane);
+      else
+        strip_product(acc, l, ST, 1, s + i * SB * ST + j * SB, ST, 1, SB / 4, 4, lane);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      double *at = tb + (i * SB + 8 * q + g) * XS + 8 * j + 2 * t;
+      at[0] = acc[j][0];
+      at[1] = acc[j][1];
+    }
+  };
+  for (int k = 0; k < nsub; ++k) {
+    const int b = k * SB;
+    double *xk = xd + k * SB * XS;
+    if (warp == 0) {
+      double v[SB];
+#pragma unroll
+      for (int j = 0; j < SB; ++j) v[j] = s[(b + lane) * ST + b + j];
       // right-looking in registers: entries of a lane above the diagonal
       // are never read by another lane
+      double piv = 0.0;
 #pragma unroll
-      for (int c = 0; c < kCholSub; ++c) {
-        const double d = __shfl_sync(0xffffffffu, v[c], c);
-        const double rs = rsqrt(d);
-        if (lane == 0) {
-          xdiag[b + c] = rs;
-          diag[b + c] = sqrt(d);
-          if (!(d > 0.0) && bad < 0 && b + c < nbj) bad = b + c;
+      for (int c = 0; c < SB; ++c) {
+        const double u = v[c];
+        ut[c * XS + lane] = u;
+        const double d = __shfl_sync(0xffffffffu, u, c);
+        const double nxt = c + 1 < SB ? __shfl_sync(0xffffffffu, u, c + 1 < SB ? c + 1 : c) : 0.0;
+        const double inv = 1.0 / d;
+        if (lane == c) {
+          piv = d;
+          diag[b + c] = d;
+          pinv[b + c] = inv;
         }
-        v[c] *= rs;
+        const double w = -u * inv;
+        if (c + 1 < SB) v[c + 1 < SB ? c + 1 : c] = fma(w, nxt, v[c + 1 < SB ? c + 1 : c]);
+        __syncwarp();
 #pragma unroll
-        for (int j = c + 1; j < kCholSub; ++j)
-          v[j] = fma(-v[c], __shfl_sync(0xffffffffu, v[c], j), v[j]);
+        for (int j = c + 2; j < SB; ++j) v[j] = fma(w, ut[c * XS + j], v[j]);
+        // eight more columns for warp 1 (a barrier of these two warps)
+        if (c % 8 == 7) asm volatile("bar.arrive %0, 64;" ::"r"(1 + c / 8) : "memory");
       }
-#pragma unroll
-      for (int j = 0; j < kCholSub; ++j)
-        if (j < lane) row[j] = v[j];
+      const double rs = rsqrt(piv);
+      xdiag[b + lane] = rs;
+      const unsigned wrong = __ballot_sync(0xffffffffu, !(piv > 0.0) && b + lane < nbj);
+      if (lane == 0 && wrong && bad < 0) bad = b + __ffs(wrong) - 1;
       __syncwarp();
-      // X_kk column `lane`: x_i = (e_lane - sum_{j < i} L_ij x_j) / L_ii,
-      // the sums carried forward so that the chain per row is one FMA
-      double x[kCholSub];
 #pragma unroll
-      for (int r = 0; r < kCholSub; ++r) x[r] = r == lane ? 1.0 : 0.0;
+      for (int c = 0; c < SB; ++c)
+        if (c < lane) s[(b + lane) * ST + b + c] = ut[c * XS + lane] * xdiag[b + c];
+    } else if (warp == 1) {
+      // X_kk column `lane` by forward substitution on U, the sums carried
+      // forward: t_i = e_i - sum_{j < i} U_ij t_j / d_j, x_i = t_i rsqrt(d_i)
+      double x[SB];
 #pragma unroll
-      for (int i = 0; i < kCholSub; ++i) {
-        x[i] *= xdiag[b + i];
+      for (int r = 0; r < SB; ++r) x[r] = r == lane ? 1.0 : 0.0;
 #pragma unroll
-        for (int r = i + 1; r < kCholSub; ++r) x[r] = fma(-s[(b + r) * ST + b + i], x[i], x[r]);
+      for (int i = 0; i < SB; ++i) {
+        if (i % 8 == 0) asm volatile("bar.sync %0, 64;" ::"r"(1 + i / 8) : "memory");
+        const double y = -x[i] * pinv[b + i];
+#pragma unroll
+        for (int r = i + 1; r < SB; ++r) x[r] = fma(ut[i * XS + r], y, x[r]);
       }
-#pragma unroll
-      for (int r = 0; r < kCholSub; ++r) xk[r * XS + lane] = x[r];
-    }
-    __syncthreads();
-    if (b + kCholSub >= NB) break;
-    // the rows below: L[i][b + j] = sum_q A[i][b + q] X_kk[j][q], two rows per warp pass
-    for (int i0 = b + kCholSub + 2 * warp; i0 < NB; i0 += 2 * nwarps) {
-      double *r0 = s + i0 * ST + b, *r1 = r0 + ST;
-      double acc0 = 0.0, acc1 = 0.0;
-#pragma unroll 8
-      for (int q = 0; q < kCholSub; ++q) {
-        const double x = xk[lane * XS + q];
-        acc0 = fma(r0[q], x, acc0);
-        acc1 = fma(r1[q], x, acc1);
-      }
+      rsx[lane] = rsqrt(diag[b + lane]);
       __syncwarp();
-      r0[lane] = acc0;
-      r1[lane] = acc1;
-      pt[lane * PT + i0] = acc0;
-      pt[lane * PT + i0 + 1] = acc1;
+      diag[b + lane] = sqrt(diag[b + lane]);
+#pragma unroll
+      for (int r = 0; r < SB; ++r) xk[r * XS + lane] = x[r] * rsx[r];
+    } else if (warp % 4 != 0) {
+      // the other warps of schedulers 1 to 3: the rest of the previous step's
+      // update (columns past this sub-block), T, and what is final
+      const int w = warp - 2 - warp / 4;  // 0 ... 10
+      if (k == 0) {
+        load_columns(SB, nr, w * 32 + lane, 11 * 32);
+      } else {
+        int item = w;
+        for (int c0 = b + SB; c0 < nr; c0 += SB) {
+          const int strips = (nr - c0) / 8;
+          for (; item < strips; item += 11) update(c0 + 8 * item, c0, b - SB);
+          item -= strips;
+        }
+        for (; item < 4 * k; item += 11) t_strip(k, item / 4, item % 4);
+        store_block(k - 1, w, 11);
+      }
     }
     __syncthreads();
-    // the trailing lower triangle -= panel panel^T, 4 x 4 tiles
-    const int base = b + kCholSub, nt = (NB - base) / 4;
-    for (int t = tid; t < nt * nt; t += blockDim.x) {
-      const int ti = t / nt, tj = t % nt;
-      if (ti < tj) continue;
-      const int i0 = base + 4 * ti, c0 = base + 4 * tj;
-      double acc[4][4] = {};
-#pragma unroll 4
-      for (int q = 0; q < kCholSub; ++q) {
-        const double2 a01 = *reinterpret_cast<const double2 *>(pt + q * PT + i0);
-        const double2 a23 = *reinterpret_cast<const double2 *>(pt + q * PT + i0 + 2);
-        const double2 b01 = *reinterpret_cast<const double2 *>(pt + q * PT + c0);
-        const double2 b23 = *reinterpret_cast<const double2 *>(pt + q * PT + c0 + 2);
-        const double av[4] = {a01.x, a01.y, a23.x, a23.y};
-        const double bv[4] = {b01.x, b01.y, b23.x, b23.y};
+    // B: panel strips below, then X strips of this block row
+    const int below = (nr - b - SB) / 8;
+    for (int item = warp; item < below + 4 * k; item += 16) {
+      double acc[4][2] = {};
+      if (item < below) {
+        const int r0 = b + SB + 8 * item;
+        strip_product(acc, s + r0 * ST + b, ST, 1, xk, XS, 1, SB / 4, 4, lane);
+        __syncwarp();  // the strip is read before it is overwritten
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int j = 0; j < 4; ++j) {
+          double *at = s + (r0 + g) * ST + b + 8 * j + 2 * t;
+          at[0] = acc[j][0];
+          at[1] = acc[j][1];
+        }
+      } else {
+        const int i = (item - below) / 4, q = (item - below) % 4;
+        strip_product(acc, xk + 8 * q * XS, XS, 1, tb + i * SB * XS, 1, XS, 2 * (q + 1), 4, lane);
 #pragma unroll
-          for (int w = 0; w < 4; ++w) acc[u][w] = fma(av[u], bv[w], acc[u][w]);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int w = 0; w < 4; ++w) s[(i0 + u) * ST + c0 + w] -= acc[u][w];
-    }
-    __syncthreads();
-  }
-  // X by block rows: T_ik = sum_{k <= j < i} L_ij X_jk, then X_ik = -X_ii T_ik;
-  // each of the 16 warps two rows (warp, warp + 16) of every block, the lanes
-  // on columns
-  for (int i = 1; i < NB / kCholSub; ++i) {
-    const double *l0 = s + (i * kCholSub + warp) * ST;
-    const double *l1 = l0 + 16 * ST;
-    for (int k = 0; k < i; ++k) {
-      double t0 = 0.0, t1 = 0.0;
-      const double *xkk = xd + k * kCholSub * XS;
-#pragma unroll 8
-      for (int q = 0; q < kCholSub; ++q) {
-        const double x = xkk[q * XS + lane];
-        t0 = fma(l0[k * kCholSub + q], x, t0);
-        t1 = fma(l1[k * kCholSub + q], x, t1);
-      }
-      for (int j = k + 1; j < i; ++j) {
-        const double *xc = s + (k * kCholSub + lane) * ST + j * kCholSub;  // X[j*32 + q][k*32 + lane]
-#pragma unroll 8
-        for (int q = 0; q < kCholSub; ++q) {
-          const double x = xc[q];
-          t0 = fma(l0[j * kCholSub + q], x, t0);
-          t1 = fma(l1[j * kCholSub + q], x, t1);
+        for (int j = 0; j < 4; ++j) {
+          double *at = s + (i * SB + 8 * j + 2 * t) * ST + b + 8 * q + g;
+          at[0] = -acc[j][0];
+          at[ST] = -acc[j][1];
         }
       }
-      tb[(k * kCholSub + warp) * XS + lane] = t0;
-      tb[(k * kCholSub + warp + 16) * XS + lane] = t1;
     }
     __syncthreads();
-    const double *xii = xd + i * kCholSub * XS;
-    for (int k = 0; k < i; ++k) {
-      double v0 = 0.0, v1 = 0.0;
-#pragma unroll 8
-      for (int q = 0; q < kCholSub; ++q) {
-        const double tq = tb[(k * kCholSub + q) * XS + lane];
-        v0 = fma(xii[warp * XS + q], tq, v0);
-        v1 = fma(xii[(warp + 16) * XS + q], tq, v1);
-      }
-      s[(k * kCholSub + lane) * ST + i * kCholSub + warp] = -v0;
-      s[(k * kCholSub + lane) * ST + i * kCholSub + warp + 16] = -v1;
-    }
+    if (k + 1 == nsub) break;
+    // C: the next sub-block's columns
+    for (int item = warp; item < below; item += 16) update(b + SB + 8 * item, b + SB, b);
     __syncthreads();
   }
-  double *ld = Linv + static_cast<int64_t>(f) * NB * NB;
-  for (int i = tid; i < nbj * nbj; i += blockDim.x) {
-    const int c = i / nbj, r = i % nbj;
-    if (r >= c) a[(j0 + c) * n + j0 + r] = r == c ? diag[c] : s[r * ST + c];
-    double x = 0.0;
-    if (r == c)
-      x = xdiag[c];
-    else if (r > c)
-      x = (r / kCholSub == c / kCholSub)
-              ? xd[(r / kCholSub) * kCholSub * XS + (r % kCholSub) * XS + c % kCholSub]
-              : s[c * ST + r];
-    ld[c * NB + r] = x;
-  }
+  store_block(nsub - 1, warp, 16);
   if (tid == 0 && bad >= 0 && info[f] == 0) info[f] = static_cast<int>(j0) + bad + 1;
 }
 
