@@ -129,28 +129,6 @@ __global__ void diag_kernel(double *a, int64_t n, double *diag, bool save) {
   }
 }
 
-// T (ib x ib, column-major) = the lower triangle of the column-major block at
-// A (leading dimension lda), zeros above the diagonal
-__global__ void lower_copy_kernel(const double *A, int64_t lda, double *T, int ib) {
-  const int64_t total = static_cast<int64_t>(ib) * ib;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t c = i / ib, r = i % ib;
-    T[i] = r >= c ? A[c * lda + r] : 0.0;
-  }
-}
-
-// zero the strict upper triangle of a column-major n x n matrix (the
-// row-major strict lower triangle of the buffer)
-__global__ void zero_strict_upper_cm_kernel(double *a, int64_t n) {
-  const int64_t total = n * n;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t c = i / n, r = i % n;  // column-major (r, c) at c * n + r
-    if (r < c) a[i] = 0.0;
-  }
-}
-
 // Inverts the nb x nb diagonal blocks of a column-major lower-triangular
 // matrix in place, one CTA per block: the block is staged row-major in shared
 // memory and inverted row by row (forward substitution against the rows
@@ -673,6 +651,25 @@ __global__ void row_dot_into_col_kernel(const double *__restrict__ G,
   if (lane == 0) out[r * ldo + p] += s;
 }
 
+// The inverted diagonal blocks of nmat factors (block j of matrix f at
+// src + f sf + j sj, element (r, c) of L^-1 at c ld + r) into the diagonal
+// blocks of the row-major V = L^-T (n x ldv each), zeros below the diagonal
+__global__ void inverse_blocks_kernel(const double *__restrict__ src, int64_t sf, int64_t sj,
+                                      int64_t ld, int64_t n, double *__restrict__ V,
+                                      int64_t ldv) {
+  const int64_t off = static_cast<int64_t>(blockIdx.x) * kCholNb;
+  const int m = static_cast<int>(min(static_cast<int64_t>(kCholNb), n - off));
+  const double *x = src + blockIdx.y * sf + blockIdx.x * sj;
+  double *v = V + blockIdx.y * n * ldv + off * ldv + off;
+  const int lane = threadIdx.x & 31;
+  for (int c = threadIdx.x >> 5; c < m; c += blockDim.x >> 5)
+#pragma unroll
+    for (int q = 0; q < kCholNb / 32; ++q) {
+      const int r = lane + 32 * q;
+      if (r < m) v[c * ldv + r] = r >= c ? x[c * ld + r] : 0.0;
+    }
+}
+
 // The batched Cholesky's inverted diagonal blocks of one matrix (block j at
 // Linv + j * step_stride, column-major, ld kCholNb) as TF32 pairs in the two
 // layouts of the triangular-inverse recursion: rows of L^-1 (r_*) and columns
@@ -731,14 +728,11 @@ void launch_diag(double *a, int64_t n, int nmat, double *diag, bool save, cudaSt
   count_launch(); diag_kernel<<<grid, 256, 0, st>>>(a, n, diag, save);
 }
 
-void launch_lower_copy(const double *A, int64_t lda, double *T, int ib, cudaStream_t st) {
+void launch_inverse_blocks(const double *src, int64_t sf, int64_t sj, int64_t ld, int64_t n,
+                           int nmat, double *V, int64_t ldv, cudaStream_t st) {
   count_launch();
-  lower_copy_kernel<<<blocks(static_cast<int64_t>(ib) * ib), 256, 0, st>>>(A, lda, T, ib);
-}
-
-void launch_zero_strict_upper_cm(double *a, int64_t n, cudaStream_t st) {
-  count_launch();
-  zero_strict_upper_cm_kernel<<<blocks(n * n), 256, 0, st>>>(a, n);
+  inverse_blocks_kernel<<<dim3(static_cast<unsigned>((n + kCholNb - 1) / kCholNb), nmat), 256, 0,
+                          st>>>(src, sf, sj, ld, n, V, ldv);
 }
 
 int launch_trtri_diag_blocks(double *A, int64_t n, int64_t lda, int nb, cudaStream_t st,

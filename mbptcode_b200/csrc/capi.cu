@@ -37,8 +37,8 @@ void launch_lu_logdet(const double *LU, const int *piv, int64_t n, double *logde
 void launch_identity(double *a, int64_t n, cudaStream_t st);
 void launch_minus_identity(double *a, int64_t n, cudaStream_t st);
 void launch_diag(double *a, int64_t n, int nmat, double *diag, bool save, cudaStream_t st);
-void launch_lower_copy(const double *A, int64_t lda, double *T, int ib, cudaStream_t st);
-void launch_zero_strict_upper_cm(double *a, int64_t n, cudaStream_t st);
+void launch_inverse_blocks(const double *src, int64_t sf, int64_t sj, int64_t ld, int64_t n,
+                           int nmat, double *V, int64_t ldv, cudaStream_t st);
 int launch_trtri_diag_blocks(double *A, int64_t n, int64_t lda, int nb, cudaStream_t st,
                              float *c_hi = nullptr, float *c_lo = nullptr, float *r_hi = nullptr,
                              float *r_lo = nullptr, int64_t ldp = 0);
@@ -386,9 +386,6 @@ int chi0_run(const double *X, const Dims &d, const double *eps, double mu, const
 }
 
 // --------------------------------------------------------------------- Dyson
-// Block size of the LAUUM below; its DGEMM/DSYRK updates carry the flops.
-constexpr int64_t kLauumBlock = 512;
-
 // Diagonal blocks of the triangular inverse, inverted all at once in shared
 // memory (one CTA per block); the recursion above them turns the rest into
 // dense products.
@@ -406,34 +403,10 @@ struct PairScratch {
   int64_t np = 0;
 };
 
-// In place: the lower-triangular column-major block at A (n x n, leading
-// dimension lda, zeros above its diagonal, its kTrtriLeaf diagonal blocks
-// already inverted) becomes its inverse, by
-// [[L11, 0], [L21, L22]]^-1 = [[L11^-1, 0], [-L22^-1 L21 L11^-1, L22^-1]]
-// with both halves inverted first (n1 a multiple of kTrtriLeaf keeps the
-// leaves on the diagonal blocks). T holds (n - n1) x n1 doubles. FP64 DGEMMs.
-int trtri_rec(Handles &h, double *A, int64_t n, int64_t lda, double *T) {
-  if (n <= kTrtriLeaf) return MBPT_OK;
-  const int64_t n1 = round_up(n / 2, kTrtriLeaf), n2 = n - n1;
-  double *L11 = A, *L21 = A + n1, *L22 = A + n1 + n1 * lda;
-  int rc = trtri_rec(h, L11, n1, lda, T);
-  if (rc) return rc;
-  rc = trtri_rec(h, L22, n2, lda, T);
-  if (rc) return rc;
-  const double one = 1.0, zero = 0.0, minus = -1.0;
-  const int i1 = static_cast<int>(n1), i2 = static_cast<int>(n2), il = static_cast<int>(lda);
-  // T = L21 L11^-1, then L21 <- -L22^-1 T
-  if (cublasDgemm(h.blas, CUBLAS_OP_N, CUBLAS_OP_N, i2, i1, i1, &one, L21, il, L11, il, &zero,
-                  T, i2) != CUBLAS_STATUS_SUCCESS ||
-      cublasDgemm(h.blas, CUBLAS_OP_N, CUBLAS_OP_N, i2, i1, i2, &minus, L22, il, T, i2, &zero,
-                  L21, il) != CUBLAS_STATUS_SUCCESS)
-    return MBPT_ERR_CUDA;
-  return MBPT_OK;
-}
-
-// The same recursion on TF32 pairs over the whole n x n factor (diagonal
-// kTrtriLeaf blocks already in IC/IR, the factor's rows in LR), level by
-// level: the nodes of one depth are independent, so each depth is two grouped
+// The triangular inverse [[L11, 0], [L21, L22]]^-1 = [[L11^-1, 0],
+// [-L22^-1 L21 L11^-1, L22^-1]] on TF32 pairs over the whole n x n factor
+// (diagonal kTrtriLeaf blocks already in IC/IR, the factor's rows in LR, both
+// halves inverted first, split at multiples of kTrtriLeaf), level by level: the nodes of one depth are independent, so each depth is two grouped
 // launches, deepest first. Each node's products have epilogues that write
 // pairs straight into the layouts the next products read, so nothing is
 // converted between them. With the engine forming P = A_e B_e^T row by row of
@@ -498,110 +471,60 @@ struct TimingTag {
   ~TimingTag() { timing_tag(-1); }
 };
 
-// W - I from the Cholesky factor L of 1 - chi0 (column-major lower, in place;
-// the row-major upper triangle of the buffer). FP64 mode: the diagonal blocks
-// of L^-1 in shared memory, the recursion above on DGEMMs, then (L^-1)^T L^-1
-// by a blocked LAUUM on cuBLAS level 3 (LAPACK's blocking) into the same
-// triangle, which the caller mirrors and shifts by -I; this replaces potri,
-// whose LAUUM half runs far below DGEMM speed. Mixed mode (`pairs`): L^-1 as
-// TF32 pairs by the tensor-core recursion, then W = (L^-1)^T L^-1 on the
-// tensor cores over the tiles on and above the diagonal (rows of (L^-1)^T
-// vanish for k < row), W - I written whole (returns with *full = true).
-int spd_inverse_from_factor(Handles &h, double *L, int64_t n, double *T, double *Tr,
-                            const PairScratch *pairs, int *err, bool *full, cudaStream_t st,
-                            const double *diag_inv = nullptr, int64_t diag_inv_stride = 0) {
-  *full = false;
+// W - I from the Cholesky factor L of 1 - chi0 in mixed mode (column-major
+// lower, in place; the row-major upper triangle of the buffer): L^-1 as TF32
+// pairs by the tensor-core recursion, then W = (L^-1)^T L^-1 on the tensor
+// cores over the tiles on and above the diagonal (rows of (L^-1)^T vanish for
+// k < row), W - I written whole. diag_inv: the batched factorisation's inverted
+// 128 x 128 diagonal blocks (null: they are inverted here).
+int tf32_inverse_from_factor(double *L, int64_t n, const PairScratch &s, int *err,
+                             cudaStream_t st, const double *diag_inv = nullptr,
+                             int64_t diag_inv_stride = 0) {
   TimingTag tag(kTimingDyson);
-  if (pairs) {
-    const PairScratch &s = *pairs;
-    const int64_t np = s.np, kp = round_up(n, 32);
-    // rows of L (its upper triangle is never read)
-    launch_strided_to_tf32(L, n, n, 1, n, s.lr_hi, s.lr_lo, np, np, st);
-    int rc = MBPT_OK;
-    if (diag_inv)
-      // the batched factorisation kept its inverted 128 x 128 diagonal blocks
-      launch_linv_blocks_to_pairs(diag_inv, diag_inv_stride, n, s.ic_hi, s.ic_lo, s.ir_hi,
-                                  s.ir_lo, np, st);
-    else
-      rc = launch_trtri_diag_blocks(L, n, n, static_cast<int>(kTrtriLeaf), st, s.ic_hi,
-                                    s.ic_lo, s.ir_hi, s.ir_lo, np);
-    if (rc) return rc;
-    rc = trtri_pairs(s, n, err, st);
-    if (rc) return rc;
-    // W - I straight into the factor's buffer as FP64 (row-major W(j, i) is
-    // the column-major W(i, j) the caller expects; W is symmetric anyway),
-    // tiles above the diagonal mirrored by the epilogue
-    SplitMat Ae{s.ic_hi, s.ic_lo, np, kp, np, true};
-    umma::EpiArgs e;
-    e.outd = L;
-    e.ld_outd = n;
-    e.nd = static_cast<int>(n);
-    e.shift = 1.0;
-    e.alpha = 1.f;
-    rc = gemm_split(umma::EPI_F64_SYM, 1, &Ae, &Ae, np, np, e, err, st,
+  const int64_t np = s.np, kp = round_up(n, 32);
+  // rows of L (its upper triangle is never read)
+  launch_strided_to_tf32(L, n, n, 1, n, s.lr_hi, s.lr_lo, np, np, st);
+  int rc = MBPT_OK;
+  if (diag_inv)
+    launch_linv_blocks_to_pairs(diag_inv, diag_inv_stride, n, s.ic_hi, s.ic_lo, s.ir_hi, s.ir_lo,
+                                np, st);
+  else
+    rc = launch_trtri_diag_blocks(L, n, n, static_cast<int>(kTrtriLeaf), st, s.ic_hi, s.ic_lo,
+                                  s.ir_hi, s.ir_lo, np);
+  if (rc) return rc;
+  rc = trtri_pairs(s, n, err, st);
+  if (rc) return rc;
+  // W - I straight into the factor's buffer as FP64 (row-major W(j, i) is
+  // the column-major W(i, j) the caller expects; W is symmetric anyway),
+  // tiles above the diagonal mirrored by the epilogue
+  SplitMat Ae{s.ic_hi, s.ic_lo, np, kp, np, true};
+  umma::EpiArgs e;
+  e.outd = L;
+  e.ld_outd = n;
+  e.nd = static_cast<int>(n);
+  e.shift = 1.0;
+  e.alpha = 1.f;
+  return gemm_split(umma::EPI_F64_SYM, 1, &Ae, &Ae, np, np, e, err, st,
                     umma::BAND_K_FROM_M | umma::BAND_K_FROM_N | umma::BAND_UPPER);
-    if (rc) return rc;
-    *full = true;
-    return MBPT_OK;
-  }
-  // the dense products of the recursion need zeros above the diagonal
-  launch_zero_strict_upper_cm(L, n, st);
-  int rc = launch_trtri_diag_blocks(L, n, n, static_cast<int>(kTrtriLeaf), st);
-  if (rc) return rc;
-  rc = trtri_rec(h, L, n, n, Tr);
-  if (rc) return rc;
-  const double one = 1.0, zero = 0.0;
-  const int lda = static_cast<int>(n);
-  for (int64_t i = 0; i < n; i += kLauumBlock) {
-    const int ib = static_cast<int>(std::min(kLauumBlock, n - i));
-    const int ii = static_cast<int>(i);
-    double *Aii = L + i + i * n;
-    // A(i:i+ib, 0:i) = A(i:i+ib, i:i+ib)^T A(i:i+ib, 0:i)
-    if (ii > 0 &&
-        cublasDtrmm(h.blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T,
-                    CUBLAS_DIAG_NON_UNIT, ib, ii, &one, Aii, lda, L + i, lda, L + i, lda) !=
-            CUBLAS_STATUS_SUCCESS)
-      return MBPT_ERR_CUDA;
-    // A(i:i+ib, i:i+ib) = L11^T L11 from a copy with its strict upper part cleared
-    launch_lower_copy(Aii, n, T, ib, st);
-    if (cublasDsyrk(h.blas, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, ib, ib, &one, T, ib, &zero,
-                    Aii, lda) != CUBLAS_STATUS_SUCCESS)
-      return MBPT_ERR_CUDA;
-    if (i + ib < n) {
-      const int rest = static_cast<int>(n - i - ib);
-      double *Abelow = L + (i + ib) + i * n;  // A(i+ib:n, i:i+ib)
-      if (ii > 0 && cublasDgemm(h.blas, CUBLAS_OP_T, CUBLAS_OP_N, ib, ii, rest, &one, Abelow,
-                                lda, L + (i + ib), lda, &one, L + i, lda) !=
-                        CUBLAS_STATUS_SUCCESS)
-        return MBPT_ERR_CUDA;
-      if (cublasDsyrk(h.blas, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, ib, rest, &one, Abelow, lda,
-                      &one, Aii, lda) != CUBLAS_STATUS_SUCCESS)
-        return MBPT_ERR_CUDA;
-    }
-  }
-  return MBPT_OK;
 }
 
 constexpr int kCholNb = 128;     // block columns of the batched Cholesky
 constexpr int kBatchedCholMin = 4;  // frequencies from which the batch beats one potrf each
 
-// Left-looking blocked Cholesky of nmat column-major n x n SPD matrices at
-// once (A_f = L_f L_f^T, L_f in the lower triangle, the strict upper triangle
-// untouched, info_f as potrf reports it). Per 128-column step j0, for all
-// matrices in one launch each: the block column is copied to P, updated by
-// one strided-batched DGEMM P -= L[j0:, :j0] L[j0:j0+nb, :j0]^T (inner
-// dimension j0, so the FP64 GEMMs run long), its diagonal block factorised
-// and inverted in shared memory, and the panel below it formed by a second
-// batched DGEMM, L[j0+nb:, j0-block] = P_below L_jj^-T. Every launch carries
+// Left-looking blocked Cholesky of I - A_f for nmat column-major n x n
+// matrices at once (I - A_f = L_f L_f^T, L_f in the lower triangle; the strict
+// upper triangle keeps A_f; info_f as potrf reports it). Per 128-column step
+// j0, for all matrices in one launch each: the block column P = (I - A)[j0:, j0:j0+nb]
+// - L[j0:, :j0] L[j0:j0+nb, :j0]^T, formed where A is first read (one FP64 tensor-core
+// kernel, or a copy and the int8 update), its diagonal block factorised and
+// inverted in shared memory, and the panel below it formed by a second
+// product, L[j0+nb:, j0-block] = P_below L_jj^-T. Every launch carries
 // the whole batch, so the latency-bound diagonal blocks cost one launch per
 // step for all frequencies. P: nmat * n * kCholNb doubles; Linv: nmat *
-// kCholNb^2 doubles per step, step j at Linv + j * linv_step_stride (0: every
-// step in the same place); info: nmat ints, zeroed by the caller.
-// one_minus: A holds chi0 and the factorised matrices are I - A_f, formed
-// where each block column is first read (A's strict upper triangle keeps
-// chi0, its diagonal and lower triangle become the factor).
+// kCholNb^2 doubles per step, step j at Linv + j * linv_step_stride; info: nmat
+// ints, zeroed by the caller.
 // The Ozaki-scheme update's buffers for one batch (null planes: the updates
-// run as cuBLAS DGEMMs): the int8 digit planes, 2^e_r per row, exact row norms.
+// run in FP64): the int8 digit planes, 2^e_r per row, exact row norms.
 struct OzakiChol {
   int8_t *planes = nullptr;
   double *scale = nullptr;
@@ -611,44 +534,35 @@ struct OzakiChol {
 };
 
 int chol_batched(double *A, int64_t n, int nmat, int *info, double *P, double *Linv,
-                 cublasHandle_t h, cudaStream_t st, int64_t linv_step_stride = 0,
-                 const OzakiChol *oz = nullptr, bool one_minus = false) {
-  const long long n2 = static_cast<long long>(n) * n;
-  const double one = 1.0, minus = -1.0, zero = 0.0;
+                 cudaStream_t st, int64_t linv_step_stride, const OzakiChol *oz) {
   const bool ozaki = oz && oz->planes;
   if (ozaki) {
-    int rc = ozaki_chol_scales(A, n, nmat, oz->scale, oz->rowsq, one_minus, st);
+    int rc = ozaki_chol_scales(A, n, nmat, oz->scale, oz->rowsq, true, st);
     if (rc) return rc;
   }
   for (int64_t j0 = 0; j0 < n; j0 += kCholNb) {
     const int nbj = static_cast<int>(std::min<int64_t>(kCholNb, n - j0));
     const int64_t m = n - j0;
-    launch_chol_copy_panel(A, n, j0, m, nbj, nmat, one_minus, P, st);
     if (ozaki) {
+      launch_chol_copy_panel(A, n, j0, m, nbj, nmat, true, P, st);
       int rc = ozaki_chol_update(A, n, nmat, j0, nbj, P, oz->scale, oz->planes, oz->slices,
                                  oz->rowsq, oz->err, st);
       if (rc) return rc;
-    } else if (j0 > 0 &&
-               cublasDgemmStridedBatched(h, CUBLAS_OP_N, CUBLAS_OP_T, static_cast<int>(m), nbj,
-                                         static_cast<int>(j0), &minus, A + j0,
-                                         static_cast<int>(n), n2, A + j0, static_cast<int>(n),
-                                         n2, &one, P, static_cast<int>(m),
-                                         static_cast<long long>(m) * nbj,
-                                         nmat) != CUBLAS_STATUS_SUCCESS) {
-      return MBPT_ERR_CUDA;
+    } else {
+      int rc = dmma::chol_update(A, n, j0, nbj, P, nmat, st);
+      if (rc) return rc;
     }
     double *Lj = Linv + (j0 / kCholNb) * linv_step_stride;
     int rc = launch_chol_diag_block(P, m, nbj, A, n, j0, nmat, Lj, info, st);
     if (rc) return rc;
     const int64_t mb = m - nbj;
-    if (mb > 0 &&
-        cublasDgemmStridedBatched(h, CUBLAS_OP_N, CUBLAS_OP_T, static_cast<int>(mb), nbj, nbj,
-                                  &one, P + nbj, static_cast<int>(m),
-                                  static_cast<long long>(m) * nbj, Lj, kCholNb,
-                                  static_cast<long long>(kCholNb) * kCholNb, &zero,
-                                  A + j0 * n + j0 + nbj, static_cast<int>(n), n2,
-                                  nmat) != CUBLAS_STATUS_SUCCESS)
-      return MBPT_ERR_CUDA;
+    // row-major: U[j0:j0+nbj, j0+nbj:] = L_jj^-1 P[:, nbj:]
+    if (mb > 0) {
+      rc = dmma::gemm({Lj, kCholNb, static_cast<int64_t>(kCholNb) * kCholNb}, false,
+                      {P + nbj, m, m * nbj}, false, nbj, mb, nbj, 1.0, 0.0,
+                      A + j0 * n + j0 + nbj, n, n * n, nmat, false, st);
+      if (rc) return rc;
+    }
     // the block column is final: cut it into digit planes for the later steps
     if (ozaki && j0 + nbj < n) {
       int rc2 = ozaki_chol_slice(A, n, nmat, j0, nbj, oz->scale, oz->planes, oz->slices,
@@ -711,8 +625,10 @@ struct DysonBufs {
   double *work;
   double *work2;  // the second factor stream's cuSOLVER workspace
   double *rhs;   // n x n right-hand side of the LU inverse of a failed frequency
+  double *V = nullptr;  // FP64 modes: inv_batch factors' inverses (n x ldv each)
+  int64_t ldv = 0;
+  int inv_batch = 0;
   double *diag;  // nfreq x n diagonals of 1 - chi0, which the factorisation overwrites
-  double *T;     // diagonal-block scratch of the LAUUM
   PairScratch pairs[kMaxInverseStreams];  // mixed mode: one per inverse stream
   int npairs = 0;
   double *chol_P = nullptr, *chol_Linv = nullptr;  // batched Cholesky scratch
@@ -733,7 +649,8 @@ int dyson_lwork(int64_t n) {
   return l1 > l3 ? l1 : l3;
 }
 
-DysonBufs carve_dyson(Arena &ar, int64_t n, int nfreq, int mode = MBPT_MODE_FP64) {
+DysonBufs carve_dyson(Arena &ar, int64_t n, int nfreq, int mode = MBPT_MODE_FP64,
+                      bool want_w = true) {
   DysonBufs b{};
   b.lwork = dyson_lwork(n);
   b.info = ar.take<int>(nfreq + 1);
@@ -742,7 +659,11 @@ DysonBufs carve_dyson(Arena &ar, int64_t n, int nfreq, int mode = MBPT_MODE_FP64
   b.work2 = ar.take<double>(b.lwork > 0 ? b.lwork : 1);
   b.rhs = ar.take<double>(n * n);
   b.diag = ar.take<double>(n * static_cast<int64_t>(nfreq));
-  b.T = ar.take<double>(kLauumBlock * kLauumBlock);
+  if (fp64_mode(mode) && want_w) {
+    b.ldv = round_up(n, 2);  // even: 16-byte copies
+    b.inv_batch = batched_chol_enabled(nfreq) ? tau_batch(nfreq, n * b.ldv) : 1;
+    b.V = ar.take<double>(b.inv_batch * n * b.ldv);
+  }
   if (batched_chol_enabled(nfreq)) {
     b.chol_P = ar.take<double>(static_cast<int64_t>(nfreq) * n * kCholNb);
     // every step's inverted diagonal blocks are kept: the mixed inverse reads them
@@ -776,9 +697,6 @@ DysonBufs carve_dyson(Arena &ar, int64_t n, int nfreq, int mode = MBPT_MODE_FP64
 struct DysonPipe {
   cudaStream_t side = nullptr;
   cudaEvent_t join = nullptr;
-  // the inverses' own cuBLAS handle (bound to `side`): the caller's handle
-  // may still be running a later wave's factorisation on the caller's stream
-  cublasHandle_t blas_side = nullptr;
   // mixed mode's further inverse streams (index i + 1 of the inverse streams)
   std::vector<cudaStream_t> isides;
   std::vector<cudaEvent_t> ijoin;
@@ -787,14 +705,12 @@ struct DysonPipe {
   // panels between DGEMM-bound updates) share the GPU
   cudaStream_t fac2 = nullptr;
   cusolverDnHandle_t solver2 = nullptr;
-  cublasHandle_t blas2 = nullptr;  // the second half of a batched factorisation
   cudaEvent_t fork = nullptr, join2 = nullptr;
   int nfac = 1;
   // groups of the batched factorisation (MBPT_DYSON_CHOL_GROUPS, default 4):
   // group 0 on the caller's stream, group 1 on fac2, the rest on these
   int groups = 2;
   std::vector<cudaStream_t> xs;
-  std::vector<cublasHandle_t> xb;
   std::vector<cudaEvent_t> xj;
   std::vector<cudaEvent_t> ev;
   int *info = nullptr;  // pinned host, `cap` ints
@@ -813,9 +729,7 @@ DysonPipe *dyson_pipe(int nfreq) {
     pipes.emplace_back(dev, DysonPipe{});
     p = &pipes.back().second;
     p->ok = cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking) == cudaSuccess &&
-            cudaEventCreateWithFlags(&p->join, cudaEventDisableTiming) == cudaSuccess &&
-            cublasCreate(&p->blas_side) == CUBLAS_STATUS_SUCCESS &&
-            cublasSetStream(p->blas_side, p->side) == CUBLAS_STATUS_SUCCESS;
+            cudaEventCreateWithFlags(&p->join, cudaEventDisableTiming) == cudaSuccess;
     // MBPT_DYSON_FACTOR_STREAMS=1 keeps every factorisation on the caller's stream
     const char *env = std::getenv("MBPT_DYSON_FACTOR_STREAMS");
     p->nfac = (env && std::atoi(env) == 1) ? 1 : 2;
@@ -824,9 +738,7 @@ DysonPipe *dyson_pipe(int nfreq) {
               cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming) == cudaSuccess &&
               cudaEventCreateWithFlags(&p->join2, cudaEventDisableTiming) == cudaSuccess &&
               cusolverDnCreate(&p->solver2) == CUSOLVER_STATUS_SUCCESS &&
-              cusolverDnSetStream(p->solver2, p->fac2) == CUSOLVER_STATUS_SUCCESS &&
-              cublasCreate(&p->blas2) == CUBLAS_STATUS_SUCCESS &&
-              cublasSetStream(p->blas2, p->fac2) == CUBLAS_STATUS_SUCCESS;
+              cusolverDnSetStream(p->solver2, p->fac2) == CUSOLVER_STATUS_SUCCESS;
     for (int i = 1; p->ok && i < kMaxInverseStreams; ++i) {
       cudaStream_t s = nullptr;
       cudaEvent_t e = nullptr;
@@ -840,14 +752,10 @@ DysonPipe *dyson_pipe(int nfreq) {
     p->groups = p->nfac == 2 ? std::max(1, std::min(6, g)) : 1;
     for (int i = 2; p->ok && i < p->groups; ++i) {
       cudaStream_t xs = nullptr;
-      cublasHandle_t xb = nullptr;
       cudaEvent_t xj = nullptr;
       p->ok = cudaStreamCreateWithFlags(&xs, cudaStreamNonBlocking) == cudaSuccess &&
-              cudaEventCreateWithFlags(&xj, cudaEventDisableTiming) == cudaSuccess &&
-              cublasCreate(&xb) == CUBLAS_STATUS_SUCCESS &&
-              cublasSetStream(xb, xs) == CUBLAS_STATUS_SUCCESS;
+              cudaEventCreateWithFlags(&xj, cudaEventDisableTiming) == cudaSuccess;
       p->xs.push_back(xs);
-      p->xb.push_back(xb);
       p->xj.push_back(xj);
     }
   }
@@ -882,7 +790,7 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
               int *info_host, int *sign_host, Arena &ar, cudaStream_t st,
               int mode = MBPT_MODE_FP64, int *err = nullptr, int *info_dev_out = nullptr) {
   const bool deferred = info_dev_out != nullptr;
-  DysonBufs b = carve_dyson(ar, n, nfreq, mode);
+  DysonBufs b = carve_dyson(ar, n, nfreq, mode, want_w != 0);
   if (ar.overflow()) return MBPT_ERR_WORKSPACE;
   Handles &h = handles(st);
   DysonPipe *pp = dyson_pipe(nfreq);
@@ -920,7 +828,6 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
     // group's DGEMMs fill the GPU while another's diagonal blocks (one CTA
     // per matrix) are factorised
     auto stream_of = [&](int g) { return g == 0 ? st : (g == 1 ? pp->fac2 : pp->xs[g - 2]); };
-    auto blas_of = [&](int g) { return g == 0 ? h.blas : (g == 1 ? pp->blas2 : pp->xb[g - 2]); };
     auto join_of = [&](int g) { return g == 1 ? pp->join2 : pp->xj[g - 2]; };
     // waves (MBPT_DYSON_WAVES=2): the frequencies factorised in two halves one
     // after the other on the same streams, the tensor-core inverses of the
@@ -959,8 +866,7 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
         rc0 = chol_batched(chi0 + f0 * n * n, n, f1 - f0, b.info + f0,
                            b.chol_P + static_cast<int64_t>(f0) * n * kCholNb,
                            b.chol_Linv + static_cast<int64_t>(f0) * kCholNb * kCholNb,
-                           blas_of(g), gs, static_cast<int64_t>(nfreq) * kCholNb * kCholNb,
-                           &oz, true);
+                           gs, static_cast<int64_t>(nfreq) * kCholNb * kCholNb, &oz);
         if (rc0) break;
         // this group's log-determinants, info words and events on its own stream
         launch_logdet_diag(chi0 + f0 * n * n, n, f1 - f0, logdet + f0, gs);
@@ -976,6 +882,18 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
           cudaStreamWaitEvent(st, join_of(g), 0) != cudaSuccess)
         return MBPT_ERR_CUDA;
     if (rc0) return rc0;
+    // FP64 modes: the inverses of as many factors at a time as the scratch holds
+    // (where a factorisation failed nothing is written)
+    if (want_w && fp64_mode(mode))
+      for (int f0 = 0; f0 < nfreq; f0 += b.inv_batch) {
+        const int nb = std::min(b.inv_batch, nfreq - f0);
+        const int64_t blk = static_cast<int64_t>(kCholNb) * kCholNb;
+        launch_inverse_blocks(b.chol_Linv + f0 * blk, blk, nfreq * blk, kCholNb, n, nb, b.V,
+                              b.ldv, st);
+        const int rc1 =
+            dmma::spd_inverse(chi0 + f0 * n * n, n, b.V, b.ldv, b.info + f0, nb, st);
+        if (rc1) return rc1;
+      }
   }
   const int nfac = nfreq > 1 && !batched ? pp->nfac : 1;
   if (nfac == 2 && (cudaEventRecord(pp->fork, st) != cudaSuccess ||
@@ -1013,7 +931,8 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
     if (sign_host) sign_host[f] = 1;
     double *m = chi0 + f * n * n;
     if (inf == 0) {
-      if (want_w) {
+      // a batch's FP64 inverses are under way already
+      if (want_w && !(batched && fp64_mode(mode))) {
         const int si = f % nsides;
         cudaStream_t ss = side_of(si);
         side_used[si] = true;
@@ -1021,14 +940,18 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
           rc = MBPT_ERR_CUDA;
           break;
         }
-        Handles hs{pp->blas_side, h.solver};
-        bool full = false;
-        rc = spd_inverse_from_factor(
-            hs, m, n, b.T, b.rhs, mode == MBPT_MODE_MIXED ? &b.pairs[si] : nullptr, err, &full,
-            ss, batched ? b.chol_Linv + static_cast<int64_t>(f) * kCholNb * kCholNb : nullptr,
-            static_cast<int64_t>(nfreq) * kCholNb * kCholNb);
+        if (mode == MBPT_MODE_MIXED) {
+          rc = tf32_inverse_from_factor(
+              m, n, b.pairs[si], err, ss,
+              batched ? b.chol_Linv + static_cast<int64_t>(f) * kCholNb * kCholNb : nullptr,
+              static_cast<int64_t>(nfreq) * kCholNb * kCholNb);
+        } else {
+          rc = launch_trtri_diag_blocks(m, n, n, static_cast<int>(kTrtriLeaf), ss);
+          if (rc) break;
+          launch_inverse_blocks(m, 0, kTrtriLeaf * n + kTrtriLeaf, n, n, 1, b.V, b.ldv, ss);
+          rc = dmma::spd_inverse(m, n, b.V, b.ldv, nullptr, 1, ss);
+        }
         if (rc) break;
-        if (!full) launch_symmetrize_minus_identity(m, n, 1, ss);
       }
       continue;
     }
@@ -1594,7 +1517,7 @@ size_t mbpt_rpa_energy_workspace_bytes(int64_t M, int64_t norb, int64_t nocc, in
   ar.take<double>(34);                                         // weights
   Arena a2 = ar;
   carve_chi0(ar, d, ntau, nfreq, mode, true);
-  carve_dyson(a2, naux, nfreq);
+  carve_dyson(a2, naux, nfreq, MBPT_MODE_FP64, false);
   return (ar.used > a2.used ? ar.used : a2.used) + 4096;
 }
 

@@ -23,14 +23,28 @@
 // launch (cuBLAS 34.1, one point a launch); smaller warp tiles (32 x 16, more
 // warps) 32.8, two CTAs per SM with a deeper ring 32.1. The sweep with it
 // (n = 400, M = naux = 2400, 20 points): chi0 36.9 -> 27.2 ms, Sigma of 400
-// states 45.0 -> 32.0 ms; E_c at M = 888, naux = 141: 1.51 -> 0.76 ms.
+// states 45.0 -> 31.8 ms; E_c at M = 888, naux = 141: 1.51 -> 0.72 ms.
+//
+// The Dyson step's FP64 products run on the same kernel, all frequencies (and
+// all halvings of one depth of the triangular inverse) in one launch: the
+// Cholesky's block-column updates and panels, V = U^-1 by halves and W = V V^T
+// over the K columns where V is not zero. One frequency at a time the library
+// took 1200 launches of small products at naux = 1500, 20 frequencies: 16.1
+// ms, now 4.0.
 #include <algorithm>
+#include <vector>
 
 #include "dmma.h"
 
 namespace mbpt {
 namespace dmma {
 namespace {
+
+// a halving of the triangular inverse: rows [o, o + n1) and the n2 after them
+struct Node {
+  int o, n1, n2;
+};
+constexpr int kMaxNodes = 32;
 
 constexpr int BM = 64, BK = 16, kStages = 3, kThreads = 128;
 constexpr int kKStride = BK + 4;  // [row][k] tiles
@@ -172,6 +186,12 @@ struct Args {
   int64_t ld_xs;
   double *out;
   int64_t s_out;
+  // Dyson step
+  const double *src;   // CHOL: the matrices whose identity complement is factorised
+  int64_t ld_src, s_src;
+  const int *info;     // matrices whose word is not zero are left alone (null: none)
+  int nnodes;
+  Node node[kMaxNodes];
 };
 
 enum Epi : int {
@@ -179,6 +199,10 @@ enum Epi : int {
   PRODUCT = 1,   // C = acc0 o acc1, mirrored
   SIGMA = 2,     // c0 = acc1 o acc0, c1 = acc2 o acc0: upper tiles, the diagonal ones halved
   ROWDOT = 3,    // out[p] += alpha sum_r xs[r, p] acc[r, p], K from the tile's first row
+  CHOL = 4,      // C = I - src - acc, on and above the diagonal
+  NODE_T = 5,    // per node: T^T = U12^T V11^T, K from the tile's first column
+  NODE_V = 6,    // per node: V12 = -T V22, K up to the tile's last column
+  INVERSE = 7,   // C = -I + V V^T, mirrored, K from the tile's first column
 };
 
 template <int BN, bool AK, bool BKC, int EPI>
@@ -191,7 +215,23 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
   const int g = lane >> 2, t = lane & 3;
   const int wm = (warp & 1) * 32, wn = (warp >> 1) * (BN / 2);
   int ti, tj;
-  if (p.upper) {
+  int rows_m = p.m, rows_n = p.n, k_end0 = p.k[0];
+  int64_t z = blockIdx.z, off_a = 0, off_b = 0, off_c = 0;
+  if constexpr (EPI == NODE_T || EPI == NODE_V) {
+    const Node &q = p.node[z % p.nnodes];
+    z /= p.nnodes;
+    const int64_t o1 = q.o, o2 = q.o + q.n1;
+    rows_m = EPI == NODE_T ? q.n2 : q.n1;
+    rows_n = EPI == NODE_T ? q.n1 : q.n2;
+    k_end0 = rows_n;
+    off_a = EPI == NODE_T ? o1 * p.a[0].ld + o2 : o2 * p.a[0].ld + o1;
+    off_b = EPI == NODE_T ? o1 * p.b[0].ld + o1 : o2 * p.b[0].ld + o2;
+    off_c = EPI == NODE_T ? o2 * p.ldc + o1 : o1 * p.ldc + o2;
+    const int tn = (rows_n + BN - 1) / BN;
+    ti = blockIdx.x / tn;
+    tj = blockIdx.x % tn;
+    if (ti * BM >= rows_m) return;
+  } else if (p.upper) {
     upper_tile(blockIdx.x, p.tiles_m, ti, tj);
   } else {
     // eight row tiles sweep the column tiles together (L2 reuse)
@@ -201,12 +241,16 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
     tj = in / rows;
   }
   const int m0 = ti * BM, n0 = tj * BN;
-  const int64_t z = blockIdx.z;
-  const int k_first = EPI == ROWDOT ? m0 : 0;
+  if constexpr (EPI >= CHOL) {
+    if (p.info && p.info[z] != 0) return;
+  }
+  if (EPI == CHOL && n0 + BN <= m0) return;
+  const int k_first = EPI == ROWDOT ? m0 : (EPI == INVERSE || EPI == NODE_T ? n0 : 0);
+  if (EPI == NODE_V) k_end0 = min(k_end0, n0 + BN);
   int tiles[NS], total = 0;
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
-    tiles[s] = (p.k[s] - k_first + BK - 1) / BK;
+    tiles[s] = ((s == 0 ? k_end0 : p.k[s]) - k_first + BK - 1) / BK;
     total += tiles[s];
   }
   // the tiles of the products, one product after the other
@@ -214,8 +258,9 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
   Stream<BKC, BN> fb;
   int fseg = EPI == SIGMA && tiles[0] == 0 ? 1 : 0, fleft = tiles[fseg], fstage = 0;
   auto open = [&](int s) {
-    fa.start(p.a[s].p + z * p.a[s].stride, p.a[s].ld, m0, p.m, k_first, p.k[s], p.wa[s]);
-    fb.start(p.b[s].p + z * p.b[s].stride, p.b[s].ld, n0, p.n, k_first, p.k[s], p.wb[s]);
+    const int ke = s == 0 ? k_end0 : p.k[s];
+    fa.start(p.a[s].p + z * p.a[s].stride + off_a, p.a[s].ld, m0, rows_m, k_first, ke, p.wa[s]);
+    fb.start(p.b[s].p + z * p.b[s].stride + off_b, p.b[s].ld, n0, rows_n, k_first, ke, p.wb[s]);
   };
   open(fseg);
   auto fetch = [&] {
@@ -242,14 +287,14 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
 #pragma unroll
     for (int i = 0; i < MI; ++i) {
       const int r = m0 + wm + 8 * i + g;
-      if (r >= p.m) continue;
+      if (r >= rows_m) continue;
 #pragma unroll
       for (int j = 0; j < NJ; ++j)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int col = n0 + wn + 8 * j + 2 * t + e;
-          if (col >= p.n) continue;
-          double *at = c + z * p.sc + static_cast<int64_t>(r) * p.ldc + col;
+          if (col >= rows_n) continue;
+          double *at = c + z * p.sc + off_c + static_cast<int64_t>(r) * p.ldc + col;
           const double v = value(i, j, e, at);
           *at = v;
           if (mirror) c[z * p.sc + static_cast<int64_t>(col) * p.ldc + r] = v;
@@ -257,6 +302,18 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
     }
   };
   clear();
+  if constexpr (EPI == INVERSE) {
+    // the sums start from -I: a diagonal entry's first term cancels it, and the
+    // small ones that follow are not rounded at the size of 1 (W - I of the
+    // mid-size test 3x nearer its value than with I taken off at the end)
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          if (m0 + wm + 8 * i + g == n0 + wn + 8 * j + 2 * t + e) acc[i][j][e] = -1.0;
+  }
   int seg_end = tiles[0];
   [[maybe_unused]] int seg = 0;
   if constexpr (EPI == SIGMA) {
@@ -320,7 +377,21 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
       }
     }
   }
-  if constexpr (EPI == STORE) {
+  if constexpr (EPI == CHOL) {
+    const double *src = p.src + z * p.s_src;
+    store(p.c0,
+          [&](int i, int j, int e, double *) {
+            const int r = m0 + wm + 8 * i + g, col = n0 + wn + 8 * j + 2 * t + e;
+            return (r == col ? 1.0 : 0.0) - src[static_cast<int64_t>(r) * p.ld_src + col] -
+                   acc[i][j][e];
+          },
+          false);
+  } else if constexpr (EPI == NODE_T || EPI == NODE_V) {
+    store(p.c0, [&](int i, int j, int e, double *) { return EPI == NODE_T ? acc[i][j][e] : -acc[i][j][e]; },
+          false);
+  } else if constexpr (EPI == INVERSE) {
+    store(p.c0, [&](int i, int j, int e, double *) { return acc[i][j][e]; }, tj > ti);
+  } else if constexpr (EPI == STORE) {
     const double alpha = p.alpha, beta = p.beta;
     store(p.c0,
           [&](int i, int j, int e, const double *at) {
@@ -366,13 +437,18 @@ int launch(Args &p, int batch, cudaStream_t st) {
   using S = Smem<BN, AK, BKC>;
   if (p.m < 1 || p.n < 1 || batch < 1 || batch > 65535) return MBPT_ERR_SHAPE;
   for (int s = 0; s < NS; ++s) {
-    if (p.k[s] < (EPI == SIGMA && s == 0 && p.zt ? 0 : 1)) return MBPT_ERR_SHAPE;
+    const bool none = (EPI == SIGMA && s == 0 && p.zt) || EPI == CHOL;
+    if (p.k[s] < (none ? 0 : 1)) return MBPT_ERR_SHAPE;
     p.wa[s] = wide(p.a[s], batch);
     p.wb[s] = wide(p.b[s], batch);
   }
   p.tiles_m = (p.m + BM - 1) / BM;
   p.tiles_n = (p.n + BN - 1) / BN;
   if (p.upper && (BN != BM || p.m != p.n)) return MBPT_ERR_SHAPE;
+  if (EPI >= CHOL && p.nnodes == 0) p.nnodes = 1;
+  if ((EPI == NODE_T || EPI == NODE_V) && static_cast<int64_t>(batch) * p.nnodes > 65535)
+    return MBPT_ERR_SHAPE;
+  if (EPI == NODE_T || EPI == NODE_V) batch *= p.nnodes;
   const int64_t grid = p.upper ? static_cast<int64_t>(p.tiles_m) * (p.tiles_m + 1) / 2
                                : static_cast<int64_t>(p.tiles_m) * p.tiles_n;
   if (grid > (int64_t{1} << 30)) return MBPT_ERR_SHAPE;
@@ -475,6 +551,74 @@ int half_quadratic(const double *h, int64_t sh, int64_t m, const double *xs, int
   p.s_out = s_out;
   if (narrow(ns)) return launch<32, true, false, ROWDOT>(p, batch, st);
   return launch<64, true, false, ROWDOT>(p, batch, st);
+}
+
+int chol_update(const double *chi0, int64_t n, int64_t j0, int nbj, double *P, int batch,
+                cudaStream_t st) {
+  const int64_t m = n - j0;
+  if (!fits(m) || nbj < 1 || nbj > m || j0 < 0) return MBPT_ERR_SHAPE;
+  Args p{};
+  p.a[0] = p.b[0] = {chi0 + j0, n, n * n};
+  p.k[0] = static_cast<int>(j0);
+  p.m = nbj;
+  p.n = static_cast<int>(m);
+  p.src = chi0 + j0 * n + j0;
+  p.ld_src = n;
+  p.s_src = n * n;
+  p.c0 = P;
+  p.ldc = m;
+  p.sc = m * nbj;
+  return launch<64, false, false, CHOL>(p, batch, st);
+}
+
+int spd_inverse(double *chi0, int64_t n, double *V, int64_t ldv, const int *info, int batch,
+                cudaStream_t st) {
+  if (!fits(n)) return MBPT_ERR_SHAPE;
+  std::vector<std::vector<Node>> levels;
+  struct Split {
+    static void add(int64_t o, int64_t len, size_t depth, std::vector<std::vector<Node>> &lv) {
+      if (len <= kInverseLeaf) return;
+      if (lv.size() <= depth) lv.resize(depth + 1);
+      const int64_t n1 = round_up(len / 2, kInverseLeaf);
+      lv[depth].push_back({static_cast<int>(o), static_cast<int>(n1), static_cast<int>(len - n1)});
+      add(o, n1, depth + 1, lv);
+      add(o + n1, len - n1, depth + 1, lv);
+    }
+  };
+  Split::add(0, n, 0, levels);
+  const int64_t sv = n * ldv;
+  for (size_t d = levels.size(); d-- > 0;)
+    for (size_t first = 0; first < levels[d].size(); first += kMaxNodes) {
+      Args p{};
+      p.nnodes = static_cast<int>(std::min<size_t>(kMaxNodes, levels[d].size() - first));
+      for (int i = 0; i < p.nnodes; ++i) {
+        p.node[i] = levels[d][first + i];
+        p.m = std::max(p.m, std::max(p.node[i].n1, p.node[i].n2));
+      }
+      p.n = p.m;
+      p.k[0] = p.m;
+      p.info = info;
+      p.c0 = V;
+      p.ldc = ldv;
+      p.sc = sv;
+      Args q = p;
+      p.a[0] = {chi0, n, n * n};
+      p.b[0] = {V, ldv, sv};
+      int rc = launch<64, false, true, NODE_T>(p, batch, st);
+      if (rc) return rc;
+      q.a[0] = q.b[0] = {V, ldv, sv};
+      rc = launch<64, false, false, NODE_V>(q, batch, st);
+      if (rc) return rc;
+    }
+  Args p{};
+  p.a[0] = p.b[0] = {V, ldv, sv};
+  p.k[0] = p.m = p.n = static_cast<int>(n);
+  p.info = info;
+  p.c0 = chi0;
+  p.ldc = n;
+  p.sc = n * n;
+  p.upper = true;
+  return launch<64, true, true, INVERSE>(p, batch, st);
 }
 
 }  // namespace dmma

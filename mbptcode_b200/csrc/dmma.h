@@ -42,5 +42,23 @@ int sigma_h(const double *zt, const Operand &u, const Operand &d, int64_t naux,
 int half_quadratic(const double *h, int64_t sh, int64_t m, const double *xs, int64_t ns,
                    double sign, double *out, int64_t s_out, int batch, cudaStream_t st);
 
+// One step of the left-looking Cholesky of I - chi0 for `batch` row-major
+// n x n matrices whose rows above j0 hold the factor U (I - chi0 = U^T U):
+// P (nbj x (n - j0)) = (I - chi0)[j0:j0+nbj, j0:] - U[:j0, j0:j0+nbj]^T U[:j0, j0:],
+// on and above the diagonal.
+int chol_update(const double *chi0, int64_t n, int64_t j0, int nbj, double *P, int batch,
+                cudaStream_t st);
+
+// The triangular inverse halves down to diagonal blocks of this many rows.
+constexpr int64_t kInverseLeaf = 128;
+
+// chi0 <- U^-1 U^-T - I for `batch` factors U (the upper triangles of the
+// row-major n x n chi0; the strict lower ones are not read), symmetric to the
+// bit. V: batch x n x ldv doubles of scratch (ldv >= n) whose kInverseLeaf
+// diagonal blocks hold the inverses of U's, zeros below the diagonal. Where a
+// matrix's info word is not zero nothing is written.
+int spd_inverse(double *chi0, int64_t n, double *V, int64_t ldv, const int *info, int batch,
+                cudaStream_t st);
+
 }  // namespace dmma
 }  // namespace mbpt

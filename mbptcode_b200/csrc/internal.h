@@ -164,7 +164,6 @@ void launch_one_minus(double *a, int64_t n, int nmat, double *trace, cudaStream_
 void launch_trace(const double *a, int64_t n, int nmat, double *trace, cudaStream_t st);
 void launch_logdet_diag(const double *L, int64_t n, int nmat, double *logdet,
                         cudaStream_t st);
-void launch_symmetrize_minus_identity(double *a, int64_t n, int nmat, cudaStream_t st);
 void launch_rowdot(const double *R, int64_t ld_r, const double *Xs, int64_t ld_x, int64_t M,
                    int64_t S, double sign, double *out, cudaStream_t st);
 void launch_gather_cols_f32(const double *X, int64_t M, int64_t n, const int64_t *states,

@@ -330,19 +330,6 @@ __global__ void logdet_kernel(const double *L, int64_t n, double *logdet) {
   if (threadIdx.x == 0) logdet[blockIdx.x] = 2.0 * part[0];
 }
 
-// The inverse lives in one triangle (row-major upper = column-major lower):
-// mirror it and subtract the identity, giving W - I.
-__global__ void symmetrize_minus_identity_kernel(double *a, int64_t n) {
-  double *m = a + static_cast<int64_t>(blockIdx.y) * n * n;
-  const int64_t total = n * n;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t r = i / n, c = i % n;
-    if (r > c) m[i] = m[c * n + r];
-    if (r == c) m[i] -= 1.0;
-  }
-}
-
 // out[p] += sign * sum_P Xs[P, p] R[P, p]
 __global__ void rowdot_kernel(const double *__restrict__ R, int64_t ld_r,
                               const double *__restrict__ Xs, int64_t ld_x, int64_t M, int64_t S,
@@ -565,11 +552,6 @@ void launch_one_minus(double *a, int64_t n, int nmat, double *trace, cudaStream_
 void launch_logdet_diag(const double *L, int64_t n, int nmat, double *logdet,
                         cudaStream_t st) {
   count_launch(); logdet_kernel<<<nmat, 256, 0, st>>>(L, n, logdet);
-}
-
-void launch_symmetrize_minus_identity(double *a, int64_t n, int nmat, cudaStream_t st) {
-  dim3 grid(static_cast<unsigned>(grid_cap(n * n) / 4 + 1), nmat);
-  count_launch(); symmetrize_minus_identity_kernel<<<grid, kThreads, 0, st>>>(a, n);
 }
 
 void launch_rowdot(const double *R, int64_t ld_r, const double *Xs, int64_t ld_x, int64_t M,
