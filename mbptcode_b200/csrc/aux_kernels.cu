@@ -190,12 +190,18 @@ __global__ void trtri_diag_blocks_kernel(double *A, int64_t n, int64_t lda, int 
 // rows x k FP64 matrix X(r, c) = src[r * rs + c * cs], through a 32 x 33
 // shared tile so that the global reads run along whichever stride is 1.
 // The pair is split from the FP64 value: hi = tf32(x), lo = tf32(x - hi).
+// Matrices over blockIdx.z (src and pairs src_stride and rows_p k_p apart);
+// lower: only the 32 x 32 tiles on and below the diagonal.
 __global__ void strided_to_tf32_kernel(const double *__restrict__ src, int64_t rows, int64_t k,
-                                       int64_t rs, int64_t cs, float *hi, float *lo,
-                                       int64_t rows_p, int64_t k_p) {
+                                       int64_t rs, int64_t cs, int64_t src_stride, float *hi,
+                                       float *lo, int64_t rows_p, int64_t k_p, bool lower) {
   __shared__ double tile[32][33];
   const int64_t r0 = static_cast<int64_t>(blockIdx.y) * 32;
   const int64_t c0 = static_cast<int64_t>(blockIdx.x) * 32;
+  if (lower && c0 > r0) return;
+  src += blockIdx.z * src_stride;
+  hi += blockIdx.z * rows_p * k_p;
+  lo += blockIdx.z * rows_p * k_p;
   const bool col_unit = cs == 1;
   for (int a = threadIdx.y; a < 32; a += blockDim.y) {
     const int64_t r = col_unit ? r0 + a : r0 + threadIdx.x;
@@ -670,26 +676,42 @@ __global__ void inverse_blocks_kernel(const double *__restrict__ src, int64_t sf
     }
 }
 
-// The batched Cholesky's inverted diagonal blocks of one matrix (block j at
-// Linv + j * step_stride, column-major, ld kCholNb) as TF32 pairs in the two
-// layouts of the triangular-inverse recursion: rows of L^-1 (r_*) and columns
-// of L^-1 as rows (c_*), zeros above the diagonal included, as
-// trtri_diag_blocks_kernel writes them. One CTA per block.
+// The batched Cholesky's inverted diagonal blocks (block j of matrix f at
+// Linv + j step_stride + f kCholNb^2, column-major, ld kCholNb) as TF32 pairs in
+// the two layouts of the triangular-inverse recursion: rows of L^-1 (r_*) and
+// columns of L^-1 as rows (c_*), zeros above the diagonal included, as
+// trtri_diag_blocks_kernel writes them; the matrices' pair arrays ldp^2 apart.
+// One 32 x 32 tile of a block per CTA, transposed through shared memory (one
+// CTA per block, strided 4-byte stores: 54 us at 7 blocks).
 __global__ void linv_blocks_to_pairs_kernel(const double *__restrict__ Linv,
                                             int64_t step_stride, int64_t n, float *c_hi,
                                             float *c_lo, float *r_hi, float *r_lo, int64_t ldp) {
-  const int64_t off = static_cast<int64_t>(blockIdx.x) * kCholNb;
+  __shared__ float th[32][33], tl[32][33];
+  const int64_t off = static_cast<int64_t>(blockIdx.y) * kCholNb;
   const int m = static_cast<int>(min(static_cast<int64_t>(kCholNb), n - off));
-  const double *X = Linv + static_cast<int64_t>(blockIdx.x) * step_stride;
-  for (int idx = threadIdx.x; idx < m * m; idx += blockDim.x) {
-    const int c = idx / m, r = idx % m;
-    const double x = X[c * kCholNb + r];
-    const float h = to_tf32(static_cast<float>(x));
-    const float l = to_tf32(static_cast<float>(x - static_cast<double>(h)));
-    r_hi[(off + r) * ldp + off + c] = h;
-    r_lo[(off + r) * ldp + off + c] = l;
-    c_hi[(off + c) * ldp + off + r] = h;
-    c_lo[(off + c) * ldp + off + r] = l;
+  const int r0 = (blockIdx.x & 3) * 32, c0 = (blockIdx.x >> 2) * 32;
+  const double *X = Linv + blockIdx.y * step_stride + blockIdx.z * int64_t{kCholNb * kCholNb};
+  const int64_t base = blockIdx.z * ldp * ldp;
+  const int x = threadIdx.x;
+  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+    const int r = r0 + x, c = c0 + k;
+    if (r < m && c < m) {
+      const double v = X[c * kCholNb + r];
+      const float h = to_tf32(static_cast<float>(v));
+      const float l = to_tf32(static_cast<float>(v - static_cast<double>(h)));
+      c_hi[base + (off + c) * ldp + off + r] = h;
+      c_lo[base + (off + c) * ldp + off + r] = l;
+      th[k][x] = h;
+      tl[k][x] = l;
+    }
+  }
+  __syncthreads();
+  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+    const int r = r0 + k, c = c0 + x;
+    if (r < m && c < m) {
+      r_hi[base + (off + r) * ldp + off + c] = th[x][k];
+      r_lo[base + (off + r) * ldp + off + c] = tl[x][k];
+    }
   }
 }
 
@@ -750,11 +772,13 @@ int launch_trtri_diag_blocks(double *A, int64_t n, int64_t lda, int nb, cudaStre
 }
 
 void launch_strided_to_tf32(const double *src, int64_t rows, int64_t k, int64_t rs, int64_t cs,
-                            float *hi, float *lo, int64_t rows_p, int64_t k_p, cudaStream_t st) {
+                            int64_t src_stride, float *hi, float *lo, int64_t rows_p,
+                            int64_t k_p, bool lower, int batch, cudaStream_t st) {
   count_launch();
-  dim3 grid(static_cast<unsigned>((k_p + 31) / 32), static_cast<unsigned>((rows_p + 31) / 32));
-  strided_to_tf32_kernel<<<grid, dim3(32, 8), 0, st>>>(src, rows, k, rs, cs, hi, lo, rows_p,
-                                                       k_p);
+  dim3 grid(static_cast<unsigned>((k_p + 31) / 32), static_cast<unsigned>((rows_p + 31) / 32),
+            static_cast<unsigned>(batch));
+  strided_to_tf32_kernel<<<grid, dim3(32, 8), 0, st>>>(src, rows, k, rs, cs, src_stride, hi, lo,
+                                                       rows_p, k_p, lower);
 }
 
 void launch_identity(double *a, int64_t n, cudaStream_t st) {
@@ -842,12 +866,15 @@ void launch_row_dot_into_col(const double *G, const double *X, int64_t nr, int64
                                                                               out, ldo, p);
 }
 
-void launch_linv_blocks_to_pairs(const double *Linv, int64_t step_stride, int64_t n,
+void launch_linv_blocks_to_pairs(const double *Linv, int64_t step_stride, int64_t n, int batch,
                                  float *c_hi, float *c_lo, float *r_hi, float *r_lo,
                                  int64_t ldp, cudaStream_t st) {
+  constexpr unsigned kTiles = (kCholNb / 32) * (kCholNb / 32);
   count_launch();
-  linv_blocks_to_pairs_kernel<<<static_cast<unsigned>((n + kCholNb - 1) / kCholNb), 256, 0,
-                                st>>>(Linv, step_stride, n, c_hi, c_lo, r_hi, r_lo, ldp);
+  linv_blocks_to_pairs_kernel<<<dim3(kTiles, static_cast<unsigned>((n + kCholNb - 1) / kCholNb),
+                                     static_cast<unsigned>(batch)),
+                                dim3(32, 8), 0, st>>>(Linv, step_stride, n, c_hi, c_lo, r_hi,
+                                                      r_lo, ldp);
 }
 
 }  // namespace mbpt

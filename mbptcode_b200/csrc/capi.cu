@@ -43,10 +43,11 @@ int launch_trtri_diag_blocks(double *A, int64_t n, int64_t lda, int nb, cudaStre
                              float *c_hi = nullptr, float *c_lo = nullptr, float *r_hi = nullptr,
                              float *r_lo = nullptr, int64_t ldp = 0);
 void launch_strided_to_tf32(const double *src, int64_t rows, int64_t k, int64_t rs, int64_t cs,
-                            float *hi, float *lo, int64_t rows_p, int64_t k_p, cudaStream_t st);
+                            int64_t src_stride, float *hi, float *lo, int64_t rows_p,
+                            int64_t k_p, bool lower, int batch, cudaStream_t st);
 void launch_row_scaled_copy(const double *X, int64_t M, int64_t n, int64_t p, double *out,
                             cudaStream_t st);
-void launch_linv_blocks_to_pairs(const double *Linv, int64_t step_stride, int64_t n,
+void launch_linv_blocks_to_pairs(const double *Linv, int64_t step_stride, int64_t n, int batch,
                                  float *c_hi, float *c_lo, float *r_hi, float *r_lo,
                                  int64_t ldp, cudaStream_t st);
 void launch_rowdot_f32(const float *R, int64_t ld_r, const double *X, int64_t ld_x, int64_t M,
@@ -213,8 +214,8 @@ struct Chi0Bufs {
   double *w;  // cosft_wt on the device
   // fp64 (Xo_s, Xv_s, Go, Y: `batch` tau points each; Gv: the int8 mode only)
   double *Xo_s, *Xv_s, *Go, *Gv, *Y, *proj;
+  // mixed (Y, Pi, Z: `batch` tau points each, stacked by rows)
   int batch;
-  // mixed
   bf16 *Dt_hi, *Dt_lo, *Pi_hi, *Pi_lo, *Z_hi, *Z_lo;
   float *Yo_hi, *Yo_lo, *Yv_hi, *Yv_lo;  // TF32 pairs of the G products
   float *proj32;
@@ -226,13 +227,18 @@ struct Chi0Bufs {
 // already fills the GPU many times over), in even batches. At M = 2400 six
 // points a launch leave 26 tiles to the busiest SM where 25.03 are the mean;
 // one point a launch would leave 6 against 5.007.
-int tau_batch(int ntau, int64_t doubles_per_tau) {
-  const int64_t cap = (int64_t{640} << 20) / 8;
+int tau_batch(int ntau, int64_t doubles_per_tau, int64_t cap_mb = 640) {
+  const int64_t cap = (cap_mb << 20) / 8;
   const int64_t most = std::max<int64_t>(1, std::min<int64_t>(
       std::min(ntau, kMaxTauBatch), cap / std::max<int64_t>(1, doubles_per_tau)));
   const int64_t batches = (ntau + most - 1) / most;
   return static_cast<int>((ntau + batches - 1) / batches);
 }
+
+// The mixed sweeps' tile pairs run 74 at a time; a product of few pairs leaves
+// the last round of them nearly empty (153 pairs at M = 4219: 3 rounds for
+// 2.07; four points a launch: 9 for 8.3), so their batches may take 2 GB.
+constexpr int64_t kMixedBatchMb = 2048;
 
 TauList tau_list(const double *tau, int count) {
   TauList l{};
@@ -264,16 +270,20 @@ Chi0Bufs carve_chi0(Arena &ar, const Dims &d, int ntau, int nfreq, int mode, boo
     b.Y = ar.take<double>(b.batch * d.M * d.naux);
     if (own_proj) b.proj = ar.take<double>(static_cast<size_t>(ntau) * d.naux * d.naux);
   } else {
+    // TF32 pairs of Y, BF16 pairs of Pi and Z per tau point, in doubles
+    b.batch = tau_batch(ntau, d.Mp * (d.Ko + d.Kv) + (d.Mp * d.Mp + d.Ap * d.Mp) / 2,
+                        kMixedBatchMb);
+    const int64_t nb = b.batch;
     b.Dt_hi = ar.take<bf16>(d.Ap * d.Mp);
     b.Dt_lo = ar.take<bf16>(d.Ap * d.Mp);
-    b.Yo_hi = ar.take<float>(d.Mp * d.Ko);
-    b.Yo_lo = ar.take<float>(d.Mp * d.Ko);
-    b.Yv_hi = ar.take<float>(d.Mp * d.Kv);
-    b.Yv_lo = ar.take<float>(d.Mp * d.Kv);
-    b.Pi_hi = ar.take<bf16>(d.Mp * d.Mp);
-    b.Pi_lo = ar.take<bf16>(d.Mp * d.Mp);
-    b.Z_hi = ar.take<bf16>(d.Ap * d.Mp);
-    b.Z_lo = ar.take<bf16>(d.Ap * d.Mp);
+    b.Yo_hi = ar.take<float>(nb * d.Mp * d.Ko);
+    b.Yo_lo = ar.take<float>(nb * d.Mp * d.Ko);
+    b.Yv_hi = ar.take<float>(nb * d.Mp * d.Kv);
+    b.Yv_lo = ar.take<float>(nb * d.Mp * d.Kv);
+    b.Pi_hi = ar.take<bf16>(nb * d.Mp * d.Mp);
+    b.Pi_lo = ar.take<bf16>(nb * d.Mp * d.Mp);
+    b.Z_hi = ar.take<bf16>(nb * d.Ap * d.Mp);
+    b.Z_lo = ar.take<bf16>(nb * d.Ap * d.Mp);
     b.proj32 = ar.take<float>(static_cast<size_t>(ntau) * d.Ap * d.Ap);
     b.eye = ar.take<double>(static_cast<size_t>(ntau) * ntau);
   }
@@ -337,14 +347,15 @@ int chi0_run(const double *X, const Dims &d, const double *eps, double mu, const
     // G_occ and G_virt in TF32x3: their K sums cancel (off-diagonal entries
     // are ~sqrt(K) below the summed terms), which the BF16 split would carry
     // into chi0 at ~1e-4 relative; the D^T Pi D products stay BF16x3
-    SplitMat Yo{b.Yo_hi, b.Yo_lo, d.Mp, d.Ko, d.Ko, true};
-    SplitMat Yv{b.Yv_hi, b.Yv_lo, d.Mp, d.Kv, d.Kv, true};
     SplitMat Dt{b.Dt_hi, b.Dt_lo, d.Ap, d.Mp, d.Mp};
-    SplitMat Pi{b.Pi_hi, b.Pi_lo, d.Mp, d.Mp, d.Mp};
-    SplitMat Z{b.Z_hi, b.Z_lo, d.Ap, d.Mp, d.Mp};
-    for (int k = 0; k < ntau; ++k) {
-      launch_prep_branches_tf32(X, d.M, d.n, d.nocc, eps, mu, tau[k], b.Yo_hi, b.Yo_lo, d.Ko,
-                                b.Yv_hi, b.Yv_lo, d.Kv, d.Mp, st);
+    for (int k = 0; k < ntau; k += b.batch) {
+      const int nb = std::min(b.batch, ntau - k);
+      SplitMat Yo{b.Yo_hi, b.Yo_lo, nb * d.Mp, d.Ko, d.Ko, true};
+      SplitMat Yv{b.Yv_hi, b.Yv_lo, nb * d.Mp, d.Kv, d.Kv, true};
+      SplitMat Pi{b.Pi_hi, b.Pi_lo, nb * d.Mp, d.Mp, d.Mp};
+      SplitMat Z{b.Z_hi, b.Z_lo, nb * d.Ap, d.Mp, d.Mp};
+      launch_prep_branches<float>(X, d.M, d.n, d.nocc, eps, mu, tau_list(tau + k, nb), b.Yo_hi,
+                                  b.Yo_lo, d.Ko, b.Yv_hi, b.Yv_lo, d.Kv, d.Mp, st);
       umma::EpiArgs e;
       // Pi = (Y_o Y_o^T) o (Y_v Y_v^T), split for the next product
       e.out0_hi = b.Pi_hi;
@@ -353,14 +364,16 @@ int chi0_run(const double *X, const Dims &d, const double *eps, double mu, const
       SplitMat A2[2] = {Yo, Yv};
       // Pi is symmetric: the tiles on and above the diagonal, mirrored by the epilogue
       int rc = gemm_split(umma::EPI_HADAMARD_SPLIT, 2, A2, A2, d.Mp, d.Mp, e, err, st,
-                          umma::BAND_UPPER);
+                          umma::BAND_UPPER,
+                          {nb, {d.Mp, d.Mp}, {d.Mp, d.Mp}, d.Mp * d.Mp});
       if (rc) return rc;
       // Z = D^T Pi  (= (Pi D)^T, Pi symmetric)
       e = umma::EpiArgs();
       e.out0_hi = b.Z_hi;
       e.out0_lo = b.Z_lo;
       e.ld_out = d.Mp;
-      rc = gemm_split(umma::EPI_SPLIT, 1, &Dt, &Pi, d.Ap, d.Mp, e, err, st);
+      rc = gemm_split(umma::EPI_SPLIT, 1, &Dt, &Pi, d.Ap, d.Mp, e, err, st, 0,
+                      {nb, {0, 0}, {d.Mp, 0}, d.Ap * d.Mp});
       if (rc) return rc;
       // proj = -2 D^T Z^T
       e = umma::EpiArgs();
@@ -368,7 +381,8 @@ int chi0_run(const double *X, const Dims &d, const double *eps, double mu, const
       e.ld_outf = d.Ap;
       e.alpha = -2.f;
       // proj = -2 D^T Pi D is symmetric: upper tiles, mirrored
-      rc = gemm_split(umma::EPI_F32, 1, &Dt, &Z, d.Ap, d.Ap, e, err, st, umma::BAND_UPPER);
+      rc = gemm_split(umma::EPI_F32, 1, &Dt, &Z, d.Ap, d.Ap, e, err, st, umma::BAND_UPPER,
+                      {nb, {0, 0}, {d.Ap, 0}, d.Ap * d.Ap});
       if (rc) return rc;
     }
     launch_transform<float>(b.proj32, d.Ap * d.Ap, d.Ap, d.naux, d.naux, b.w, nfreq, ntau,
@@ -427,12 +441,13 @@ void collect_nodes(int64_t o, int64_t n, size_t depth,
   collect_nodes(o + n1, n - n1, depth + 1, levels);
 }
 
-int trtri_pairs(const PairScratch &s, int64_t n, int *err, cudaStream_t st) {
+int trtri_pairs(const PairScratch &s, int64_t n, int nb, int *err, cudaStream_t st) {
   std::vector<std::vector<std::pair<int64_t, int64_t>>> levels;
   collect_nodes(0, n, 0, levels);
-  const int64_t ld = s.np;
-  const SplitMat IC{s.ic_hi, s.ic_lo, ld, ld, ld, true}, IR{s.ir_hi, s.ir_lo, ld, ld, ld, true};
-  const SplitMat LR{s.lr_hi, s.lr_lo, ld, ld, ld, true}, TT{s.tt_hi, s.tt_lo, ld, ld, ld, true};
+  const int64_t ld = s.np, rows = nb * ld;
+  const SplitMat IC{s.ic_hi, s.ic_lo, rows, ld, ld, true}, IR{s.ir_hi, s.ir_lo, rows, ld, ld, true};
+  const SplitMat LR{s.lr_hi, s.lr_lo, rows, ld, ld, true}, TT{s.tt_hi, s.tt_lo, rows, ld, ld, true};
+  const GemmBatch batch{nb, {ld, 0}, {ld, 0}, ld * ld};
   std::vector<GemmGroup> g1, g2;
   for (size_t d = levels.size(); d-- > 0;) {
     g1.clear();
@@ -449,7 +464,8 @@ int trtri_pairs(const PairScratch &s, int64_t n, int *err, cudaStream_t st) {
     e1.ld_p = ld;
     e1.alpha = 1.f;
     int rc = gemm_split_grouped(umma::EPI_TF32_PAIR, IC, LR, g1.data(),
-                                static_cast<int>(g1.size()), e1, err, st, umma::BAND_K_FROM_M);
+                                static_cast<int>(g1.size()), e1, err, st, umma::BAND_K_FROM_M,
+                                batch);
     if (rc) return rc;
     umma::EpiArgs e2;
     e2.p_hi = s.ic_hi;
@@ -460,7 +476,7 @@ int trtri_pairs(const PairScratch &s, int64_t n, int *err, cudaStream_t st) {
     e2.ld_t = ld;
     e2.alpha = -1.f;
     rc = gemm_split_grouped(umma::EPI_TF32_PAIR, TT, IR, g2.data(), static_cast<int>(g2.size()),
-                            e2, err, st, umma::BAND_K_TO_N);
+                            e2, err, st, umma::BAND_K_TO_N, batch);
     if (rc) return rc;
   }
   return MBPT_OK;
@@ -471,33 +487,34 @@ struct TimingTag {
   ~TimingTag() { timing_tag(-1); }
 };
 
-// W - I from the Cholesky factor L of 1 - chi0 in mixed mode (column-major
-// lower, in place; the row-major upper triangle of the buffer): L^-1 as TF32
-// pairs by the tensor-core recursion, then W = (L^-1)^T L^-1 on the tensor
-// cores over the tiles on and above the diagonal (rows of (L^-1)^T vanish for
-// k < row), W - I written whole. diag_inv: the batched factorisation's inverted
-// 128 x 128 diagonal blocks (null: they are inverted here).
-int tf32_inverse_from_factor(double *L, int64_t n, const PairScratch &s, int *err,
-                             cudaStream_t st, const double *diag_inv = nullptr,
-                             int64_t diag_inv_stride = 0) {
+// W - I from the Cholesky factors L of nb matrices 1 - chi0 in mixed mode
+// (column-major lower, in place; the row-major upper triangles of the buffers):
+// L^-1 as TF32 pairs by the tensor-core recursion, then W = (L^-1)^T L^-1 on
+// the tensor cores over the tiles on and above the diagonal (rows of (L^-1)^T
+// vanish for k < row), W - I written whole. diag_inv: the batched
+// factorisation's inverted 128 x 128 diagonal blocks (null: they are inverted
+// here, nb 1). info: a matrix whose word is not zero is left as it is.
+int tf32_inverse_from_factor(double *L, int64_t n, int nb, const PairScratch &s, int *err,
+                             cudaStream_t st, const int *info = nullptr,
+                             const double *diag_inv = nullptr, int64_t diag_inv_stride = 0) {
   TimingTag tag(kTimingDyson);
   const int64_t np = s.np, kp = round_up(n, 32);
-  // rows of L (its upper triangle is never read)
-  launch_strided_to_tf32(L, n, n, 1, n, s.lr_hi, s.lr_lo, np, np, st);
+  // rows of L below the diagonal
+  launch_strided_to_tf32(L, n, n, 1, n, n * n, s.lr_hi, s.lr_lo, np, np, true, nb, st);
   int rc = MBPT_OK;
   if (diag_inv)
-    launch_linv_blocks_to_pairs(diag_inv, diag_inv_stride, n, s.ic_hi, s.ic_lo, s.ir_hi, s.ir_lo,
-                                np, st);
+    launch_linv_blocks_to_pairs(diag_inv, diag_inv_stride, n, nb, s.ic_hi, s.ic_lo, s.ir_hi,
+                                s.ir_lo, np, st);
   else
     rc = launch_trtri_diag_blocks(L, n, n, static_cast<int>(kTrtriLeaf), st, s.ic_hi, s.ic_lo,
                                   s.ir_hi, s.ir_lo, np);
   if (rc) return rc;
-  rc = trtri_pairs(s, n, err, st);
+  rc = trtri_pairs(s, n, nb, err, st);
   if (rc) return rc;
   // W - I straight into the factor's buffer as FP64 (row-major W(j, i) is
   // the column-major W(i, j) the caller expects; W is symmetric anyway),
   // tiles above the diagonal mirrored by the epilogue
-  SplitMat Ae{s.ic_hi, s.ic_lo, np, kp, np, true};
+  SplitMat Ae{s.ic_hi, s.ic_lo, nb * np, kp, np, true};
   umma::EpiArgs e;
   e.outd = L;
   e.ld_outd = n;
@@ -505,7 +522,8 @@ int tf32_inverse_from_factor(double *L, int64_t n, const PairScratch &s, int *er
   e.shift = 1.0;
   e.alpha = 1.f;
   return gemm_split(umma::EPI_F64_SYM, 1, &Ae, &Ae, np, np, e, err, st,
-                    umma::BAND_K_FROM_M | umma::BAND_K_FROM_N | umma::BAND_UPPER);
+                    umma::BAND_K_FROM_M | umma::BAND_K_FROM_N | umma::BAND_UPPER,
+                    {nb, {np, 0}, {np, 0}, n * n, 0, 0, info});
 }
 
 constexpr int kCholNb = 128;     // block columns of the batched Cholesky
@@ -594,20 +612,22 @@ int ozaki_slices(int mode, int64_t n) {
   return (v == 6 || v == 7 || v == 8) ? v : 8;
 }
 
-// Mixed mode: the tensor-core inverses of that many frequencies run at once,
-// each on its own side stream with its own TF32 pair scratch (8 n_p^2 floats):
-// the recursion's deep levels are small products that leave most of the GPU
-// idle when one frequency runs alone. MBPT_DYSON_INVERSE_STREAMS (1 to 4,
-// default 4), read once per process so that the size query and the call see
-// the same count.
-constexpr int kMaxInverseStreams = 4;
-int inverse_streams() {
-  static const int v = [] {
+// Mixed mode: the tensor-core inverses of that many frequencies share each
+// launch (the recursion's deep levels are small products that leave most of
+// the GPU idle when one frequency runs alone), with 8 n_p^2 floats of TF32 pair
+// scratch each: as many as 1 GB holds, four at least.
+// MBPT_DYSON_INVERSE_STREAMS (1 to 4) sets the number instead, read once per
+// process so that the size query and the call see the same.
+int inverses_in_flight(int64_t np, int nfreq) {
+  static const int env = [] {
     const char *e = std::getenv("MBPT_DYSON_INVERSE_STREAMS");
-    const int k = e ? std::atoi(e) : kMaxInverseStreams;
-    return std::max(1, std::min(kMaxInverseStreams, k));
+    return e ? std::max(1, std::min(4, std::atoi(e))) : 0;
   }();
-  return v;
+  const int64_t fit = (int64_t{1} << 30) / (32 * np * np);
+  const int most = static_cast<int>(std::max<int64_t>(
+      1, std::min<int64_t>(nfreq, env ? env : std::max<int64_t>(4, fit))));
+  const int rounds = (nfreq + most - 1) / most;
+  return (nfreq + rounds - 1) / rounds;
 }
 
 bool batched_chol_enabled(int nfreq) {
@@ -629,7 +649,7 @@ struct DysonBufs {
   int64_t ldv = 0;
   int inv_batch = 0;
   double *diag;  // nfreq x n diagonals of 1 - chi0, which the factorisation overwrites
-  PairScratch pairs[kMaxInverseStreams];  // mixed mode: one per inverse stream
+  PairScratch pairs;  // mixed mode: npairs frequencies' arrays, stacked
   int npairs = 0;
   double *chol_P = nullptr, *chol_Linv = nullptr;  // batched Cholesky scratch
   int8_t *oz_planes = nullptr;                       // Ozaki digit planes (all frequencies)
@@ -678,14 +698,12 @@ DysonBufs carve_dyson(Arena &ar, int64_t n, int nfreq, int mode = MBPT_MODE_FP64
   }
   if (mode == MBPT_MODE_MIXED) {
     const int64_t np = round_up(n, 128), cap = np * np;
-    b.npairs = std::min(inverse_streams(), std::max(1, nfreq));
-    for (int i = 0; i < b.npairs; ++i) {
-      PairScratch &q = b.pairs[i];
-      q.np = np;
-      for (float **f : {&q.lr_hi, &q.lr_lo, &q.ic_hi, &q.ic_lo, &q.ir_hi, &q.ir_lo, &q.tt_hi,
-                        &q.tt_lo})
-        *f = ar.take<float>(cap);
-    }
+    b.npairs = batched_chol_enabled(nfreq) ? inverses_in_flight(np, nfreq) : 1;
+    PairScratch &q = b.pairs;
+    q.np = np;
+    for (float **f : {&q.lr_hi, &q.lr_lo, &q.ic_hi, &q.ic_lo, &q.ir_hi, &q.ir_lo, &q.tt_hi,
+                      &q.tt_lo})
+      *f = ar.take<float>(b.npairs * cap);
   }
   return b;
 }
@@ -697,9 +715,6 @@ DysonBufs carve_dyson(Arena &ar, int64_t n, int nfreq, int mode = MBPT_MODE_FP64
 struct DysonPipe {
   cudaStream_t side = nullptr;
   cudaEvent_t join = nullptr;
-  // mixed mode's further inverse streams (index i + 1 of the inverse streams)
-  std::vector<cudaStream_t> isides;
-  std::vector<cudaEvent_t> ijoin;
   // second factor stream: odd frequencies factorise there with their own
   // cuSOLVER handle, so that two Cholesky factorisations (latency-bound
   // panels between DGEMM-bound updates) share the GPU
@@ -739,14 +754,6 @@ DysonPipe *dyson_pipe(int nfreq) {
               cudaEventCreateWithFlags(&p->join2, cudaEventDisableTiming) == cudaSuccess &&
               cusolverDnCreate(&p->solver2) == CUSOLVER_STATUS_SUCCESS &&
               cusolverDnSetStream(p->solver2, p->fac2) == CUSOLVER_STATUS_SUCCESS;
-    for (int i = 1; p->ok && i < kMaxInverseStreams; ++i) {
-      cudaStream_t s = nullptr;
-      cudaEvent_t e = nullptr;
-      p->ok = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess &&
-              cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
-      p->isides.push_back(s);
-      p->ijoin.push_back(e);
-    }
     const char *genv = std::getenv("MBPT_DYSON_CHOL_GROUPS");
     const int g = genv ? std::atoi(genv) : 4;
     p->groups = p->nfac == 2 ? std::max(1, std::min(6, g)) : 1;
@@ -808,19 +815,15 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
   // the diagonal (of chi0 in a batch, of 1 - chi0 otherwise), for the LU fallback
   launch_diag(chi0, n, nfreq, b.diag, true, st);
   if (mode == MBPT_MODE_MIXED && want_w) {
-    // the pair arrays are read as zeros wherever the recursion does not write
-    // (padding, above the diagonal blocks); every frequency writes the rest
-    for (int i = 0; i < b.npairs; ++i) {
-      const PairScratch &q = b.pairs[i];
-      const size_t bytes = sizeof(float) * q.np * q.np;
-      for (float *f : {q.lr_hi, q.lr_lo, q.ic_hi, q.ic_lo, q.ir_hi, q.ir_lo, q.tt_hi, q.tt_lo})
-        if (cudaMemsetAsync(f, 0, bytes, st) != cudaSuccess) return MBPT_ERR_CUDA;
-    }
+    // the inverse's pair arrays are read as zeros wherever the recursion does
+    // not write (padding, above the diagonal blocks); every frequency writes
+    // the rest, and all that is read of the other arrays
+    const PairScratch &q = b.pairs;
+    for (float *f : {q.ic_hi, q.ic_lo, q.ir_hi, q.ir_lo})
+      if (cudaMemsetAsync(f, 0, sizeof(float) * b.npairs * q.np * q.np, st) != cudaSuccess)
+        return MBPT_ERR_CUDA;
   }
-  // the inverse streams: FP64 mode's cuBLAS inverse on the side stream only
-  const int nsides = mode == MBPT_MODE_MIXED ? b.npairs : 1;
-  auto side_of = [&](int i) { return i == 0 ? pp->side : pp->isides[i - 1]; };
-  bool side_used[kMaxInverseStreams] = {};
+  bool side_used = false;
   if (batched) {
     if (cudaMemsetAsync(b.info, 0, sizeof(int) * nfreq, st) != cudaSuccess) return MBPT_ERR_CUDA;
     // groups of frequencies on their own streams (four by default, each of
@@ -829,71 +832,60 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
     // per matrix) are factorised
     auto stream_of = [&](int g) { return g == 0 ? st : (g == 1 ? pp->fac2 : pp->xs[g - 2]); };
     auto join_of = [&](int g) { return g == 1 ? pp->join2 : pp->xj[g - 2]; };
-    // waves (MBPT_DYSON_WAVES=2): the frequencies factorised in two halves one
-    // after the other on the same streams, the tensor-core inverses of the
-    // first half (on the side stream, issued as soon as its factors are done)
-    // running beside the second half's FP64 factorisation. Off by default:
-    // at naux 7200, 24 frequencies it measured 155.6 ms against 154.0 ms for
-    // one wave (the overlap does not pay for the smaller batches)
-    const char *wenv = std::getenv("MBPT_DYSON_WAVES");
-    const int want_waves = wenv ? std::max(1, std::atoi(wenv)) : 1;
-    const int waves = (want_w && nfreq >= 2 * kBatchedCholMin) ? std::min(want_waves, 2) : 1;
-    int G = 1;
-    for (int w = 0; w < waves; ++w) {
-      const int n_w = nfreq * (w + 1) / waves - nfreq * w / waves;
-      G = std::max(G, std::min(pp->groups, n_w / kBatchedCholMin));
-    }
+    const int G = std::max(1, std::min(pp->groups, nfreq / kBatchedCholMin));
     if (G > 1 && cudaEventRecord(pp->fork, st) != cudaSuccess) return MBPT_ERR_CUDA;
     for (int g = 1; g < G; ++g)
       if (cudaStreamWaitEvent(stream_of(g), pp->fork, 0) != cudaSuccess) return MBPT_ERR_CUDA;
     int rc0 = MBPT_OK;
-    for (int w = 0; w < waves && !rc0; ++w) {
-      const int w0 = nfreq * w / waves, nw = nfreq * (w + 1) / waves - w0;
-      const int Gw = std::max(1, std::min(G, nw / kBatchedCholMin));
-      for (int g = 0; g < Gw && !rc0; ++g) {
-        const int f0 = w0 + static_cast<int>(static_cast<int64_t>(nw) * g / Gw);
-        const int f1 = w0 + static_cast<int>(static_cast<int64_t>(nw) * (g + 1) / Gw);
-        cudaStream_t gs = stream_of(g);
-        OzakiChol oz;
-        if (b.oz_planes) {
-          // this group's frequencies own a contiguous share of each buffer
-          oz.planes = b.oz_planes + ozaki_planes_bytes(n, f0, b.oz_slices);
-          oz.scale = b.oz_scale + static_cast<int64_t>(f0) * n;
-          oz.rowsq = b.oz_rowsq + static_cast<int64_t>(f0) * n;
-          oz.slices = b.oz_slices;
-          oz.err = err;
-        }
-        rc0 = chol_batched(chi0 + f0 * n * n, n, f1 - f0, b.info + f0,
-                           b.chol_P + static_cast<int64_t>(f0) * n * kCholNb,
-                           b.chol_Linv + static_cast<int64_t>(f0) * kCholNb * kCholNb,
-                           gs, static_cast<int64_t>(nfreq) * kCholNb * kCholNb, &oz);
-        if (rc0) break;
-        // this group's log-determinants, info words and events on its own stream
-        launch_logdet_diag(chi0 + f0 * n * n, n, f1 - f0, logdet + f0, gs);
-        if (!deferred && cudaMemcpyAsync(pp->info + f0, b.info + f0, sizeof(int) * (f1 - f0),
-                                         cudaMemcpyDeviceToHost, gs) != cudaSuccess)
-          rc0 = MBPT_ERR_CUDA;
-        for (int f = f0; f < f1 && !rc0; ++f)
-          if (cudaEventRecord(pp->ev[f], gs) != cudaSuccess) rc0 = MBPT_ERR_CUDA;
+    for (int g = 0; g < G && !rc0; ++g) {
+      const int f0 = static_cast<int>(static_cast<int64_t>(nfreq) * g / G);
+      const int f1 = static_cast<int>(static_cast<int64_t>(nfreq) * (g + 1) / G);
+      cudaStream_t gs = stream_of(g);
+      OzakiChol oz;
+      if (b.oz_planes) {
+        // this group's frequencies own a contiguous share of each buffer
+        oz.planes = b.oz_planes + ozaki_planes_bytes(n, f0, b.oz_slices);
+        oz.scale = b.oz_scale + static_cast<int64_t>(f0) * n;
+        oz.rowsq = b.oz_rowsq + static_cast<int64_t>(f0) * n;
+        oz.slices = b.oz_slices;
+        oz.err = err;
       }
+      rc0 = chol_batched(chi0 + f0 * n * n, n, f1 - f0, b.info + f0,
+                         b.chol_P + static_cast<int64_t>(f0) * n * kCholNb,
+                         b.chol_Linv + static_cast<int64_t>(f0) * kCholNb * kCholNb,
+                         gs, static_cast<int64_t>(nfreq) * kCholNb * kCholNb, &oz);
+      if (rc0) break;
+      // this group's log-determinants, info words and events on its own stream
+      launch_logdet_diag(chi0 + f0 * n * n, n, f1 - f0, logdet + f0, gs);
+      if (!deferred && cudaMemcpyAsync(pp->info + f0, b.info + f0, sizeof(int) * (f1 - f0),
+                                       cudaMemcpyDeviceToHost, gs) != cudaSuccess)
+        rc0 = MBPT_ERR_CUDA;
+      for (int f = f0; f < f1 && !rc0; ++f)
+        if (cudaEventRecord(pp->ev[f], gs) != cudaSuccess) rc0 = MBPT_ERR_CUDA;
     }
     for (int g = 1; g < G; ++g)
       if (cudaEventRecord(join_of(g), stream_of(g)) != cudaSuccess ||
           cudaStreamWaitEvent(st, join_of(g), 0) != cudaSuccess)
         return MBPT_ERR_CUDA;
     if (rc0) return rc0;
-    // FP64 modes: the inverses of as many factors at a time as the scratch holds
-    // (where a factorisation failed nothing is written)
-    if (want_w && fp64_mode(mode))
-      for (int f0 = 0; f0 < nfreq; f0 += b.inv_batch) {
-        const int nb = std::min(b.inv_batch, nfreq - f0);
-        const int64_t blk = static_cast<int64_t>(kCholNb) * kCholNb;
-        launch_inverse_blocks(b.chol_Linv + f0 * blk, blk, nfreq * blk, kCholNb, n, nb, b.V,
-                              b.ldv, st);
-        const int rc1 =
-            dmma::spd_inverse(chi0 + f0 * n * n, n, b.V, b.ldv, b.info + f0, nb, st);
-        if (rc1) return rc1;
+    // the inverses of as many factors at a time as the scratch holds (where a
+    // factorisation failed nothing is written)
+    const int nbi = mode == MBPT_MODE_MIXED ? b.npairs : b.inv_batch;
+    const int64_t blk = static_cast<int64_t>(kCholNb) * kCholNb;
+    for (int f0 = 0; want_w && f0 < nfreq; f0 += nbi) {
+      const int nb = std::min(nbi, nfreq - f0);
+      double *m = chi0 + f0 * n * n;
+      const double *dinv = b.chol_Linv + f0 * blk;
+      int rc1;
+      if (mode == MBPT_MODE_MIXED) {
+        rc1 = tf32_inverse_from_factor(m, n, nb, b.pairs, err, st, b.info + f0, dinv,
+                                       nfreq * blk);
+      } else {
+        launch_inverse_blocks(dinv, blk, nfreq * blk, kCholNb, n, nb, b.V, b.ldv, st);
+        rc1 = dmma::spd_inverse(m, n, b.V, b.ldv, b.info + f0, nb, st);
       }
+      if (rc1) return rc1;
+    }
   }
   const int nfac = nfreq > 1 && !batched ? pp->nfac : 1;
   if (nfac == 2 && (cudaEventRecord(pp->fork, st) != cudaSuccess ||
@@ -931,20 +923,15 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
     if (sign_host) sign_host[f] = 1;
     double *m = chi0 + f * n * n;
     if (inf == 0) {
-      // a batch's FP64 inverses are under way already
-      if (want_w && !(batched && fp64_mode(mode))) {
-        const int si = f % nsides;
-        cudaStream_t ss = side_of(si);
-        side_used[si] = true;
+      if (want_w && !batched) {  // a batch's inverses are under way already
+        cudaStream_t ss = pp->side;
+        side_used = true;
         if (cudaStreamWaitEvent(ss, pp->ev[f], 0) != cudaSuccess) {
           rc = MBPT_ERR_CUDA;
           break;
         }
         if (mode == MBPT_MODE_MIXED) {
-          rc = tf32_inverse_from_factor(
-              m, n, b.pairs[si], err, ss,
-              batched ? b.chol_Linv + static_cast<int64_t>(f) * kCholNb * kCholNb : nullptr,
-              static_cast<int64_t>(nfreq) * kCholNb * kCholNb);
+          rc = tf32_inverse_from_factor(m, n, 1, b.pairs, err, ss);
         } else {
           rc = launch_trtri_diag_blocks(m, n, n, static_cast<int>(kTrtriLeaf), ss);
           if (rc) break;
@@ -959,9 +946,7 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
     // restore 1 - chi0 from its untouched triangle, then LU for log|det| (and
     // the inverse), as the reference's slogdet/inv
     bad = true;
-    for (int i = 1; i < nsides; ++i)
-      if (cudaStreamSynchronize(side_of(i)) != cudaSuccess) rc = MBPT_ERR_CUDA;
-    if (rc || cudaStreamSynchronize(pp->side) != cudaSuccess ||
+    if (cudaStreamSynchronize(pp->side) != cudaSuccess ||
         (nfac == 2 && cudaStreamSynchronize(pp->fac2) != cudaSuccess) ||
         cudaStreamSynchronize(st) != cudaSuccess) {
       rc = MBPT_ERR_CUDA;
@@ -997,11 +982,9 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
     }
     if (sign_host) sign_host[f] = sgn;
   }
-  for (int i = 0; i < nsides; ++i) {
-    if (!side_used[i]) continue;
-    cudaEvent_t j = i == 0 ? pp->join : pp->ijoin[i - 1];
-    cudaEventRecord(j, side_of(i));
-    cudaStreamWaitEvent(st, j, 0);
+  if (side_used) {
+    cudaEventRecord(pp->join, pp->side);
+    cudaStreamWaitEvent(st, pp->join, 0);
   }
   if (nfac == 2) {
     cudaEventRecord(pp->join2, pp->fac2);
@@ -1020,8 +1003,8 @@ struct SigmaBufs {
   // fp64 (U, Ws, Hl, Hg, Xo_s, Xv_s: `batch` tau points each; Zt alone where
   // W = I; Hl as G and R: the int8 mode)
   double *U, *Ws, *Zt, *Hl, *Hg, *Xo_s, *Xv_s, *Xs, *R;
+  // mixed (W, U, Y, Zf, Hl, Hg: `batch` tau points each, stacked by rows)
   int batch;
-  // mixed
   bf16 *D_hi, *D_lo, *W_hi, *W_lo, *U_hi, *U_lo, *Yo_hi, *Yo_lo, *Yv_hi, *Yv_lo, *Hl_hi,
       *Hl_lo, *Hg_hi, *Hg_lo, *XsT_hi, *XsT_lo;
   float *xs, *Zf;
@@ -1054,24 +1037,22 @@ SigmaBufs carve_sigma(Arena &ar, const Dims &d, int ntau, int nstates, int mode)
     b.R = ar.take<double>(d.M * static_cast<int64_t>(nstates));
   } else {
     const int64_t Sp = pad_states(nstates);
+    // BF16 pairs of W, U, Y, H^< and H^> and FP32 Zt per tau point, in doubles
+    b.batch = tau_batch(ntau, (d.Ap * d.Ap + d.Mp * (d.Ap + d.Ko + d.Kv) + 3 * d.Mp * d.Mp) / 2,
+                        kMixedBatchMb);
+    const int64_t nb = b.batch;
     b.D_hi = ar.take<bf16>(d.Mp * d.Ap);
     b.D_lo = ar.take<bf16>(d.Mp * d.Ap);
-    b.W_hi = ar.take<bf16>(d.Ap * d.Ap);
-    b.W_lo = ar.take<bf16>(d.Ap * d.Ap);
-    b.U_hi = ar.take<bf16>(d.Mp * d.Ap);
-    b.U_lo = ar.take<bf16>(d.Mp * d.Ap);
-    b.Yo_hi = ar.take<bf16>(d.Mp * d.Ko);
-    b.Yo_lo = ar.take<bf16>(d.Mp * d.Ko);
-    b.Yv_hi = ar.take<bf16>(d.Mp * d.Kv);
-    b.Yv_lo = ar.take<bf16>(d.Mp * d.Kv);
-    b.Hl_hi = ar.take<bf16>(d.Mp * d.Mp);
-    b.Hl_lo = ar.take<bf16>(d.Mp * d.Mp);
-    b.Hg_hi = ar.take<bf16>(d.Mp * d.Mp);
-    b.Hg_lo = ar.take<bf16>(d.Mp * d.Mp);
+    for (bf16 **q : {&b.W_hi, &b.W_lo}) *q = ar.take<bf16>(nb * d.Ap * d.Ap);
+    for (bf16 **q : {&b.U_hi, &b.U_lo}) *q = ar.take<bf16>(nb * d.Mp * d.Ap);
+    for (bf16 **q : {&b.Yo_hi, &b.Yo_lo}) *q = ar.take<bf16>(nb * d.Mp * d.Ko);
+    for (bf16 **q : {&b.Yv_hi, &b.Yv_lo}) *q = ar.take<bf16>(nb * d.Mp * d.Kv);
+    for (bf16 **q : {&b.Hl_hi, &b.Hl_lo, &b.Hg_hi, &b.Hg_lo})
+      *q = ar.take<bf16>(nb * d.Mp * d.Mp);
     b.XsT_hi = ar.take<bf16>(Sp * d.Mp);
     b.XsT_lo = ar.take<bf16>(Sp * d.Mp);
     b.xs = ar.take<float>(d.Mp * Sp);
-    b.Zf = ar.take<float>(d.Mp * d.Mp);
+    b.Zf = ar.take<float>(nb * d.Mp * d.Mp);
     b.sig = ar.take<double>(2 * static_cast<int64_t>(ntau) * Sp);
   }
   return b;
@@ -1158,24 +1139,28 @@ int sigma_run(const double *X, const Dims &d, const double *eps, double mu, cons
     launch_gather_cols_split_t(X, d.M, d.n, states, S, b.XsT_hi, b.XsT_lo, d.Mp, Sp, d.Mp, st);
     cudaMemsetAsync(b.sig, 0, sizeof(double) * 2 * ntau * Sp, st);
     SplitMat Dm{b.D_hi, b.D_lo, d.Mp, d.Ap, d.Ap};
-    SplitMat Wm{b.W_hi, b.W_lo, d.Ap, d.Ap, d.Ap};
-    SplitMat Um{b.U_hi, b.U_lo, d.Mp, d.Ap, d.Ap};
-    SplitMat Yo{b.Yo_hi, b.Yo_lo, d.Mp, d.Ko, d.Ko}, Yv{b.Yv_hi, b.Yv_lo, d.Mp, d.Kv, d.Kv};
-    SplitMat Hl{b.Hl_hi, b.Hl_lo, d.Mp, d.Mp, d.Mp}, Hg{b.Hg_hi, b.Hg_lo, d.Mp, d.Mp, d.Mp};
     SplitMat XsT{b.XsT_hi, b.XsT_lo, Sp, d.Mp, d.Mp};
-    for (int k = 0; k < ntau; ++k) {
-      launch_prep_branches(X, d.M, d.n, d.nocc, eps, mu, tau[k], b.Yo_hi, b.Yo_lo, d.Ko,
-                           b.Yv_hi, b.Yv_lo, d.Kv, d.Mp, st);
+    const int64_t m2 = d.Mp * d.Mp;
+    for (int k = 0; k < ntau; k += b.batch) {
+      const int nb = std::min(b.batch, ntau - k);
+      SplitMat Wm{b.W_hi, b.W_lo, nb * d.Ap, d.Ap, d.Ap};
+      SplitMat Um{b.U_hi, b.U_lo, nb * d.Mp, d.Ap, d.Ap};
+      SplitMat Yo{b.Yo_hi, b.Yo_lo, nb * d.Mp, d.Ko, d.Ko};
+      SplitMat Yv{b.Yv_hi, b.Yv_lo, nb * d.Mp, d.Kv, d.Kv};
+      SplitMat Hl{b.Hl_hi, b.Hl_lo, nb * d.Mp, d.Mp, d.Mp};
+      SplitMat Hg{b.Hg_hi, b.Hg_lo, nb * d.Mp, d.Mp, d.Mp};
+      launch_prep_branches<bf16>(X, d.M, d.n, d.nocc, eps, mu, tau_list(tau + k, nb), b.Yo_hi,
+                                 b.Yo_lo, d.Ko, b.Yv_hi, b.Yv_lo, d.Kv, d.Mp, st);
       umma::EpiArgs e;
       int rc = MBPT_OK;
       if (Wt) {
         // U = D Wt (Wt symmetric); without Wt, W = I and U = D
-        launch_split_pad<double>(Wt + k * a2, d.naux, d.naux, d.naux, 1.f, b.W_hi, b.W_lo,
-                                 d.Ap, d.Ap, d.Ap, false, st);
+        launch_split_pad_batch(Wt + k * a2, d.naux, d.naux, b.W_hi, b.W_lo, d.Ap, d.Ap, nb, st);
         e.out0_hi = b.U_hi;
         e.out0_lo = b.U_lo;
         e.ld_out = d.Ap;
-        rc = gemm_split(umma::EPI_SPLIT, 1, &Dm, &Wm, d.Mp, d.Ap, e, err, st);
+        rc = gemm_split(umma::EPI_SPLIT, 1, &Dm, &Wm, d.Mp, d.Ap, e, err, st, 0,
+                        {nb, {0, 0}, {d.Ap, 0}, d.Mp * d.Ap});
         if (rc) return rc;
       }
       // Zt = U D^T (= D W D^T, symmetric) whole in FP32: upper 256 x 256 tiles
@@ -1185,7 +1170,7 @@ int sigma_run(const double *X, const Dims &d, const double *eps, double mu, cons
       e.ld_outf = d.Mp;
       e.alpha = 1.f;
       rc = gemm_split(umma::EPI_F32, 1, Wt ? &Um : &Dm, &Dm, d.Mp, d.Mp, e, err, st,
-                      umma::BAND_UPPER);
+                      umma::BAND_UPPER, {nb, {Wt ? d.Mp : 0, 0}, {0, 0}, m2});
       if (rc) return rc;
       // G_occ, G_virt (short K) -> H< = G_occ o Zt, H> = G_virt o Zt; all four
       // symmetric: upper tiles, mirrored by the epilogue
@@ -1199,7 +1184,7 @@ int sigma_run(const double *X, const Dims &d, const double *eps, double mu, cons
       e.ld_zt = d.Mp;
       SplitMat A2g[2] = {Yo, Yv};
       rc = gemm_split(umma::EPI_SIGMA_HZ, 2, A2g, A2g, d.Mp, d.Mp, e, err, st,
-                      umma::BAND_UPPER);
+                      umma::BAND_UPPER, {nb, {d.Mp, d.Mp}, {d.Mp, d.Mp}, m2, m2});
       if (rc) return rc;
       // branch sums: sum_P X_s[P,p] (H X_s)[P,p]
       e = umma::EpiArgs();
@@ -1208,7 +1193,8 @@ int sigma_run(const double *X, const Dims &d, const double *eps, double mu, cons
       e.sig0 = b.sig + static_cast<int64_t>(k) * Sp;
       e.sig1 = b.sig + static_cast<int64_t>(ntau + k) * Sp;
       SplitMat A2[2] = {Hl, Hg}, B2[2] = {XsT, XsT};
-      rc = gemm_split(umma::EPI_ROWDOT2, 2, A2, B2, d.Mp, Sp, e, err, st);
+      rc = gemm_split(umma::EPI_ROWDOT2, 2, A2, B2, d.Mp, Sp, e, err, st, 0,
+                      {nb, {d.Mp, d.Mp}, {0, 0}, 0, 0, Sp});
       if (rc) return rc;
     }
     cudaMemcpy2DAsync(branch, sizeof(double) * S, b.sig, sizeof(double) * Sp,
@@ -1751,7 +1737,7 @@ int mbpt_sigma_ao(const double *X_ao, int64_t M, int64_t nao, const double *mo_c
   SplitMat Hl{b.Hl_hi, b.Hl_lo, d.Mp, d.Mp, d.Mp}, Hg{b.Hg_hi, b.Hg_lo, d.Mp, d.Mp, d.Mp};
   SplitMat XaT{b.XaT_hi, b.XaT_lo, naop, d.Mp, d.Mp}, RT{b.RT_hi, b.RT_lo, naop, d.Mp, d.Mp};
   for (int k = 0; k < ntau; ++k) {
-    launch_prep_branches(b.Xmo, M, norb, nocc, eps, mu, tau_host[k], b.Yo_hi, b.Yo_lo, d.Ko,
+    launch_prep_branches<bf16>(b.Xmo, M, norb, nocc, eps, mu, tau_list(tau_host + k, 1), b.Yo_hi, b.Yo_lo, d.Ko,
                          b.Yv_hi, b.Yv_lo, d.Kv, d.Mp, st);
     launch_split_pad<double>(Wt + k * a2, naux, naux, naux, 1.f, b.W_hi, b.W_lo, d.Ap, d.Ap,
                              d.Ap, false, st);

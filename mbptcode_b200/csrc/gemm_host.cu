@@ -67,17 +67,23 @@ bool make_tmap(CUtensorMap *m, const void *base, int64_t rows, int64_t cols, int
 // spans per pair.
 template <int NACC, int BN, int EPI, bool TF32, int DRAIN, int CTAS = 1>
 int launch(const SplitMat *A, const SplitMat *B, int64_t m_rows, int64_t n_rows,
-           const umma::EpiArgs &e, int *err, cudaStream_t st, int band = 0) {
+           const umma::EpiArgs &e, int *err, cudaStream_t st, const GemmBatch &batch,
+           int band = 0) {
   using L = umma::Layout<NACC, BN, (DRAIN > 0), CTAS>;
+  if (batch.n < 1 || batch.n > 65535) return MBPT_ERR_SHAPE;
   // the last column tile may overhang a multiple of 128 (BN = 256): its
   // B rows read as zeros and its dead columns are not stored
   if (m_rows % umma::BM || n_rows % 128 || m_rows <= 0 || n_rows <= 0) return MBPT_ERR_SHAPE;
   const int64_t bk = TF32 ? 32 : 64;
   umma::Params<NACC> p;
   for (int j = 0; j < NACC; ++j) {
-    if (A[j].cols != B[j].cols || A[j].cols <= 0 || A[j].rows < m_rows || B[j].rows < n_rows ||
-        A[j].tf32 != TF32 || B[j].tf32 != TF32)
+    if (A[j].cols != B[j].cols || A[j].cols <= 0 ||
+        A[j].rows < m_rows + (batch.n - 1) * batch.a_rows[j] ||
+        B[j].rows < n_rows + (batch.n - 1) * batch.b_rows[j] || A[j].tf32 != TF32 ||
+        B[j].tf32 != TF32 || A[j].rows > INT32_MAX || B[j].rows > INT32_MAX)
       return MBPT_ERR_SHAPE;
+    p.bs_a[j] = static_cast<int>(batch.a_rows[j]);
+    p.bs_b[j] = static_cast<int>(batch.b_rows[j]);
     if (!make_tmap(&p.tm[4 * j + 0], A[j].hi, A[j].rows, A[j].cols, A[j].ld, umma::BM, TF32) ||
         !make_tmap(&p.tm[4 * j + 1], A[j].lo, A[j].rows, A[j].cols, A[j].ld, umma::BM, TF32) ||
         !make_tmap(&p.tm[4 * j + 2], B[j].hi, B[j].rows, B[j].cols, B[j].ld, BN / CTAS,
@@ -91,6 +97,10 @@ int launch(const SplitMat *A, const SplitMat *B, int64_t m_rows, int64_t n_rows,
   p.n_valid = static_cast<int>(n_rows);
   p.m_valid = static_cast<int>(m_rows);
   p.band = band;
+  p.bs_out = batch.out;
+  p.bs_zt = batch.zt;
+  p.bs_sig = batch.sig;
+  p.skip = batch.skip;
   p.ngroups = 0;
   p.epi = e;
   p.err = err;
@@ -110,7 +120,8 @@ int launch(const SplitMat *A, const SplitMat *B, int64_t m_rows, int64_t n_rows,
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(static_cast<unsigned>(2 * ((p.tiles_m + 1) / 2) * p.tiles_n));
+    cfg.gridDim = dim3(static_cast<unsigned>(2 * ((p.tiles_m + 1) / 2) * p.tiles_n),
+                       static_cast<unsigned>(batch.n));
     cfg.blockDim = dim3(64 + BN);
     cfg.dynamicSmemBytes = L::kSmemBytes;
     cfg.stream = st;
@@ -120,7 +131,8 @@ int launch(const SplitMat *A, const SplitMat *B, int64_t m_rows, int64_t n_rows,
     if (timed) timing_end(st, EPI, ev0, ev1);
     return rc == cudaSuccess ? MBPT_OK : MBPT_ERR_CUDA;
   } else {
-    kern<<<p.tiles_m * p.tiles_n, 64 + BN, L::kSmemBytes, st>>>(p);
+    kern<<<dim3(static_cast<unsigned>(p.tiles_m * p.tiles_n), static_cast<unsigned>(batch.n)),
+           64 + BN, L::kSmemBytes, st>>>(p);
     if (timed) timing_end(st, EPI, ev0, ev1);
     return cudaGetLastError() == cudaSuccess ? MBPT_OK : MBPT_ERR_CUDA;
   }
@@ -140,8 +152,13 @@ constexpr int kMaxGroups = 32;
 // and stores nothing (each group's m_valid / n_valid).
 template <int EPI, int DRAIN, int BN = 128, int CTAS = 1>
 int launch_grouped(const SplitMat &A, const SplitMat &B, const GemmGroup *g, int ng,
-                   const umma::EpiArgs &e, int *err, cudaStream_t st, int band) {
+                   const umma::EpiArgs &e, int *err, cudaStream_t st, int band,
+                   const GemmBatch &batch) {
   using L = umma::Layout<1, BN, (DRAIN > 0), CTAS>;
+  if (batch.n < 1 || batch.n > 65535 || A.rows > INT32_MAX || B.rows > INT32_MAX)
+    return MBPT_ERR_SHAPE;
+  const int64_t ra = A.rows - (batch.n - 1) * batch.a_rows[0];  // rows of one member
+  const int64_t rb = B.rows - (batch.n - 1) * batch.b_rows[0];
   if (!A.tf32 || !B.tf32 || ng < 1 || ng > kMaxGroups) return MBPT_ERR_SHAPE;
   umma::Params<1, kMaxGroups> p;
   if (!make_tmap(&p.tm[0], A.hi, A.rows, A.cols, A.ld, umma::BM, true) ||
@@ -156,7 +173,7 @@ int launch_grouped(const SplitMat &A, const SplitMat &B, const GemmGroup *g, int
     // every block inside its array, K origins on 32-element slabs
     if (q.m_rows <= 0 || q.n_rows <= 0 || q.m_rows % umma::BM || q.n_rows % 128 || q.k <= 0 ||
         q.a_k0 % 32 || q.b_k0 % 32 || q.a_row0 < 0 || q.b_row0 < 0 ||
-        q.a_row0 + q.m_rows > A.rows || q.b_row0 + q.n_rows > B.rows ||
+        q.a_row0 + q.m_rows > ra || q.b_row0 + q.n_rows > rb ||
         q.a_k0 + kp > A.cols || q.b_k0 + kp > B.cols)
       return MBPT_ERR_SHAPE;
     umma::Group &G = p.grp[i];
@@ -176,6 +193,11 @@ int launch_grouped(const SplitMat &A, const SplitMat &B, const GemmGroup *g, int
     tiles += (CTAS == 2 ? (G.tiles_m + 1) / 2 : G.tiles_m) * G.tiles_n;
   }
   p.ngroups = ng;
+  p.bs_a[0] = static_cast<int>(batch.a_rows[0]);
+  p.bs_b[0] = static_cast<int>(batch.b_rows[0]);
+  p.bs_out = batch.out;
+  p.bs_zt = p.bs_sig = 0;
+  p.skip = batch.skip;
   p.k_tiles[0] = 0;
   p.tiles_m = p.tiles_n = 0;
   p.n_valid = 1 << 30;
@@ -198,7 +220,7 @@ int launch_grouped(const SplitMat &A, const SplitMat &B, const GemmGroup *g, int
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(static_cast<unsigned>(2 * tiles));
+    cfg.gridDim = dim3(static_cast<unsigned>(2 * tiles), static_cast<unsigned>(batch.n));
     cfg.blockDim = dim3(64 + BN);
     cfg.dynamicSmemBytes = L::kSmemBytes;
     cfg.stream = st;
@@ -206,7 +228,8 @@ int launch_grouped(const SplitMat &A, const SplitMat &B, const GemmGroup *g, int
     cfg.numAttrs = 1;
     rc = cudaLaunchKernelEx(&cfg, kern, p);
   } else {
-    kern<<<tiles, 64 + BN, L::kSmemBytes, st>>>(p);
+    kern<<<dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(batch.n)), 64 + BN,
+           L::kSmemBytes, st>>>(p);
     rc = cudaGetLastError();
   }
   if (timed) timing_end(st, EPI, ev0, ev1);
@@ -217,7 +240,7 @@ int launch_grouped(const SplitMat &A, const SplitMat &B, const GemmGroup *g, int
 
 int gemm_split_grouped(int epi, const SplitMat &A, const SplitMat &B, const GemmGroup *groups,
                        int ngroups, const umma::EpiArgs &e, int *err, cudaStream_t st,
-                       int band) {
+                       int band, const GemmBatch &batch) {
   constexpr int kDrain = 2;
   for (int first = 0; first < ngroups; first += kMaxGroups) {
     const int ng = std::min(kMaxGroups, ngroups - first);
@@ -225,9 +248,9 @@ int gemm_split_grouped(int epi, const SplitMat &A, const SplitMat &B, const Gemm
     if (epi == umma::EPI_TF32_PAIR)
       rc = engine_pairs()
                ? launch_grouped<umma::EPI_TF32_PAIR, kDrain, 256, 2>(A, B, groups + first, ng, e,
-                                                                     err, st, band)
+                                                                     err, st, band, batch)
                : launch_grouped<umma::EPI_TF32_PAIR, kDrain>(A, B, groups + first, ng, e, err,
-                                                             st, band);
+                                                             st, band, batch);
     if (rc) return rc;
   }
   return MBPT_OK;
@@ -339,7 +362,8 @@ int gemm_timing(int enable, double *total_ms, long long *launches) {
 }
 
 int gemm_split(int epi, int nacc, const SplitMat *A, const SplitMat *B, int64_t m_rows,
-               int64_t n_rows, const umma::EpiArgs &e, int *err, cudaStream_t st, int band) {
+               int64_t n_rows, const umma::EpiArgs &e, int *err, cudaStream_t st, int band,
+               const GemmBatch &batch) {
   using namespace umma;
   // K slabs per drained chunk of the last accumulator: 24 accumulation steps
   // (~1e-6 relative truncation bias, against ~4e-5 for an undrained K = 7296)
@@ -354,30 +378,30 @@ int gemm_split(int epi, int nacc, const SplitMat *A, const SplitMat *B, int64_t 
         // other reuses one of its TMEM buffers; the Hadamard is symmetric
         const SplitMat A2[2] = {A[1], A[0]}, B2[2] = {B[1], B[0]};
         return launch<2, 256, EPI_HADAMARD_SPLIT, true, kDrain, 2>(A2, B2, m_rows, n_rows, e,
-                                                                   err, st, band);
+                                                                   err, st, batch, band);
       }
       return launch<2, 128, EPI_HADAMARD_SPLIT, true, kDrain>(A, B, m_rows, n_rows, e, err, st,
-                                                              band);
+                                                              batch, band);
     }
     if (!tf && nacc == 1 && epi == EPI_F32)
       return engine_pairs()
                  ? launch<1, 256, EPI_F32, false, kDrain, 2>(A, B, m_rows, n_rows, e, err, st,
-                                                            band)
+                                                            batch, band)
                  : launch<1, 256, EPI_F32, false, kDrain>(A, B, m_rows, n_rows, e, err, st,
-                                                         band);
+                                                         batch, band);
     // the two G products of Sigma's H (short K: not drained) against a stored Zt
     if (!tf && nacc == 2 && epi == EPI_SIGMA_HZ)
       return engine_pairs()
                  ? launch<2, 256, EPI_SIGMA_HZ, false, 0, 2>(A, B, m_rows, n_rows, e, err, st,
-                                                            band)
+                                                            batch, band)
                  : launch<2, 256, EPI_SIGMA_HZ, false, 0>(A, B, m_rows, n_rows, e, err, st,
-                                                         band);
+                                                         batch, band);
     if (!tf && nacc == 1 && epi == EPI_F64_SYM)
       return engine_pairs()
                  ? launch<1, 256, EPI_F64_SYM, false, kDrain, 2>(A, B, m_rows, n_rows, e, err,
-                                                                st, band)
+                                                                st, batch, band)
                  : launch<1, 256, EPI_F64_SYM, false, kDrain>(A, B, m_rows, n_rows, e, err, st,
-                                                             band);
+                                                             batch, band);
     return MBPT_ERR_UNSUPPORTED;
   }
   if (band) {
@@ -388,45 +412,45 @@ int gemm_split(int epi, int nacc, const SplitMat *A, const SplitMat *B, int64_t 
     if ((band & BAND_UPPER) && m_rows != n_rows) return MBPT_ERR_SHAPE;
     if (epi == EPI_TF32_PAIR)
       return launch<1, 128, EPI_TF32_PAIR, true, kDrain>(A, B, m_rows, n_rows, e, err, st,
-                                                         band);
+                                                         batch, band);
     // the symmetric FP64 store (W = L^-T L^-1): 128 x 256 tiles, which halve
     // the A reads through shared memory for the three TF32 products
     if (epi == EPI_F64_SYM && (band & BAND_UPPER))
       return engine_pairs()
                  ? launch<1, 256, EPI_F64_SYM, true, kDrain, 2>(A, B, m_rows, n_rows, e, err,
-                                                               st, band)
+                                                               st, batch, band)
                  : launch<1, 256, EPI_F64_SYM, true, kDrain>(A, B, m_rows, n_rows, e, err, st,
-                                                            band);
+                                                            batch, band);
     if (epi == EPI_F64_SYM)
-      return launch<1, 128, EPI_F64_SYM, true, kDrain>(A, B, m_rows, n_rows, e, err, st, band);
-    return launch<1, 128, EPI_F32, true, kDrain>(A, B, m_rows, n_rows, e, err, st, band);
+      return launch<1, 128, EPI_F64_SYM, true, kDrain>(A, B, m_rows, n_rows, e, err, st, batch, band);
+    return launch<1, 128, EPI_F32, true, kDrain>(A, B, m_rows, n_rows, e, err, st, batch, band);
   }
   if (tf) {
     if (nacc == 2 && epi == EPI_HADAMARD_SPLIT)
-      return launch<2, 128, EPI_HADAMARD_SPLIT, true, kDrain>(A, B, m_rows, n_rows, e, err, st);
+      return launch<2, 128, EPI_HADAMARD_SPLIT, true, kDrain>(A, B, m_rows, n_rows, e, err, st, batch);
     if (nacc == 1 && epi == EPI_F32)
-      return launch<1, 128, EPI_F32, true, kDrain>(A, B, m_rows, n_rows, e, err, st);
+      return launch<1, 128, EPI_F32, true, kDrain>(A, B, m_rows, n_rows, e, err, st, batch);
     if (nacc == 1 && epi == EPI_TF32_PAIR)
-      return launch<1, 128, EPI_TF32_PAIR, true, kDrain>(A, B, m_rows, n_rows, e, err, st);
+      return launch<1, 128, EPI_TF32_PAIR, true, kDrain>(A, B, m_rows, n_rows, e, err, st, batch);
     return MBPT_ERR_UNSUPPORTED;
   }
   // the non-symmetric N^3 products: 128 x 256 tiles (a quarter fewer operand
   // bytes per flop through the shared-memory ring than 128 x 128)
   if (nacc == 1 && epi == EPI_SPLIT)
     return engine_pairs()
-               ? launch<1, 256, EPI_SPLIT, false, kDrain, 2>(A, B, m_rows, n_rows, e, err, st)
-               : launch<1, 256, EPI_SPLIT, false, kDrain>(A, B, m_rows, n_rows, e, err, st);
+               ? launch<1, 256, EPI_SPLIT, false, kDrain, 2>(A, B, m_rows, n_rows, e, err, st, batch)
+               : launch<1, 256, EPI_SPLIT, false, kDrain>(A, B, m_rows, n_rows, e, err, st, batch);
   if (nacc == 1 && epi == EPI_F32)
-    return launch<1, 128, EPI_F32, false, kDrain>(A, B, m_rows, n_rows, e, err, st);
+    return launch<1, 128, EPI_F32, false, kDrain>(A, B, m_rows, n_rows, e, err, st, batch);
   if (nacc == 1 && epi == EPI_F32_ACC)
-    return launch<1, 128, EPI_F32_ACC, false, kDrain>(A, B, m_rows, n_rows, e, err, st);
+    return launch<1, 128, EPI_F32_ACC, false, kDrain>(A, B, m_rows, n_rows, e, err, st, batch);
   if (nacc == 2 && epi == EPI_HADAMARD_SPLIT)
-    return launch<2, 128, EPI_HADAMARD_SPLIT, false, kDrain>(A, B, m_rows, n_rows, e, err, st);
+    return launch<2, 128, EPI_HADAMARD_SPLIT, false, kDrain>(A, B, m_rows, n_rows, e, err, st, batch);
   // the row contraction: two undrained accumulators, 256-wide on CTA pairs
   if (nacc == 2 && epi == EPI_ROWDOT2)
     return engine_pairs()
-               ? launch<2, 256, EPI_ROWDOT2, false, 0, 2>(A, B, m_rows, n_rows, e, err, st)
-               : launch<2, 128, EPI_ROWDOT2, false, 0>(A, B, m_rows, n_rows, e, err, st);
+               ? launch<2, 256, EPI_ROWDOT2, false, 0, 2>(A, B, m_rows, n_rows, e, err, st, batch)
+               : launch<2, 128, EPI_ROWDOT2, false, 0>(A, B, m_rows, n_rows, e, err, st, batch);
   return MBPT_ERR_UNSUPPORTED;
 }
 

@@ -18,12 +18,23 @@ struct SplitMat {
   bool tf32 = false;
 };
 
+// Several products of one shape in one launch: member b reads A[j] from row b
+// a_rows[j] and B[j] from row b b_rows[j] of the stacked operands (0: shared), and
+// writes its outputs b out elements further on (zt, sig likewise). skip: device
+// words, one per member; a member whose word is not zero is left out.
+struct GemmBatch {
+  int n = 1;
+  int64_t a_rows[2] = {0, 0}, b_rows[2] = {0, 0};
+  int64_t out = 0, zt = 0, sig = 0;
+  const int *skip = nullptr;
+};
+
 // C (m_rows x n_rows tile grid, both multiples of 128) from nacc problems
 // A[j] B[j]^T with the fused epilogue `epi`. band: umma::Band flags of
 // triangular operands (the TF32 single-product FP32 store only).
 int gemm_split(int epi, int nacc, const SplitMat *A, const SplitMat *B, int64_t m_rows,
                int64_t n_rows, const umma::EpiArgs &e, int *err, cudaStream_t st,
-               int band = 0);
+               int band = 0, const GemmBatch &batch = GemmBatch());
 
 // One product of a grouped launch: an m_rows x n_rows output block (multiples
 // of 128) from the A rows [a_row0, +m_rows) and B rows [b_row0, +n_rows), K
@@ -38,7 +49,7 @@ struct GemmGroup {
 // as few launches as possible (up to 32 per launch); EPI_TF32_PAIR only.
 int gemm_split_grouped(int epi, const SplitMat &A, const SplitMat &B, const GemmGroup *groups,
                        int ngroups, const umma::EpiArgs &e, int *err, cudaStream_t st,
-                       int band = 0);
+                       int band = 0, const GemmBatch &batch = GemmBatch());
 
 // The engine's bounded barrier wait on a barrier that is (arrive = 1) or is
 // never (arrive = 0) completed, giving up after limit_us microseconds.
@@ -121,14 +132,6 @@ template <typename T>
 void launch_split_pad(const T *src, int64_t rows, int64_t cols, int64_t ld_src, float scale,
                       bf16 *hi, bf16 *lo, int64_t ld_dst, int64_t rows_p, int64_t cols_p,
                       bool transpose, cudaStream_t st);
-void launch_prep_branches(const double *X, int64_t M, int64_t n, int64_t nocc,
-                          const double *eps, double mu, double tau, bf16 *o_hi, bf16 *o_lo,
-                          int64_t ld_o, bf16 *v_hi, bf16 *v_lo, int64_t ld_v, int64_t Mp,
-                          cudaStream_t st);
-void launch_prep_branches_tf32(const double *X, int64_t M, int64_t n, int64_t nocc,
-                               const double *eps, double mu, double tau, float *o_hi,
-                               float *o_lo, int64_t ld_o, float *v_hi, float *v_lo,
-                               int64_t ld_v, int64_t Mp, cudaStream_t st);
 void launch_split_pad_colscale(const double *src, int64_t rows, int64_t cols, int64_t ld_src,
                                const double *f, double s, bf16 *hi, bf16 *lo, int64_t ld_dst,
                                int64_t rows_p, int64_t cols_p, cudaStream_t st);
@@ -144,6 +147,16 @@ struct TauList {
   double t[kMaxTauBatch];
   int n;
 };
+// `batch` rows x cols matrices, one after the other, as BF16 pairs zero-padded
+// to rows_p x cols_p each
+void launch_split_pad_batch(const double *src, int64_t rows, int64_t cols, bf16 *hi, bf16 *lo,
+                            int64_t rows_p, int64_t cols_p, int batch, cudaStream_t st);
+// Y_o (n taus x Mp x ld_o) and Y_v (n taus x Mp x ld_v) as BF16 or TF32 pairs
+template <typename T>
+void launch_prep_branches(const double *X, int64_t M, int64_t n, int64_t nocc,
+                          const double *eps, double mu, const TauList &taus, T *o_hi, T *o_lo,
+                          int64_t ld_o, T *v_hi, T *v_lo, int64_t ld_v, int64_t Mp,
+                          cudaStream_t st);
 // Xo_s (n taus x M x nocc) and Xv_s (n taus x M x (norb - nocc)), power 1
 void launch_scaled_branches_batch(const double *X, int64_t M, int64_t n, int64_t nocc,
                                   const double *eps, double mu, const TauList &taus,

@@ -94,6 +94,12 @@ struct Params {
   int n_valid;  // output columns to store (tiles_n * BN unless the last tile overhangs)
   int m_valid;  // output rows to store (a CTA pair's second tile may lie past them)
   int band;  // Band flags (0: dense)
+  // batch member b (blockIdx.y): its rows of A and B start b bs rows further
+  // down (0: an operand of all members), its outputs b bs_out elements, its
+  // zt b bs_zt and its sig sums b bs_sig elements further on
+  int bs_a[NACC], bs_b[NACC];
+  int64_t bs_out, bs_zt, bs_sig;
+  const int *skip;  // members whose word here is not zero are left out (null: none)
   int ngroups;
   Group grp[NGRP > 0 ? NGRP : 1];
   EpiArgs epi;
@@ -460,6 +466,8 @@ __global__ void __launch_bounds__(64 + BN, 1)
   // rank in the pair (0 issues the MMAs); 0 without pairs
   const uint32_t rank = kPair ? cluster_rank() : 0u;
   const bool leader = rank == 0;
+  const int by = static_cast<int>(blockIdx.y);
+  const int64_t ob = by * p.bs_out;
   // this CTA's product (grouped launches) and its origins
   int pid = kPair ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
   int tiles_m = p.tiles_m, tiles_n = p.tiles_n;
@@ -478,8 +486,8 @@ __global__ void __launch_bounds__(64 + BN, 1)
     b_row0 = G.b_row0;
     b_k0 = G.b_k0;
     grp_k_tiles = G.k_tiles;
-    p_off = G.p_off;
-    t_off = G.t_off;
+    p_off = G.p_off + ob;
+    t_off = G.t_off + ob;
     m_valid = G.m_valid;
     n_valid = G.n_valid;
   }
@@ -507,6 +515,7 @@ __global__ void __launch_bounds__(64 + BN, 1)
   // a symmetric product skips tiles whose last 128-column block lies below
   // the diagonal
   if ((p.band & BAND_UPPER) && (n0 + BN) / 128 - 1 < tm_pair) return;
+  if (p.skip && p.skip[by] != 0) return;
   // K slabs [kb, ke) of accumulator j that can hold nonzeros for this tile (a
   // pair's: both CTAs run its rows' span; the slabs one CTA adds are zeros)
   constexpr int kSlab = TF32 ? 32 : BK;
@@ -569,6 +578,7 @@ __global__ void __launch_bounds__(64 + BN, 1)
       for (int j = 0; j < NACC && ok; ++j) {
         int kb, ke;
         k_span(j, kb, ke);
+        const int ya = a_row0 + by * p.bs_a[j] + m0, yb = b_row0 + by * p.bs_b[j] + n0;
         for (int kt = kb; kt < ke; ++kt, ++it) {
           const int s = it % L::kStages;
           const uint32_t ph = (it / L::kStages) & 1;
@@ -581,19 +591,18 @@ __global__ void __launch_bounds__(64 + BN, 1)
           const int kx = kt * kSlab;
           if constexpr (kPair) {
             const uint32_t bar = cluster_addr(&full[s], 0);
-            const int nb = b_row0 + n0 + static_cast<int>(rank) * (BN / 2);
-            tma_load_2d_pair(st, &p.tm[4 * j + 0], a_k0 + kx, a_row0 + m0, bar);
-            tma_load_2d_pair(st + L::kABytes, &p.tm[4 * j + 1], a_k0 + kx, a_row0 + m0, bar);
+            const int nb = yb + static_cast<int>(rank) * (BN / 2);
+            tma_load_2d_pair(st, &p.tm[4 * j + 0], a_k0 + kx, ya, bar);
+            tma_load_2d_pair(st + L::kABytes, &p.tm[4 * j + 1], a_k0 + kx, ya, bar);
             tma_load_2d_pair(st + 2 * L::kABytes, &p.tm[4 * j + 2], b_k0 + kx, nb, bar);
             tma_load_2d_pair(st + 2 * L::kABytes + L::kBBytes, &p.tm[4 * j + 3], b_k0 + kx, nb,
                              bar);
           } else {
-            tma_load_2d(st, &p.tm[4 * j + 0], a_k0 + kx, a_row0 + m0, &full[s]);
-            tma_load_2d(st + L::kABytes, &p.tm[4 * j + 1], a_k0 + kx, a_row0 + m0, &full[s]);
-            tma_load_2d(st + 2 * L::kABytes, &p.tm[4 * j + 2], b_k0 + kx, b_row0 + n0,
+            tma_load_2d(st, &p.tm[4 * j + 0], a_k0 + kx, ya, &full[s]);
+            tma_load_2d(st + L::kABytes, &p.tm[4 * j + 1], a_k0 + kx, ya, &full[s]);
+            tma_load_2d(st + 2 * L::kABytes, &p.tm[4 * j + 2], b_k0 + kx, yb, &full[s]);
+            tma_load_2d(st + 2 * L::kABytes + L::kBBytes, &p.tm[4 * j + 3], b_k0 + kx, yb,
                         &full[s]);
-            tma_load_2d(st + 2 * L::kABytes + L::kBBytes, &p.tm[4 * j + 3], b_k0 + kx,
-                        b_row0 + n0, &full[s]);
           }
         }
       }
@@ -784,9 +793,10 @@ __global__ void __launch_bounds__(64 + BN, 1)
         if constexpr (EPI == EPI_SPLIT) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) v0[i] *= e.alpha;
-          store_split32(e.out0_hi + row * e.ld_out + col, e.out0_lo + row * e.ld_out + col, v0);
+          store_split32(e.out0_hi + ob + row * e.ld_out + col,
+                        e.out0_lo + ob + row * e.ld_out + col, v0);
         } else if constexpr (EPI == EPI_F32 || EPI == EPI_F32_ACC) {
-          float4 *dst = reinterpret_cast<float4 *>(e.outf + row * e.ld_outf + col);
+          float4 *dst = reinterpret_cast<float4 *>(e.outf + ob + row * e.ld_outf + col);
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             float4 o = make_float4(e.alpha * v0[4 * q], e.alpha * v0[4 * q + 1],
@@ -801,19 +811,19 @@ __global__ void __launch_bounds__(64 + BN, 1)
             if (mirror) {
 #pragma unroll
               for (int i = 0; i < 32; ++i)
-                e.outf[static_cast<int64_t>(col + i) * e.ld_outf + row] = e.alpha * v0[i];
+                e.outf[ob + static_cast<int64_t>(col + i) * e.ld_outf + row] = e.alpha * v0[i];
             }
           }
         } else if constexpr (EPI == EPI_F64_SYM) {
           if (row < e.nd) {
-            double *dst = e.outd + static_cast<int64_t>(row) * e.ld_outd + col;
+            double *dst = e.outd + ob + static_cast<int64_t>(row) * e.ld_outd + col;
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
               if (col + i < e.nd) {
                 const double v = static_cast<double>(e.alpha * v0[i]) -
                                  (row == col + i ? e.shift : 0.0);
                 dst[i] = v;
-                if (mirror) e.outd[static_cast<int64_t>(col + i) * e.ld_outd + row] = v;
+                if (mirror) e.outd[ob + static_cast<int64_t>(col + i) * e.ld_outd + row] = v;
               }
             }
           }
@@ -846,14 +856,17 @@ __global__ void __launch_bounds__(64 + BN, 1)
           load(1, c, v1);
 #pragma unroll
           for (int i = 0; i < 32; ++i) v0[i] *= v1[i];
-          store_split32(e.out0_hi + row * e.ld_out + col, e.out0_lo + row * e.ld_out + col, v0);
+          store_split32(e.out0_hi + ob + row * e.ld_out + col,
+                        e.out0_lo + ob + row * e.ld_out + col, v0);
           if (mirror)
-            store_split32_t(e.out0_hi + static_cast<int64_t>(col) * e.ld_out + row,
-                            e.out0_lo + static_cast<int64_t>(col) * e.ld_out + row, e.ld_out, v0);
+            store_split32_t(e.out0_hi + ob + static_cast<int64_t>(col) * e.ld_out + row,
+                            e.out0_lo + ob + static_cast<int64_t>(col) * e.ld_out + row,
+                            e.ld_out, v0);
         } else if constexpr (EPI == EPI_SIGMA_HZ) {
           // acc0 = G_occ, acc1 = G_virt; Zt (symmetric, stored whole) from memory
           float z[32], v1[32];
-          const float4 *zs = reinterpret_cast<const float4 *>(e.zt + row * e.ld_zt + col);
+          const float4 *zs =
+              reinterpret_cast<const float4 *>(e.zt + by * p.bs_zt + row * e.ld_zt + col);
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             const float4 t = zs[q];
@@ -861,17 +874,21 @@ __global__ void __launch_bounds__(64 + BN, 1)
           }
 #pragma unroll
           for (int i = 0; i < 32; ++i) v0[i] *= z[i];
-          store_split32(e.out0_hi + row * e.ld_out + col, e.out0_lo + row * e.ld_out + col, v0);
+          store_split32(e.out0_hi + ob + row * e.ld_out + col,
+                        e.out0_lo + ob + row * e.ld_out + col, v0);
           if (mirror)
-            store_split32_t(e.out0_hi + static_cast<int64_t>(col) * e.ld_out + row,
-                            e.out0_lo + static_cast<int64_t>(col) * e.ld_out + row, e.ld_out, v0);
+            store_split32_t(e.out0_hi + ob + static_cast<int64_t>(col) * e.ld_out + row,
+                            e.out0_lo + ob + static_cast<int64_t>(col) * e.ld_out + row,
+                            e.ld_out, v0);
           load(1, c, v1);
 #pragma unroll
           for (int i = 0; i < 32; ++i) v1[i] *= z[i];
-          store_split32(e.out1_hi + row * e.ld_out + col, e.out1_lo + row * e.ld_out + col, v1);
+          store_split32(e.out1_hi + ob + row * e.ld_out + col,
+                        e.out1_lo + ob + row * e.ld_out + col, v1);
           if (mirror)
-            store_split32_t(e.out1_hi + static_cast<int64_t>(col) * e.ld_out + row,
-                            e.out1_lo + static_cast<int64_t>(col) * e.ld_out + row, e.ld_out, v1);
+            store_split32_t(e.out1_hi + ob + static_cast<int64_t>(col) * e.ld_out + row,
+                            e.out1_lo + ob + static_cast<int64_t>(col) * e.ld_out + row,
+                            e.ld_out, v1);
         } else if constexpr (EPI == EPI_ROWDOT2) {
           float v1[32], xs[32];
           load(1, c, v1);
@@ -888,8 +905,8 @@ __global__ void __launch_bounds__(64 + BN, 1)
           }
           const float s0 = warp_column_sum(v0, lane);
           const float s1 = warp_column_sum(v1, lane);
-          atomicAdd(e.sig0 + col + lane, static_cast<double>(s0));
-          atomicAdd(e.sig1 + col + lane, -static_cast<double>(s1));
+          atomicAdd(e.sig0 + by * p.bs_sig + col + lane, static_cast<double>(s0));
+          atomicAdd(e.sig1 + by * p.bs_sig + col + lane, -static_cast<double>(s1));
         }
       }
     }
