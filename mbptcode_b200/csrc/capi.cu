@@ -60,8 +60,6 @@ void launch_row_scale_acc(const double *a, int64_t lda, int64_t p, const double 
                           int64_t nc, double *out, cudaStream_t st);
 void launch_row_dot_into_col(const double *G, const double *X, int64_t nr, int64_t nc,
                              double *out, int64_t ldo, int64_t p, cudaStream_t st);
-void launch_chol_copy_panel(const double *A, int64_t n, int64_t j0, int64_t m, int nbj,
-                            int nmat, bool one_minus, double *P, cudaStream_t st);
 int launch_chol_diag_block(const double *P, int64_t m, int nbj, double *A, int64_t n,
                            int64_t j0, int nmat, double *Linv, int *info, cudaStream_t st);
 void launch_sigma_back_gather(const double *X, int64_t M, int64_t n, const int64_t *states,
@@ -534,7 +532,7 @@ constexpr int kBatchedCholMin = 4;  // frequencies from which the batch beats on
 // upper triangle keeps A_f; info_f as potrf reports it). Per 128-column step
 // j0, for all matrices in one launch each: the block column P = (I - A)[j0:, j0:j0+nb]
 // - L[j0:, :j0] L[j0:j0+nb, :j0]^T, formed where A is first read (one FP64 tensor-core
-// kernel, or a copy and the int8 update), its diagonal block factorised and
+// kernel, or the int8 update), its diagonal block factorised and
 // inverted in shared memory, and the panel below it formed by a second
 // product, L[j0+nb:, j0-block] = P_below L_jj^-T. Every launch carries
 // the whole batch, so the latency-bound diagonal blocks cost one launch per
@@ -551,44 +549,43 @@ struct OzakiChol {
   int *err = nullptr;
 };
 
-int chol_batched(double *A, int64_t n, int nmat, int *info, double *P, double *Linv,
-                 cudaStream_t st, int64_t linv_step_stride, const OzakiChol *oz) {
-  const bool ozaki = oz && oz->planes;
-  if (ozaki) {
-    int rc = ozaki_chol_scales(A, n, nmat, oz->scale, oz->rowsq, true, st);
-    if (rc) return rc;
-  }
-  for (int64_t j0 = 0; j0 < n; j0 += kCholNb) {
-    const int nbj = static_cast<int>(std::min<int64_t>(kCholNb, n - j0));
-    const int64_t m = n - j0;
-    if (ozaki) {
-      launch_chol_copy_panel(A, n, j0, m, nbj, nmat, true, P, st);
-      int rc = ozaki_chol_update(A, n, nmat, j0, nbj, P, oz->scale, oz->planes, oz->slices,
-                                 oz->rowsq, oz->err, st);
-      if (rc) return rc;
-    } else {
-      int rc = dmma::chol_update(A, n, j0, nbj, P, nmat, st);
-      if (rc) return rc;
-    }
-    double *Lj = Linv + (j0 / kCholNb) * linv_step_stride;
-    int rc = launch_chol_diag_block(P, m, nbj, A, n, j0, nmat, Lj, info, st);
-    if (rc) return rc;
-    const int64_t mb = m - nbj;
-    // row-major: U[j0:j0+nbj, j0+nbj:] = L_jj^-1 P[:, nbj:]
-    if (mb > 0) {
-      rc = dmma::gemm({Lj, kCholNb, static_cast<int64_t>(kCholNb) * kCholNb}, false,
-                      {P + nbj, m, m * nbj}, false, nbj, mb, nbj, 1.0, 0.0,
-                      A + j0 * n + j0 + nbj, n, n * n, nmat, false, st);
-      if (rc) return rc;
-    }
-    // the block column is final: cut it into digit planes for the later steps
-    if (ozaki && j0 + nbj < n) {
-      int rc2 = ozaki_chol_slice(A, n, nmat, j0, nbj, oz->scale, oz->planes, oz->slices,
-                                 oz->rowsq, st);
-      if (rc2) return rc2;
-    }
-  }
-  return cudaGetLastError() == cudaSuccess ? MBPT_OK : MBPT_ERR_CUDA;
+// One group of matrices of the batch, on its own stream.
+struct CholGroup {
+  double *A;
+  int nmat;
+  int *info;
+  double *P, *Linv;
+  cudaStream_t st;
+  OzakiChol oz;
+};
+
+// The step at column j0 of one group (j0 = 0 also sets the row scales).
+int chol_step(const CholGroup &g, int64_t n, int64_t j0, int64_t linv_step_stride) {
+  const bool ozaki = g.oz.planes != nullptr;
+  const int nbj = static_cast<int>(std::min<int64_t>(kCholNb, n - j0));
+  const int64_t m = n - j0, mb = m - nbj;
+  int rc = MBPT_OK;
+  if (ozaki && j0 == 0)
+    rc = ozaki_chol_scales(g.A, n, g.nmat, g.oz.scale, g.oz.rowsq, true, g.st);
+  if (rc) return rc;
+  if (ozaki && j0 > 0)
+    rc = ozaki_chol_update(g.A, n, g.nmat, j0, nbj, g.P, g.oz.scale, g.oz.planes, g.oz.slices,
+                           g.oz.rowsq, g.oz.err, g.st);
+  else
+    rc = dmma::chol_update(g.A, n, j0, nbj, g.P, g.nmat, g.st);
+  if (rc) return rc;
+  double *Lj = g.Linv + (j0 / kCholNb) * linv_step_stride;
+  rc = launch_chol_diag_block(g.P, m, nbj, g.A, n, j0, g.nmat, Lj, g.info, g.st);
+  if (rc || mb == 0) return rc;
+  // row-major: U[j0:j0+nbj, j0+nbj:] = L_jj^-1 P[:, nbj:]
+  rc = dmma::gemm({Lj, kCholNb, static_cast<int64_t>(kCholNb) * kCholNb}, false,
+                  {g.P + nbj, m, m * nbj}, false, nbj, mb, nbj, 1.0, 0.0,
+                  g.A + j0 * n + j0 + nbj, n, n * n, g.nmat, false, g.st);
+  // the block column is final: cut it into digit planes for the later steps
+  if (!rc && ozaki)
+    rc = ozaki_chol_slice(g.A, n, g.nmat, j0, nbj, g.oz.scale, g.oz.planes, g.oz.slices,
+                          g.oz.rowsq, g.st);
+  return rc;
 }
 
 // The batched Cholesky's trailing updates: on the int8 tensor cores (the
@@ -637,6 +634,18 @@ bool batched_chol_enabled(int nfreq) {
     return e ? std::atoi(e) : 1;
   }();
   return env != 0 && nfreq >= kBatchedCholMin;
+}
+
+// Groups of the batched factorisation where MBPT_DYSON_CHOL_GROUPS names none.
+// A few steps of small products cannot hide each other's diagonal blocks, and
+// each further group is five more launches a step: 20 matrices of 141 rows
+// take 0.21 ms (with W) in one group, 0.25 in four; 24 of 786 rows (mixed)
+// 1.27, 1.24, 1.24 and 1.34 in 1, 2, 4 and 6; 24 of 2400 rows 8.25, 7.82,
+// 7.71 and 7.61; of 5400 rows 44.0, 42.4, 42.2 and 42.3.
+constexpr int kMostCholGroups = 6;
+int chol_groups(int64_t n, int asked) {
+  if (asked > 0) return asked;
+  return n <= 384 ? 1 : (n <= 1024 ? 2 : 4);
 }
 
 struct DysonBufs {
@@ -722,9 +731,9 @@ struct DysonPipe {
   cusolverDnHandle_t solver2 = nullptr;
   cudaEvent_t fork = nullptr, join2 = nullptr;
   int nfac = 1;
-  // groups of the batched factorisation (MBPT_DYSON_CHOL_GROUPS, default 4):
-  // group 0 on the caller's stream, group 1 on fac2, the rest on these
-  int groups = 2;
+  // groups of the batched factorisation as MBPT_DYSON_CHOL_GROUPS asks (0: by
+  // size): group 0 on the caller's stream, group 1 on fac2, the rest on these
+  int groups = 0;
   std::vector<cudaStream_t> xs;
   std::vector<cudaEvent_t> xj;
   std::vector<cudaEvent_t> ev;
@@ -755,9 +764,9 @@ DysonPipe *dyson_pipe(int nfreq) {
               cusolverDnCreate(&p->solver2) == CUSOLVER_STATUS_SUCCESS &&
               cusolverDnSetStream(p->solver2, p->fac2) == CUSOLVER_STATUS_SUCCESS;
     const char *genv = std::getenv("MBPT_DYSON_CHOL_GROUPS");
-    const int g = genv ? std::atoi(genv) : 4;
-    p->groups = p->nfac == 2 ? std::max(1, std::min(6, g)) : 1;
-    for (int i = 2; p->ok && i < p->groups; ++i) {
+    if (genv) p->groups = std::max(1, std::min(kMostCholGroups, std::atoi(genv)));
+    if (p->nfac != 2) p->groups = 1;
+    for (int i = 2; p->ok && i < kMostCholGroups; ++i) {
       cudaStream_t xs = nullptr;
       cudaEvent_t xj = nullptr;
       p->ok = cudaStreamCreateWithFlags(&xs, cudaStreamNonBlocking) == cudaSuccess &&
@@ -826,35 +835,39 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
   bool side_used = false;
   if (batched) {
     if (cudaMemsetAsync(b.info, 0, sizeof(int) * nfreq, st) != cudaSuccess) return MBPT_ERR_CUDA;
-    // groups of frequencies on their own streams (four by default, each of
-    // at least kBatchedCholMin frequencies): one
-    // group's DGEMMs fill the GPU while another's diagonal blocks (one CTA
-    // per matrix) are factorised
+    // groups of frequencies on their own streams (each of at least
+    // kBatchedCholMin frequencies): one group's products fill the GPU while
+    // another's diagonal blocks (one CTA per matrix) are factorised
     auto stream_of = [&](int g) { return g == 0 ? st : (g == 1 ? pp->fac2 : pp->xs[g - 2]); };
     auto join_of = [&](int g) { return g == 1 ? pp->join2 : pp->xj[g - 2]; };
-    const int G = std::max(1, std::min(pp->groups, nfreq / kBatchedCholMin));
+    const int G = std::max(1, std::min(chol_groups(n, pp->groups), nfreq / kBatchedCholMin));
     if (G > 1 && cudaEventRecord(pp->fork, st) != cudaSuccess) return MBPT_ERR_CUDA;
     for (int g = 1; g < G; ++g)
       if (cudaStreamWaitEvent(stream_of(g), pp->fork, 0) != cudaSuccess) return MBPT_ERR_CUDA;
-    int rc0 = MBPT_OK;
-    for (int g = 0; g < G && !rc0; ++g) {
-      const int f0 = static_cast<int>(static_cast<int64_t>(nfreq) * g / G);
-      const int f1 = static_cast<int>(static_cast<int64_t>(nfreq) * (g + 1) / G);
-      cudaStream_t gs = stream_of(g);
-      OzakiChol oz;
+    const int64_t blk = static_cast<int64_t>(kCholNb) * kCholNb;
+    auto first_of = [&](int g) { return static_cast<int>(static_cast<int64_t>(nfreq) * g / G); };
+    std::vector<CholGroup> grp(G);
+    for (int g = 0; g < G; ++g) {
+      const int f0 = first_of(g);
+      grp[g] = {chi0 + f0 * n * n, first_of(g + 1) - f0, b.info + f0, b.chol_P + f0 * n * kCholNb,
+                b.chol_Linv + f0 * blk, stream_of(g), OzakiChol()};
       if (b.oz_planes) {
         // this group's frequencies own a contiguous share of each buffer
+        OzakiChol &oz = grp[g].oz;
         oz.planes = b.oz_planes + ozaki_planes_bytes(n, f0, b.oz_slices);
         oz.scale = b.oz_scale + static_cast<int64_t>(f0) * n;
         oz.rowsq = b.oz_rowsq + static_cast<int64_t>(f0) * n;
         oz.slices = b.oz_slices;
         oz.err = err;
       }
-      rc0 = chol_batched(chi0 + f0 * n * n, n, f1 - f0, b.info + f0,
-                         b.chol_P + static_cast<int64_t>(f0) * n * kCholNb,
-                         b.chol_Linv + static_cast<int64_t>(f0) * kCholNb * kCholNb,
-                         gs, static_cast<int64_t>(nfreq) * kCholNb * kCholNb, &oz);
-      if (rc0) break;
+    }
+    // step by step over the groups, so that all of them are under way early
+    int rc0 = MBPT_OK;
+    for (int64_t j0 = 0; j0 < n && !rc0; j0 += kCholNb)
+      for (int g = 0; g < G && !rc0; ++g) rc0 = chol_step(grp[g], n, j0, nfreq * blk);
+    for (int g = 0; g < G && !rc0; ++g) {
+      const int f0 = first_of(g), f1 = first_of(g + 1);
+      cudaStream_t gs = stream_of(g);
       // this group's log-determinants, info words and events on its own stream
       launch_logdet_diag(chi0 + f0 * n * n, n, f1 - f0, logdet + f0, gs);
       if (!deferred && cudaMemcpyAsync(pp->info + f0, b.info + f0, sizeof(int) * (f1 - f0),
@@ -871,7 +884,6 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
     // the inverses of as many factors at a time as the scratch holds (where a
     // factorisation failed nothing is written)
     const int nbi = mode == MBPT_MODE_MIXED ? b.npairs : b.inv_batch;
-    const int64_t blk = static_cast<int64_t>(kCholNb) * kCholNb;
     for (int f0 = 0; want_w && f0 < nfreq; f0 += nbi) {
       const int nb = std::min(nbi, nfreq - f0);
       double *m = chi0 + f0 * n * n;

@@ -83,7 +83,7 @@ int ozaki_chol_scales(const double *A, int64_t n, int nmat, double *scale, doubl
 int ozaki_chol_slice(const double *A, int64_t n, int nmat, int64_t j0, int nb,
                      const double *scale, int8_t *planes, int slices, double *rownorm,
                      cudaStream_t st);
-// P -= L[j0:, :j0] L[j0:j0+nb, :j0]^T for every matrix from the digit planes
+// P = (I - A)[j0:, j0:j0+nb] - L[j0:, :j0] L[j0:j0+nb, :j0]^T for every matrix from the digit planes
 // (the diagonal entries from the exact FP64 running row norms, nmat x n).
 int ozaki_chol_update(double *A, int64_t n, int nmat, int64_t j0, int nb, double *P,
                       const double *scale, const int8_t *planes, int slices, double *rowsq,

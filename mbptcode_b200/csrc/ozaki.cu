@@ -143,7 +143,7 @@ __device__ __forceinline__ int8_t next_digit(double &t, double base) {
 }
 
 enum Epi : int {
-  EPI_CHOL = 0,  // the Cholesky panel: P -= product, column-major, exact diagonal
+  EPI_CHOL = 0,  // the Cholesky panel: P = I - chi0 - product, column-major, exact diagonal
   EPI_GEMM = 1,  // C = alpha product + beta C, row-major
 };
 
@@ -156,6 +156,7 @@ struct UpdateArgs {
   int nmat;            // planes per digit level (matrices of a batch)
   int a_row0, b_row0;  // first plane rows of the A and B operands
   int tiles_n;         // 64-column tiles per row of tiles
+  const double *A0;    // Cholesky: nmat n x n chi0, I - chi0 being factorised
   double *P;           // nmat panels, column-major m x nb (ld m), m = n - j0
   int64_t p_stride;    // elements between panels
   const double *scale; // Cholesky: nmat x n, 2^e_r; GEMM: the rows of A
@@ -329,11 +330,12 @@ __global__ void __launch_bounds__(192, 1) chol_update_kernel(const __grid_consta
           for (int i = 0; i < 32; ++i) acc[i] += static_cast<double>(v[i]) * w;
         }
         if (EPI == EPI_CHOL && live) {
-          // all 32 loads first (P's column entries and the columns' scales),
+          // all 32 loads first (chi0's column entries and the columns' scales),
           // then the stores: one memory round trip per chunk instead of one
           // per column, which the compiler cannot reorder across the stores
           // (two halves of 16 columns: the registers hold acc and one half)
           double *Prow = P + pr;   // column pc of the panel at Prow + pc m
+          const double *Arow = p.A0 + f * p.n * p.n + p.j0 * (p.n + 1) + pr;
           // the diagonal entry from the exact running row norm
           const int pd = pr - c0 - ch * 32;
           const double diag = (pd >= 0 && pd < 32 && pr < p.nb)
@@ -344,7 +346,7 @@ __global__ void __launch_bounds__(192, 1) chol_update_kernel(const __grid_consta
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
               const int pc = c0 + ch * 32 + h + i;  // panel column
-              old[i] = pc < p.nb ? Prow[static_cast<int64_t>(pc) * m] : 0.0;
+              old[i] = (pr == pc ? 1.0 : 0.0) - (pc < p.nb ? Arow[pc * p.n] : 0.0);
               scol[i] = pc < p.nb ? sc[p.j0 + pc] : 0.0;
             }
 #pragma unroll
@@ -705,6 +707,7 @@ int ozaki_chol_update(double *A, int64_t n, int nmat, int64_t j0, int nb, double
   p.nb = nb;
   p.k_tiles = static_cast<int>(j0 / ozaki::BKB);
   p.nmat = nmat;
+  p.A0 = A;
   p.P = P;
   p.p_stride = m * nb;
   p.scale = scale;
