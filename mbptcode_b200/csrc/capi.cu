@@ -177,13 +177,17 @@ bool gemm_f64(cublasHandle_t h, bool ta, bool tb, int64_t m, int64_t n, int64_t 
 
 // the forward sweeps' FP64 products: native in MBPT_MODE_FP64, on the Ozaki
 // product in MBPT_MODE_FP64_INT8; `sym`: the n x n product is symmetric, and
-// the Ozaki product forms its upper tiles only (the native one forms all)
+// the Ozaki product forms its upper tiles only (the native one forms all); a, b:
+// operands cut beforehand for it
 bool gemm_mode(int mode, cublasHandle_t h, bool ta, bool tb, int64_t m, int64_t n, int64_t k,
                double alpha, const double *A, int64_t lda, const double *B, int64_t ldb,
-               double beta, double *C, int64_t ldc, bool sym = false) {
+               double beta, double *C, int64_t ldc, bool sym = false,
+               const OzakiOperand *a = nullptr, const OzakiOperand *b = nullptr) {
   if (mode == MBPT_MODE_FP64_INT8) {
     OzakiEpi e;
     e.sym = sym;
+    e.a = a;
+    e.b = b;
     return gemm_ozaki(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, &e);
   }
   return dgemm_rm(h, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
@@ -212,6 +216,7 @@ struct Chi0Bufs {
   double *w;  // cosft_wt on the device
   // fp64 (Xo_s, Xv_s, Go, Y: `batch` tau points each; Gv: the int8 mode only)
   double *Xo_s, *Xv_s, *Go, *Gv, *Y, *proj;
+  int8_t *Dt_cut;  // int8 mode: D^T's digit planes
   // mixed (Y, Pi, Z: `batch` tau points each, stacked by rows)
   int batch;
   bf16 *Dt_hi, *Dt_lo, *Pi_hi, *Pi_lo, *Z_hi, *Z_lo;
@@ -259,7 +264,10 @@ Chi0Bufs carve_chi0(Arena &ar, const Dims &d, int ntau, int nfreq, int mode, boo
   Chi0Bufs b{};
   b.w = ar.take<double>(static_cast<size_t>(nfreq) * ntau);
   if (fp64_mode(mode)) {
-    b.batch = mode == MBPT_MODE_FP64 ? tau_batch(ntau, d.M * (d.M + d.naux + d.n)) : 1;
+    // the int8 products go one tau point at a time, Pi is formed in batches
+    b.batch = tau_batch(ntau, d.M * (d.M + d.naux + d.n));
+    if (mode == MBPT_MODE_FP64_INT8)
+      b.Dt_cut = ar.take<int8_t>(ozaki_operand_bytes(d.naux, d.M));
     b.Xo_s = ar.take<double>(b.batch * d.M * d.nocc);
     b.Xv_s = ar.take<double>(b.batch * d.M * d.nv);
     // the library products hold one tau point's G_occ and G_virt
@@ -297,8 +305,14 @@ int chi0_run(const double *X, const Dims &d, const double *eps, double mu, const
   const int64_t a2 = d.naux * d.naux;
   double top = 0.0;
   for (int i = 0; i < nfreq * ntau; ++i) top = std::max(top, std::fabs(cw[i]));
-  if (mode == MBPT_MODE_FP64 && top <= kAmplifyingWeight) {
+  if (fp64_mode(mode) && (mode == MBPT_MODE_FP64_INT8 || top <= kAmplifyingWeight)) {
     double *proj = proj_out ? proj_out : b.proj;
+    cublasHandle_t h = handles(st).blas;
+    OzakiOperand Dt;
+    if (mode == MBPT_MODE_FP64_INT8) {
+      const int rc = ozaki_cut(D, d.naux, d.M, d.naux, true, b.Dt_cut, &Dt, st);
+      if (rc) return rc;
+    }
     const int64_t mo = d.M * d.nocc, mv = d.M * d.nv, m2 = d.M * d.M, ma = d.M * d.naux;
     for (int k = 0; k < ntau; k += b.batch) {
       const int nb = std::min(b.batch, ntau - k);
@@ -309,8 +323,15 @@ int chi0_run(const double *X, const Dims &d, const double *eps, double mu, const
       int rc = dmma::hadamard_product({b.Xo_s, d.nocc, mo}, {X, d.n, 0}, d.nocc,
                                       {b.Xv_s, d.nv, mv}, {X + d.nocc, d.n, 0}, d.nv, d.M, b.Go,
                                       d.M, m2, nb, st);
-      if (!rc)
-        rc = dmma::gemm({b.Go, d.M, m2}, true, {D, d.naux, 0}, false, d.M, d.naux, d.M, 1.0, 0.0,
+      for (int i = 0; mode == MBPT_MODE_FP64_INT8 && !rc && i < nb; ++i)
+        if (!gemm_mode(mode, h, false, false, d.M, d.naux, d.M, 1.0, b.Go + i * m2, d.M, D, d.naux,
+                       0.0, b.Y, d.naux, false, nullptr, &Dt) ||
+            !gemm_mode(mode, h, true, false, d.naux, d.naux, d.M, -2.0, D, d.naux, b.Y, d.naux,
+                       0.0, proj + (k + i) * a2, d.naux, true, &Dt))
+          rc = MBPT_ERR_CUDA;
+      if (rc) return rc;
+      if (mode == MBPT_MODE_FP64_INT8) continue;
+      rc = dmma::gemm({b.Go, d.M, m2}, true, {D, d.naux, 0}, false, d.M, d.naux, d.M, 1.0, 0.0,
                         b.Y, d.naux, ma, nb, false, st);
       if (!rc)
         rc = dmma::gemm({D, d.naux, 0}, false, {b.Y, d.naux, ma}, false, d.naux, d.naux, d.M,
@@ -325,16 +346,16 @@ int chi0_run(const double *X, const Dims &d, const double *eps, double mu, const
     for (int k = 0; k < ntau; ++k) {
       launch_scaled_branches(X, d.M, d.n, d.nocc, eps, mu, tau[k], 1.0, b.Xo_s, b.Xv_s, st);
       // G_occ = (X_o e^{e_o tau}) X_o^T, G_virt likewise (MBPTcode space_time.py:525-526)
-      if (!gemm_mode(mode, h, false, true, d.M, d.M, d.nocc, 1.0, b.Xo_s, d.nocc, X, d.n, 0.0,
+      if (!dgemm_rm(h, false, true, d.M, d.M, d.nocc, 1.0, b.Xo_s, d.nocc, X, d.n, 0.0,
                      b.Go, d.M) ||
-          !gemm_mode(mode, h, false, true, d.M, d.M, d.nv, 1.0, b.Xv_s, d.nv, X + d.nocc, d.n,
+          !dgemm_rm(h, false, true, d.M, d.M, d.nv, 1.0, b.Xv_s, d.nv, X + d.nocc, d.n,
                      0.0, b.Gv, d.M))
         return MBPT_ERR_CUDA;
       launch_hadamard(b.Go, b.Gv, d.M * d.M, st);
-      if (!gemm_mode(mode, h, false, false, d.M, d.naux, d.M, 1.0, b.Go, d.M, D, d.naux, 0.0,
+      if (!dgemm_rm(h, false, false, d.M, d.naux, d.M, 1.0, b.Go, d.M, D, d.naux, 0.0,
                      b.Y, d.naux) ||
-          !gemm_mode(mode, h, true, false, d.naux, d.naux, d.M, -2.0, D, d.naux, b.Y, d.naux,
-                     0.0, proj + k * a2, d.naux, true))
+          !dgemm_rm(h, true, false, d.naux, d.naux, d.M, -2.0, D, d.naux, b.Y, d.naux,
+                     0.0, proj + k * a2, d.naux))
         return MBPT_ERR_CUDA;
     }
     launch_transform<double>(proj, a2, d.naux, d.naux, d.naux, b.w, nfreq, ntau, chi0, a2,
@@ -1012,9 +1033,10 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
 
 // -------------------------------------------------------------------- Sigma
 struct SigmaBufs {
-  // fp64 (U, Ws, Hl, Hg, Xo_s, Xv_s: `batch` tau points each; Zt alone where
-  // W = I; Hl as G and R: the int8 mode)
-  double *U, *Ws, *Zt, *Hl, *Hg, *Xo_s, *Xv_s, *Xs, *R;
+  // fp64 (U, Ws, Hl, Hg, Xo_s, Xv_s: `batch` tau points each, one in the int8
+  // mode; Zt: there, and where W = I)
+  double *U, *Ws, *Zt, *Hl, *Hg, *Xo_s, *Xv_s, *Xs;
+  int8_t *D_cut;  // int8 mode: D's digit planes
   // mixed (W, U, Y, Zf, Hl, Hg: `batch` tau points each, stacked by rows)
   int batch;
   bf16 *D_hi, *D_lo, *W_hi, *W_lo, *U_hi, *U_lo, *Yo_hi, *Yo_lo, *Yv_hi, *Yv_lo, *Hl_hi,
@@ -1041,12 +1063,11 @@ SigmaBufs carve_sigma(Arena &ar, const Dims &d, int ntau, int nstates, int mode)
     b.Xs = ar.take<double>(d.M * static_cast<int64_t>(nstates));
   } else if (fp64_mode(mode)) {
     b.U = ar.take<double>(d.M * d.naux);
-    b.Zt = ar.take<double>(d.M * d.M);
-    b.Hl = ar.take<double>(d.M * d.M);
+    for (double **q : {&b.Zt, &b.Hl, &b.Hg}) *q = ar.take<double>(d.M * d.M);
     b.Xo_s = ar.take<double>(d.M * d.nocc);
     b.Xv_s = ar.take<double>(d.M * d.nv);
     b.Xs = ar.take<double>(d.M * static_cast<int64_t>(nstates));
-    b.R = ar.take<double>(d.M * static_cast<int64_t>(nstates));
+    b.D_cut = ar.take<int8_t>(ozaki_operand_bytes(d.M, d.naux));
   } else {
     const int64_t Sp = pad_states(nstates);
     // BF16 pairs of W, U, Y, H^< and H^> and FP32 Zt per tau point, in doubles
@@ -1113,36 +1134,30 @@ int sigma_run(const double *X, const Dims &d, const double *eps, double mu, cons
   } else if (fp64_mode(mode)) {
     cublasHandle_t h = handles(st).blas;
     launch_gather_cols_f64(X, d.M, d.n, states, S, b.Xs, st);
-    for (int k = 0; k < ntau; ++k) {
-      // Zt = D Wt D^T (MBPTcode imaginary_time.py:508, :513); Wt = I without Wt
+    if (cudaMemsetAsync(branch, 0, sizeof(double) * 2 * ntau * S, st) != cudaSuccess)
+      return MBPT_ERR_CUDA;
+    OzakiOperand Dr;
+    int rc = ozaki_cut(D, d.M, d.naux, d.naux, false, b.D_cut, &Dr, st);
+    for (int k = 0; k < ntau && !rc; ++k) {
+      // the two N^3 products of Zt = D Wt D^T (symmetric) on the int8 tensor
+      // cores; W = I without Wt
       if (Wt && !gemm_mode(mode, h, false, false, d.M, d.naux, d.naux, 1.0, D, d.naux,
-                           Wt + k * a2, d.naux, 0.0, b.U, d.naux))
+                           Wt + k * a2, d.naux, 0.0, b.U, d.naux, false, &Dr))
         return MBPT_ERR_CUDA;
       if ((Wt || k == 0) && !gemm_mode(mode, h, false, true, d.M, d.M, d.naux, 1.0,
-                                       Wt ? b.U : D, d.naux, D, d.naux, 0.0, b.Zt, d.M, true))
+                                       Wt ? b.U : D, d.naux, D, d.naux, 0.0, b.Zt, d.M, true,
+                                       Wt ? nullptr : &Dr, &Dr))
         return MBPT_ERR_CUDA;
+      // then as in the FP64 mode
       launch_scaled_branches(X, d.M, d.n, d.nocc, eps, mu, tau[k], 1.0, b.Xo_s, b.Xv_s, st);
-      double *out_l = branch + static_cast<int64_t>(k) * S;
-      double *out_g = branch + static_cast<int64_t>(ntau + k) * S;
-      // lesser branch: G_occ o Zt contracted with X_s on both sides
-      if (!gemm_mode(mode, h, false, true, d.M, d.M, d.nocc, 1.0, b.Xo_s, d.nocc, X, d.n, 0.0,
-                     b.Hl, d.M))
-        return MBPT_ERR_CUDA;
-      launch_hadamard(b.Hl, b.Zt, d.M * d.M, st);
-      if (!gemm_mode(mode, h, false, false, d.M, S, d.M, 1.0, b.Hl, d.M, b.Xs, S, 0.0, b.R, S))
-        return MBPT_ERR_CUDA;
-      cudaMemsetAsync(out_l, 0, sizeof(double) * S, st);
-      launch_rowdot(b.R, S, b.Xs, S, d.M, S, 1.0, out_l, st);
-      // greater branch, with its minus sign
-      if (!gemm_mode(mode, h, false, true, d.M, d.M, d.nv, 1.0, b.Xv_s, d.nv, X + d.nocc, d.n,
-                     0.0, b.Hl, d.M))
-        return MBPT_ERR_CUDA;
-      launch_hadamard(b.Hl, b.Zt, d.M * d.M, st);
-      if (!gemm_mode(mode, h, false, false, d.M, S, d.M, 1.0, b.Hl, d.M, b.Xs, S, 0.0, b.R, S))
-        return MBPT_ERR_CUDA;
-      cudaMemsetAsync(out_g, 0, sizeof(double) * S, st);
-      launch_rowdot(b.R, S, b.Xs, S, d.M, S, -1.0, out_g, st);
+      rc = dmma::sigma_h(b.Zt, {}, {}, d.naux, {b.Xo_s, d.nocc, 0}, {X, d.n, 0}, d.nocc,
+                         {b.Xv_s, d.nv, 0}, {X + d.nocc, d.n, 0}, d.nv, d.M, b.Hl, b.Hg, 0, 1,
+                         st);
+      if (!rc) rc = dmma::half_quadratic(b.Hl, 0, d.M, b.Xs, S, 1.0, branch + k * S, S, 1, st);
+      if (!rc)
+        rc = dmma::half_quadratic(b.Hg, 0, d.M, b.Xs, S, -1.0, branch + (ntau + k) * S, S, 1, st);
     }
+    if (rc) return rc;
   } else {
     const int64_t Sp = pad_states(nstates);
     launch_split_pad<double>(D, d.M, d.naux, d.naux, 1.f, b.D_hi, b.D_lo, d.Ap, d.Mp, d.Ap,
@@ -1218,10 +1233,12 @@ int sigma_run(const double *X, const Dims &d, const double *eps, double mu, cons
 // ------------------------------------------------------------- chi0 adjoint
 struct BackBufs {
   double *pb, *E, *Xo_s, *Xv_s, *Go, *Gv, *P, *T, *GoX, *GvX;
+  int8_t *D_cut;  // int8 mode: D's digit planes
 };
 
-BackBufs carve_back(Arena &ar, const Dims &d) {
+BackBufs carve_back(Arena &ar, const Dims &d, int mode) {
   BackBufs b{};
+  if (mode == MBPT_MODE_FP64_INT8) b.D_cut = ar.take<int8_t>(ozaki_operand_bytes(d.M, d.naux));
   b.pb = ar.take<double>(d.naux * d.naux);
   b.E = ar.take<double>(d.M * d.naux);
   b.Xo_s = ar.take<double>(d.M * d.nocc);
@@ -1238,26 +1255,42 @@ BackBufs carve_back(Arena &ar, const Dims &d) {
 int back_run(const double *pbar, const double *X, const Dims &d, const double *eps, double mu,
              const double *D, const double *tau, int ntau, double *eps_bar, double *X_bar,
              double *D_bar, Arena &ar, cudaStream_t st, int mode) {
-  BackBufs b = carve_back(ar, d);
+  BackBufs b = carve_back(ar, d, mode);
   if (ar.overflow()) return MBPT_ERR_WORKSPACE;
   cublasHandle_t h = handles(st).blas;
   const int64_t a2 = d.naux * d.naux;
   cudaMemsetAsync(eps_bar, 0, sizeof(double) * d.n, st);
   cudaMemsetAsync(X_bar, 0, sizeof(double) * d.M * d.n, st);
   cudaMemsetAsync(D_bar, 0, sizeof(double) * d.M * d.naux, st);
+  const bool int8 = mode == MBPT_MODE_FP64_INT8;
+  OzakiOperand Dr;  // D's rows, an operand of two products per tau point
+  if (int8) {
+    const int rc = ozaki_cut(D, d.M, d.naux, d.naux, false, b.D_cut, &Dr, st);
+    if (rc) return rc;
+  }
   for (int k = 0; k < ntau; ++k) {
     // MBPTcode gradients/rpa/space_time_adjoint.py:196-217, one row tile
     launch_sym_half(pbar + k * a2, b.pb, d.naux, 1, st);
     if (!gemm_mode(mode, h, false, false, d.M, d.naux, d.naux, -2.0, D, d.naux, b.pb, d.naux, 0.0,
-                  b.E, d.naux))
+                  b.E, d.naux, false, &Dr))
       return MBPT_ERR_CUDA;
     launch_scaled_branches(X, d.M, d.n, d.nocc, eps, mu, tau[k], 1.0, b.Xo_s, b.Xv_s, st);
-    if (!gemm_mode(mode, h, false, true, d.M, d.M, d.nocc, 1.0, b.Xo_s, d.nocc, X, d.n, 0.0, b.Go,
-                  d.M) ||
-        !gemm_mode(mode, h, false, true, d.M, d.M, d.nv, 1.0, b.Xv_s, d.nv, X + d.nocc, d.n, 0.0,
-                  b.Gv, d.M))
-      return MBPT_ERR_CUDA;
-    launch_hadamard3(b.P, b.Go, b.Gv, d.M * d.M, st);  // Pi
+    if (int8) {
+      // the short inner dimensions leave the int8 product nothing but its
+      // operands' cutting and its stores: G_occ, G_virt and Pi in one FP64
+      // kernel, upper tiles (M = 2400, n = 400: 133 us instead of 350)
+      const int rc = dmma::hadamard_product(
+          {b.Xo_s, d.nocc, 0}, {X, d.n, 0}, d.nocc, {b.Xv_s, d.nv, 0}, {X + d.nocc, d.n, 0}, d.nv,
+          d.M, b.P, d.M, 0, 1, st, b.Go, b.Gv);
+      if (rc) return rc;
+    } else {
+      if (!dgemm_rm(h, false, true, d.M, d.M, d.nocc, 1.0, b.Xo_s, d.nocc, X, d.n, 0.0, b.Go,
+                    d.M) ||
+          !dgemm_rm(h, false, true, d.M, d.M, d.nv, 1.0, b.Xv_s, d.nv, X + d.nocc, d.n, 0.0, b.Gv,
+                    d.M))
+        return MBPT_ERR_CUDA;
+      launch_hadamard3(b.P, b.Go, b.Gv, d.M * d.M, st);  // Pi
+    }
     if (!gemm_mode(mode, h, false, false, d.M, d.naux, d.M, 2.0, b.P, d.M, b.E, d.naux, 1.0, D_bar,
                   d.naux))
       return MBPT_ERR_CUDA;
@@ -1265,9 +1298,10 @@ int back_run(const double *pbar, const double *X, const Dims &d, const double *e
     // Pi_bar o Gv, Gv_bar = Pi_bar o Go: on the Ozaki product both straight
     // from its epilogue (Pi_bar never stored), else through Pi_bar
     double *go_bar = b.P, *gv_bar = b.T;
-    if (mode == MBPT_MODE_FP64_INT8 && d.naux <= kOzakiKChunk) {
+    if (int8 && d.naux <= kOzakiKChunk) {
       OzakiEpi e;
       e.sym = true;
+      e.b = &Dr;
       e.h1 = b.Gv;
       e.h2 = b.Go;
       e.c2 = gv_bar;
@@ -1295,6 +1329,7 @@ int back_run(const double *pbar, const double *X, const Dims &d, const double *e
 // ------------------------------------------------------- self-energy adjoint
 struct SigBackBufs {
   double *Xo_s, *Xv_s, *Go, *Gv, *Zt, *Al, *Ag, *U, *Xs, *Xl, *Xg, *T1, *GoX, *GvX;
+  int8_t *D_cut, *Dt_cut;  // D's and D^T's digit planes (int8 mode)
 };
 
 SigBackBufs carve_sigma_back(Arena &ar, const Dims &d, int64_t S) {
@@ -1306,6 +1341,8 @@ SigBackBufs carve_sigma_back(Arena &ar, const Dims &d, int64_t S) {
   for (double **m : {&b.Xs, &b.Xl, &b.Xg, &b.T1}) *m = ar.take<double>(d.M * S);
   b.GoX = ar.take<double>(d.M * d.nocc);
   b.GvX = ar.take<double>(d.M * d.nv);
+  b.D_cut = ar.take<int8_t>(ozaki_operand_bytes(d.M, d.naux));
+  b.Dt_cut = ar.take<int8_t>(ozaki_operand_bytes(d.naux, d.M));
   return b;
 }
 
@@ -1333,6 +1370,12 @@ int sigma_back_run(const double *X, const Dims &d, const double *eps, double mu,
   cudaMemsetAsync(eps_bar, 0, sizeof(double) * d.n, st);
   cudaMemsetAsync(X_bar, 0, sizeof(double) * M * d.n, st);
   cudaMemsetAsync(D_bar, 0, sizeof(double) * M * A, st);
+  OzakiOperand Dr, Dt;
+  if (mode == MBPT_MODE_FP64_INT8) {
+    int rc = ozaki_cut(D, M, A, A, false, b.D_cut, &Dr, st);
+    if (!rc) rc = ozaki_cut(D, A, M, A, true, b.Dt_cut, &Dt, st);
+    if (rc) return rc;
+  }
   for (int k = 0; k < ntau; ++k) {
     const double *Wk = Wt + k * a2;
     launch_scaled_branches(X, M, d.n, d.nocc, eps, mu, tau[k], 1.0, b.Xo_s, b.Xv_s, st);
@@ -1341,8 +1384,9 @@ int sigma_back_run(const double *X, const Dims &d, const double *eps, double mu,
     if (!gemm_mode(mode, h, false, true, M, M, d.nocc, 1.0, b.Xo_s, d.nocc, X, d.n, 0.0, b.Go, M) ||
         !gemm_mode(mode, h, false, true, M, M, d.nv, 1.0, b.Xv_s, d.nv, X + d.nocc, d.n, 0.0, b.Gv,
                   M) ||
-        !gemm_mode(mode, h, false, false, M, A, A, 1.0, D, A, Wk, A, 0.0, b.U, A) ||
-        !gemm_mode(mode, h, false, true, M, M, A, 1.0, b.U, A, D, A, 0.0, b.Zt, M, true) ||
+        !gemm_mode(mode, h, false, false, M, A, A, 1.0, D, A, Wk, A, 0.0, b.U, A, false, &Dr) ||
+        !gemm_mode(mode, h, false, true, M, M, A, 1.0, b.U, A, D, A, 0.0, b.Zt, M, true, nullptr,
+                  &Dr) ||
         !gemm_mode(mode, h, false, true, M, M, S, 1.0, b.Xl, S, b.Xs, S, 0.0, b.Al, M) ||
         !gemm_mode(mode, h, false, true, M, M, S, 1.0, b.Xg, S, b.Xs, S, 0.0, b.Ag, M))
       return MBPT_ERR_CUDA;
@@ -1358,8 +1402,10 @@ int sigma_back_run(const double *X, const Dims &d, const double *eps, double mu,
       return MBPT_ERR_CUDA;
     launch_xbar_update(b.GoX, b.GvX, X, M, d.n, d.nocc, eps, mu, tau[k], X_bar, eps_bar, st);
     // U <- Zt_bar D, then Wt_bar = D^T U and D_bar += 2 U Wt (Zt_bar and Wt symmetric)
-    if (!gemm_mode(mode, h, false, false, M, A, M, 1.0, b.Zt, M, D, A, 0.0, b.U, A) ||
-        !gemm_mode(mode, h, true, false, A, A, M, 1.0, D, A, b.U, A, 0.0, Wt_bar + k * a2, A) ||
+    if (!gemm_mode(mode, h, false, false, M, A, M, 1.0, b.Zt, M, D, A, 0.0, b.U, A, false, nullptr,
+                  &Dt) ||
+        !gemm_mode(mode, h, true, false, A, A, M, 1.0, D, A, b.U, A, 0.0, Wt_bar + k * a2, A, false,
+                  &Dt) ||
         !gemm_mode(mode, h, false, false, M, A, A, 2.0, b.U, A, Wk, A, 1.0, D_bar, A))
       return MBPT_ERR_CUDA;
   }
@@ -1625,7 +1671,7 @@ size_t mbpt_chi0_backward_workspace_bytes(int64_t M, int64_t norb, int64_t nocc,
   Dims d(M, norb, nocc, naux);
   Arena ar;
   ar.counting = true;
-  carve_back(ar, d);
+  carve_back(ar, d, mode);
   return ar.used + 2048;
 }
 

@@ -179,7 +179,7 @@ struct Args {
   int m, n, tiles_m, tiles_n;
   bool upper;
   double alpha, beta;
-  double *c0, *c1;
+  double *c0, *c1, *c2;  // PRODUCT: c1, c2 the factors themselves (null: not kept)
   int64_t ldc, sc;
   const double *zt;    // SIGMA: Zt as stored (ld m) instead of the first product
   const double *xs;    // row contraction
@@ -402,6 +402,10 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
   } else if constexpr (EPI == PRODUCT) {
     store(p.c0, [&](int i, int j, int e, double *) { return acc[i][j][e] * keep[i][j][e]; },
           tj > ti);
+    if (p.c1) {
+      store(p.c1, [&](int i, int j, int e, double *) { return keep[i][j][e]; }, tj > ti);
+      store(p.c2, [&](int i, int j, int e, double *) { return acc[i][j][e]; }, tj > ti);
+    }
   } else if constexpr (EPI == SIGMA) {
     const double f = ti == tj ? 0.5 : 1.0;
     store(p.c1, [&](int i, int j, int e, double *) { return acc[i][j][e] * keep[i][j][e] * f; },
@@ -495,7 +499,7 @@ int gemm(const Operand &a, bool a_k, const Operand &b, bool b_k, int64_t m, int6
 
 int hadamard_product(const Operand &a0, const Operand &b0, int64_t k0, const Operand &a1,
                      const Operand &b1, int64_t k1, int64_t m, double *c, int64_t ldc,
-                     int64_t sc, int batch, cudaStream_t st) {
+                     int64_t sc, int batch, cudaStream_t st, double *g0, double *g1) {
   if (!fits(m) || !fits(k0) || !fits(k1)) return MBPT_ERR_SHAPE;
   Args p{};
   p.a[0] = a0;
@@ -506,6 +510,8 @@ int hadamard_product(const Operand &a0, const Operand &b0, int64_t k0, const Ope
   p.k[1] = static_cast<int>(k1);
   p.m = p.n = static_cast<int>(m);
   p.c0 = c;
+  p.c1 = g0;
+  p.c2 = g1;
   p.ldc = ldc;
   p.sc = sc;
   p.upper = true;

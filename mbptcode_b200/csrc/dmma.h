@@ -22,10 +22,12 @@ int gemm(const Operand &a, bool a_k, const Operand &b, bool b_k, int64_t m, int6
          cudaStream_t st);
 
 // C (m x m) = (A0 B0^T) o (A1 B1^T), both symmetric: Pi = G_occ o G_virt.
-// All operands K-contiguous.
+// All operands K-contiguous. g0, g1: the two factors as well, laid out as C
+// (both or neither).
 int hadamard_product(const Operand &a0, const Operand &b0, int64_t k0, const Operand &a1,
                      const Operand &b1, int64_t k1, int64_t m, double *c, int64_t ldc,
-                     int64_t sc, int batch, cudaStream_t st);
+                     int64_t sc, int batch, cudaStream_t st, double *g0 = nullptr,
+                     double *g1 = nullptr);
 
 // Zt = U D^T, hl = (Xo_s Xo^T) o Zt and hg = (Xv_s Xv^T) o Zt (all symmetric,
 // K-contiguous operands), leading dimension m, as `half_quadratic` reads

@@ -98,12 +98,26 @@ int ozaki_chol_update(double *A, int64_t n, int nmat, int64_t j0, int nb, double
 //   h1 (and h2): C = (alpha op(A) op(B)) o h1 and C2 = (alpha op(A) op(B)) o h2,
 //        element-wise, h1, h2 and C2 with C's leading dimension; needs beta
 //        0 and k <= kOzakiKChunk (the product complete in one pass).
+//   a, b: op(A)'s rows, op(B)^T's rows cut beforehand by ozaki_cut (slices 8; A, B
+//        are then not read; a cut that was not made, k too large, is ignored).
+struct OzakiOperand {
+  int8_t *planes = nullptr;
+  double *scale = nullptr;
+  int64_t rows = 0, k = 0;
+};
 struct OzakiEpi {
   bool sym = false;
+  const OzakiOperand *a = nullptr, *b = nullptr;
   const double *h1 = nullptr, *h2 = nullptr;
   double *c2 = nullptr;
 };
 constexpr int64_t kOzakiKChunk = 32768;
+// The digit planes of an operand that several products share: x(i, k) =
+// src[i ld + k], or src[k ld + i] with trans, into buf (ozaki_operand_bytes,
+// 16-byte aligned).
+size_t ozaki_operand_bytes(int64_t rows, int64_t k);
+int ozaki_cut(const double *src, int64_t rows, int64_t k, int64_t ld, bool trans, void *buf,
+              OzakiOperand *op, cudaStream_t st);
 size_t ozaki_gemm_scratch_bytes(int64_t m, int64_t n, int64_t k, int slices);
 int ozaki_dgemm(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha,
                 const double *A, int64_t lda, const double *B, int64_t ldb, double beta,

@@ -756,6 +756,49 @@ size_t ozaki_gemm_scratch_bytes(int64_t m, int64_t n, int64_t k, int slices) {
   return static_cast<size_t>(slices) * (mp + np) * kc + 16 * (mp + np) + 4096;
 }
 
+// The row maxima and digit planes of `count` operands (their rowmax words
+// zeroed by the caller).
+static int cut_operands(const ozaki::Sources &src, int count, int slices, cudaStream_t st) {
+  if (count == 0) return MBPT_OK;
+  int64_t rmax = 0, kmax = 0, kpmax = 0;
+  for (int i = 0; i < count; ++i) {
+    rmax = std::max(rmax, src.s[i].rows_pad);
+    kmax = std::max(kmax, src.s[i].kdim);
+    kpmax = std::max(kpmax, src.s[i].k_pad);
+  }
+  const dim3 gm(static_cast<unsigned>((kmax + ozaki::kMaxK - 1) / ozaki::kMaxK),
+                static_cast<unsigned>(rmax / ozaki::kMaxRows), count);
+  const dim3 gs(static_cast<unsigned>(kpmax / 128), static_cast<unsigned>(rmax / 32), count);
+  count_launch(2);
+  ozaki::row_max_kernel<<<gm, 256, 0, st>>>(src);
+  if (slices == 8)
+    ozaki::operand_slice_kernel<8><<<gs, 256, 0, st>>>(src);
+  else
+    ozaki::operand_slice_kernel<7><<<gs, 256, 0, st>>>(src);
+  return cudaGetLastError() == cudaSuccess ? MBPT_OK : MBPT_ERR_CUDA;
+}
+
+size_t ozaki_operand_bytes(int64_t rows, int64_t k) {
+  const int64_t rp = round_up(rows, 128);
+  return static_cast<size_t>(8) * rp * round_up(k, 128) + 16 * rp + 1024;
+}
+
+int ozaki_cut(const double *src, int64_t rows, int64_t k, int64_t ld, bool trans, void *buf,
+              OzakiOperand *op, cudaStream_t st) {
+  *op = OzakiOperand();
+  if (k > kOzakiKChunk || k < 1 || rows < 1) return MBPT_OK;  // cut chunk by chunk instead
+  const int64_t rp = round_up(rows, 128), kp = round_up(k, 128);
+  int8_t *planes = static_cast<int8_t *>(buf);
+  double *scale = reinterpret_cast<double *>(planes + 8 * rp * kp);
+  unsigned long long *rowmax = reinterpret_cast<unsigned long long *>(scale + rp);
+  if (cudaMemsetAsync(rowmax, 0, sizeof(unsigned long long) * rp, st) != cudaSuccess)
+    return MBPT_ERR_CUDA;
+  ozaki::Sources s{};
+  s.s[0] = {src, rows, k, ld, trans ? 1 : 0, rowmax, scale, planes, rp, kp};
+  *op = {planes, scale, rows, k};
+  return cut_operands(s, 1, 8, st);
+}
+
 int ozaki_dgemm(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha,
                 const double *A, int64_t lda, const double *B, int64_t ldb, double beta,
                 double *C, int64_t ldc, int slices, void *scratch, size_t scratch_bytes,
@@ -767,6 +810,12 @@ int ozaki_dgemm(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha,
   if (x.sym && m != n) return MBPT_ERR_SHAPE;
   if (x.h1 && (beta != 0.0 || k > kOzakiKChunk || (x.h2 && !x.c2))) return MBPT_ERR_SHAPE;
   if (scratch_bytes < ozaki_gemm_scratch_bytes(m, n, k, slices)) return MBPT_ERR_WORKSPACE;
+  // operands cut beforehand (one pass, 8 digits)
+  const bool one = k <= kOzakiKChunk && slices == 8;
+  const OzakiOperand *ca = one && x.a && x.a->planes ? x.a : nullptr;
+  const OzakiOperand *cb = one && x.b && x.b->planes ? x.b : nullptr;
+  if ((ca && (ca->rows != m || ca->k != k)) || (cb && (cb->rows != n || cb->k != k)))
+    return MBPT_ERR_SHAPE;
   const int64_t mp = round_up(m, 128), np = round_up(n, 128);
   static std::atomic<uint64_t> attr8{0}, attr7{0};
   for (int64_t kb = 0; kb < k; kb += kOzakiKChunk) {
@@ -782,20 +831,23 @@ int ozaki_dgemm(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha,
     unsigned long long *ma = reinterpret_cast<unsigned long long *>(sb + np), *mb = ma + mp;
     // op(A) rows are K-contiguous unless ta; op(B) = B^T rows unless tb
     ozaki::Sources src{};
-    src.s[0] = {ta ? A + kb * lda : A + kb, m, kc, lda, ta ? 1 : 0, ma, sa, pa, mp, kp};
-    src.s[1] = {tb ? B + kb : B + kb * ldb, n, kc, ldb, tb ? 0 : 1, mb, sb, pb, np, kp};
-    if (cudaMemsetAsync(ma, 0, sizeof(unsigned long long) * (mp + np), st) != cudaSuccess)
+    int count = 0;
+    if (!ca)
+      src.s[count++] = {ta ? A + kb * lda : A + kb, m, kc, lda, ta ? 1 : 0, ma, sa, pa, mp, kp};
+    if (!cb)
+      src.s[count++] = {tb ? B + kb : B + kb * ldb, n, kc, ldb, tb ? 0 : 1, mb, sb, pb, np, kp};
+    if (count && cudaMemsetAsync(ma, 0, sizeof(unsigned long long) * (mp + np), st) != cudaSuccess)
       return MBPT_ERR_CUDA;
-    const int64_t rmax = std::max(mp, np);
-    const dim3 gm(static_cast<unsigned>((kc + ozaki::kMaxK - 1) / ozaki::kMaxK),
-                  static_cast<unsigned>(rmax / ozaki::kMaxRows), 2);
-    const dim3 gs(static_cast<unsigned>(kp / 128), static_cast<unsigned>(rmax / 32), 2);
-    count_launch(2);
-    ozaki::row_max_kernel<<<gm, 256, 0, st>>>(src);
-    if (slices == 8)
-      ozaki::operand_slice_kernel<8><<<gs, 256, 0, st>>>(src);
-    else
-      ozaki::operand_slice_kernel<7><<<gs, 256, 0, st>>>(src);
+    const int rc = cut_operands(src, count, slices, st);
+    if (rc) return rc;
+    if (ca) {
+      pa = ca->planes;
+      sa = ca->scale;
+    }
+    if (cb) {
+      pb = cb->planes;
+      sb = cb->scale;
+    }
     ozaki::UpdateArgs p{};
     if (!ozaki::make_operand_map(&p.tm_a, pa, kp, mp, slices, ozaki::BM) ||
         !ozaki::make_operand_map(&p.tm_b, pb, kp, np, slices, ozaki::BN))
