@@ -193,6 +193,29 @@ def host_array(a):
     return arr, arr.ctypes.data_as(C.c_void_p)
 
 
+#: host arrays up to this many bytes cross in `upload` without a host wait
+UPLOAD_BYTES = 1 << 20
+
+
+def upload(a, device, dtype=torch.float64, stream=None):
+    """A small host array on `device`, through a pinned staging block of
+    torch's host allocator, so that the copy is ordered on the caller's stream
+    and the host goes on (a copy from pageable memory waits for everything
+    queued before it: 20-50 us with the GPU idle after each). A call that runs
+    on a `stream` of its own, or a large array, takes the waiting copy."""
+    import numpy as np
+    arr = np.ascontiguousarray(a)
+    if not arr.flags.writeable:   # a broadcast view: torch wants memory it may own
+        arr = arr.copy()
+    t = torch.from_numpy(arr)
+    if t.numel() * t.element_size() > UPLOAD_BYTES or not (
+            stream is None or stream == torch.cuda.current_stream(device)):
+        return t.to(device=device, dtype=dtype)
+    pin = torch.empty(t.shape, dtype=dtype, pin_memory=True)
+    pin.copy_(t)
+    return pin.to(device, non_blocking=True)
+
+
 class Workspace:
     """A grow-only device scratch buffer per device, reused across calls."""
 

@@ -9,6 +9,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <mutex>
 #include <algorithm>
 #include <tuple>
@@ -823,9 +824,11 @@ DysonPipe *dyson_pipe(int nfreq) {
 // LU). Non-null: no host wait; every frequency's inverse is issued from its
 // factor and the info words land in info_dev_out, where a nonzero word marks
 // a frequency whose W - I and log-determinant are not valid.
+// tail: launches onto `st` what needs the log-determinants of all frequencies.
 int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, double *trace,
               int *info_host, int *sign_host, Arena &ar, cudaStream_t st,
-              int mode = MBPT_MODE_FP64, int *err = nullptr, int *info_dev_out = nullptr) {
+              int mode = MBPT_MODE_FP64, int *err = nullptr, int *info_dev_out = nullptr,
+              const std::function<void()> &tail = nullptr) {
   const bool deferred = info_dev_out != nullptr;
   DysonBufs b = carve_dyson(ar, n, nfreq, mode, want_w != 0);
   if (ar.overflow()) return MBPT_ERR_WORKSPACE;
@@ -942,6 +945,9 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
       return MBPT_ERR_CUDA;
     return MBPT_OK;
   };
+  // the host only reads info words from here on: what follows on the device
+  // runs meanwhile, and again below if a frequency took the LU route
+  if (batched && tail) tail();
   bool bad = false;
   int rc = MBPT_OK;
   for (int f = 0; f < nfac && f < nfreq && rc == MBPT_OK; ++f) rc = factor(f);
@@ -1024,6 +1030,7 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
     cudaStreamWaitEvent(st, pp->join2, 0);
   }
   if (rc) return rc;
+  if (tail && (bad || !batched)) tail();
   if (deferred && cudaMemcpyAsync(info_dev_out, b.info, sizeof(int) * nfreq,
                                   cudaMemcpyDeviceToDevice, st) != cudaSuccess)
     return MBPT_ERR_CUDA;
@@ -1583,10 +1590,11 @@ int mbpt_rpa_energy(const double *X, int64_t M, int64_t norb, int64_t nocc, cons
   int rc = chi0_run(X, d, eps, mu, D, tau, ntau, cw, nfreq, mode, chi0, proj, rest, err, st);
   if (rc) return rc;
   rest = ar;
-  rc = dyson_run(chi0, naux, nfreq, 0, logdet, trace, info_host, nullptr, rest, st);
-  if (rc && rc != MBPT_ERR_NOT_SPD) return rc;
   cudaMemcpyAsync(w, ow, sizeof(double) * nfreq, cudaMemcpyHostToDevice, st);
-  launch_energy_sum(logdet, trace, w, nfreq, e_c, st);
+  rc = dyson_run(chi0, naux, nfreq, 0, logdet, trace, info_host, nullptr, rest, st,
+                 MBPT_MODE_FP64, nullptr, nullptr,
+                 [&] { launch_energy_sum(logdet, trace, w, nfreq, e_c, st); });
+  if (rc && rc != MBPT_ERR_NOT_SPD) return rc;
   if (cudaGetLastError() != cudaSuccess) return MBPT_ERR_CUDA;
   return rc;
 }

@@ -15,7 +15,8 @@ import warnings
 import numpy as np
 import torch
 
-from ._lib import BUFFERS, WORKSPACE, check, host_array, lib, ptr, require_device, stream_ptr
+from ._lib import (BUFFERS, WORKSPACE, check, host_array, lib, ptr, require_device, stream_ptr,
+                   upload)
 from .grids import space_time_axes, space_time_axes_unrestricted
 from .space_time import (_Err, _eps_host, _mode, check_mixed_weights, chi0_sweep,
                          dyson_batch, to_device, transform)
@@ -136,10 +137,10 @@ def sigma_branch_sums(X, D, Wt, eps, nocc, tau_points, states, mu, precision=Non
     Wt = None if Wt is None else to_device(Wt, dev)
     Xd, Dd = to_device(X, dev), to_device(D, dev)
     eps_h = _eps_host(eps)
-    ed = to_device(eps_h, dev)
+    ed = upload(eps_h, dev, stream=stream)
     M, norb = Xd.shape
     naux = Dd.shape[1]
-    st = torch.as_tensor(np.asarray(states, dtype=np.int64), device=dev)
+    st = upload(np.asarray(states, dtype=np.int64), dev, torch.int64, stream)
     S = st.numel()
     tau_h, tp = host_array(tau_points)
     ntau = len(tau_h)
@@ -166,8 +167,7 @@ def sigma_frequency(branch, C, S, stream=None):
     (nstates, npade) device tensor: ``imaginary_time.py:525-532``."""
     dev = branch.device
     ntau, nstates = branch.shape[1], branch.shape[2]
-    Cd = torch.as_tensor(np.ascontiguousarray(C, dtype=np.float64), device=dev)
-    Sd = torch.as_tensor(np.ascontiguousarray(S, dtype=np.float64), device=dev)
+    Cd, Sd = upload(C, dev, stream=stream), upload(S, dev, stream=stream)
     npade = Cd.shape[0]
     out = torch.empty((nstates, npade, 2), dtype=torch.float64, device=dev)
     bc = branch.contiguous()  # held until the call has launched its kernel
@@ -188,10 +188,13 @@ def qp_solve(sigma, pade_freq, eps_anchor, states, nocc, mu, xc=None, greedy=Tru
     sig = torch.view_as_real(sigma.contiguous()).contiguous()
     S, npade = sigma.shape
     pf_h, pp = host_array(pade_freq)
-    ea = to_device(eps_anchor, dev)
-    st = torch.as_tensor(np.asarray(states, dtype=np.int64), device=dev)
-    xcd = None if xc is None else to_device(np.broadcast_to(np.asarray(xc, float), (S,))
-                                            if not isinstance(xc, torch.Tensor) else xc, dev)
+    ea = (to_device(eps_anchor, dev) if isinstance(eps_anchor, torch.Tensor)
+          else upload(eps_anchor, dev, stream=stream))
+    st = upload(np.asarray(states, dtype=np.int64), dev, torch.int64, stream)
+    if xc is None or isinstance(xc, torch.Tensor):
+        xcd = None if xc is None else to_device(xc, dev)
+    else:
+        xcd = upload(np.broadcast_to(np.asarray(xc, float), (S,)), dev, stream=stream)
     wd = None if warm is None else to_device(warm, dev)
     roots = torch.empty(S, dtype=torch.float64, device=dev)
     z = torch.empty(S, dtype=torch.float64, device=dev)
@@ -353,7 +356,7 @@ def gw_sweep(X, D, eps, nocc, states=None, ntau='auto', axes=None, precision=Non
             ev[1].record()
             ev[2].record()
         e_c = torch.empty((), dtype=torch.float64, device=dev)
-        ow = torch.as_tensor(np.asarray(axes.grid.omega_weights, float), device=dev)
+        ow = upload(np.asarray(axes.grid.omega_weights, float), dev, stream=stream)
         check(lib().mbpt_energy_sum(ptr(logdet), ptr(trace), ptr(ow), len(ow), ptr(e_c),
                                     stream_ptr(stream)), 'mbpt_energy_sum')
         return _sweep_tail(X, D, eps_h, nocc, states, axes, precision, eps_anchor, xc_diagonal,
@@ -370,7 +373,7 @@ def gw_sweep(X, D, eps, nocc, states=None, ntau='auto', axes=None, precision=Non
                                          precision=precision, err=err, deferred=_deferred)
     # E_c from the same factorisations: the frequency axis is a minimax quadrature
     e_c = torch.empty((), dtype=torch.float64, device=dev)
-    ow = torch.as_tensor(np.asarray(axes.grid.omega_weights, float), device=dev)
+    ow = upload(np.asarray(axes.grid.omega_weights, float), dev, stream=stream)
     check(lib().mbpt_energy_sum(ptr(logdet), ptr(trace), ptr(ow), len(ow), ptr(e_c),
                                 stream_ptr(stream)), 'mbpt_energy_sum')
     if ev:
@@ -501,7 +504,7 @@ def gw_sweep_unrestricted(X_mos, D, spectra, noccs, states=None, ntau='auto', ax
     logdet, trace, info, _ = dyson_batch(chi0, want_w=True, stream=stream,
                                          precision=precision, err=err)
     e_c = torch.empty((), dtype=torch.float64, device=dev)
-    ow = torch.as_tensor(np.asarray(axes.grid.omega_weights, float), device=dev)
+    ow = upload(np.asarray(axes.grid.omega_weights, float), dev, stream=stream)
     check(lib().mbpt_energy_sum(ptr(logdet), ptr(trace), ptr(ow), len(ow), ptr(e_c),
                                 stream_ptr(stream)), 'mbpt_energy_sum')
     Wt = w_tau_from_frequencies(

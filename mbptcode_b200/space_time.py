@@ -19,7 +19,8 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import MODES, WORKSPACE, check, host_array, lib, ptr, require_device, stream_ptr
+from ._lib import (MODES, WORKSPACE, check, host_array, lib, ptr, require_device, stream_ptr,
+                   upload)
 
 _DEFAULT_PRECISION = ['fp64']
 
@@ -114,7 +115,7 @@ def chi0_sweep(X, D, eps, nocc, tau_points, cosft_wt, mu=None, precision=None,
     dev = require_device()
     Xd, Dd = to_device(X, dev), to_device(D, dev)
     eps_h = _eps_host(eps)
-    ed = to_device(eps_h, dev)
+    ed = upload(eps_h, dev, stream=stream)
     if mu is None:
         mu = particle_hole_window(eps_h, nocc)[2]
     M, norb = Xd.shape
@@ -427,14 +428,14 @@ def _flag_nonpositive(where, sign, flags):
         flags.setdefault('nonpositive_det', []).append(where)
 
 
-def rpa_energy_device(X, D, eps, nocc, tau_points, cosft_wt, omega_weights, mu=None,
-                      precision=None, want_proj=False, stream=None):
-    """(E_c as a 0-d device tensor, info, proj or None): chi0 sweep, Cholesky
-    log-determinants and the weighted frequency sum in one library call."""
+def _rpa_energy(X, D, eps, nocc, tau_points, cosft_wt, omega_weights, mu, precision, want_proj,
+                stream):
+    """(out, info, proj): `rpa_energy_device` before its device error word is
+    read; out is a device array, E_c and the words of that int32 pair."""
     dev = require_device()
     Xd, Dd = to_device(X, dev), to_device(D, dev)
     eps_h = _eps_host(eps)
-    ed = to_device(eps_h, dev)
+    ed = upload(eps_h, dev, stream=stream)
     if mu is None:
         mu = particle_hole_window(eps_h, nocc)[2]
     M, norb = Xd.shape
@@ -445,22 +446,40 @@ def rpa_energy_device(X, D, eps, nocc, tau_points, cosft_wt, omega_weights, mu=N
     ntau, nfreq = len(tau_h), cw_h.shape[0]
     mode = _mode(precision)
     check_mixed_weights(precision, cw_h)
-    e_c = torch.empty((), dtype=torch.float64, device=dev)
+    out = torch.zeros(2, dtype=torch.float64, device=dev)
     proj = (torch.empty((ntau, naux, naux), dtype=torch.float64, device=dev)
             if want_proj else None)
     info = np.zeros(nfreq, dtype=np.int32)
     nbytes = lib().mbpt_rpa_energy_workspace_bytes(M, norb, nocc, naux, ntau, nfreq, mode)
     ws = WORKSPACE.get(nbytes, dev)
-    err = _Err(dev)
     import ctypes
     rc = lib().mbpt_rpa_energy(ptr(Xd), M, norb, nocc, ptr(ed), float(mu), ptr(Dd), naux, tp,
-                               ntau, cp, op, nfreq, mode, ptr(e_c), ptr(proj),
+                               ntau, cp, op, nfreq, mode, ptr(out), ptr(proj),
                                info.ctypes.data_as(ctypes.c_void_p), ptr(ws), ws.numel(),
-                               ptr(err.t), stream_ptr(stream))
+                               ptr(out[1:]), stream_ptr(stream))
     if rc not in (_lib.OK, _lib.ERR_NOT_SPD):
         check(rc, 'mbpt_rpa_energy')
-    err.check('mbpt_rpa_energy')
-    return e_c, info, proj
+    return out, info, proj
+
+
+def _energy_and_check(out):
+    """E_c of `_rpa_energy`'s output on the host, its error word checked."""
+    host = torch.empty(2, dtype=torch.float64, pin_memory=True).copy_(out, non_blocking=True)
+    torch.cuda.current_stream(out.device).synchronize()
+    e_c, word = host.numpy()[0], host.numpy().view(np.int32)[2]
+    if word:
+        raise _lib.MBPTError(int(word), 'mbpt_rpa_energy (device)')
+    return float(e_c)
+
+
+def rpa_energy_device(X, D, eps, nocc, tau_points, cosft_wt, omega_weights, mu=None,
+                      precision=None, want_proj=False, stream=None):
+    """(E_c as a 0-d device tensor, info, proj or None): chi0 sweep, Cholesky
+    log-determinants and the weighted frequency sum in one library call."""
+    out, info, proj = _rpa_energy(X, D, eps, nocc, tau_points, cosft_wt, omega_weights, mu,
+                                  precision, want_proj, stream)
+    _energy_and_check(out)
+    return out[0], info, proj
 
 
 def rpa_correlation_energy_space_time(X, D, eps, nocc, grid, mu=None, tile_gb=None,
@@ -474,15 +493,14 @@ def rpa_correlation_energy_space_time(X, D, eps, nocc, grid, mu=None, tile_gb=No
         raise NotImplementedError('the solvent-folded energy is not on the device route')
     if comm is not None and getattr(comm, 'Get_size', lambda: 1)() > 1:
         raise NotImplementedError('the device route runs on one GPU, without MPI ranks')
-    e_c, info, proj = rpa_energy_device(X, D, eps, nocc, grid.tau_points, grid.cosft_wt,
-                                        grid.omega_weights, mu=mu, precision=precision,
-                                        want_proj=want_tape)
+    out, info, proj = _rpa_energy(X, D, eps, nocc, grid.tau_points, grid.cosft_wt,
+                                  grid.omega_weights, mu, precision, want_tape, None)
+    value = _energy_and_check(out)
     bad = [int(k) for k in np.nonzero(info)[0]]
     for k in bad:
         _flag_nonpositive(k, -1, None)
     if flags is not None and bad:
         flags.setdefault('nonpositive_det', []).extend(bad)
-    value = float(e_c.item())
     if not want_tape:
         return value
     from types import SimpleNamespace
@@ -495,7 +513,7 @@ def transform(values, weights, stream=None, out=None, accumulate=False):
     `out` with `accumulate`)."""
     dev = values.device
     K, n = values.shape[0], values.shape[-1]
-    w = torch.as_tensor(np.ascontiguousarray(weights, dtype=np.float64), device=dev)
+    w = upload(weights, dev, stream=stream)
     J = w.shape[0]
     if out is None:
         if accumulate:
