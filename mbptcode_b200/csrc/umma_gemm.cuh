@@ -361,30 +361,83 @@ __device__ __forceinline__ void tmem_ld32(uint32_t addr, float (&v)[32]) {
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ void store_split32(bf16 *hi, bf16 *lo, const float (&v)[32]) {
+// ---- stores of a warp's 32 x 32 block (lane = row, v = its 32 columns) ----
+// A lane that stores its own row touches 32 rows per instruction, 16 bytes of a
+// 32-byte sector in each; a transposed BF16 store moves 64 bytes per
+// instruction. The blocks are therefore turned in shared memory (the operand
+// ring, free once the accumulators are complete; kStageWarp bytes per warp) so that
+// every store instruction writes whole sectors of consecutive memory.
+constexpr int kStageBf16Row = 80;   // bytes per row of 32 BF16: 64 and a 16-byte skew
+constexpr int kStageF32Row = 144;   // bytes per row of 32 FP32: 128 and a 16-byte skew
+constexpr int kStageWarp = 128 * kStageBf16Row;  // four BF16 blocks, or two FP32 ones
+
+// rows of `buf` (32 BF16 each) to out[r ld ...]: four lanes a row
+__device__ __forceinline__ void flush_bf16(const uint8_t *buf, bf16 *out, int64_t ld, int lane) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = 8 * i + (lane >> 2), seg = lane & 3;
+    *reinterpret_cast<uint4 *>(out + r * ld + 8 * seg) =
+        *reinterpret_cast<const uint4 *>(buf + r * kStageBf16Row + 16 * seg);
+  }
+}
+
+// The block as a BF16 pair at hi / lo (its row 0, column 0, leading dimension
+// ld); with t_hi, also transposed there (element (r, c) at c ld + r).
+__device__ __forceinline__ void store_split32(uint8_t *buf, bf16 *hi, bf16 *lo, bf16 *t_hi,
+                                              bf16 *t_lo, int64_t ld, const float (&v)[32],
+                                              int lane) {
+  uint8_t *bh = buf, *bl = buf + 32 * kStageBf16Row;
+  bf16 *th = reinterpret_cast<bf16 *>(buf + 64 * kStageBf16Row) + lane;
+  bf16 *tl = th + 32 * (kStageBf16Row / 2);
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     __align__(16) bf16 h[8];
     __align__(16) bf16 l[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) split_bf16(v[8 * q + i], h[i], l[i]);
-    reinterpret_cast<uint4 *>(hi)[q] = *reinterpret_cast<const uint4 *>(h);
-    reinterpret_cast<uint4 *>(lo)[q] = *reinterpret_cast<const uint4 *>(l);
+    for (int i = 0; i < 8; ++i) {
+      split_bf16(v[8 * q + i], h[i], l[i]);
+      if (t_hi) {
+        th[(8 * q + i) * (kStageBf16Row / 2)] = h[i];
+        tl[(8 * q + i) * (kStageBf16Row / 2)] = l[i];
+      }
+    }
+    *reinterpret_cast<uint4 *>(bh + lane * kStageBf16Row + 16 * q) =
+        *reinterpret_cast<const uint4 *>(h);
+    *reinterpret_cast<uint4 *>(bl + lane * kStageBf16Row + 16 * q) =
+        *reinterpret_cast<const uint4 *>(l);
   }
+  __syncwarp();
+  flush_bf16(bh, hi, ld, lane);
+  flush_bf16(bl, lo, ld, lane);
+  if (t_hi) {
+    flush_bf16(buf + 64 * kStageBf16Row, t_hi, ld, lane);
+    flush_bf16(buf + 96 * kStageBf16Row, t_lo, ld, lane);
+  }
+  __syncwarp();
 }
 
-// The transposed store of store_split32: v[i] goes to hi/lo[i * ld] (base at
-// the mirrored position); across the warp, lanes (consecutive rows) write
-// consecutive elements of each mirrored row.
-__device__ __forceinline__ void store_split32_t(bf16 *hi, bf16 *lo, int64_t ld,
-                                                const float (&v)[32]) {
+// The block as FP32 at out (row 0, column 0, leading dimension ld), added to
+// what is there with ACC.
+template <bool ACC>
+__device__ __forceinline__ void store_f32(uint8_t *buf, float *out, int64_t ld,
+                                          const float (&v)[32], int lane) {
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    bf16 h, l;
-    split_bf16(v[i], h, l);
-    hi[i * ld] = h;
-    lo[i * ld] = l;
+  for (int q = 0; q < 8; ++q)
+    *reinterpret_cast<float4 *>(buf + lane * kStageF32Row + 16 * q) =
+        make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = 4 * i + (lane >> 3), seg = lane & 7;
+    float4 o = *reinterpret_cast<const float4 *>(buf + r * kStageF32Row + 16 * seg);
+    float4 *dst = reinterpret_cast<float4 *>(out + r * ld + 4 * seg);
+    if constexpr (ACC) {
+      const float4 prev = *dst;
+      o.x += prev.x; o.y += prev.y; o.z += prev.z; o.w += prev.w;
+    }
+    *dst = o;
   }
+  __syncwarp();
 }
 
 // Lane l ends with the warp sum of column l of the 32 x 32 block v (row = lane).
@@ -713,6 +766,34 @@ __global__ void __launch_bounds__(64 + BN, 1)
     const int cb = ((warp - 2) >> 2) * 128;
     const uint32_t taddr = tmem + (static_cast<uint32_t>(sp * 32) << 16);
     bool ok = true;
+    // symmetric output, per 128-column block tb of this warp: a block below
+    // the diagonal is not stored, one above it also fills its mirror; columns
+    // past n_valid (a 256-wide tile over a 128-multiple edge) are not stored,
+    // nor the rows of a pair's second tile past m_valid
+    const int tb = (n0 + cb) / 128;
+    const bool upper = (p.band & BAND_UPPER) != 0;
+    const bool mirror = upper && tb > tm;
+    const bool live = n0 + cb < n_valid && m0 < m_valid && !(upper && tb < tm);
+    // Zt of the warp's 32 x 128 entries while the products run; above the
+    // diagonal block from its mirror (the same bits), whose rows lie along the
+    // lanes. Read after the products, a row per lane, it cost the epilogue a
+    // memory round trip per 32 columns
+    float z[EPI == EPI_SIGMA_HZ ? 128 : 1];
+    if constexpr (EPI == EPI_SIGMA_HZ) {
+      const float *zp = p.epi.zt + by * p.bs_zt;
+      const int64_t zr = m0 + sp * 32 + lane, zc = n0 + cb;
+      if (live && mirror) {
+#pragma unroll
+        for (int i = 0; i < 128; ++i) z[i] = zp[(zc + i) * p.epi.ld_zt + zr];
+      } else if (live) {
+        const float4 *zs = reinterpret_cast<const float4 *>(zp + zr * p.epi.ld_zt + zc);
+#pragma unroll
+        for (int q = 0; q < 32; ++q) {
+          const float4 t = zs[q];
+          z[4 * q] = t.x; z[4 * q + 1] = t.y; z[4 * q + 2] = t.z; z[4 * q + 3] = t.w;
+        }
+      }
+    }
     float acc[DRAIN > 0 ? 128 : 1];
     if constexpr (DRAIN > 0) {
 #pragma unroll
@@ -754,13 +835,9 @@ __global__ void __launch_bounds__(64 + BN, 1)
       if (lane == 0) DevErr{p.err}.set(MBPT_ERR_TIMEOUT);
     } else {
       tc_fence_after();
-      const int row = m0 + sp * 32 + lane;
+      const int row0 = m0 + sp * 32, row = row0 + lane;
       const EpiArgs &e = p.epi;
-      // symmetric output, per 128-column block tb of this warp: a block below
-      // the diagonal is not stored, one above it also fills its mirror
-      const int tb = (n0 + cb) / 128;
-      const bool upper = (p.band & BAND_UPPER) != 0;
-      const bool mirror = upper && tb > tm;
+      uint8_t *stage = smem + (warp - 2) * kStageWarp;
       // 32 columns starting at the warp's column c of accumulator j (the
       // drained one from registers)
       int col_of[NACC];
@@ -781,51 +858,50 @@ __global__ void __launch_bounds__(64 + BN, 1)
         }
         tmem_ld32(taddr + static_cast<uint32_t>(col_of[j] + cb + c), v);
       };
-      // columns past n_valid (a 256-wide tile over a 128-multiple edge) are not
-      // stored, nor the rows of a pair's second tile past m_valid
-      const bool live = n0 + cb < n_valid && m0 < m_valid && !(upper && tb < tm);
 #pragma unroll
       for (int c = 0; c < 128; c += 32) {
         if (!live) break;
         const int col = n0 + cb + c;
+        const int64_t at = static_cast<int64_t>(row0), ac = static_cast<int64_t>(col);
         float v0[32];
         load(0, c, v0);
         if constexpr (EPI == EPI_SPLIT) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) v0[i] *= e.alpha;
-          store_split32(e.out0_hi + ob + row * e.ld_out + col,
-                        e.out0_lo + ob + row * e.ld_out + col, v0);
+          const int64_t o = ob + at * e.ld_out + ac;
+          store_split32(stage, e.out0_hi + o, e.out0_lo + o, nullptr, nullptr, e.ld_out, v0, lane);
         } else if constexpr (EPI == EPI_F32 || EPI == EPI_F32_ACC) {
-          float4 *dst = reinterpret_cast<float4 *>(e.outf + ob + row * e.ld_outf + col);
 #pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            float4 o = make_float4(e.alpha * v0[4 * q], e.alpha * v0[4 * q + 1],
-                                   e.alpha * v0[4 * q + 2], e.alpha * v0[4 * q + 3]);
-            if constexpr (EPI == EPI_F32_ACC) {
-              const float4 prev = dst[q];
-              o.x += prev.x; o.y += prev.y; o.z += prev.z; o.w += prev.w;
-            }
-            dst[q] = o;
-          }
+          for (int i = 0; i < 32; ++i) v0[i] *= e.alpha;
+          store_f32<EPI == EPI_F32_ACC>(stage, e.outf + ob + at * e.ld_outf + ac, e.ld_outf, v0,
+                                        lane);
           if constexpr (EPI == EPI_F32) {
             if (mirror) {
 #pragma unroll
-              for (int i = 0; i < 32; ++i)
-                e.outf[ob + static_cast<int64_t>(col + i) * e.ld_outf + row] = e.alpha * v0[i];
+              for (int i = 0; i < 32; ++i) e.outf[ob + (ac + i) * e.ld_outf + row] = v0[i];
             }
           }
         } else if constexpr (EPI == EPI_F64_SYM) {
-          if (row < e.nd) {
-            double *dst = e.outd + ob + static_cast<int64_t>(row) * e.ld_outd + col;
+          float *fs = reinterpret_cast<float *>(stage);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              if (col + i < e.nd) {
-                const double v = static_cast<double>(e.alpha * v0[i]) -
-                                 (row == col + i ? e.shift : 0.0);
-                dst[i] = v;
-                if (mirror) e.outd[ob + static_cast<int64_t>(col + i) * e.ld_outd + row] = v;
-              }
-            }
+          for (int i = 0; i < 32; ++i) {
+            v0[i] *= e.alpha;
+            fs[lane * 33 + i] = v0[i];
+          }
+          __syncwarp();
+          double *dst = e.outd + ob + at * e.ld_outd + ac + lane;
+          if (col + lane < e.nd) {
+#pragma unroll 8
+            for (int r = 0; r < 32; ++r)
+              if (row0 + r < e.nd)
+                dst[r * e.ld_outd] = static_cast<double>(fs[r * 33 + lane]) -
+                                     (row0 + r == col + lane ? e.shift : 0.0);
+          }
+          __syncwarp();
+          if (mirror && row < e.nd) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (col + i < e.nd) e.outd[ob + (ac + i) * e.ld_outd + row] = static_cast<double>(v0[i]);
           }
         } else if constexpr (EPI == EPI_TF32_PAIR) {
           float hi[32], lo[32];
@@ -835,20 +911,15 @@ __global__ void __launch_bounds__(64 + BN, 1)
             hi[i] = to_tf32(v);
             lo[i] = to_tf32(v - hi[i]);
           }
-          float4 *dh = reinterpret_cast<float4 *>(e.p_hi + p_off + row * e.ld_p + col);
-          float4 *dl = reinterpret_cast<float4 *>(e.p_lo + p_off + row * e.ld_p + col);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            dh[q] = make_float4(hi[4 * q], hi[4 * q + 1], hi[4 * q + 2], hi[4 * q + 3]);
-            dl[q] = make_float4(lo[4 * q], lo[4 * q + 1], lo[4 * q + 2], lo[4 * q + 3]);
-          }
+          store_f32<false>(stage, e.p_hi + p_off + at * e.ld_p + ac, e.ld_p, hi, lane);
+          store_f32<false>(stage, e.p_lo + p_off + at * e.ld_p + ac, e.ld_p, lo, lane);
           if (e.t_hi) {
             // column col + i of the tile is row col + i of t: the warp's 32
             // consecutive rows land on 32 consecutive floats
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
-              e.t_hi[t_off + static_cast<int64_t>(col + i) * e.ld_t + row] = hi[i];
-              e.t_lo[t_off + static_cast<int64_t>(col + i) * e.ld_t + row] = lo[i];
+              e.t_hi[t_off + (ac + i) * e.ld_t + row] = hi[i];
+              e.t_lo[t_off + (ac + i) * e.ld_t + row] = lo[i];
             }
           }
         } else if constexpr (EPI == EPI_HADAMARD_SPLIT) {
@@ -856,39 +927,21 @@ __global__ void __launch_bounds__(64 + BN, 1)
           load(1, c, v1);
 #pragma unroll
           for (int i = 0; i < 32; ++i) v0[i] *= v1[i];
-          store_split32(e.out0_hi + ob + row * e.ld_out + col,
-                        e.out0_lo + ob + row * e.ld_out + col, v0);
-          if (mirror)
-            store_split32_t(e.out0_hi + ob + static_cast<int64_t>(col) * e.ld_out + row,
-                            e.out0_lo + ob + static_cast<int64_t>(col) * e.ld_out + row,
-                            e.ld_out, v0);
+          const int64_t o = ob + at * e.ld_out + ac, m = ob + ac * e.ld_out + at;
+          store_split32(stage, e.out0_hi + o, e.out0_lo + o, mirror ? e.out0_hi + m : nullptr,
+                        e.out0_lo + m, e.ld_out, v0, lane);
         } else if constexpr (EPI == EPI_SIGMA_HZ) {
-          // acc0 = G_occ, acc1 = G_virt; Zt (symmetric, stored whole) from memory
-          float z[32], v1[32];
-          const float4 *zs =
-              reinterpret_cast<const float4 *>(e.zt + by * p.bs_zt + row * e.ld_zt + col);
+          // acc0 = G_occ, acc1 = G_virt; Zt (symmetric, stored whole) read above
+          const int64_t o = ob + at * e.ld_out + ac, m = ob + ac * e.ld_out + at;
 #pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const float4 t = zs[q];
-            z[4 * q] = t.x; z[4 * q + 1] = t.y; z[4 * q + 2] = t.z; z[4 * q + 3] = t.w;
-          }
+          for (int i = 0; i < 32; ++i) v0[i] *= z[c + i];
+          store_split32(stage, e.out0_hi + o, e.out0_lo + o, mirror ? e.out0_hi + m : nullptr,
+                        e.out0_lo + m, e.ld_out, v0, lane);
+          load(1, c, v0);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v0[i] *= z[i];
-          store_split32(e.out0_hi + ob + row * e.ld_out + col,
-                        e.out0_lo + ob + row * e.ld_out + col, v0);
-          if (mirror)
-            store_split32_t(e.out0_hi + ob + static_cast<int64_t>(col) * e.ld_out + row,
-                            e.out0_lo + ob + static_cast<int64_t>(col) * e.ld_out + row,
-                            e.ld_out, v0);
-          load(1, c, v1);
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v1[i] *= z[i];
-          store_split32(e.out1_hi + ob + row * e.ld_out + col,
-                        e.out1_lo + ob + row * e.ld_out + col, v1);
-          if (mirror)
-            store_split32_t(e.out1_hi + ob + static_cast<int64_t>(col) * e.ld_out + row,
-                            e.out1_lo + ob + static_cast<int64_t>(col) * e.ld_out + row,
-                            e.ld_out, v1);
+          for (int i = 0; i < 32; ++i) v0[i] *= z[c + i];
+          store_split32(stage, e.out1_hi + o, e.out1_lo + o, mirror ? e.out1_hi + m : nullptr,
+                        e.out1_lo + m, e.ld_out, v0, lane);
         } else if constexpr (EPI == EPI_ROWDOT2) {
           float v1[32], xs[32];
           load(1, c, v1);
