@@ -52,9 +52,9 @@ HARTREE_EV = 27.211386245988
 N_ORB, NOCC, M, NTAU = 1200, 120, 7200, 24
 SEED = 2024
 
-# algorithmic FLOPs of one launch of each engine kernel at this workload
+# algorithmic FLOPs of one product of each engine kernel at this workload
 # (the split products' 3x and the padding are not counted). Pi, proj and H are
-# symmetric: those launches form the 128 x 128 tiles on and above the
+# symmetric: those products form the 128 x 128 tiles on and above the
 # diagonal only (T (T + 1) / 2 of T^2, T = 57 tile rows) and count that work.
 _T = -(-M // 128)
 SYM = (_T * (_T + 1) / 2) / (_T * _T)
@@ -65,7 +65,14 @@ FLOPS = {
     'sigma_hadamard': SYM * 2.0 * M * M * N_ORB,        # G_occ, G_virt (o Zt)
     'row_contraction': 2.0 * 2.0 * M * M * N_ORB,       # (G o Zt) X_s, both branches
 }
-# DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the
+# products of one sweep: chi0's hadamard, split and f32 and Sigma's split, f32,
+# sigma_hadamard and row_contraction at each tau point, and the last three once
+# more for the exchange. A launch takes several tau points (as many as the
+# workspace holds), so a kernel's work is counted from the sweep and not from
+# its launches
+PRODUCTS = {'hadamard': NTAU, 'split': 2 * NTAU, 'f32': 2 * NTAU + 1,
+            'sigma_hadamard': NTAU + 1, 'row_contraction': NTAU + 1}
+# DRAM bytes per product (dram__bytes_read.sum + dram__bytes_write.sum) of the
 # engine kernels at this workload, from one ncu capture of a tau point at full
 # size (python bench_cases.py tau --M 7200 --n 1200 --nocc 120
 # --states 1200, the seven engine launches of one tau point)
@@ -404,13 +411,16 @@ def main():
     fixed = {k: v for k, v in kern.items() if k in FLOPS}
     top, (top_ms, top_n) = max(fixed.items(), key=lambda kv: kv[1][0]) if fixed else ('', (0, 0))
     peak = float(pk.get('bf16_tflops_sustained', pk.get('bf16_tflops')))
-    def alg_tflops(k, ms, n):
-        return FLOPS.get(k, 0.0) / (ms / max(n, 1) / 1e3) / 1e12
+    def products(k):
+        return PRODUCTS.get(k, 0) * args.steps
 
-    achieved = alg_tflops(top, top_ms, top_n) if top_n else None
+    def alg_tflops(k, ms):
+        return FLOPS.get(k, 0.0) * products(k) / max(ms / 1e3, 1e-9) / 1e12
+
+    achieved = alg_tflops(top, top_ms) if top_n else None
     kernels = {k: {'launches': n, 'total_ms': round(ms, 3),
                    'avg_ms': round(ms / max(n, 1), 4),
-                   'tflops_alg': round(alg_tflops(k, ms, n), 1)}
+                   'tflops_alg': round(alg_tflops(k, ms), 1)}
                for k, (ms, n) in kern.items()}
     if fam:
         ms, n = fam
@@ -418,7 +428,7 @@ def main():
             'launches': n, 'total_ms': round(ms, 3), 'avg_ms': round(ms / max(n, 1), 4),
             'tflops_alg': round(DYSON_INV_FLOPS * NTAU / (ms / 1e3) / 1e12, 1),
             'note': 'one sweep outside the timed region; summed over the family'}
-    traffic = TRAFFIC_BYTES.get(top)
+    traffic = TRAFFIC_BYTES[top] * products(top) / top_n if top_n else None  # per launch
 
     cpu = None
     if rank == 0 and not args.no_cpu:
