@@ -23,19 +23,25 @@ __global__ void chi0_bar_seed_kernel(double *a, int64_t n, const double *w) {
     m[i] *= s;
 }
 
-// out = (in + in^T) / 2 for each n x n slice: one 32 x 32 tile and its mirror
-// per block, both halves through shared memory so that every access runs
-// along rows
+// out = (in + in^T) / 2 for each n x n slice, `in` the sum of `parts` arrays
+// part_stride apart: one 32 x 32 tile and its mirror per block, both halves
+// through shared memory so that every access runs along rows
 __global__ void sym_half_kernel(const double *__restrict__ in, double *__restrict__ out,
-                                int64_t n) {
+                                int64_t n, int parts, int64_t part_stride) {
   __shared__ double lo[32][33], up[32][33];
   if (blockIdx.x < blockIdx.y) return;
   const int64_t base = static_cast<int64_t>(blockIdx.z) * n * n;
   const int64_t r0 = static_cast<int64_t>(blockIdx.y) * 32, c0 = static_cast<int64_t>(blockIdx.x) * 32;
   const int x = threadIdx.x;
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    up[k][x] = r0 + k < n && c0 + x < n ? in[base + (r0 + k) * n + c0 + x] : 0.0;
-    lo[k][x] = c0 + k < n && r0 + x < n ? in[base + (c0 + k) * n + r0 + x] : 0.0;
+    double u = 0.0, l = 0.0;
+    for (int p = 0; p < parts; ++p) {
+      const double *a = in + p * part_stride + base;
+      if (r0 + k < n && c0 + x < n) u += a[(r0 + k) * n + c0 + x];
+      if (c0 + k < n && r0 + x < n) l += a[(c0 + k) * n + r0 + x];
+    }
+    up[k][x] = u;
+    lo[k][x] = l;
   }
   __syncthreads();
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
@@ -705,10 +711,11 @@ void launch_chi0_bar_seed(double *a, int64_t n, int nfreq, const double *w, cuda
   count_launch(); chi0_bar_seed_kernel<<<grid, 256, 0, st>>>(a, n, w);
 }
 
-void launch_sym_half(const double *in, double *out, int64_t n, int batch, cudaStream_t st) {
+void launch_sym_half(const double *in, double *out, int64_t n, int batch, cudaStream_t st,
+                     int parts) {
   const unsigned t = static_cast<unsigned>((n + 31) / 32);
   count_launch();
-  sym_half_kernel<<<dim3(t, t, batch), dim3(32, 8), 0, st>>>(in, out, n);
+  sym_half_kernel<<<dim3(t, t, batch), dim3(32, 8), 0, st>>>(in, out, n, parts, batch * n * n);
 }
 
 void launch_xbar_update(const double *GoX, const double *GvX, const double *X, int64_t M,

@@ -28,7 +28,8 @@ int launch_pade_eval(const double *sigma, const double *pade_freq, int npade,
                      const double *query, int nq, double *out, cudaStream_t st);
 void launch_chi0_bar_seed(double *a, int64_t n, int nfreq, const double *scale,
                           cudaStream_t st);
-void launch_sym_half(const double *in, double *out, int64_t n, int batch, cudaStream_t st);
+void launch_sym_half(const double *in, double *out, int64_t n, int batch, cudaStream_t st,
+                     int parts = 1);
 void launch_xbar_update(const double *GoX, const double *GvX, const double *X, int64_t M,
                         int64_t n, int64_t nocc, const double *eps, double mu, double tau,
                         double *X_bar, double *eps_bar, cudaStream_t st);
@@ -261,6 +262,22 @@ TauList tau_list(const double *tau, int count) {
 // below 1e3.
 constexpr double kAmplifyingWeight = 1e6;
 
+// Whether chi0's FP64 products take Pi by halves: Pi = T + T^T with T the upper
+// tiles, so D^T Pi D = S + S^T with S = D^T (T D). T D is half of Pi D's work
+// (M^2 naux for 2 M^2 naux), S cannot leave out half of its tiles (2 M naux^2
+// for M naux^2): fewer operations from M = naux on, 7 % fewer at M = 5/4 naux.
+// A launch of about one round of CTAs takes as long as its longest sum, which
+// the halves leave as it is, and S + S^T is a pass of its own. Measured (chi0
+// of 20 points, whole and by halves, us; M x naux): 400 x 150 217 and 236,
+// 480 x 200 262 and 257, 600 x 150 278 and 261, 888 x 141 398 and 334, 1332 x
+// 236 915 and 680; at M = 5/4 naux 600 x 470 523 and 529, 888 x 700 1159 and
+// 1167, 1500 x 1200 5325 and 5190, 2400 x 1920 19950 and 18950; 1500 x 1500
+// 7039 and 7186.
+bool half_pi(const Dims &d, int batch) {
+  const int64_t ctas = (d.M + 63) / 64 * ((d.naux + 63) / 64) * batch;
+  return (2 * d.M >= 3 * d.naux && ctas >= 592) || (4 * d.M >= 5 * d.naux && ctas >= 4096);
+}
+
 Chi0Bufs carve_chi0(Arena &ar, const Dims &d, int ntau, int nfreq, int mode, bool own_proj) {
   Chi0Bufs b{};
   b.w = ar.take<double>(static_cast<size_t>(nfreq) * ntau);
@@ -315,6 +332,7 @@ int chi0_run(const double *X, const Dims &d, const double *eps, double mu, const
       if (rc) return rc;
     }
     const int64_t mo = d.M * d.nocc, mv = d.M * d.nv, m2 = d.M * d.M, ma = d.M * d.naux;
+    const bool half = mode == MBPT_MODE_FP64 && half_pi(d, b.batch);
     for (int k = 0; k < ntau; k += b.batch) {
       const int nb = std::min(b.batch, ntau - k);
       launch_scaled_branches_batch(X, d.M, d.n, d.nocc, eps, mu, tau_list(tau + k, nb), b.Xo_s,
@@ -323,7 +341,7 @@ int chi0_run(const double *X, const Dims &d, const double *eps, double mu, const
       // (MBPTcode space_time.py:525-526), Y = Pi D, proj = -2 D^T Y
       int rc = dmma::hadamard_product({b.Xo_s, d.nocc, mo}, {X, d.n, 0}, d.nocc,
                                       {b.Xv_s, d.nv, mv}, {X + d.nocc, d.n, 0}, d.nv, d.M, b.Go,
-                                      d.M, m2, nb, st);
+                                      d.M, m2, nb, st, nullptr, nullptr, half);
       for (int i = 0; mode == MBPT_MODE_FP64_INT8 && !rc && i < nb; ++i)
         if (!gemm_mode(mode, h, false, false, d.M, d.naux, d.M, 1.0, b.Go + i * m2, d.M, D, d.naux,
                        0.0, b.Y, d.naux, false, nullptr, &Dt) ||
@@ -333,10 +351,18 @@ int chi0_run(const double *X, const Dims &d, const double *eps, double mu, const
       if (rc) return rc;
       if (mode == MBPT_MODE_FP64_INT8) continue;
       rc = dmma::gemm({b.Go, d.M, m2}, true, {D, d.naux, 0}, false, d.M, d.naux, d.M, 1.0, 0.0,
-                        b.Y, d.naux, ma, nb, false, st);
-      if (!rc)
+                      b.Y, d.naux, ma, nb, false, st, half);
+      if (!rc && half) {
+        // Z = -4 D^T (T D) where Pi = T + T^T was, proj = (Z + Z^T) / 2; the
+        // parts of Z fit where Pi was
+        const int parts = std::min<int64_t>(dmma::product_parts(d.naux, d.naux, d.M, nb), m2 / a2);
+        rc = dmma::gemm_parts({D, d.naux, 0}, {b.Y, d.naux, ma}, d.naux, d.naux, d.M, -4.0, b.Go,
+                              d.naux, a2, nb, parts, st);
+        launch_sym_half(b.Go, proj + k * a2, d.naux, nb, st, parts);
+      } else if (!rc) {
         rc = dmma::gemm({D, d.naux, 0}, false, {b.Y, d.naux, ma}, false, d.naux, d.naux, d.M,
                         -2.0, 0.0, proj + k * a2, d.naux, a2, nb, true, st);
+      }
       if (rc) return rc;
     }
     launch_transform<double>(proj, a2, d.naux, d.naux, d.naux, b.w, nfreq, ntau, chi0, a2,

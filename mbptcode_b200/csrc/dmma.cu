@@ -24,6 +24,12 @@
 // warps) 32.8, two CTAs per SM with a deeper ring 32.1. The sweep with it
 // (n = 400, M = naux = 2400, 20 points): chi0 36.9 -> 27.2 ms, Sigma of 400
 // states 45.0 -> 31.8 ms; E_c at M = 888, naux = 141: 1.51 -> 0.72 ms.
+// With Pi by halves (half: the product with T reads K from each row tile's
+// first row, every member's longest sums first: 179 -> 103 us at M = 888, naux
+// = 141, 20 points), D^T Y cut along K where its CTAs are few (72 -> 49 us
+// there), no DMMAs on the padding of a product's last K tile (Pi of 5 + 38
+// orbitals at M = 888: 65 -> 46 us) and 16-byte stores: E_c of that case 0.58
+// -> 0.49 ms, G0W0 at M = 1332 2.07 -> 1.72 ms.
 //
 // The Dyson step's FP64 products run on the same kernel, all frequencies (and
 // all halvings of one depth of the triangular inverse) in one launch: the
@@ -178,6 +184,11 @@ struct Args {
   bool wa[3], wb[3];  // 16-byte copies
   int m, n, tiles_m, tiles_n;
   bool upper;
+  bool half;       // PRODUCT: upper tiles only, the diagonal ones halved; STORE: A is such a half
+  bool pairs;      // 16-byte stores
+  int members;     // half: the batch, all in one grid dimension
+  int ksplit;      // STORE: K in so many parts, each with a result of its own
+  int64_t s_part;
   double alpha, beta;
   double *c0, *c1, *c2;  // PRODUCT: c1, c2 the factors themselves (null: not kept)
   int64_t ldc, sc;
@@ -194,9 +205,14 @@ struct Args {
   Node node[kMaxNodes];
 };
 
+// the K columns of one of `parts` parts of k: whole tiles
+__host__ __device__ constexpr int round_to(int k, int parts) {
+  return ((k + parts - 1) / parts + BK - 1) / BK * BK;
+}
+
 enum Epi : int {
-  STORE = 0,     // C = alpha acc + beta C (upper: and its mirror)
-  PRODUCT = 1,   // C = acc0 o acc1, mirrored
+  STORE = 0,     // C = alpha acc + beta C (upper: and its mirror; half: K from the tile's first row)
+  PRODUCT = 1,   // C = acc0 o acc1, mirrored (half: as SIGMA's)
   SIGMA = 2,     // c0 = acc1 o acc0, c1 = acc2 o acc0: upper tiles, the diagonal ones halved
   ROWDOT = 3,    // out[p] += alpha sum_r xs[r, p] acc[r, p], K from the tile's first row
   CHOL = 4,      // C = I - src - acc, on and above the diagonal
@@ -217,6 +233,8 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
   int ti, tj;
   int rows_m = p.m, rows_n = p.n, k_end0 = p.k[0];
   int64_t z = blockIdx.z, off_a = 0, off_b = 0, off_c = 0;
+  unsigned tile = blockIdx.x;
+  int k_begin = 0;
   if constexpr (EPI == NODE_T || EPI == NODE_V) {
     const Node &q = p.node[z % p.nnodes];
     z /= p.nnodes;
@@ -228,15 +246,27 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
     off_b = EPI == NODE_T ? o1 * p.b[0].ld + o1 : o2 * p.b[0].ld + o2;
     off_c = EPI == NODE_T ? o2 * p.ldc + o1 : o1 * p.ldc + o2;
     const int tn = (rows_n + BN - 1) / BN;
-    ti = blockIdx.x / tn;
-    tj = blockIdx.x % tn;
+    ti = tile / tn;
+    tj = tile % tn;
     if (ti * BM >= rows_m) return;
   } else if (p.upper) {
-    upper_tile(blockIdx.x, p.tiles_m, ti, tj);
+    upper_tile(tile, p.tiles_m, ti, tj);
   } else {
+    if constexpr (EPI == STORE) {
+      if (p.half) {  // the longest sums of all members first
+        z = tile % p.members;
+        tile /= p.members;
+      } else if (p.ksplit > 1) {
+        const int part = z % p.ksplit, per = round_to(p.k[0], p.ksplit);
+        k_begin = part * per;
+        k_end0 = min(k_end0, k_begin + per);
+        off_c = part * p.s_part;
+        z /= p.ksplit;
+      }
+    }
     // eight row tiles sweep the column tiles together (L2 reuse)
-    const int per = 8 * p.tiles_n, grp = blockIdx.x / per, first = grp * 8;
-    const int rows = min(8, p.tiles_m - first), in = blockIdx.x % per;
+    const int per = 8 * p.tiles_n, grp = tile / per, first = grp * 8;
+    const int rows = min(8, p.tiles_m - first), in = tile % per;
     ti = first + in % rows;
     tj = in / rows;
   }
@@ -245,18 +275,20 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
     if (p.info && p.info[z] != 0) return;
   }
   if (EPI == CHOL && n0 + BN <= m0) return;
-  const int k_first = EPI == ROWDOT ? m0 : (EPI == INVERSE || EPI == NODE_T ? n0 : 0);
+  const int k_first = EPI == ROWDOT || (EPI == STORE && p.half)
+                          ? m0
+                          : (EPI == INVERSE || EPI == NODE_T ? n0 : k_begin);
   if (EPI == NODE_V) k_end0 = min(k_end0, n0 + BN);
-  int tiles[NS], total = 0;
+  // a product's K columns and tiles
+  auto depth = [&](int s) { return (s == 0 ? k_end0 : p.k[s]) - k_first; };
+  auto tiles = [&](int s) { return (depth(s) + BK - 1) / BK; };
+  int total = 0;
 #pragma unroll
-  for (int s = 0; s < NS; ++s) {
-    tiles[s] = ((s == 0 ? k_end0 : p.k[s]) - k_first + BK - 1) / BK;
-    total += tiles[s];
-  }
+  for (int s = 0; s < NS; ++s) total += tiles(s);
   // the tiles of the products, one product after the other
   Stream<AK, BM> fa;
   Stream<BKC, BN> fb;
-  int fseg = EPI == SIGMA && tiles[0] == 0 ? 1 : 0, fleft = tiles[fseg], fstage = 0;
+  int fseg = EPI == SIGMA && k_end0 == 0 ? 1 : 0, fleft = tiles(fseg), fstage = 0;
   auto open = [&](int s) {
     const int ke = s == 0 ? k_end0 : p.k[s];
     fa.start(p.a[s].p + z * p.a[s].stride + off_a, p.a[s].ld, m0, rows_m, k_first, ke, p.wa[s]);
@@ -270,7 +302,7 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
     fstage = fstage + 1 == kStages ? 0 : fstage + 1;
     if (NS > 1 && --fleft == 0 && fseg + 1 < NS) {
       ++fseg;
-      fleft = tiles[fseg < NS ? fseg : 0];
+      fleft = tiles(fseg < NS ? fseg : 0);
       open(fseg < NS ? fseg : 0);
     }
   };
@@ -289,16 +321,24 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
       const int r = m0 + wm + 8 * i + g;
       if (r >= rows_m) continue;
 #pragma unroll
-      for (int j = 0; j < NJ; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int col = n0 + wn + 8 * j + 2 * t + e;
-          if (col >= rows_n) continue;
-          double *at = c + z * p.sc + off_c + static_cast<int64_t>(r) * p.ldc + col;
-          const double v = value(i, j, e, at);
-          *at = v;
-          if (mirror) c[z * p.sc + static_cast<int64_t>(col) * p.ldc + r] = v;
+      for (int j = 0; j < NJ; ++j) {
+        const int col = n0 + wn + 8 * j + 2 * t;
+        if (col >= rows_n) continue;
+        double *at = c + z * p.sc + off_c + static_cast<int64_t>(r) * p.ldc + col;
+        const bool two = col + 1 < rows_n;
+        const double v0 = value(i, j, 0, at), v1 = two ? value(i, j, 1, at + 1) : 0.0;
+        if (two && p.pairs) {
+          *reinterpret_cast<double2 *>(at) = make_double2(v0, v1);
+        } else {
+          at[0] = v0;
+          if (two) at[1] = v1;
         }
+        if (mirror) {
+          double *tr = c + z * p.sc + static_cast<int64_t>(col) * p.ldc + r;
+          tr[0] = v0;
+          if (two) tr[p.ldc] = v1;
+        }
+      }
     }
   };
   clear();
@@ -314,12 +354,12 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
         for (int e = 0; e < 2; ++e)
           if (m0 + wm + 8 * i + g == n0 + wn + 8 * j + 2 * t + e) acc[i][j][e] = -1.0;
   }
-  int seg_end = tiles[0];
+  int seg_end = tiles(0);
   [[maybe_unused]] int seg = 0;
   if constexpr (EPI == SIGMA) {
     if (p.zt) {
       seg = 1;
-      seg_end = tiles[1];
+      seg_end = tiles(1);
 #pragma unroll
       for (int i = 0; i < MI; ++i)
 #pragma unroll
@@ -344,8 +384,7 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
     cp_commit();
     const double *sa = sm + stage * S::kStage, *sb = sa + S::kA;
     stage = stage + 1 == kStages ? 0 : stage + 1;
-#pragma unroll
-    for (int kk = 0; kk < BK; kk += 4) {
+    auto step = [&](int kk) {
       double a[MI], b[NJ];
 #pragma unroll
       for (int i = 0; i < MI; ++i) a[i] = sa[Tile<AK, BM>::at(wm + 8 * i + g, kk + t)];
@@ -355,6 +394,16 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
       for (int i = 0; i < MI; ++i)
 #pragma unroll
         for (int j = 0; j < NJ; ++j) mma(acc[i][j], a[i], b[j]);
+    };
+    // a product's last tile takes the steps that it has columns for (5 occupied
+    // and 53 virtual orbitals: 16 steps instead of 20)
+    if (it + 1 == seg_end) {
+      const int left = (depth(seg) - 1) % BK;
+#pragma unroll 1
+      for (int kk = 0; kk <= left; kk += 4) step(kk);
+    } else {
+#pragma unroll
+      for (int kk = 0; kk < BK; kk += 4) step(kk);
     }
     if constexpr (NS > 1) {
       if (it + 1 == seg_end && seg + 1 < NS) {
@@ -373,7 +422,7 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
         }
         clear();
         ++seg;
-        seg_end += tiles[seg < NS ? seg : 0];
+        seg_end += tiles(seg < NS ? seg : 0);
       }
     }
   }
@@ -400,8 +449,9 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
           },
           p.upper && tj > ti);
   } else if constexpr (EPI == PRODUCT) {
-    store(p.c0, [&](int i, int j, int e, double *) { return acc[i][j][e] * keep[i][j][e]; },
-          tj > ti);
+    const double f = p.half && ti == tj ? 0.5 : 1.0;
+    store(p.c0, [&](int i, int j, int e, double *) { return acc[i][j][e] * keep[i][j][e] * f; },
+          !p.half && tj > ti);
     if (p.c1) {
       store(p.c1, [&](int i, int j, int e, double *) { return keep[i][j][e]; }, tj > ti);
       store(p.c2, [&](int i, int j, int e, double *) { return acc[i][j][e]; }, tj > ti);
@@ -446,6 +496,10 @@ int launch(Args &p, int batch, cudaStream_t st) {
     p.wa[s] = wide(p.a[s], batch);
     p.wb[s] = wide(p.b[s], batch);
   }
+  // the second and third results lie as the first
+  p.pairs = p.ldc % 2 == 0 && (batch <= 1 || p.sc % 2 == 0) && p.s_part % 2 == 0 &&
+            ((reinterpret_cast<uintptr_t>(p.c0) | reinterpret_cast<uintptr_t>(p.c1) |
+              reinterpret_cast<uintptr_t>(p.c2)) & 15) == 0;
   p.tiles_m = (p.m + BM - 1) / BM;
   p.tiles_n = (p.n + BN - 1) / BN;
   if (p.upper && (BN != BM || p.m != p.n)) return MBPT_ERR_SHAPE;
@@ -453,9 +507,21 @@ int launch(Args &p, int batch, cudaStream_t st) {
   if ((EPI == NODE_T || EPI == NODE_V) && static_cast<int64_t>(batch) * p.nnodes > 65535)
     return MBPT_ERR_SHAPE;
   if (EPI == NODE_T || EPI == NODE_V) batch *= p.nnodes;
-  const int64_t grid = p.upper ? static_cast<int64_t>(p.tiles_m) * (p.tiles_m + 1) / 2
-                               : static_cast<int64_t>(p.tiles_m) * p.tiles_n;
+  int64_t grid = p.upper ? static_cast<int64_t>(p.tiles_m) * (p.tiles_m + 1) / 2
+                         : static_cast<int64_t>(p.tiles_m) * p.tiles_n;
   if (grid > (int64_t{1} << 30)) return MBPT_ERR_SHAPE;
+  if (EPI == STORE && p.half) {
+    p.members = batch;
+    if (grid * batch > (int64_t{1} << 30)) return MBPT_ERR_SHAPE;
+    grid *= batch;
+    batch = 1;
+  } else if (EPI == STORE && p.ksplit > 1) {
+    // every part has a first column
+    if (round_to(p.k[0], p.ksplit) * (p.ksplit - 1) >= p.k[0] ||
+        static_cast<int64_t>(batch) * p.ksplit > 65535 || p.upper)
+      return MBPT_ERR_SHAPE;
+    batch *= p.ksplit;
+  }
   auto kern = dmma_kernel<BN, AK, BKC, EPI>;
   static std::atomic<uint64_t> attr{0};
   if (!allow_smem(reinterpret_cast<const void *>(kern), S::kBytes, attr)) return MBPT_ERR_CUDA;
@@ -470,13 +536,17 @@ int launch(Args &p, int batch, cudaStream_t st) {
 // alike; 24.7 against 21.1 at n = 141, 160 columns against 192).
 bool narrow(int64_t n) { return round_up(n, 64) * 20 >= round_up(n, 32) * 21; }
 
+// A product with fewer CTAs than four per SM is cut along K.
+constexpr int64_t kFewCtas = 4 * 148;
+
 bool fits(int64_t v) { return v > 0 && v <= (int64_t{1} << 30); }
 
 }  // namespace
 
 int gemm(const Operand &a, bool a_k, const Operand &b, bool b_k, int64_t m, int64_t n, int64_t k,
          double alpha, double beta, double *c, int64_t ldc, int64_t sc, int batch, bool upper,
-         cudaStream_t st) {
+         cudaStream_t st, bool half) {
+  if (half && (!a_k || m != k)) return MBPT_ERR_SHAPE;
   if (!fits(m) || !fits(n) || !fits(k)) return MBPT_ERR_SHAPE;
   Args p{};
   p.a[0] = a;
@@ -490,6 +560,7 @@ int gemm(const Operand &a, bool a_k, const Operand &b, bool b_k, int64_t m, int6
   p.ldc = ldc;
   p.sc = sc;
   p.upper = upper;
+  p.half = half;
   if (a_k && b_k) return launch<64, true, true, STORE>(p, batch, st);
   if (a_k && narrow(n)) return launch<32, true, false, STORE>(p, batch, st);
   if (a_k) return launch<64, true, false, STORE>(p, batch, st);
@@ -497,9 +568,35 @@ int gemm(const Operand &a, bool a_k, const Operand &b, bool b_k, int64_t m, int6
   return MBPT_ERR_UNSUPPORTED;
 }
 
+int product_parts(int64_t m, int64_t n, int64_t k, int batch) {
+  const int64_t ctas = ((m + BM - 1) / BM) * ((n + 63) / 64) * batch;
+  int parts = 1;
+  while (parts < kMaxParts && ctas * parts < kFewCtas && k >= 128 * (parts + 1)) ++parts;
+  return parts;
+}
+
+int gemm_parts(const Operand &a, const Operand &b, int64_t m, int64_t n, int64_t k, double alpha,
+               double *c, int64_t ldc, int64_t sc, int batch, int parts, cudaStream_t st) {
+  if (!fits(m) || !fits(n) || !fits(k)) return MBPT_ERR_SHAPE;
+  Args p{};
+  p.a[0] = a;
+  p.b[0] = b;
+  p.k[0] = static_cast<int>(k);
+  p.m = static_cast<int>(m);
+  p.n = static_cast<int>(n);
+  p.alpha = alpha;
+  p.c0 = c;
+  p.ldc = ldc;
+  p.sc = sc;
+  p.ksplit = parts;
+  p.s_part = sc * batch;
+  return launch<64, false, false, STORE>(p, batch, st);
+}
+
 int hadamard_product(const Operand &a0, const Operand &b0, int64_t k0, const Operand &a1,
                      const Operand &b1, int64_t k1, int64_t m, double *c, int64_t ldc,
-                     int64_t sc, int batch, cudaStream_t st, double *g0, double *g1) {
+                     int64_t sc, int batch, cudaStream_t st, double *g0, double *g1,
+                     bool half) {
   if (!fits(m) || !fits(k0) || !fits(k1)) return MBPT_ERR_SHAPE;
   Args p{};
   p.a[0] = a0;
@@ -515,6 +612,7 @@ int hadamard_product(const Operand &a0, const Operand &b0, int64_t k0, const Ope
   p.ldc = ldc;
   p.sc = sc;
   p.upper = true;
+  p.half = half;
   return launch<64, true, true, PRODUCT>(p, batch, st);
 }
 

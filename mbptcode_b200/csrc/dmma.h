@@ -16,18 +16,30 @@ struct Operand {
 // C (m x n, row-major, ldc) = alpha A B^T + beta C per batch member, A (m x k)
 // and B (n x k) K-contiguous (a_k, b_k) or row-contiguous (not A
 // row-contiguous with B K-contiguous). upper: the product is symmetric (m ==
-// n): the tiles on and above the diagonal are formed and mirrored.
+// n): the tiles on and above the diagonal are formed and mirrored. half: A
+// (m x m, K-contiguous) is held by halves (below): of each row tile, K runs
+// from the tile's first row on.
 int gemm(const Operand &a, bool a_k, const Operand &b, bool b_k, int64_t m, int64_t n, int64_t k,
          double alpha, double beta, double *c, int64_t ldc, int64_t sc, int batch, bool upper,
-         cudaStream_t st);
+         cudaStream_t st, bool half = false);
+
+// C_0 + ... + C_{parts-1} = alpha A B^T, A and B row-contiguous: each part sums
+// its own range of K and lies batch sc doubles after the one before.
+// product_parts: the number of parts that fills the GPU (1 to kMaxParts).
+constexpr int kMaxParts = 8;
+int product_parts(int64_t m, int64_t n, int64_t k, int batch);
+int gemm_parts(const Operand &a, const Operand &b, int64_t m, int64_t n, int64_t k, double alpha,
+               double *c, int64_t ldc, int64_t sc, int batch, int parts, cudaStream_t st);
 
 // C (m x m) = (A0 B0^T) o (A1 B1^T), both symmetric: Pi = G_occ o G_virt.
 // All operands K-contiguous. g0, g1: the two factors as well, laid out as C
-// (both or neither).
+// (both or neither). half: C is held by halves, the 64 x 64 tiles on and above
+// the diagonal only, the diagonal ones times 1/2, so that C = T + T^T for the
+// T that is stored.
 int hadamard_product(const Operand &a0, const Operand &b0, int64_t k0, const Operand &a1,
                      const Operand &b1, int64_t k1, int64_t m, double *c, int64_t ldc,
                      int64_t sc, int batch, cudaStream_t st, double *g0 = nullptr,
-                     double *g1 = nullptr);
+                     double *g1 = nullptr, bool half = false);
 
 // Zt = U D^T, hl = (Xo_s Xo^T) o Zt and hg = (Xv_s Xv^T) o Zt (all symmetric,
 // K-contiguous operands), leading dimension m, as `half_quadratic` reads
