@@ -26,7 +26,7 @@
 // columns), warp 0 the TMA producer (64-byte swizzled boxes of 64 K), warp 1
 // the TMEM owner and MMA issuer (the S(S+1)/2 products of a 32-wide K step
 // as one MMA per A plane and group of up to four B planes), warps
-// 2-5 the epilogue; two pipeline stages of S A-planes and S B-planes; every
+// 2-9 the epilogue; two pipeline stages of S A-planes and S B-planes; every
 // mbarrier wait bounded, as in the split engine.
 #include <algorithm>
 
@@ -62,10 +62,11 @@ struct Layout {
   static constexpr int kStageBytes = S * (kAPlane + kBPlane);
   // as many stages as 196 KB hold: 2 for S = 7 and 8 (84 and 96 KB each)
   static constexpr int kStages = (196 * 1024) / kStageBytes < 8 ? (196 * 1024) / kStageBytes : 8;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
+  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 512;
   static constexpr int kLevels = S;
   static constexpr int kTmemCols = 512;
   static_assert(kLevels * BN <= 512, "levels exceed TMEM");
+  static_assert(kStages * kStageBytes >= 16 * 32 * 33 * 8, "the epilogue's blocks");
 };
 
 __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *tm, int x, int y,
@@ -121,6 +122,18 @@ __device__ __forceinline__ void tmem_ld32_s32(uint32_t addr, int (&v)[32]) {
       : "memory");
 }
 
+__device__ __forceinline__ void tmem_ld16_s32(uint32_t addr, int (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
+        "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(addr)
+      : "memory");
+}
+
 // Shared tile of the cutting kernels, 32 rows x 128 columns: one double of
 // padding per 16 columns and a row stride of 137, so that a half warp hits 16
 // different 8-byte banks when it writes 16 columns or 16 rows, and 15 when it
@@ -140,6 +153,12 @@ __device__ __forceinline__ int8_t next_digit(double &t, double base) {
   const double r = t + kMagic;
   t = (t - (r - kMagic)) * base;
   return static_cast<int8_t>(__double2loint(r));
+}
+
+// An int32 as a double by one FP64 addition (the conversion unit takes 16 lanes
+// per clock and SM, a quarter of the FP64 pipe's rate)
+__device__ __forceinline__ double exact_double(int v) {
+  return __hiloint2double(0x43300000, v ^ static_cast<int>(0x80000000u)) - 4503601774854144.0;
 }
 
 enum Epi : int {
@@ -173,22 +192,81 @@ struct UpdateArgs {
   int *err;
 };
 
+// Weights of the levels: 2^(2 - 7 l), and 127^-2 254^-(l - 2) for the 8-bit
+// digits (the powers of 254 are exact, so each is one rounding), l = 2 on.
+__constant__ double kLevel7[8] = {0x1p-12, 0x1p-19, 0x1p-26, 0x1p-33,
+                                  0x1p-40, 0x1p-47, 0x1p-54, 0x1p-61};
+__constant__ double kLevel6[6] = {1.0 / 16129.0,
+                                  1.0 / (16129.0 * 254.0),
+                                  1.0 / (16129.0 * 254.0 * 254.0),
+                                  1.0 / (16129.0 * 254.0 * 254.0 * 254.0),
+                                  1.0 / (16129.0 * 254.0 * 254.0 * 254.0 * 254.0),
+                                  1.0 / (16129.0 * 254.0 * 254.0 * 254.0 * 254.0 * 254.0)};
+constexpr int kThreads = 320;
+
+// The N columns at taddr of all levels, combined: smallest levels first.
+template <int S, int N>
+__device__ __forceinline__ void levels(uint32_t taddr, double (&acc)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) acc[i] = 0.0;
+#pragma unroll 1
+  for (int lev = S - 1; lev >= 0; --lev) {
+    int v[N];
+    if constexpr (N == 16)
+      tmem_ld16_s32(taddr + static_cast<uint32_t>(lev * BN), v);
+    else
+      tmem_ld32_s32(taddr + static_cast<uint32_t>(lev * BN), v);
+    const double w = S == 6 ? kLevel6[lev] : kLevel7[lev];
+#pragma unroll
+    for (int i = 0; i < N; ++i) acc[i] += exact_double(v[i]) * w;
+  }
+}
+
+// What the epilogue takes matters as much as the products' rate: combining
+// eight levels costs 1.6e5 FP64 operations a tile, and a tile's products last
+// 57 us at K = 2400. With four warps that loaded and stored 64 columns of
+// their own rows in eight round trips it was 16 us on top (the tensor pipe
+// idle); eight warps, blocks turned in shared memory and the Cholesky's
+// chi0 entries fetched while the products run: 3.3 us. Measured: products of
+// 1000, 2400 and 4096 with their operand cutting 70, 467 and 1890 -> 57, 402
+// and 1690 us, the factor of 24 x 5400 (six digits) 19.3 -> 17.1 ms, of 24 x
+// 2400 3.35 -> 2.90. What is left is the products' operand traffic: a stage
+// (two K steps) of S = 8 reads 96 KB of A and 144 KB of B from shared memory
+// and has 96 KB written to it, 2690 clocks at 128 bytes a clock where its MMAs
+// take 2300; 2684 measured.
 template <int S, int EPI>
-__global__ void __launch_bounds__(192, 1) chol_update_kernel(const __grid_constant__ UpdateArgs p) {
+__global__ void __launch_bounds__(kThreads, 1) chol_update_kernel(const __grid_constant__ UpdateArgs p) {
   static_assert(S != 6 || EPI == EPI_CHOL, "8-bit digits: the Cholesky's planes only");
   using L = Layout<S>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  // A stage is filled and freed in G chunks of C A planes: full[0] covers the
+  // first chunk and all B planes, full[g] chunk g; empty[g] the A planes of
+  // chunk g and the B planes that no later step reads. One barrier per stage
+  // refills it only once all of its products are done, and the next stage's
+  // products are short cover for that on a few K steps: the Cholesky's factor
+  // of 24 x 5400 21.2 -> 19.3 ms with chunks of two, 2400 3.55 -> 3.35 (one
+  // plane a chunk: 20.9 and 3.51); a product at 3100 1.01 -> 0.99 ms with four.
+  constexpr int C = EPI == EPI_CHOL ? 2 : 4, G = (S + C - 1) / C;
   uint64_t *full = reinterpret_cast<uint64_t *>(smem + L::kStages * L::kStageBytes);
-  uint64_t *empty = full + L::kStages;
-  uint64_t *accum = empty + L::kStages;
+  uint64_t *empty = full + L::kStages * G;
+  uint64_t *accum = empty + L::kStages * G;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(accum + 1);
   int *fail = reinterpret_cast<int *>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int f = blockIdx.y;
-  const int tm = blockIdx.x / p.tiles_n, tn = blockIdx.x % p.tiles_n;
+  int tm = blockIdx.x / p.tiles_n, tn = blockIdx.x % p.tiles_n;
+  if (EPI == EPI_GEMM) {
+    // down strips of 16 column tiles: the CTAs in flight read 9 rows of A
+    // tiles and 16 of B instead of 3 and all of them (from memory once the
+    // planes outgrow L2: 3100 0.99 -> 0.97 ms, 4096 1.90 -> 1.88)
+    const int per = 16 * p.tiles_m, first = blockIdx.x / per * 16, in = blockIdx.x % per;
+    const int cols = min(16, p.tiles_n - first);
+    tm = in / cols;
+    tn = first + in % cols;
+  }
   const int r0 = tm * BM;       // tile row (Cholesky: matrix row j0 + r0)
   const int c0 = tn * BN;       // tile column
   // uniform: the second half of a narrow last panel, a tile below the
@@ -198,10 +276,7 @@ __global__ void __launch_bounds__(192, 1) chol_update_kernel(const __grid_consta
   const int m = static_cast<int>(p.n - p.j0);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < L::kStages; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], 1);
-    }
+    for (int s = 0; s < 2 * L::kStages * G; ++s) mbar_init(&full[s], 1);
     mbar_init(accum, 1);
     *fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -223,53 +298,63 @@ __global__ void __launch_bounds__(192, 1) chol_update_kernel(const __grid_consta
     if (lane == 0) {
       bool ok = true;
       int it = 0;
-      for (int kt = 0; kt < p.k_tiles; ++kt, ++it) {
+      for (int kt = 0; kt < p.k_tiles && ok; ++kt, ++it) {
         const int s = it % L::kStages;
         const uint32_t ph = (it / L::kStages) & 1;
-        if (!mbar_wait(&empty[s], ph ^ 1)) { ok = false; break; }
-        mbar_expect_tx(&full[s], L::kStageBytes);
         uint8_t *st = smem + s * L::kStageBytes;
+        uint64_t *fs = full + s * G, *es = empty + s * G;
         const int kx = kt * BKB;
 #pragma unroll
-        for (int q = 0; q < S; ++q) {
-          const int plane = q * p.nmat + f;
-          tma_load_3d(st + q * L::kAPlane, &p.tm_a, kx, p.a_row0 + r0, plane, &full[s]);
-          tma_load_3d(st + S * L::kAPlane + q * L::kBPlane, &p.tm_b, kx, p.b_row0 + c0, plane,
-                      &full[s]);
+        for (int g = 0; g < G; ++g) {
+          if (!mbar_wait(&es[g], ph ^ 1)) { ok = false; break; }
+          const int q1 = (g + 1) * C < S ? (g + 1) * C : S;
+          mbar_expect_tx(&fs[g], (q1 - g * C) * L::kAPlane + (g == 0 ? S * L::kBPlane : 0));
+#pragma unroll
+          for (int q = g * C; q < q1; ++q) {
+            const int t = G > 1 ? S - 1 - q : q;
+            tma_load_3d(st + q * L::kAPlane, &p.tm_a, kx, p.a_row0 + r0, q * p.nmat + f, &fs[g]);
+            tma_load_3d(st + S * L::kAPlane + t * L::kBPlane, &p.tm_b, kx, p.b_row0 + c0,
+                        t * p.nmat + f, &fs[0]);
+          }
         }
       }
       if (!ok) {
         atomicExch(fail, 1);
         DevErr{p.err}.set(MBPT_ERR_TIMEOUT);
       }
-      for (int q = max(0, it - L::kStages); q < it; ++q)
-        mbar_wait(&full[q % L::kStages], (q / L::kStages) & 1);
+      for (int k = max(0, it - L::kStages); k < it; ++k)
+        for (int g = 0; g < G; ++g)
+          mbar_wait(&full[k % L::kStages * G + g], (k / L::kStages) & 1);
     }
     __syncwarp();
   } else if (warp == 1) {
     if (lane == 0) {
       bool ok = true;
-      for (int kt = 0; kt < p.k_tiles; ++kt) {
+      for (int kt = 0; kt < p.k_tiles && ok; ++kt) {
         const int s = kt % L::kStages;
         const uint32_t ph = (kt / L::kStages) & 1;
-        if (!mbar_wait(&full[s], ph) || *reinterpret_cast<volatile int *>(fail)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
         const uint32_t st = smem_u32(smem + s * L::kStageBytes);
+        // A plane sa against the B planes 1 .. S + 1 - sa stacked as one
+        // operand (they lie back to back, 64 rows each): product (sa, t)
+        // lands in column block sa + t - 2, its level's accumulator, so one
+        // MMA of up to 256 columns serves four levels and A is read from
+        // shared memory once per four products. Plane 1 covers every
+        // level, so its MMAs open the accumulators. After step sa its A plane
+        // and B plane S + 1 - sa are not read again.
 #pragma unroll
-        for (int kk = 0; kk < BKB / 32; ++kk) {
-          const uint64_t adv = static_cast<uint64_t>(kk * 2);  // 32 bytes >> 4
-          const bool first = kt == 0 && kk == 0;
-          // A plane sa against the B planes 1 .. S + 1 - sa stacked as one
-          // operand (they lie back to back, 64 rows each): product (sa, t)
-          // lands in column block sa + t - 2, its level's accumulator, so one
-          // MMA of up to 256 columns serves four levels and A is read from
-          // shared memory once per four products. Plane 1 covers every
-          // level, so its MMAs open the accumulators.
+        for (int sa = 1; sa <= S; ++sa) {
+          if ((sa - 1) % C == 0) {
+            if (!mbar_wait(&full[s * G + (sa - 1) / C], ph) ||
+                *reinterpret_cast<volatile int *>(fail)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+          }
 #pragma unroll
-          for (int sa = 1; sa <= S; ++sa) {
+          for (int kk = 0; kk < BKB / 32; ++kk) {
+            const uint64_t adv = static_cast<uint64_t>(kk * 2);  // 32 bytes >> 4
+            const bool first = kt == 0 && kk == 0;
             const uint64_t da = kmajor_desc(st + (sa - 1) * L::kAPlane) + adv;
 #pragma unroll
             for (int t0 = 1; t0 <= S + 1 - sa; t0 += kStackPlanes) {
@@ -281,8 +366,8 @@ __global__ void __launch_bounds__(192, 1) chol_update_kernel(const __grid_consta
               mma_s8(d, da, db, idesc_s8(cnt * BN), (first && sa == 1) ? 0u : 1u);
             }
           }
+          if (sa % C == 0 || sa == S) mma_commit(&empty[s * G + (sa - 1) / C]);
         }
-        mma_commit(&empty[s]);
       }
       if (!ok) {
         atomicExch(fail, 1);
@@ -293,112 +378,116 @@ __global__ void __launch_bounds__(192, 1) chol_update_kernel(const __grid_consta
     }
     __syncwarp();
   } else {
-    const int sp = warp & 3;
-    const uint32_t taddr = tmem + (static_cast<uint32_t>(sp * 32) << 16);
+    // eight warps: rows by the TMEM lanes a warp reaches, columns by halves
+    const int sp = warp & 3, ch = (warp - 2) >> 2;
+    const uint32_t taddr = tmem + (static_cast<uint32_t>(sp * 32) << 16) + ch * 32;
+    const int pr = r0 + sp * 32 + lane;             // tile row of this thread
+    const int cb = c0 + ch * 32;                    // the warp's first column
+    double old[EPI == EPI_CHOL ? 32 : 1], scol = 0.0, srow = 0.0, diag = 0.0;
+    const bool live = EPI == EPI_CHOL && pr < m;
+    if constexpr (EPI == EPI_CHOL) {
+      // what the result takes from memory, while the products run
+      const double *sc = p.scale + static_cast<int64_t>(f) * p.n + p.j0;
+      const double *Arow = p.A0 + f * p.n * p.n + p.j0 * (p.n + 1) + pr;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const int pc = cb + i;  // panel column
+        old[i] = (pr == pc ? 1.0 : 0.0) - (live && pc < p.nb ? Arow[pc * p.n] : 0.0);
+      }
+      srow = live ? sc[pr] : 0.0;
+      scol = cb + lane < p.nb ? sc[cb + lane] : 0.0;
+      // the diagonal entry comes from the exact running row norm
+      if (pr >= cb && pr < cb + 32 && pr < p.nb)
+        diag = p.rowsq[static_cast<int64_t>(f) * p.n + p.j0 + pr];
+    } else {
+      srow = pr < p.m_rows ? p.alpha * p.scale[pr] : 0.0;
+      scol = cb + lane < p.n_cols ? p.scale_b[cb + lane] : 0.0;
+    }
     const bool ok = mbar_wait(accum, 0) && !*reinterpret_cast<volatile int *>(fail);
     __syncwarp();
     if (!ok) {
       if (lane == 0) DevErr{p.err}.set(MBPT_ERR_TIMEOUT);
     } else {
       tc_fence_after();
-      const int pr = r0 + sp * 32 + lane;             // tile row of this thread
-      const bool live = EPI == EPI_CHOL ? pr < m : pr < p.m_rows;
-      const int64_t row = EPI == EPI_CHOL ? p.j0 + pr : pr;
-      const double *sc = p.scale + (EPI == EPI_CHOL ? static_cast<int64_t>(f) * p.n : 0);
-      const double srow = live ? sc[row] : 0.0;
-      double *P = EPI == EPI_CHOL ? p.P + static_cast<int64_t>(f) * p.p_stride : nullptr;
-#pragma unroll 1
-      for (int ch = 0; ch < BN / 32; ++ch) {
-        double acc[32];
+      if constexpr (EPI == EPI_CHOL) {
+        double *Prow = p.P + static_cast<int64_t>(f) * p.p_stride + pr;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) acc[i] = 0.0;
-        // smallest levels first
-#pragma unroll 1
-        for (int lev = S + 1; lev >= 2; --lev) {
-          int v[32];
-          tmem_ld32_s32(taddr + static_cast<uint32_t>((lev - 2) * BN + ch * 32), v);
-          double w;
-          if constexpr (S == 6) {
-            // 1 / (127^2 254^(lev - 2)): the power is an exact integer below 2^53
-            double pw = 16129.0;
-            for (int q = 2; q < lev; ++q) pw *= 254.0;
-            w = 1.0 / pw;
-          } else {
-            w = ldexp(1.0, 2 - 7 * lev);
+        for (int h = 0; h < 32; h += 16) {
+          double acc[16];
+          levels<S>(taddr + h, acc);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const int pc = cb + h + i;
+            const double s = __shfl_sync(0xffffffffu, scol, h + i);
+            if (live && pc < p.nb)
+              Prow[static_cast<int64_t>(pc) * m] = pr == pc ? old[h + i] - diag
+                                                            : old[h + i] - acc[i] * srow * s;
           }
-#pragma unroll
-          for (int i = 0; i < 32; ++i) acc[i] += static_cast<double>(v[i]) * w;
         }
-        if (EPI == EPI_CHOL && live) {
-          // all 32 loads first (chi0's column entries and the columns' scales),
-          // then the stores: one memory round trip per chunk instead of one
-          // per column, which the compiler cannot reorder across the stores
-          // (two halves of 16 columns: the registers hold acc and one half)
-          double *Prow = P + pr;   // column pc of the panel at Prow + pc m
-          const double *Arow = p.A0 + f * p.n * p.n + p.j0 * (p.n + 1) + pr;
-          // the diagonal entry from the exact running row norm
-          const int pd = pr - c0 - ch * 32;
-          const double diag = (pd >= 0 && pd < 32 && pr < p.nb)
-                                  ? p.rowsq[static_cast<int64_t>(f) * p.n + p.j0 + pr] : 0.0;
+      } else {
+        double acc[32];
+        levels<S>(taddr, acc);
+        // the warp's 32 x 32 block through shared memory (the ring is free), so
+        // that rows are read and written 256 bytes at a time
+        constexpr int kRow = 33;
+        double *blk = reinterpret_cast<double *>(smem) + (warp - 2) * 32 * kRow;
 #pragma unroll
-          for (int h = 0; h < 32; h += 16) {
-            double old[16], scol[16];
+        for (int i = 0; i < 32; ++i) blk[lane * kRow + i] = srow * acc[i];
+        __syncwarp();
+        const int col = cb + lane, rb = r0 + sp * 32;
+        double *b2 = reinterpret_cast<double *>(smem) + (8 + warp - 2) * 32 * kRow;
+        const bool two = p.H1 && p.H2;
+        // this column's rows that are stored end here
+        const int last = col < p.n_cols ? (p.sym ? min(p.m_rows, col + 1) : p.m_rows) - rb : 0;
+#pragma unroll 1
+        for (int h = 0; h < 32; h += 16) {
+          double *c = p.C + static_cast<int64_t>(rb + h) * p.ldc + col;
+          const int n_in = last - h;
+          double v[16], g[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = blk[(h + i) * kRow + lane] * scol;
+          if (two) {
+            const double *h2 = p.H2 + (c - p.C);
+            double *c2 = p.C2 + (c - p.C);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) g[i] = i < n_in ? h2[i * p.ldc] : 0.0;
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
-              const int pc = c0 + ch * 32 + h + i;  // panel column
-              old[i] = (pr == pc ? 1.0 : 0.0) - (pc < p.nb ? Arow[pc * p.n] : 0.0);
-              scol[i] = pc < p.nb ? sc[p.j0 + pc] : 0.0;
-            }
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const int pc = c0 + ch * 32 + h + i;
-              if (pc < p.nb)
-                Prow[static_cast<int64_t>(pc) * m] =
-                    pr == pc ? old[i] - diag : old[i] - acc[h + i] * srow * scol[i];
+              g[i] *= v[i];
+              if (i < n_in) c2[i * p.ldc] = g[i];
+              if (p.sym) b2[(h + i) * kRow + lane] = g[i];
             }
           }
-        } else if (EPI == EPI_GEMM && live) {
-          const int64_t ro = static_cast<int64_t>(pr) * p.ldc;
-          const double a = p.alpha * srow;
-          // eight columns at a time: their loads (column scales, factors, the
-          // old C) ahead of their stores, one memory round trip per eight
+          if (p.H1) {
+            const double *h1 = p.H1 + (c - p.C);
 #pragma unroll
-          for (int h = 0; h < 32; h += 8) {
-            double sb[8], f1[8], f2[8], cold[8];
+            for (int i = 0; i < 16; ++i) g[i] = i < n_in ? h1[i * p.ldc] : 0.0;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int col = c0 + ch * 32 + h + i;
-              const bool in = col < p.n_cols && (!p.sym || col >= pr);
-              sb[i] = in ? p.scale_b[col] : 0.0;
-              f1[i] = in && p.H1 ? p.H1[ro + col] : 0.0;
-              f2[i] = in && p.H1 && p.H2 ? p.H2[ro + col] : 0.0;
-              cold[i] = in && !p.H1 && p.beta != 0.0 ? p.C[ro + col] : 0.0;
-            }
+            for (int i = 0; i < 16; ++i) v[i] *= g[i];
+          } else if (p.beta != 0.0) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int col = c0 + ch * 32 + h + i;
-              // symmetric: the upper triangle, each entry also at its mirror
-              // (the lanes' rows are consecutive, so the mirrored stores of
-              // one column coalesce)
-              if (col < p.n_cols && (!p.sym || col >= pr)) {
-                const double v = a * acc[h + i] * sb[i];
-                const int64_t mo = static_cast<int64_t>(col) * p.ldc + pr;
-                const bool mirror = p.sym && col > pr;
-                if (p.H1) {
-                  const double o1 = v * f1[i];
-                  p.C[ro + col] = o1;
-                  if (mirror) p.C[mo] = o1;
-                  if (p.H2) {
-                    const double o2 = v * f2[i];
-                    p.C2[ro + col] = o2;
-                    if (mirror) p.C2[mo] = o2;
-                  }
-                } else {
-                  const double o = p.beta == 0.0 ? v : v + p.beta * cold[i];
-                  p.C[ro + col] = o;
-                  if (mirror) p.C[mo] = o;
-                }
-              }
+            for (int i = 0; i < 16; ++i) g[i] = i < n_in ? c[i * p.ldc] : 0.0;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = v[i] + p.beta * g[i];
+          }
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if (i < n_in) c[i * p.ldc] = v[i];
+          if (p.sym) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) blk[(h + i) * kRow + lane] = v[i];
+          }
+        }
+        if (p.sym && cb + 31 > rb) {
+          // each entry above the diagonal also at its mirror
+          __syncwarp();
+#pragma unroll 8
+          for (int i = 0; i < 32; ++i) {
+            const int c = cb + i;
+            if (pr < p.m_rows && c < p.n_cols && c > pr) {
+              const int64_t mo = static_cast<int64_t>(c) * p.ldc + pr;
+              p.C[mo] = blk[lane * kRow + i];
+              if (two) p.C2[mo] = b2[lane * kRow + i];
             }
           }
         }
@@ -728,19 +817,19 @@ int ozaki_chol_update(double *A, int64_t n, int nmat, int64_t j0, int nb, double
     const int smem = ozaki::Layout<6>::kSmemBytes;
     if (!allow_smem(reinterpret_cast<const void *>(kern), smem, attr6)) return MBPT_ERR_CUDA;
     count_launch();
-    kern<<<grid, 192, smem, st>>>(p);
+    kern<<<grid, ozaki::kThreads, smem, st>>>(p);
   } else if (slices == 8) {
     auto kern = ozaki::chol_update_kernel<8, ozaki::EPI_CHOL>;
     const int smem = ozaki::Layout<8>::kSmemBytes;
     if (!allow_smem(reinterpret_cast<const void *>(kern), smem, attr8)) return MBPT_ERR_CUDA;
     count_launch();
-    kern<<<grid, 192, smem, st>>>(p);
+    kern<<<grid, ozaki::kThreads, smem, st>>>(p);
   } else if (slices == 7) {
     auto kern = ozaki::chol_update_kernel<7, ozaki::EPI_CHOL>;
     const int smem = ozaki::Layout<7>::kSmemBytes;
     if (!allow_smem(reinterpret_cast<const void *>(kern), smem, attr7)) return MBPT_ERR_CUDA;
     count_launch();
-    kern<<<grid, 192, smem, st>>>(p);
+    kern<<<grid, ozaki::kThreads, smem, st>>>(p);
   } else {
     return MBPT_ERR_SHAPE;
   }
@@ -882,12 +971,12 @@ int ozaki_dgemm(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha,
       auto kern = ozaki::chol_update_kernel<8, ozaki::EPI_GEMM>;
       const int smem = ozaki::Layout<8>::kSmemBytes;
       if (!allow_smem(reinterpret_cast<const void *>(kern), smem, attr8)) return MBPT_ERR_CUDA;
-      kern<<<grid, 192, smem, st>>>(p);
+      kern<<<grid, ozaki::kThreads, smem, st>>>(p);
     } else {
       auto kern = ozaki::chol_update_kernel<7, ozaki::EPI_GEMM>;
       const int smem = ozaki::Layout<7>::kSmemBytes;
       if (!allow_smem(reinterpret_cast<const void *>(kern), smem, attr7)) return MBPT_ERR_CUDA;
-      kern<<<grid, 192, smem, st>>>(p);
+      kern<<<grid, ozaki::kThreads, smem, st>>>(p);
     }
     if (cudaGetLastError() != cudaSuccess) return MBPT_ERR_CUDA;
   }
