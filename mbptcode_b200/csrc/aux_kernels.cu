@@ -668,8 +668,13 @@ __global__ void inverse_blocks_kernel(const double *__restrict__ src, int64_t sf
 // The batched Cholesky's inverted diagonal blocks (block j of matrix f at
 // Linv + j step_stride + f kCholNb^2, column-major, ld kCholNb) as TF32 pairs in
 // the two layouts of the triangular-inverse recursion: rows of L^-1 (r_*) and
-// columns of L^-1 as rows (c_*), zeros above the diagonal included, as
-// trtri_diag_blocks_kernel writes them; the matrices' pair arrays ldp^2 apart.
+// columns of L^-1 as rows (c_*), zeros above the diagonal and past row n
+// included; the matrices' pair arrays ldp^2 apart. The recursion and the product
+// after it start (end) K at the first row (last row) of a tile of up to 256, so
+// beside the blocks they write they read one block on the zero side of the
+// diagonal: that one is zeroed here too, c_* left of each block but the first
+// and r_* right of each but the last, and nothing else has to be (clearing the
+// four arrays took 57 of 2220 us in G0W0 at naux = 786, 330 of 40600 at 5400).
 // One 32 x 32 tile of a block per CTA, transposed through shared memory (one
 // CTA per block, strided 4-byte stores: 54 us at 7 blocks).
 __global__ void linv_blocks_to_pairs_kernel(const double *__restrict__ Linv,
@@ -684,23 +689,24 @@ __global__ void linv_blocks_to_pairs_kernel(const double *__restrict__ Linv,
   const int x = threadIdx.x;
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
     const int r = r0 + x, c = c0 + k;
-    if (r < m && c < m) {
-      const double v = X[c * kCholNb + r];
-      const float h = to_tf32(static_cast<float>(v));
-      const float l = to_tf32(static_cast<float>(v - static_cast<double>(h)));
-      c_hi[base + (off + c) * ldp + off + r] = h;
-      c_lo[base + (off + c) * ldp + off + r] = l;
-      th[k][x] = h;
-      tl[k][x] = l;
-    }
+    const double v = r < m && c < m ? X[c * kCholNb + r] : 0.0;
+    const float h = to_tf32(static_cast<float>(v));
+    const float l = to_tf32(static_cast<float>(v - static_cast<double>(h)));
+    float *at = c_hi + base + (off + c) * ldp + off + r;
+    float *al = c_lo + base + (off + c) * ldp + off + r;
+    *at = h;
+    *al = l;
+    if (off > 0) at[-kCholNb] = al[-kCholNb] = 0.f;
+    th[k][x] = h;
+    tl[k][x] = l;
   }
   __syncthreads();
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    const int r = r0 + k, c = c0 + x;
-    if (r < m && c < m) {
-      r_hi[base + (off + r) * ldp + off + c] = th[x][k];
-      r_lo[base + (off + r) * ldp + off + c] = tl[x][k];
-    }
+    float *at = r_hi + base + (off + r0 + k) * ldp + off + c0 + x;
+    float *al = r_lo + base + (off + r0 + k) * ldp + off + c0 + x;
+    *at = th[x][k];
+    *al = tl[x][k];
+    if (off + kCholNb < n) at[kCholNb] = al[kCholNb] = 0.f;
   }
 }
 

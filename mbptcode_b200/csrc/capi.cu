@@ -452,7 +452,8 @@ int chi0_run(const double *X, const Dims &d, const double *eps, double mu, const
 constexpr int64_t kTrtriLeaf = 128;
 
 // Mixed-mode scratch of the inverse: TF32 hi/lo pair arrays, np x np each
-// (np = n rounded up to 128), zero outside what the recursion writes.
+// (np = n rounded up to 128), zero on the far side of the diagonal as far as
+// a tile reaches.
 //   LR: rows of the factor L (row i along k);
 //   IC: columns of L^-1 as rows, IC(j, k) = L^-1(k, j);
 //   IR: rows of L^-1, IR(i, k) = L^-1(i, k);
@@ -873,10 +874,10 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
     launch_one_minus(chi0, n, nfreq, trace, st);
   // the diagonal (of chi0 in a batch, of 1 - chi0 otherwise), for the LU fallback
   launch_diag(chi0, n, nfreq, b.diag, true, st);
-  if (mode == MBPT_MODE_MIXED && want_w) {
-    // the inverse's pair arrays are read as zeros wherever the recursion does
-    // not write (padding, above the diagonal blocks); every frequency writes
-    // the rest, and all that is read of the other arrays
+  if (mode == MBPT_MODE_MIXED && want_w && !batched) {
+    // the inverse's pair arrays are read as zeros beside what the recursion
+    // writes (padding, above the diagonal blocks); a batch's diagonal blocks
+    // come with the zeros around them
     const PairScratch &q = b.pairs;
     for (float *f : {q.ic_hi, q.ic_lo, q.ir_hi, q.ir_lo})
       if (cudaMemsetAsync(f, 0, sizeof(float) * b.npairs * q.np * q.np, st) != cudaSuccess)
