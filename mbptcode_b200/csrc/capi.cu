@@ -1159,10 +1159,8 @@ int sigma_run(const double *X, const Dims &d, const double *eps, double mu, cons
                          {b.Xo_s, d.nocc, mo}, {X, d.n, 0}, d.nocc, {b.Xv_s, d.nv, mv},
                          {X + d.nocc, d.n, 0}, d.nv, d.M, b.Hl, b.Hg, m2, nb, st);
       if (!rc)
-        rc = dmma::half_quadratic(b.Hl, m2, d.M, b.Xs, S, 1.0, branch + k * S, S, nb, st);
-      if (!rc)
-        rc = dmma::half_quadratic(b.Hg, m2, d.M, b.Xs, S, -1.0, branch + (ntau + k) * S, S, nb,
-                                  st);
+        rc = dmma::half_quadratic(b.Hl, b.Hg, m2, d.M, b.Xs, S, branch + k * S,
+                                  branch + (ntau + k) * S, S, nb, st);
     }
     if (rc) return rc;
   } else if (fp64_mode(mode)) {
@@ -1187,9 +1185,9 @@ int sigma_run(const double *X, const Dims &d, const double *eps, double mu, cons
       rc = dmma::sigma_h(b.Zt, {}, {}, d.naux, {b.Xo_s, d.nocc, 0}, {X, d.n, 0}, d.nocc,
                          {b.Xv_s, d.nv, 0}, {X + d.nocc, d.n, 0}, d.nv, d.M, b.Hl, b.Hg, 0, 1,
                          st);
-      if (!rc) rc = dmma::half_quadratic(b.Hl, 0, d.M, b.Xs, S, 1.0, branch + k * S, S, 1, st);
       if (!rc)
-        rc = dmma::half_quadratic(b.Hg, 0, d.M, b.Xs, S, -1.0, branch + (ntau + k) * S, S, 1, st);
+        rc = dmma::half_quadratic(b.Hl, b.Hg, 0, d.M, b.Xs, S, branch + k * S,
+                                  branch + (ntau + k) * S, S, 1, st);
     }
     if (rc) return rc;
   } else {

@@ -27,7 +27,8 @@
 // With Pi by halves (half: the product with T reads K from each row tile's
 // first row, every member's longest sums first: 179 -> 103 us at M = 888, naux
 // = 141, 20 points), D^T Y cut along K where its CTAs are few (72 -> 49 us
-// there), no DMMAs on the padding of a product's last K tile (Pi of 5 + 38
+// there), both branches' contractions with the states in one launch, the longest
+// sums first (157 -> 87 us for 58 states at M = 1332, 20 points), no DMMAs on the padding of a product's last K tile (Pi of 5 + 38
 // orbitals at M = 888: 65 -> 46 us) and 16-byte stores: E_c of that case 0.58
 // -> 0.49 ms, G0W0 at M = 1332 2.07 -> 1.72 ms.
 //
@@ -186,7 +187,7 @@ struct Args {
   bool upper;
   bool half;       // PRODUCT: upper tiles only, the diagonal ones halved; STORE: A is such a half
   bool pairs;      // 16-byte stores
-  int members;     // half: the batch, all in one grid dimension
+  int members;     // half, ROWDOT: the batch, all in one grid dimension
   int ksplit;      // STORE: K in so many parts, each with a result of its own
   int64_t s_part;
   double alpha, beta;
@@ -195,7 +196,7 @@ struct Args {
   const double *zt;    // SIGMA: Zt as stored (ld m) instead of the first product
   const double *xs;    // row contraction
   int64_t ld_xs;
-  double *out;
+  double *out, *out2;
   int64_t s_out;
   // Dyson step
   const double *src;   // CHOL: the matrices whose identity complement is factorised
@@ -214,7 +215,8 @@ enum Epi : int {
   STORE = 0,     // C = alpha acc + beta C (upper: and its mirror; half: K from the tile's first row)
   PRODUCT = 1,   // C = acc0 o acc1, mirrored (half: as SIGMA's)
   SIGMA = 2,     // c0 = acc1 o acc0, c1 = acc2 o acc0: upper tiles, the diagonal ones halved
-  ROWDOT = 3,    // out[p] += alpha sum_r xs[r, p] acc[r, p], K from the tile's first row
+  ROWDOT = 3,    // out[p] += 2 sum_r xs[r, p] acc[r, p], K from the tile's first row; the
+                 // second half of the members a[1]'s, out2[p] -= ...
   CHOL = 4,      // C = I - src - acc, on and above the diagonal
   NODE_T = 5,    // per node: T^T = U12^T V11^T, K from the tile's first column
   NODE_V = 6,    // per node: V12 = -T V22, K up to the tile's last column
@@ -235,6 +237,7 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
   int64_t z = blockIdx.z, off_a = 0, off_b = 0, off_c = 0;
   unsigned tile = blockIdx.x;
   int k_begin = 0;
+  [[maybe_unused]] bool second = false;
   if constexpr (EPI == NODE_T || EPI == NODE_V) {
     const Node &q = p.node[z % p.nnodes];
     z /= p.nnodes;
@@ -252,8 +255,14 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
   } else if (p.upper) {
     upper_tile(tile, p.tiles_m, ti, tj);
   } else {
+    if constexpr (EPI == ROWDOT) {  // the longest sums of all members first
+      z = tile % p.members;
+      tile /= p.members;
+      second = 2 * z >= p.members;
+      if (second) z -= p.members / 2;
+    }
     if constexpr (EPI == STORE) {
-      if (p.half) {  // the longest sums of all members first
+      if (p.half) {
         z = tile % p.members;
         tile /= p.members;
       } else if (p.ksplit > 1) {
@@ -291,7 +300,8 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
   int fseg = EPI == SIGMA && k_end0 == 0 ? 1 : 0, fleft = tiles(fseg), fstage = 0;
   auto open = [&](int s) {
     const int ke = s == 0 ? k_end0 : p.k[s];
-    fa.start(p.a[s].p + z * p.a[s].stride + off_a, p.a[s].ld, m0, rows_m, k_first, ke, p.wa[s]);
+    const Operand &oa = p.a[EPI == ROWDOT && second ? 1 : s];
+    fa.start(oa.p + z * oa.stride + off_a, oa.ld, m0, rows_m, k_first, ke, p.wa[s]);
     fb.start(p.b[s].p + z * p.b[s].stride + off_b, p.b[s].ld, n0, rows_n, k_first, ke, p.wb[s]);
   };
   open(fseg);
@@ -475,7 +485,8 @@ __global__ void __launch_bounds__(kThreads, BN == 32 ? 4 : 3) dmma_kernel(const 
         }
 #pragma unroll
         for (int d = 4; d < 32; d <<= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-        if (g == 0 && col < p.n) atomicAdd(p.out + z * p.s_out + col, p.alpha * s);
+        if (g == 0 && col < p.n)
+          atomicAdd((second ? p.out2 : p.out) + z * p.s_out + col, (second ? -2.0 : 2.0) * s);
       }
   }
 }
@@ -510,7 +521,11 @@ int launch(Args &p, int batch, cudaStream_t st) {
   int64_t grid = p.upper ? static_cast<int64_t>(p.tiles_m) * (p.tiles_m + 1) / 2
                          : static_cast<int64_t>(p.tiles_m) * p.tiles_n;
   if (grid > (int64_t{1} << 30)) return MBPT_ERR_SHAPE;
-  if (EPI == STORE && p.half) {
+  if (EPI == ROWDOT) {
+    p.wa[0] = p.wa[0] && wide(p.a[1], batch);
+    batch *= 2;
+  }
+  if (EPI == ROWDOT || (EPI == STORE && p.half)) {
     p.members = batch;
     if (grid * batch > (int64_t{1} << 30)) return MBPT_ERR_SHAPE;
     grid *= batch;
@@ -639,19 +654,21 @@ int sigma_h(const double *zt, const Operand &u, const Operand &d, int64_t naux,
   return launch<64, true, true, SIGMA>(p, batch, st);
 }
 
-int half_quadratic(const double *h, int64_t sh, int64_t m, const double *xs, int64_t ns,
-                   double sign, double *out, int64_t s_out, int batch, cudaStream_t st) {
+int half_quadratic(const double *hl, const double *hg, int64_t sh, int64_t m, const double *xs,
+                   int64_t ns, double *out_l, double *out_g, int64_t s_out, int batch,
+                   cudaStream_t st) {
   if (!fits(m) || !fits(ns)) return MBPT_ERR_SHAPE;
   Args p{};
-  p.a[0] = {h, m, sh};
+  p.a[0] = {hl, m, sh};
+  p.a[1] = {hg, m, sh};
   p.b[0] = {xs, ns, 0};
   p.k[0] = static_cast<int>(m);
   p.m = static_cast<int>(m);
   p.n = static_cast<int>(ns);
-  p.alpha = 2.0 * sign;
   p.xs = xs;
   p.ld_xs = ns;
-  p.out = out;
+  p.out = out_l;
+  p.out2 = out_g;
   p.s_out = s_out;
   if (narrow(ns)) return launch<32, true, false, ROWDOT>(p, batch, st);
   return launch<64, true, false, ROWDOT>(p, batch, st);

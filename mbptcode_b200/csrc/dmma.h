@@ -51,10 +51,12 @@ int sigma_h(const double *zt, const Operand &u, const Operand &d, int64_t naux,
             const Operand &xv, int64_t nv, int64_t m, double *hl, double *hg, int64_t sh,
             int batch, cudaStream_t st);
 
-// out[p] += sign x_p^T H x_p for the ns columns x_p of xs (m x ns) and the
-// symmetric H held as sigma_h leaves it: twice the sum over its tiles.
-int half_quadratic(const double *h, int64_t sh, int64_t m, const double *xs, int64_t ns,
-                   double sign, double *out, int64_t s_out, int batch, cudaStream_t st);
+// out_l[p] += x_p^T Hl x_p and out_g[p] -= x_p^T Hg x_p for the ns columns x_p
+// of xs (m x ns) and the symmetric Hl and Hg held as sigma_h leaves them: twice
+// the sum over their tiles.
+int half_quadratic(const double *hl, const double *hg, int64_t sh, int64_t m, const double *xs,
+                   int64_t ns, double *out_l, double *out_g, int64_t s_out, int batch,
+                   cudaStream_t st);
 
 // One step of the left-looking Cholesky of I - chi0 for `batch` row-major
 // n x n matrices whose rows above j0 hold the factor U (I - chi0 = U^T U):
