@@ -9,16 +9,18 @@
  *   - Calls are stream-ordered on `stream` (a cudaStream_t, NULL = legacy
  *     default stream) and take their scratch from the caller's `workspace`
  *     of `ws_bytes` bytes, sized by the matching *_workspace_bytes query.
- *     The FP64 products and the Cholesky/LU factorisations go through
- *     cuBLAS/cuSOLVER handles created on first use (per host thread);
+ *     The reverse sweeps' and the contour rows' FP64 products and the LU
+ *     factorisations go through cuBLAS/cuSOLVER handles created on first use
+ *     (per host thread);
  *     mbpt_dyson (and mbpt_rpa_energy through it) synchronises `stream`
  *     once to read the factorisations' info words.
  *   - The return value is an mbpt_status. Errors found on the device (a
  *     bounded wait that ran out) are written to the int at `err_dev`
  *     (zeroed by the caller before the call, read after it); NULL skips.
- *   - mode MBPT_MODE_FP64 runs every product in FP64 (cuBLAS DGEMM, the plain
- *     GPU path); MBPT_MODE_MIXED runs the N^3 products on the tcgen05 tensor
- *     cores as split (3-term) products with FP32 accumulation: BF16 pairs for
+ *   - mode MBPT_MODE_FP64 runs every product in FP64 (the forward sweeps and the
+ *     Dyson step on the library's own kernels for the FP64 tensor pipe, the
+ *     rest on cuBLAS DGEMM: the plain GPU path); MBPT_MODE_MIXED runs the N^3
+ *     products on the tcgen05 tensor cores as split (3-term) products with FP32 accumulation: BF16 pairs for
  *     the Coulomb-side products, TF32 pairs for G_occ / G_virt and for the
  *     inverse of the Dyson step. The tau <-> omega transforms, the
  *     Cholesky/log-det, the quadrature sums and the QP root search are FP64
@@ -76,7 +78,8 @@ int mbpt_device_supported(int device);
 
 /* Instrumentation (no counterpart in MBPTcode, which has no device code):
  * the number of this library's kernels launched by the process so far, and
- * CUDA-event timing of the tensor-core engine's launches. mbpt_gemm_timing
+ * CUDA-event timing of the tensor-core engine's launches (one launch covers
+ * several tau points or frequencies). mbpt_gemm_timing
  * with enable = 1 starts recording on the launching streams (enable = 2: all
  * but category 7, whose many small launches the event pairs would slow down);
  * a call with
@@ -123,7 +126,7 @@ int mbpt_chi0_sweep(const double *X_dev, int64_t M, int64_t norb, int64_t nocc,
  * by a Cholesky factorisation of 1 - chi0 at each frequency (FP64). From
  * four frequencies on, one batched factorisation of all of them, whose
  * trailing updates run on the int8 tensor cores (the Ozaki scheme,
- * FP64-accurate) in MBPT_MODE_MIXED and as native FP64 DGEMMs in
+ * FP64-accurate) in MBPT_MODE_MIXED and on the FP64 tensor pipe in
  * MBPT_MODE_FP64 (the environment variable MBPT_DYSON_OZAKI=1 or =0 forces
  * either).
  * chi0_dev (nfreq, naux, naux): in chi0; out W - I = [1 - chi0]^-1 - 1 when
@@ -134,8 +137,8 @@ int mbpt_chi0_sweep(const double *X_dev, int64_t M, int64_t norb, int64_t nocc,
  * is the determinant's sign); the call then returns MBPT_ERR_NOT_SPD after
  * finishing every frequency. info_host/sign_host may be NULL.
  * mode: the factorisation and log-determinant are FP64 either way; the inverse
- * W = L^-T L^-1 is formed from the FP64 factor by cuBLAS level-3 products
- * (MBPT_MODE_FP64) or, with MBPT_MODE_MIXED, by TF32x3 tensor-core products
+ * W = L^-T L^-1 is formed from the FP64 factor by FP64 products (the FP64
+ * modes; W - I is then symmetric to the bit) or, with MBPT_MODE_MIXED, by TF32x3 tensor-core products
  * (the triangular inverse's off-diagonal blocks and L^-T L^-1): a few 2^-22
  * absolute on W - I, whose entries are bounded by 1. */
 size_t mbpt_dyson_workspace_bytes(int64_t naux, int nfreq, int mode);

@@ -1,7 +1,10 @@
 // C entry points of libmbpt_b200: orchestration of the route on the caller's
-// stream over the caller's workspace. FP64 mode runs the N^3 products through
-// cuBLAS DGEMM (the plain GPU path); mixed mode through the tcgen05 split
-// engine (umma_gemm.cuh). The Cholesky factorisations use cuSOLVER in FP64.
+// stream over the caller's workspace. FP64 mode runs the sweeps' and the Dyson
+// step's N^3 products on the FP64 tensor pipe (dmma.cu), many tau points or
+// frequencies per launch (the library's products where a grid's weights would
+// amplify their last bits, and in the reverse sweeps); mixed mode runs them on
+// the tcgen05 split engine (umma_gemm.cuh). Fewer than four frequencies are
+// factorised by cuSOLVER, one at a time.
 #include <cublas_v2.h>
 #include <cusolverDn.h>
 

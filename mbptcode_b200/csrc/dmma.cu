@@ -23,21 +23,22 @@
 // launch (cuBLAS 34.1, one point a launch); smaller warp tiles (32 x 16, more
 // warps) 32.8, two CTAs per SM with a deeper ring 32.1. The sweep with it
 // (n = 400, M = naux = 2400, 20 points): chi0 36.9 -> 27.2 ms, Sigma of 400
-// states 45.0 -> 31.8 ms; E_c at M = 888, naux = 141: 1.51 -> 0.72 ms.
-// With Pi by halves (half: the product with T reads K from each row tile's
-// first row, every member's longest sums first: 179 -> 103 us at M = 888, naux
-// = 141, 20 points), D^T Y cut along K where its CTAs are few (72 -> 49 us
-// there), both branches' contractions with the states in one launch, the longest
-// sums first (157 -> 87 us for 58 states at M = 1332, 20 points), no DMMAs on the padding of a product's last K tile (Pi of 5 + 38
-// orbitals at M = 888: 65 -> 46 us) and 16-byte stores: E_c of that case 0.58
-// -> 0.49 ms, G0W0 at M = 1332 2.07 -> 1.72 ms.
+// states 45.0 -> 31.1 ms; E_c at M = 888, naux = 141: 1.51 -> 0.49 ms.
+// What small sizes took beyond that (20 points): Pi by halves, the product with
+// it reading K from each row tile's first row, every member's longest sums
+// first (179 -> 103 us at M = 888, naux = 141); D^T Y cut along K where its
+// CTAs are few (72 -> 49 us there); no DMMAs on the padding of a product's
+// last K tile and 16-byte stores (Pi of 5 + 38 orbitals at M = 888: 65 -> 46
+// us); both branches' contractions with the states in one launch, the longest
+// sums first (58 states at M = 1332: 157 -> 87 us). E_c of the first case
+// 0.58 -> 0.49 ms, G0W0 of the last 2.07 -> 1.67 ms.
 //
 // The Dyson step's FP64 products run on the same kernel, all frequencies (and
 // all halvings of one depth of the triangular inverse) in one launch: the
 // Cholesky's block-column updates and panels, V = U^-1 by halves and W = V V^T
 // over the K columns where V is not zero. One frequency at a time the library
 // took 1200 launches of small products at naux = 1500, 20 frequencies: 16.1
-// ms, now 4.0.
+// ms, now 3.85.
 #include <algorithm>
 #include <vector>
 
