@@ -446,7 +446,8 @@ def _rpa_energy(X, D, eps, nocc, tau_points, cosft_wt, omega_weights, mu, precis
     ntau, nfreq = len(tau_h), cw_h.shape[0]
     mode = _mode(precision)
     check_mixed_weights(precision, cw_h)
-    out = torch.zeros(2, dtype=torch.float64, device=dev)
+    with torch.cuda.stream(stream):  # its fill runs ahead of the kernels that write there
+        out = torch.zeros(2, dtype=torch.float64, device=dev)
     proj = (torch.empty((ntau, naux, naux), dtype=torch.float64, device=dev)
             if want_proj else None)
     info = np.zeros(nfreq, dtype=np.int32)
@@ -462,10 +463,12 @@ def _rpa_energy(X, D, eps, nocc, tau_points, cosft_wt, omega_weights, mu, precis
     return out, info, proj
 
 
-def _energy_and_check(out):
-    """E_c of `_rpa_energy`'s output on the host, its error word checked."""
-    host = torch.empty(2, dtype=torch.float64, pin_memory=True).copy_(out, non_blocking=True)
-    torch.cuda.current_stream(out.device).synchronize()
+def _energy_and_check(out, stream=None):
+    """E_c of `_rpa_energy`'s output on the host, its error word checked: read
+    on the call's own stream, behind the kernels that write it."""
+    with torch.cuda.stream(stream):
+        host = torch.empty(2, dtype=torch.float64, pin_memory=True).copy_(out, non_blocking=True)
+        torch.cuda.current_stream(out.device).synchronize()
     e_c, word = host.numpy()[0], host.numpy().view(np.int32)[2]
     if word:
         raise _lib.MBPTError(int(word), 'mbpt_rpa_energy (device)')
@@ -478,7 +481,7 @@ def rpa_energy_device(X, D, eps, nocc, tau_points, cosft_wt, omega_weights, mu=N
     log-determinants and the weighted frequency sum in one library call."""
     out, info, proj = _rpa_energy(X, D, eps, nocc, tau_points, cosft_wt, omega_weights, mu,
                                   precision, want_proj, stream)
-    _energy_and_check(out)
+    _energy_and_check(out, stream)
     return out[0], info, proj
 
 
