@@ -211,7 +211,7 @@ def upload(a, device, dtype=torch.float64, stream=None):
     if t.numel() * t.element_size() > UPLOAD_BYTES or not (
             stream is None or stream == torch.cuda.current_stream(device)):
         return t.to(device=device, dtype=dtype)
-    pin = torch.empty(t.shape, dtype=dtype, pin_memory=True)
+    pin = torch.empty(t.shape, dtype=dtype, device='cpu', pin_memory=True)
     pin.copy_(t)
     return pin.to(device, non_blocking=True)
 

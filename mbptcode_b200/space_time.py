@@ -467,7 +467,8 @@ def _energy_and_check(out, stream=None):
     """E_c of `_rpa_energy`'s output on the host, its error word checked: read
     on the call's own stream, behind the kernels that write it."""
     with torch.cuda.stream(stream):
-        host = torch.empty(2, dtype=torch.float64, pin_memory=True).copy_(out, non_blocking=True)
+        host = torch.empty(2, dtype=torch.float64, device='cpu', pin_memory=True)
+        host.copy_(out, non_blocking=True)
         torch.cuda.current_stream(out.device).synchronize()
     e_c, word = host.numpy()[0], host.numpy().view(np.int32)[2]
     if word:
