@@ -167,7 +167,7 @@ def sigma_frequency(branch, C, S, stream=None):
     (nstates, npade) device tensor: ``imaginary_time.py:525-532``."""
     dev = branch.device
     ntau, nstates = branch.shape[1], branch.shape[2]
-    Cd, Sd = upload(C, dev, stream=stream), upload(S, dev, stream=stream)
+    Cd, Sd = (upload(np.asarray(m, dtype=np.float64), dev, stream=stream) for m in (C, S))
     npade = Cd.shape[0]
     out = torch.empty((nstates, npade, 2), dtype=torch.float64, device=dev)
     bc = branch.contiguous()  # held until the call has launched its kernel

@@ -517,7 +517,7 @@ def transform(values, weights, stream=None, out=None, accumulate=False):
     `out` with `accumulate`)."""
     dev = values.device
     K, n = values.shape[0], values.shape[-1]
-    w = upload(weights, dev, stream=stream)
+    w = upload(np.asarray(weights, dtype=np.float64), dev, stream=stream)
     J = w.shape[0]
     if out is None:
         if accumulate:
