@@ -142,8 +142,9 @@ __global__ void diag_kernel(double *a, int64_t n, double *diag, bool save) {
   }
 }
 
-// Inverts the nb x nb diagonal blocks of a column-major lower-triangular
-// matrix in place, one CTA per block: the block is staged row-major in shared
+// Inverts the nb x nb diagonal blocks of column-major lower-triangular n x n
+// matrices (blockIdx.y, one after the other; the pair arrays ldp^2 apart) in
+// place, one CTA per block: the block is staged row-major in shared
 // memory and inverted row by row (forward substitution against the rows
 // already inverted), so the block never leaves the SM until it is done.
 // With c_hi set, the inverted blocks go out as TF32 pairs instead, in two
@@ -154,9 +155,11 @@ __global__ void diag_kernel(double *a, int64_t n, double *diag, bool save) {
 // with a padded row stride so the parts' reads fall in different banks.
 constexpr int kDiagParts = 4;
 
-__global__ void trtri_diag_blocks_kernel(double *A, int64_t n, int64_t lda, int nb, float *c_hi,
-                                         float *c_lo, float *r_hi, float *r_lo, int64_t ldp) {
+__global__ void trtri_diag_blocks_kernel(double *A, int64_t n, int nb, float *c_hi, float *c_lo,
+                                         float *r_hi, float *r_lo, int64_t ldp) {
   extern __shared__ double s[];  // m x m row-major block (stride m + 1), then one row of L
+  const int64_t lda = n, pairs = blockIdx.y * ldp * ldp;
+  A += blockIdx.y * n * n;
   const int64_t off = static_cast<int64_t>(blockIdx.x) * nb;
   const int m = static_cast<int>(min(static_cast<int64_t>(nb), n - off));
   const int ls = m + 1;
@@ -186,10 +189,10 @@ __global__ void trtri_diag_blocks_kernel(double *A, int64_t n, int64_t lda, int 
       const double x = s[r * ls + c];
       const float h = to_tf32(static_cast<float>(x));
       const float l = to_tf32(static_cast<float>(x - static_cast<double>(h)));
-      r_hi[(off + r) * ldp + off + c] = h;
-      r_lo[(off + r) * ldp + off + c] = l;
-      c_hi[(off + c) * ldp + off + r] = h;
-      c_lo[(off + c) * ldp + off + r] = l;
+      r_hi[pairs + (off + r) * ldp + off + c] = h;
+      r_lo[pairs + (off + r) * ldp + off + c] = l;
+      c_hi[pairs + (off + c) * ldp + off + r] = h;
+      c_lo[pairs + (off + c) * ldp + off + r] = l;
     }
     return;
   }
@@ -760,7 +763,7 @@ void launch_inverse_blocks(const double *src, int64_t sf, int64_t sj, int64_t ld
                           st>>>(src, sf, sj, ld, n, V, ldv);
 }
 
-int launch_trtri_diag_blocks(double *A, int64_t n, int64_t lda, int nb, cudaStream_t st,
+int launch_trtri_diag_blocks(double *A, int64_t n, int nmat, int nb, cudaStream_t st,
                              float *c_hi, float *c_lo, float *r_hi, float *r_lo, int64_t ldp) {
   if (nb < 1 || nb > 128) return MBPT_ERR_SHAPE;  // one thread group of kDiagParts per column
   const size_t smem = sizeof(double) * (static_cast<size_t>(nb) * (nb + 1) + nb);
@@ -769,8 +772,8 @@ int launch_trtri_diag_blocks(double *A, int64_t n, int64_t lda, int nb, cudaStre
                            static_cast<int>(smem)) != cudaSuccess)
     return MBPT_ERR_CUDA;
   count_launch();
-  trtri_diag_blocks_kernel<<<static_cast<unsigned>((n + nb - 1) / nb), nb * kDiagParts, smem,
-                             st>>>(A, n, lda, nb, c_hi, c_lo, r_hi, r_lo, ldp);
+  trtri_diag_blocks_kernel<<<dim3(static_cast<unsigned>((n + nb - 1) / nb), nmat),
+                             nb * kDiagParts, smem, st>>>(A, n, nb, c_hi, c_lo, r_hi, r_lo, ldp);
   return cudaGetLastError() == cudaSuccess ? MBPT_OK : MBPT_ERR_CUDA;
 }
 

@@ -44,7 +44,7 @@ void launch_minus_identity(double *a, int64_t n, cudaStream_t st);
 void launch_diag(double *a, int64_t n, int nmat, double *diag, bool save, cudaStream_t st);
 void launch_inverse_blocks(const double *src, int64_t sf, int64_t sj, int64_t ld, int64_t n,
                            int nmat, double *V, int64_t ldv, cudaStream_t st);
-int launch_trtri_diag_blocks(double *A, int64_t n, int64_t lda, int nb, cudaStream_t st,
+int launch_trtri_diag_blocks(double *A, int64_t n, int nmat, int nb, cudaStream_t st,
                              float *c_hi = nullptr, float *c_lo = nullptr, float *r_hi = nullptr,
                              float *r_lo = nullptr, int64_t ldp = 0);
 void launch_strided_to_tf32(const double *src, int64_t rows, int64_t k, int64_t rs, int64_t cs,
@@ -543,7 +543,7 @@ struct TimingTag {
 // the tensor cores over the tiles on and above the diagonal (rows of (L^-1)^T
 // vanish for k < row), W - I written whole. diag_inv: the batched
 // factorisation's inverted 128 x 128 diagonal blocks (null: they are inverted
-// here, nb 1). info: a matrix whose word is not zero is left as it is.
+// here). info: W - I of a matrix whose word is not zero is not formed.
 int tf32_inverse_from_factor(double *L, int64_t n, int nb, const PairScratch &s, int *err,
                              cudaStream_t st, const int *info = nullptr,
                              const double *diag_inv = nullptr, int64_t diag_inv_stride = 0) {
@@ -556,7 +556,7 @@ int tf32_inverse_from_factor(double *L, int64_t n, int nb, const PairScratch &s,
     launch_linv_blocks_to_pairs(diag_inv, diag_inv_stride, n, nb, s.ic_hi, s.ic_lo, s.ir_hi,
                                 s.ir_lo, np, st);
   else
-    rc = launch_trtri_diag_blocks(L, n, n, static_cast<int>(kTrtriLeaf), st, s.ic_hi, s.ic_lo,
+    rc = launch_trtri_diag_blocks(L, n, nb, static_cast<int>(kTrtriLeaf), st, s.ic_hi, s.ic_lo,
                                   s.ir_hi, s.ir_lo, np);
   if (rc) return rc;
   rc = trtri_pairs(s, n, nb, err, st);
@@ -742,7 +742,7 @@ DysonBufs carve_dyson(Arena &ar, int64_t n, int nfreq, int mode = MBPT_MODE_FP64
   b.diag = ar.take<double>(n * static_cast<int64_t>(nfreq));
   if (fp64_mode(mode) && want_w) {
     b.ldv = round_up(n, 2);  // even: 16-byte copies
-    b.inv_batch = batched_chol_enabled(nfreq) ? tau_batch(nfreq, n * b.ldv) : 1;
+    b.inv_batch = tau_batch(nfreq, n * b.ldv);
     b.V = ar.take<double>(b.inv_batch * n * b.ldv);
   }
   if (batched_chol_enabled(nfreq)) {
@@ -759,7 +759,7 @@ DysonBufs carve_dyson(Arena &ar, int64_t n, int nfreq, int mode = MBPT_MODE_FP64
   }
   if (mode == MBPT_MODE_MIXED) {
     const int64_t np = round_up(n, 128), cap = np * np;
-    b.npairs = batched_chol_enabled(nfreq) ? inverses_in_flight(np, nfreq) : 1;
+    b.npairs = inverses_in_flight(np, nfreq);
     PairScratch &q = b.pairs;
     q.np = np;
     for (float **f : {&q.lr_hi, &q.lr_lo, &q.ic_hi, &q.ic_lo, &q.ir_hi, &q.ir_lo, &q.tt_hi,
@@ -769,13 +769,10 @@ DysonBufs carve_dyson(Arena &ar, int64_t n, int nfreq, int mode = MBPT_MODE_FP64
   return b;
 }
 
-// Per host thread and device: a side stream on which the inverse of one
-// frequency runs while the next frequency factorises on the caller's stream,
-// one event per frequency (its factor, log-determinant and info word are
-// done) and a pinned host copy of the info words.
+// Per host thread and device: the streams beside the caller's on which
+// factorisations run, one event per frequency (its factor, log-determinant
+// and info word are done) and a pinned host copy of the info words.
 struct DysonPipe {
-  cudaStream_t side = nullptr;
-  cudaEvent_t join = nullptr;
   // second factor stream: odd frequencies factorise there with their own
   // cuSOLVER handle, so that two Cholesky factorisations (latency-bound
   // panels between DGEMM-bound updates) share the GPU
@@ -791,7 +788,7 @@ struct DysonPipe {
   std::vector<cudaEvent_t> ev;
   int *info = nullptr;  // pinned host, `cap` ints
   int cap = 0;
-  bool ok = false;
+  bool ok = true;
 };
 
 DysonPipe *dyson_pipe(int nfreq) {
@@ -804,12 +801,10 @@ DysonPipe *dyson_pipe(int nfreq) {
   if (!p) {
     pipes.emplace_back(dev, DysonPipe{});
     p = &pipes.back().second;
-    p->ok = cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking) == cudaSuccess &&
-            cudaEventCreateWithFlags(&p->join, cudaEventDisableTiming) == cudaSuccess;
     // MBPT_DYSON_FACTOR_STREAMS=1 keeps every factorisation on the caller's stream
     const char *env = std::getenv("MBPT_DYSON_FACTOR_STREAMS");
     p->nfac = (env && std::atoi(env) == 1) ? 1 : 2;
-    if (p->ok && p->nfac == 2)
+    if (p->nfac == 2)
       p->ok = cudaStreamCreateWithFlags(&p->fac2, cudaStreamNonBlocking) == cudaSuccess &&
               cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming) == cudaSuccess &&
               cudaEventCreateWithFlags(&p->join2, cudaEventDisableTiming) == cudaSuccess &&
@@ -842,18 +837,18 @@ DysonPipe *dyson_pipe(int nfreq) {
   return p->ok ? p : nullptr;
 }
 
-// Factorise the frequencies on two streams (even ones on `st`, odd ones on the
-// pipe's second factor stream, two ahead of the host); as soon as frequency
-// f's info word is on the host, its inverse goes to the side stream, so that
-// the tensor-core (or DGEMM) inverse of f overlaps the FP64 Cholesky
-// factorisations of f + 1 and f + 2. A frequency that is not positive definite
-// falls back to LU with every stream drained first. The caller's stream waits
-// for the other two at the end.
-// info_dev_out null: the host reads each frequency's info word before its
-// inverse (a positive definite frequency's W from the factor, any other by
-// LU). Non-null: no host wait; every frequency's inverse is issued from its
-// factor and the info words land in info_dev_out, where a nonzero word marks
-// a frequency whose W - I and log-determinant are not valid.
+// Four frequencies or more are factorised together (chol_step, in groups on
+// their own streams), fewer by one potrf each, even ones on `st` and odd ones
+// on the pipe's second factor stream. The inverses of as many factors as the
+// scratch holds then share their launches on `st`, a matrix whose info word is
+// not zero being left out. With two or three frequencies that is one chain of
+// short launches at the end, where one chain per frequency on a side stream
+// took longer than the factors it ran beside (B200, three frequencies, mixed:
+// n = 300 980 us, now 631; 1200 1990, 1632; 3600 6150, 5260).
+// info_dev_out null: the host then reads the info words, and a frequency that
+// is not positive definite takes the LU route with `st` drained first.
+// Non-null: no host wait; the info words land in info_dev_out, where a nonzero
+// word marks a frequency whose W - I and log-determinant are not valid.
 // tail: launches onto `st` what needs the log-determinants of all frequencies.
 int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, double *trace,
               int *info_host, int *sign_host, Arena &ar, cudaStream_t st,
@@ -866,8 +861,6 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
   DysonPipe *pp = dyson_pipe(nfreq);
   if (!pp) return MBPT_ERR_CUDA;
   const int ni = static_cast<int>(n);
-  // many frequencies: one batched factorisation of all of them, then the
-  // per-frequency loop below only reads their info words
   const bool batched = b.chol_P != nullptr;
   // the batch forms 1 - chi0 where it first reads each block column (no pass
   // of its own over the matrices); one potrf per frequency needs it whole
@@ -886,7 +879,7 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
       if (cudaMemsetAsync(f, 0, sizeof(float) * b.npairs * q.np * q.np, st) != cudaSuccess)
         return MBPT_ERR_CUDA;
   }
-  bool side_used = false;
+  const int64_t blk = static_cast<int64_t>(kCholNb) * kCholNb;
   if (batched) {
     if (cudaMemsetAsync(b.info, 0, sizeof(int) * nfreq, st) != cudaSuccess) return MBPT_ERR_CUDA;
     // groups of frequencies on their own streams (each of at least
@@ -898,7 +891,6 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
     if (G > 1 && cudaEventRecord(pp->fork, st) != cudaSuccess) return MBPT_ERR_CUDA;
     for (int g = 1; g < G; ++g)
       if (cudaStreamWaitEvent(stream_of(g), pp->fork, 0) != cudaSuccess) return MBPT_ERR_CUDA;
-    const int64_t blk = static_cast<int64_t>(kCholNb) * kCholNb;
     auto first_of = [&](int g) { return static_cast<int>(static_cast<int64_t>(nfreq) * g / G); };
     std::vector<CholGroup> grp(G);
     for (int g = 0; g < G; ++g) {
@@ -935,54 +927,57 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
           cudaStreamWaitEvent(st, join_of(g), 0) != cudaSuccess)
         return MBPT_ERR_CUDA;
     if (rc0) return rc0;
-    // the inverses of as many factors at a time as the scratch holds (where a
-    // factorisation failed nothing is written)
-    const int nbi = mode == MBPT_MODE_MIXED ? b.npairs : b.inv_batch;
-    for (int f0 = 0; want_w && f0 < nfreq; f0 += nbi) {
-      const int nb = std::min(nbi, nfreq - f0);
-      double *m = chi0 + f0 * n * n;
-      const double *dinv = b.chol_Linv + f0 * blk;
-      int rc1;
-      if (mode == MBPT_MODE_MIXED) {
-        rc1 = tf32_inverse_from_factor(m, n, nb, b.pairs, err, st, b.info + f0, dinv,
-                                       nfreq * blk);
-      } else {
-        launch_inverse_blocks(dinv, blk, nfreq * blk, kCholNb, n, nb, b.V, b.ldv, st);
-        rc1 = dmma::spd_inverse(m, n, b.V, b.ldv, b.info + f0, nb, st);
-      }
-      if (rc1) return rc1;
+  } else {
+    const int nfac = nfreq > 1 ? pp->nfac : 1;
+    if (nfac == 2 && (cudaEventRecord(pp->fork, st) != cudaSuccess ||
+                      cudaStreamWaitEvent(pp->fac2, pp->fork, 0) != cudaSuccess))
+      return MBPT_ERR_CUDA;
+    for (int f = 0; f < nfreq; ++f) {
+      double *m = chi0 + f * n * n;
+      const bool second = nfac == 2 && (f & 1);
+      cudaStream_t fs = second ? pp->fac2 : st;
+      if (cusolverDnDpotrf(second ? pp->solver2 : h.solver, CUBLAS_FILL_MODE_LOWER, ni, m, ni,
+                           second ? b.work2 : b.work, b.lwork,
+                           b.info + f) != CUSOLVER_STATUS_SUCCESS)
+        return MBPT_ERR_CUDA;
+      // log det from the factor's diagonal before the inverse overwrites it
+      // (replaced below where the factorisation failed)
+      launch_logdet_diag(m, n, 1, logdet + f, fs);
+      if ((!deferred && cudaMemcpyAsync(pp->info + f, b.info + f, sizeof(int),
+                                        cudaMemcpyDeviceToHost, fs) != cudaSuccess) ||
+          cudaEventRecord(pp->ev[f], fs) != cudaSuccess)
+        return MBPT_ERR_CUDA;
     }
+    if (nfac == 2 && (cudaEventRecord(pp->join2, pp->fac2) != cudaSuccess ||
+                      cudaStreamWaitEvent(st, pp->join2, 0) != cudaSuccess))
+      return MBPT_ERR_CUDA;
   }
-  const int nfac = nfreq > 1 && !batched ? pp->nfac : 1;
-  if (nfac == 2 && (cudaEventRecord(pp->fork, st) != cudaSuccess ||
-                    cudaStreamWaitEvent(pp->fac2, pp->fork, 0) != cudaSuccess))
-    return MBPT_ERR_CUDA;
-  auto factor = [&](int f) -> int {
-    if (batched) return MBPT_OK;
-    double *m = chi0 + f * n * n;
-    const bool second = nfac == 2 && (f & 1);
-    cudaStream_t fs = second ? pp->fac2 : st;
-    if (cusolverDnDpotrf(second ? pp->solver2 : h.solver, CUBLAS_FILL_MODE_LOWER, ni, m, ni,
-                         second ? b.work2 : b.work, b.lwork,
-                         b.info + f) != CUSOLVER_STATUS_SUCCESS)
-      return MBPT_ERR_CUDA;
-    // log det from the factor's diagonal before the inverse overwrites it
-    // (replaced below where the factorisation failed)
-    launch_logdet_diag(m, n, 1, logdet + f, fs);
-    if (cudaMemcpyAsync(pp->info + f, b.info + f, sizeof(int), cudaMemcpyDeviceToHost, fs) !=
-            cudaSuccess ||
-        cudaEventRecord(pp->ev[f], fs) != cudaSuccess)
-      return MBPT_ERR_CUDA;
-    return MBPT_OK;
-  };
+  const int nbi = mode == MBPT_MODE_MIXED ? b.npairs : b.inv_batch;
+  for (int f0 = 0; want_w && f0 < nfreq; f0 += nbi) {
+    const int nb = std::min(nbi, nfreq - f0);
+    double *m = chi0 + f0 * n * n;
+    // a batch's factorisation kept its inverted diagonal blocks
+    const double *dinv = batched ? b.chol_Linv + f0 * blk : nullptr;
+    int rc1 = MBPT_OK;
+    if (mode == MBPT_MODE_MIXED) {
+      rc1 = tf32_inverse_from_factor(m, n, nb, b.pairs, err, st, b.info + f0, dinv, nfreq * blk);
+    } else {
+      if (batched) {
+        launch_inverse_blocks(dinv, blk, nfreq * blk, kCholNb, n, nb, b.V, b.ldv, st);
+      } else {
+        rc1 = launch_trtri_diag_blocks(m, n, nb, static_cast<int>(kTrtriLeaf), st);
+        launch_inverse_blocks(m, n * n, kTrtriLeaf * n + kTrtriLeaf, n, n, nb, b.V, b.ldv, st);
+      }
+      if (!rc1) rc1 = dmma::spd_inverse(m, n, b.V, b.ldv, b.info + f0, nb, st);
+    }
+    if (rc1) return rc1;
+  }
   // the host only reads info words from here on: what follows on the device
   // runs meanwhile, and again below if a frequency took the LU route
-  if (batched && tail) tail();
+  if (tail) tail();
   bool bad = false;
   int rc = MBPT_OK;
-  for (int f = 0; f < nfac && f < nfreq && rc == MBPT_OK; ++f) rc = factor(f);
   for (int f = 0; f < nfreq && rc == MBPT_OK; ++f) {
-    if (f + nfac < nfreq && (rc = factor(f + nfac)) != MBPT_OK) break;
     if (!deferred && cudaEventSynchronize(pp->ev[f]) != cudaSuccess) {
       rc = MBPT_ERR_CUDA;
       break;
@@ -991,33 +986,12 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
     if (info_host && !deferred) info_host[f] = inf;
     if (sign_host) sign_host[f] = 1;
     double *m = chi0 + f * n * n;
-    if (inf == 0) {
-      if (want_w && !batched) {  // a batch's inverses are under way already
-        cudaStream_t ss = pp->side;
-        side_used = true;
-        if (cudaStreamWaitEvent(ss, pp->ev[f], 0) != cudaSuccess) {
-          rc = MBPT_ERR_CUDA;
-          break;
-        }
-        if (mode == MBPT_MODE_MIXED) {
-          rc = tf32_inverse_from_factor(m, n, 1, b.pairs, err, ss);
-        } else {
-          rc = launch_trtri_diag_blocks(m, n, n, static_cast<int>(kTrtriLeaf), ss);
-          if (rc) break;
-          launch_inverse_blocks(m, 0, kTrtriLeaf * n + kTrtriLeaf, n, n, 1, b.V, b.ldv, ss);
-          rc = dmma::spd_inverse(m, n, b.V, b.ldv, nullptr, 1, ss);
-        }
-        if (rc) break;
-      }
-      continue;
-    }
-    // not positive definite: drain every stream (the LU shares the scratch),
+    if (inf == 0) continue;
+    // not positive definite: drain the stream (the LU shares the scratch),
     // restore 1 - chi0 from its untouched triangle, then LU for log|det| (and
     // the inverse), as the reference's slogdet/inv
     bad = true;
-    if (cudaStreamSynchronize(pp->side) != cudaSuccess ||
-        (nfac == 2 && cudaStreamSynchronize(pp->fac2) != cudaSuccess) ||
-        cudaStreamSynchronize(st) != cudaSuccess) {
+    if (cudaStreamSynchronize(st) != cudaSuccess) {
       rc = MBPT_ERR_CUDA;
       break;
     }
@@ -1051,16 +1025,8 @@ int dyson_run(double *chi0, int64_t n, int nfreq, int want_w, double *logdet, do
     }
     if (sign_host) sign_host[f] = sgn;
   }
-  if (side_used) {
-    cudaEventRecord(pp->join, pp->side);
-    cudaStreamWaitEvent(st, pp->join, 0);
-  }
-  if (nfac == 2) {
-    cudaEventRecord(pp->join2, pp->fac2);
-    cudaStreamWaitEvent(st, pp->join2, 0);
-  }
   if (rc) return rc;
-  if (tail && (bad || !batched)) tail();
+  if (tail && bad) tail();
   if (deferred && cudaMemcpyAsync(info_dev_out, b.info, sizeof(int) * nfreq,
                                   cudaMemcpyDeviceToDevice, st) != cudaSuccess)
     return MBPT_ERR_CUDA;
