@@ -23,6 +23,17 @@ __global__ void chi0_bar_seed_kernel(double *a, int64_t n, const double *w) {
     m[i] *= s;
 }
 
+// a[i] = the sum of a[i + p n] over the parts p, i < n
+__global__ void sum_parts_kernel(double *a, int64_t n, int parts) {
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    double s = a[i];
+#pragma unroll 4
+    for (int p = 1; p < parts; ++p) s += a[i + p * n];
+    a[i] = s;
+  }
+}
+
 // out = (in + in^T) / 2 for each n x n slice, `in` the sum of `parts` arrays
 // part_stride apart: one 32 x 32 tile and its mirror per block, both halves
 // through shared memory so that every access runs along rows
@@ -36,6 +47,7 @@ __global__ void sym_half_kernel(const double *__restrict__ in, double *__restric
   // eight loads in flight per thread (one row of both tiles at a time: 31 us
   // for one slice of n = 2400, now 24)
   double u[4] = {}, l[4] = {};
+#pragma unroll 2
   for (int p = 0; p < parts; ++p) {
     const double *a = in + p * part_stride + base;
 #pragma unroll
@@ -732,6 +744,11 @@ void launch_sym_half(const double *in, double *out, int64_t n, int batch, cudaSt
   const unsigned t = static_cast<unsigned>((n + 31) / 32);
   count_launch();
   sym_half_kernel<<<dim3(t, t, batch), dim3(32, 8), 0, st>>>(in, out, n, parts, batch * n * n);
+}
+
+void launch_sum_parts(double *a, int64_t n, int parts, cudaStream_t st) {
+  count_launch();
+  sum_parts_kernel<<<blocks(n), 256, 0, st>>>(a, n, parts);
 }
 
 void launch_xbar_update(const double *GoX, const double *GvX, const double *X, int64_t M,

@@ -33,6 +33,7 @@ void launch_chi0_bar_seed(double *a, int64_t n, int nfreq, const double *scale,
                           cudaStream_t st);
 void launch_sym_half(const double *in, double *out, int64_t n, int batch, cudaStream_t st,
                      int parts = 1);
+void launch_sum_parts(double *a, int64_t n, int parts, cudaStream_t st);
 void launch_xbar_update(const double *GoX, const double *GvX, const double *X, int64_t M,
                         int64_t n, int64_t nocc, const double *eps, double mu, double tau,
                         double *X_bar, double *eps_bar, cudaStream_t st);
@@ -219,8 +220,10 @@ struct Dims {
 // ---------------------------------------------------------------- chi0 sweep
 struct Chi0Bufs {
   double *w;  // cosft_wt on the device
-  // fp64 (Xo_s, Xv_s, Go, Y: `batch` tau points each; Gv: the int8 mode only)
+  // fp64 (Xo_s, Xv_s, Go, Y: `batch` tau points each, Y y_parts times; Gv: the
+  // library products only)
   double *Xo_s, *Xv_s, *Go, *Gv, *Y, *proj;
+  int y_parts;
   int8_t *Dt_cut;  // int8 mode: D^T's digit planes
   // mixed (Y, Pi, Z: `batch` tau points each, stacked by rows)
   int batch;
@@ -294,7 +297,8 @@ Chi0Bufs carve_chi0(Arena &ar, const Dims &d, int ntau, int nfreq, int mode, boo
     // the library products hold one tau point's G_occ and G_virt
     b.Go = ar.take<double>(std::max(b.batch, 2) * d.M * d.M);
     b.Gv = ar.counting ? nullptr : b.Go + d.M * d.M;
-    b.Y = ar.take<double>(b.batch * d.M * d.naux);
+    b.y_parts = mode == MBPT_MODE_FP64 ? dmma::cut_parts(d.M, d.naux, d.M, b.batch) : 1;
+    b.Y = ar.take<double>(b.y_parts * b.batch * d.M * d.naux);
     if (own_proj) b.proj = ar.take<double>(static_cast<size_t>(ntau) * d.naux * d.naux);
   } else {
     // TF32 pairs of Y, BF16 pairs of Pi and Z per tau point, in doubles
@@ -353,14 +357,24 @@ int chi0_run(const double *X, const Dims &d, const double *eps, double mu, const
           rc = MBPT_ERR_CUDA;
       if (rc) return rc;
       if (mode == MBPT_MODE_FP64_INT8) continue;
-      rc = dmma::gemm({b.Go, d.M, m2}, true, {D, d.naux, 0}, false, d.M, d.naux, d.M, 1.0, 0.0,
-                      b.Y, d.naux, ma, nb, false, st, half);
-      if (!rc && half) {
-        // Z = -4 D^T (T D) where Pi = T + T^T was, proj = (Z + Z^T) / 2; the
-        // parts of Z fit where Pi was
-        const int parts = std::min<int64_t>(dmma::product_parts(d.naux, d.naux, d.M, nb), m2 / a2);
-        rc = dmma::gemm_parts({D, d.naux, 0}, {b.Y, d.naux, ma}, d.naux, d.naux, d.M, -4.0, b.Go,
-                              d.naux, a2, nb, parts, st);
+      if (b.y_parts > 1) {  // never by halves, which have their CTAs
+        rc = dmma::gemm_parts({b.Go, d.M, m2}, true, {D, d.naux, 0}, d.M, d.naux, d.M, 1.0, b.Y,
+                              d.naux, ma, nb, b.y_parts, st);
+        launch_sum_parts(b.Y, nb * ma, b.y_parts, st);
+      } else {
+        rc = dmma::gemm({b.Go, d.M, m2}, true, {D, d.naux, 0}, false, d.M, d.naux, d.M, 1.0, 0.0,
+                        b.Y, d.naux, ma, nb, false, st, half);
+      }
+      // D^T Y cut along K, into as many parts as fit where Pi was: by halves
+      // Z = -4 D^T (T D), and where few tiles leave the GPU idle Z = -2 D^T Y,
+      // both triangles formed; proj = (Z + Z^T) / 2
+      const int64_t fit = std::max(b.batch, 2) * m2 / (nb * a2);
+      const int parts = static_cast<int>(std::min(
+          fit, int64_t{half ? dmma::product_parts(d.naux, d.naux, d.M, nb)
+                            : dmma::square_parts(d.naux, d.M, nb)}));
+      if (!rc && (half || parts > 1)) {
+        rc = dmma::gemm_parts({D, d.naux, 0}, false, {b.Y, d.naux, ma}, d.naux, d.naux, d.M,
+                              half ? -4.0 : -2.0, b.Go, d.naux, a2, nb, parts, st);
         launch_sym_half(b.Go, proj + k * a2, d.naux, nb, st, parts);
       } else if (!rc) {
         rc = dmma::gemm({D, d.naux, 0}, false, {b.Y, d.naux, ma}, false, d.naux, d.naux, d.M,

@@ -555,6 +555,28 @@ bool narrow(int64_t n) { return round_up(n, 64) * 20 >= round_up(n, 32) * 21; }
 // A product with fewer CTAs than four per SM is cut along K.
 constexpr int64_t kFewCtas = 4 * 148;
 
+// Whether 64-wide tiles leave SMs without a CTA: 32-wide ones then take 0.6 us
+// per 16 K columns instead of 0.93 (Pi D at 200 x 60: 14.2 -> 9.7 us).
+bool lone(int64_t m, int64_t n, int batch) {
+  return ((m + BM - 1) / BM) * ((n + 63) / 64) * batch <= 148;
+}
+
+// What a K tile of `ctas` CTAs takes, in units of an SM's time for one at its
+// full rate (0.55 us): one CTA per SM 1.7, two 2.2, three 3, then the rest.
+double rounds(int64_t ctas) {
+  const double busy[4] = {0.0, 1.7, 2.2, 3.0};
+  return 3.0 * (ctas / 444) + busy[(ctas % 444 + 147) / 148];
+}
+
+// Parts that K is cut into so that `ctas` CTAs fill the GPU: four K tiles each
+// at least, the last one not empty.
+int fill_parts(int64_t ctas, int64_t k) {
+  auto ok = [k](int p) { return k >= 4 * BK * p && round_to(static_cast<int>(k), p) * (p - 1) < k; };
+  int parts = 1;
+  while (parts < kMaxParts && ctas * parts < kFewCtas && ok(parts + 1)) ++parts;
+  return parts;
+}
+
 bool fits(int64_t v) { return v > 0 && v <= (int64_t{1} << 30); }
 
 }  // namespace
@@ -578,7 +600,7 @@ int gemm(const Operand &a, bool a_k, const Operand &b, bool b_k, int64_t m, int6
   p.upper = upper;
   p.half = half;
   if (a_k && b_k) return launch<64, true, true, STORE>(p, batch, st);
-  if (a_k && narrow(n)) return launch<32, true, false, STORE>(p, batch, st);
+  if (a_k && (narrow(n) || lone(m, n, batch))) return launch<32, true, false, STORE>(p, batch, st);
   if (a_k) return launch<64, true, false, STORE>(p, batch, st);
   if (!b_k) return launch<64, false, false, STORE>(p, batch, st);
   return MBPT_ERR_UNSUPPORTED;
@@ -591,8 +613,19 @@ int product_parts(int64_t m, int64_t n, int64_t k, int batch) {
   return parts;
 }
 
-int gemm_parts(const Operand &a, const Operand &b, int64_t m, int64_t n, int64_t k, double alpha,
-               double *c, int64_t ldc, int64_t sc, int batch, int parts, cudaStream_t st) {
+int cut_parts(int64_t m, int64_t n, int64_t k, int batch) {
+  const int64_t ctas = ((m + BM - 1) / BM) * ((n + 63) / 64) * batch;
+  return (rounds(ctas) - ctas / 148.0) * k > 44.0 * BK ? fill_parts(ctas, k) : 1;
+}
+
+int square_parts(int64_t n, int64_t k, int batch) {
+  const int64_t t = (n + BM - 1) / BM, whole = t * t * batch, upper = t * (t + 1) / 2 * batch;
+  return (rounds(upper) - whole / 148.0) * k > 30.0 * BK ? fill_parts(whole, k) : 1;
+}
+
+int gemm_parts(const Operand &a, bool a_k, const Operand &b, int64_t m, int64_t n, int64_t k,
+               double alpha, double *c, int64_t ldc, int64_t sc, int batch, int parts,
+               cudaStream_t st) {
   if (!fits(m) || !fits(n) || !fits(k)) return MBPT_ERR_SHAPE;
   Args p{};
   p.a[0] = a;
@@ -606,6 +639,8 @@ int gemm_parts(const Operand &a, const Operand &b, int64_t m, int64_t n, int64_t
   p.sc = sc;
   p.ksplit = parts;
   p.s_part = sc * batch;
+  if (a_k && (narrow(n) || lone(m, n, batch))) return launch<32, true, false, STORE>(p, batch, st);
+  if (a_k) return launch<64, true, false, STORE>(p, batch, st);
   return launch<64, false, false, STORE>(p, batch, st);
 }
 

@@ -23,13 +23,26 @@ int gemm(const Operand &a, bool a_k, const Operand &b, bool b_k, int64_t m, int6
          double alpha, double beta, double *c, int64_t ldc, int64_t sc, int batch, bool upper,
          cudaStream_t st, bool half = false);
 
-// C_0 + ... + C_{parts-1} = alpha A B^T, A and B row-contiguous: each part sums
-// its own range of K and lies batch sc doubles after the one before.
+// C_0 + ... + C_{parts-1} = alpha A B^T, A K-contiguous (a_k) or row-contiguous,
+// B row-contiguous: each part sums its own range of K and lies batch sc doubles
+// after the one before.
 // product_parts: the number of parts that fills the GPU (1 to kMaxParts).
+// cut_parts: 1 unless the time that uneven rounds of CTAs cost (0.55 us per 16
+// columns of K and round) is well above that of a pass that adds the parts, 24
+// us. square_parts: the same for a symmetric n x n product, all of it in parts
+// against its upper tiles in one piece, 16 us. chi0 of one tau point, in one
+// piece, cut, and by the library's products (M x naux, us): 444 x 100 164, 132
+// and 133; 888 x 141 193, 147 and 150; 1332 x 236 265, 181 and 187; 1332 x 700
+// 303, 281 and 298; 2000 x 300 402, 272 and 289; of two points 2000 x 300 504,
+// 393 and 484. Not worth it, in one piece and cut: 444 x 300 of four points 163
+// and 170, 444 x 100 of twenty 188 and 196.
 constexpr int kMaxParts = 8;
 int product_parts(int64_t m, int64_t n, int64_t k, int batch);
-int gemm_parts(const Operand &a, const Operand &b, int64_t m, int64_t n, int64_t k, double alpha,
-               double *c, int64_t ldc, int64_t sc, int batch, int parts, cudaStream_t st);
+int cut_parts(int64_t m, int64_t n, int64_t k, int batch);
+int square_parts(int64_t n, int64_t k, int batch);
+int gemm_parts(const Operand &a, bool a_k, const Operand &b, int64_t m, int64_t n, int64_t k,
+               double alpha, double *c, int64_t ldc, int64_t sc, int batch, int parts,
+               cudaStream_t st);
 
 // C (m x m) = (A0 B0^T) o (A1 B1^T), both symmetric: Pi = G_occ o G_virt.
 // All operands K-contiguous. g0, g1: the two factors as well, laid out as C
