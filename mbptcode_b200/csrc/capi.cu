@@ -632,7 +632,7 @@ int chol_step(const CholGroup &g, int64_t n, int64_t j0, int64_t linv_step_strid
   const int64_t m = n - j0, mb = m - nbj;
   int rc = MBPT_OK;
   if (ozaki && j0 == 0)
-    rc = ozaki_chol_scales(g.A, n, g.nmat, g.oz.scale, g.oz.rowsq, true, g.st);
+    rc = ozaki_chol_scales(g.A, n, g.nmat, g.oz.scale, g.oz.rowsq, g.st);
   if (rc) return rc;
   if (ozaki && j0 > 0)
     rc = ozaki_chol_update(g.A, n, g.nmat, j0, nbj, g.P, g.oz.scale, g.oz.planes, g.oz.slices,
@@ -655,13 +655,13 @@ int chol_step(const CholGroup &g, int64_t n, int64_t j0, int64_t linv_step_strid
 }
 
 // The batched Cholesky's trailing updates: on the int8 tensor cores (the
-// Ozaki scheme) in mixed mode, as native FP64 DGEMMs in FP64 mode (the plain
+// Ozaki scheme) in mixed mode, on the FP64 tensor pipe in FP64 mode (the plain
 // FP64 path the mixed one is measured against). Digits per operand: in
 // mixed mode 6 signed 8-bit digits (the log-determinant within 1e-14 of
 // LAPACK, W from the factor within ~2e-12 of its largest entry; W is formed
 // from it by TF32x3 products there), 8 when forced in FP64 mode
 // (W within ~1e-14). MBPT_DYSON_OZAKI=1 / =0 forces the int8 path or the
-// DGEMMs in both modes, MBPT_DYSON_OZAKI_SLICES=6 / 7 / 8 the digits (6:
+// FP64 one in both modes, MBPT_DYSON_OZAKI_SLICES=6 / 7 / 8 the digits (6:
 // signed 8-bit digits, whose exact int32 level sums hold K below 22 016, so
 // larger matrices take 7). Read at every call, so the size query and the call
 // that follows it must see the same setting.

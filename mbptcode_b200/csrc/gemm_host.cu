@@ -407,12 +407,9 @@ int gemm_split(int epi, int nacc, const SplitMat *A, const SplitMat *B, int64_t 
   if (band) {
     // triangular K spans: the single drained FP32-store TF32 product only (its
     // spans are never empty for the operand shapes the flags describe)
-    if (!tf || nacc != 1 || (epi != EPI_F32 && epi != EPI_TF32_PAIR && epi != EPI_F64_SYM))
+    if (!tf || nacc != 1 || (epi != EPI_F32 && epi != EPI_F64_SYM))
       return MBPT_ERR_UNSUPPORTED;
     if ((band & BAND_UPPER) && m_rows != n_rows) return MBPT_ERR_SHAPE;
-    if (epi == EPI_TF32_PAIR)
-      return launch<1, 128, EPI_TF32_PAIR, true, kDrain>(A, B, m_rows, n_rows, e, err, st,
-                                                         batch, band);
     // the symmetric FP64 store (W = L^-T L^-1): 128 x 256 tiles, which halve
     // the A reads through shared memory for the three TF32 products
     if (epi == EPI_F64_SYM && (band & BAND_UPPER))
@@ -430,8 +427,6 @@ int gemm_split(int epi, int nacc, const SplitMat *A, const SplitMat *B, int64_t 
       return launch<2, 128, EPI_HADAMARD_SPLIT, true, kDrain>(A, B, m_rows, n_rows, e, err, st, batch);
     if (nacc == 1 && epi == EPI_F32)
       return launch<1, 128, EPI_F32, true, kDrain>(A, B, m_rows, n_rows, e, err, st, batch);
-    if (nacc == 1 && epi == EPI_TF32_PAIR)
-      return launch<1, 128, EPI_TF32_PAIR, true, kDrain>(A, B, m_rows, n_rows, e, err, st, batch);
     return MBPT_ERR_UNSUPPORTED;
   }
   // the non-symmetric N^3 products: 128 x 256 tiles (a quarter fewer operand
@@ -442,8 +437,6 @@ int gemm_split(int epi, int nacc, const SplitMat *A, const SplitMat *B, int64_t 
                : launch<1, 256, EPI_SPLIT, false, kDrain>(A, B, m_rows, n_rows, e, err, st, batch);
   if (nacc == 1 && epi == EPI_F32)
     return launch<1, 128, EPI_F32, false, kDrain>(A, B, m_rows, n_rows, e, err, st, batch);
-  if (nacc == 1 && epi == EPI_F32_ACC)
-    return launch<1, 128, EPI_F32_ACC, false, kDrain>(A, B, m_rows, n_rows, e, err, st, batch);
   if (nacc == 2 && epi == EPI_HADAMARD_SPLIT)
     return launch<2, 128, EPI_HADAMARD_SPLIT, false, kDrain>(A, B, m_rows, n_rows, e, err, st, batch);
   // the row contraction: two undrained accumulators, 256-wide on CTA pairs

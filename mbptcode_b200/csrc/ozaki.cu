@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(kThreads, 1) chol_update_kernel(const __grid_c
           mbar_expect_tx(&fs[g], (q1 - g * C) * L::kAPlane + (g == 0 ? S * L::kBPlane : 0));
 #pragma unroll
           for (int q = g * C; q < q1; ++q) {
-            const int t = G > 1 ? S - 1 - q : q;
+            const int t = S - 1 - q;
             tma_load_3d(st + q * L::kAPlane, &p.tm_a, kx, p.a_row0 + r0, q * p.nmat + f, &fs[g]);
             tma_load_3d(st + S * L::kAPlane + t * L::kBPlane, &p.tm_b, kx, p.b_row0 + c0,
                         t * p.nmat + f, &fs[0]);
@@ -505,17 +505,16 @@ __global__ void __launch_bounds__(kThreads, 1) chol_update_kernel(const __grid_c
   }
 }
 
-// scale[f][r] = 2^e_r with e_r = ceil(log2(sqrt(A_rr))) (A column-major, ld n);
+// scale[f][r] = 2^e_r with e_r = ceil(log2(sqrt((I - A_f)_rr))) (A column-major, ld n);
 // 1 for a diagonal that is not positive and finite (that matrix fails its
 // factorisation and is redone by LU; its digits only need to stay in range).
 __global__ void chol_scale_kernel(const double *A, int64_t n, int64_t mat_stride, int nmat,
-                                  bool one_minus, double *scale) {
+                                  double *scale) {
   const int64_t total = n * nmat;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t f = i / n, r = i % n;
-    const double d = A[f * mat_stride + r * n + r];
-    const double a = one_minus ? 1.0 - d : d;  // the diagonal of I - A_f
+    const double a = 1.0 - A[f * mat_stride + r * n + r];
     double s = 1.0;
     if (a > 0.0 && a < 1e300) {
       int e;
@@ -606,7 +605,8 @@ struct Sources {
 // The row maxima of one or two operands (blockIdx.z). Two passes over memory
 // (this and the cutting, the second mostly from L2) are what the scheme needs;
 // a block takes 32 rows x 256 K columns, so that both layouts are read along
-// their contiguous index with 32 loads in flight per thread and K is spread
+// their contiguous index with eight loads in flight per thread (32 where K runs
+// along memory) and K is spread
 // over blocks: with one thread per row of a transposed operand, walking all
 // of K, a 2400 x 2400 operand took 200 us of latency; now 7 us. The maximum
 // of non-negative doubles is that of their bits; NaN counts as nothing.
@@ -753,12 +753,12 @@ size_t ozaki_planes_bytes(int64_t n, int nmat, int slices) {
 }
 
 int ozaki_chol_scales(const double *A, int64_t n, int nmat, double *scale, double *rownorm,
-                      bool one_minus, cudaStream_t st) {
+                      cudaStream_t st) {
   if (cudaMemsetAsync(rownorm, 0, sizeof(double) * n * nmat, st) != cudaSuccess)
     return MBPT_ERR_CUDA;
   count_launch();
   ozaki::chol_scale_kernel<<<ozaki::grid_blocks(n * nmat), 256, 0, st>>>(A, n, n * n, nmat,
-                                                                         one_minus, scale);
+                                                                         scale);
   return cudaGetLastError() == cudaSuccess ? MBPT_OK : MBPT_ERR_CUDA;
 }
 
@@ -782,7 +782,7 @@ int ozaki_chol_slice(const double *A, int64_t n, int nmat, int64_t j0, int nb,
   return cudaGetLastError() == cudaSuccess ? MBPT_OK : MBPT_ERR_CUDA;
 }
 
-int ozaki_chol_update(double *A, int64_t n, int nmat, int64_t j0, int nb, double *P,
+int ozaki_chol_update(const double *A, int64_t n, int nmat, int64_t j0, int nb, double *P,
                       const double *scale, const int8_t *planes, int slices, double *rowsq,
                       int *err, cudaStream_t st) {
   if (j0 <= 0) return MBPT_OK;

@@ -29,8 +29,8 @@ enum Epi : int {
   EPI_HADAMARD_SPLIT = 2,  // out0 = acc0 o acc1, BF16 hi/lo   (Pi = Go o Gv)
   EPI_SIGMA_HZ = 3,        // out0 = acc0 o Zt, out1 = acc1 o Zt, Zt read (FP32) at zt
   EPI_ROWDOT2 = 4,         // sig0[c] += sum_r xs[r,c] acc0[r,c], sig1[c] -= ... acc1
-  EPI_F32_ACC = 5,         // outf += alpha * acc0, FP32 read-modify-write
-  EPI_TF32_PAIR = 6,       // alpha * acc0 as a TF32 hi/lo pair at p (and transposed at t)
+  EPI_TF32_PAIR = 6,       // alpha * acc0 as a TF32 hi/lo pair at p (and transposed at t),
+                           // grouped launches only
   EPI_F64_SYM = 7,         // outd = alpha * acc0 - shift [row == col], FP64, rows and
                            // columns below nd, mirrored (with BAND_UPPER)
 };
@@ -416,9 +416,7 @@ __device__ __forceinline__ void store_split32(uint8_t *buf, bf16 *hi, bf16 *lo, 
   __syncwarp();
 }
 
-// The block as FP32 at out (row 0, column 0, leading dimension ld), added to
-// what is there with ACC.
-template <bool ACC>
+// The block as FP32 at out (row 0, column 0, leading dimension ld).
 __device__ __forceinline__ void store_f32(uint8_t *buf, float *out, int64_t ld,
                                           const float (&v)[32], int lane) {
 #pragma unroll
@@ -429,13 +427,8 @@ __device__ __forceinline__ void store_f32(uint8_t *buf, float *out, int64_t ld,
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int r = 4 * i + (lane >> 3), seg = lane & 7;
-    float4 o = *reinterpret_cast<const float4 *>(buf + r * kStageF32Row + 16 * seg);
-    float4 *dst = reinterpret_cast<float4 *>(out + r * ld + 4 * seg);
-    if constexpr (ACC) {
-      const float4 prev = *dst;
-      o.x += prev.x; o.y += prev.y; o.z += prev.z; o.w += prev.w;
-    }
-    *dst = o;
+    *reinterpret_cast<float4 *>(out + r * ld + 4 * seg) =
+        *reinterpret_cast<const float4 *>(buf + r * kStageF32Row + 16 * seg);
   }
   __syncwarp();
 }
@@ -870,10 +863,10 @@ __global__ void __launch_bounds__(64 + BN, 1)
           for (int i = 0; i < 32; ++i) v0[i] *= e.alpha;
           const int64_t o = ob + at * e.ld_out + ac;
           store_split32(stage, e.out0_hi + o, e.out0_lo + o, nullptr, nullptr, e.ld_out, v0, lane);
-        } else if constexpr (EPI == EPI_F32 || EPI == EPI_F32_ACC) {
+        } else if constexpr (EPI == EPI_F32) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) v0[i] *= e.alpha;
-          store_f32<EPI == EPI_F32_ACC>(stage, e.outf + ob + at * e.ld_outf + ac, e.ld_outf, v0,
+          store_f32(stage, e.outf + ob + at * e.ld_outf + ac, e.ld_outf, v0,
                                         lane);
           if constexpr (EPI == EPI_F32) {
             if (mirror) {
@@ -911,8 +904,8 @@ __global__ void __launch_bounds__(64 + BN, 1)
             hi[i] = to_tf32(v);
             lo[i] = to_tf32(v - hi[i]);
           }
-          store_f32<false>(stage, e.p_hi + p_off + at * e.ld_p + ac, e.ld_p, hi, lane);
-          store_f32<false>(stage, e.p_lo + p_off + at * e.ld_p + ac, e.ld_p, lo, lane);
+          store_f32(stage, e.p_hi + p_off + at * e.ld_p + ac, e.ld_p, hi, lane);
+          store_f32(stage, e.p_lo + p_off + at * e.ld_p + ac, e.ld_p, lo, lane);
           if (e.t_hi) {
             // column col + i of the tile is row col + i of t: the warp's 32
             // consecutive rows land on 32 consecutive floats
