@@ -47,16 +47,17 @@ __global__ void sym_half_kernel(const double *__restrict__ in, double *__restric
   // eight loads in flight per thread (one row of both tiles at a time: 31 us
   // for one slice of n = 2400, now 24)
   double u[4] = {}, l[4] = {};
-#pragma unroll 2
-  for (int p = 0; p < parts; ++p) {
-    const double *a = in + p * part_stride + base;
+  auto add = [&](const double *a) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int k = threadIdx.y + 8 * q;
       if (r0 + k < n && c0 + x < n) u[q] += a[(r0 + k) * n + c0 + x];
       if (c0 + k < n && r0 + x < n) l[q] += a[(c0 + k) * n + r0 + x];
     }
-  }
+  };
+  add(in + base);
+#pragma unroll 2
+  for (int p = 1; p < parts; ++p) add(in + p * part_stride + base);
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     up[threadIdx.y + 8 * q][x] = u[q];

@@ -14,6 +14,7 @@ with FP32 accumulation; transforms, Cholesky and sums stay FP64).
 from __future__ import annotations
 
 import warnings
+from contextlib import nullcontext
 
 import numpy as np
 import torch
@@ -428,6 +429,11 @@ def _flag_nonpositive(where, sign, flags):
         flags.setdefault('nonpositive_det', []).append(where)
 
 
+def _on(stream):
+    """torch's own work of a call on the call's stream."""
+    return nullcontext() if stream is None else torch.cuda.stream(stream)
+
+
 def _rpa_energy(X, D, eps, nocc, tau_points, cosft_wt, omega_weights, mu, precision, want_proj,
                 stream):
     """(out, info, proj): `rpa_energy_device` before its device error word is
@@ -446,7 +452,7 @@ def _rpa_energy(X, D, eps, nocc, tau_points, cosft_wt, omega_weights, mu, precis
     ntau, nfreq = len(tau_h), cw_h.shape[0]
     mode = _mode(precision)
     check_mixed_weights(precision, cw_h)
-    with torch.cuda.stream(stream):  # its fill runs ahead of the kernels that write there
+    with _on(stream):  # its fill runs ahead of the kernels that write there
         out = torch.zeros(2, dtype=torch.float64, device=dev)
     proj = (torch.empty((ntau, naux, naux), dtype=torch.float64, device=dev)
             if want_proj else None)
@@ -466,7 +472,7 @@ def _rpa_energy(X, D, eps, nocc, tau_points, cosft_wt, omega_weights, mu, precis
 def _energy_and_check(out, stream=None):
     """E_c of `_rpa_energy`'s output on the host, its error word checked: read
     on the call's own stream, behind the kernels that write it."""
-    with torch.cuda.stream(stream):
+    with _on(stream):
         host = torch.empty(2, dtype=torch.float64, device='cpu', pin_memory=True)
         host.copy_(out, non_blocking=True)
         torch.cuda.current_stream(out.device).synchronize()
