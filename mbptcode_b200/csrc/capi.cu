@@ -4,7 +4,7 @@
 // frequencies per launch (the library's products where a grid's weights would
 // amplify their last bits, and in the reverse sweeps); mixed mode runs them on
 // the tcgen05 split engine (umma_gemm.cuh). Fewer than four frequencies are
-// factorised by cuSOLVER, one at a time.
+// factorised by cuSOLVER, each by itself.
 #include <cublas_v2.h>
 #include <cusolverDn.h>
 

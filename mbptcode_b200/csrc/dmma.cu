@@ -31,7 +31,9 @@
 // last K tile and 16-byte stores (Pi of 5 + 38 orbitals at M = 888: 65 -> 46
 // us); both branches' contractions with the states in one launch, the longest
 // sums first (58 states at M = 1332: 157 -> 87 us). E_c of the first case
-// 0.58 -> 0.49 ms, G0W0 of the last 2.07 -> 1.67 ms.
+// 0.58 -> 0.49 ms, G0W0 of the last 2.07 -> 1.67 ms. A product of one or two
+// points that leaves SMs without a CTA is cut along K, its parts added by a
+// pass of their own (chi0 of one point at M = 1332, naux = 236: 265 -> 181 us).
 //
 // The Dyson step's FP64 products run on the same kernel, all frequencies (and
 // all halvings of one depth of the triangular inverse) in one launch: the
